@@ -1,0 +1,121 @@
+// What the tensor-core Gemm kernels share: vector stores / residual loads of the epilogue and
+// the activation arithmetic that runs beside the tensor pipe.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "activation.cuh"
+#include "ptx_sm100.cuh"
+
+namespace mdc {
+
+// The epilogue's thread owns one row: it moves 32 bytes (one DRAM sector) per access.
+__device__ __forceinline__ void ld_global_32B(const void *src, uint32_t *r) {
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(src));
+}
+__device__ __forceinline__ void st_global_32B(void *dst, const uint32_t *r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+template <typename T16>
+__device__ __forceinline__ uint32_t pack_pair(float a, float b);
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+// 16 values of a row as TOut; dst is 32-byte aligned
+template <typename TOut>
+__device__ __forceinline__ void store_out16(TOut *dst, const float *v) {
+  uint32_t q[16];
+  if constexpr (sizeof(TOut) == 4) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[i] = __float_as_uint(v[i]);
+    st_global_32B(dst, q);
+    st_global_32B(dst + 8, q + 8);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = pack_pair<TOut>(v[2 * i], v[2 * i + 1]);
+    st_global_32B(dst, q);
+  }
+}
+// eight 16-bit residual values (four registers) as fp32
+template <typename T16>
+__device__ __forceinline__ void unpack_res8(const uint32_t *r, float *v) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 f;
+    if constexpr (sizeof(T16) == 2 && std::is_same<T16, __half>::value)
+      f = __half22float2(*reinterpret_cast<const __half2 *>(r + i));
+    else
+      f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(r + i));
+    v[2 * i] = f.x, v[2 * i + 1] = f.y;
+  }
+}
+
+// Activation for the Gemm epilogue.  The epilogue runs beside the tensor pipe and must keep
+// up with it; its scarce resource is the special-function unit (16 results per clock and SM,
+// shared with the 16-bit conversions).  The exact-erf GELU therefore uses ONE special-function
+// operation per element:
+//   gelu(v) = max(v, 0) - 0.5 |v| erfc(|v| / sqrt 2),     erfc(t) = 2^P(t),
+// P a degree-8 polynomial fitted (minimax, t in [0, 5.7]) to log2(erfc(t)); beyond 5.7 the
+// erfc term is below 1e-15 |v| and t is clamped.  Against the double-precision erf form the
+// result is within 1e-6 absolute and 1.1e-5 relative over [-12, 12] (fp32 evaluation), 50 times
+// below the rounding of a 16-bit output.  (The rational form of Abramowitz & Stegun 7.1.26 used
+// before needs a reciprocal as well as an exponential.)
+__device__ __forceinline__ float ex2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+using ptx::F2;
+using ptx::f2;
+using ptx::f2_add;
+using ptx::f2_fma;
+using ptx::f2_get;
+using ptx::f2_mul;
+
+__device__ __forceinline__ void gelu_erf_pair(float &va, float &vb) {
+  const float aa = fabsf(va), ab = fabsf(vb);
+  const F2 T = f2(fminf(aa * 0.70710678f, 5.7f), fminf(ab * 0.70710678f, 5.7f));
+#define MDC_C2(x) f2(x, x)
+  F2 P = f2_fma(MDC_C2(1.1948015981033677e-06f), T, MDC_C2(-4.147788058617152e-05f));
+  P = f2_fma(P, T, MDC_C2(0.0006375535158440471f));
+  P = f2_fma(P, T, MDC_C2(-0.005785022862255573f));
+  P = f2_fma(P, T, MDC_C2(0.03505704924464226f));
+  P = f2_fma(P, T, MDC_C2(-0.1536988914012909f));
+  P = f2_fma(P, T, MDC_C2(-0.9163860082626343f));
+  P = f2_fma(P, T, MDC_C2(-1.628216028213501f));
+  P = f2_fma(P, T, MDC_C2(7.682551768084522e-06f));
+#undef MDC_C2
+  float pa, pb;
+  f2_get(P, pa, pb);
+  const F2 E = f2(ex2_approx(pa), ex2_approx(pb));
+  const F2 G = f2_fma(f2(-0.5f * aa, -0.5f * ab), E, f2(fmaxf(va, 0.f), fmaxf(vb, 0.f)));
+  f2_get(G, va, vb);
+}
+
+// Applies the activation to n (even) values in place.
+template <int ACT, int N>
+__device__ __forceinline__ void act_fast_n(float *v) {
+  if constexpr (ACT == kActGeluErf) {
+#pragma unroll
+    for (int j = 0; j < N; j += 2) gelu_erf_pair(v[j], v[j + 1]);
+  } else if constexpr (ACT != kActNone) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = act_apply_t<ACT>(v[j]);
+  }
+}
+
+}  // namespace mdc

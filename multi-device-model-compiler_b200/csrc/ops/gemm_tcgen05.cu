@@ -5,17 +5,18 @@
 //
 // Structure (one persistent CTA per SM, 10 warps):
 //   warp 0   TMA producer: cp.async.bulk.tensor tiles of A (128 x 64) and W (256 x 64) into
-//            a 4-stage ring of 128-byte-swizzled shared memory, completion on mbarriers.
-//   warp 1   MMA issuer: one thread issues tcgen05.mma (M=128, N=256, K=16) reading the
-//            shared-memory tiles through matrix descriptors; tcgen05.commit releases the
-//            stage to the producer and, after the last k-block, hands the accumulator over.
+//            a ring of 128-byte-swizzled shared memory, completion on mbarriers.
+//   warp 1   MMA issuer: tcgen05.mma (M=128, N=256, K=16) reading the shared-memory tiles
+//            through matrix descriptors; tcgen05.commit releases the stage to the producer
+//            and, after the last k-block, hands the accumulator over.  Both loops are run by the
+//            whole warp with the elected lane issuing (see ptx_sm100.cuh: the one-lane form was
+//            bound by instruction issue, 590 cycles per k-block where the MMAs need 512).
 //   warps 2-9 epilogue: tcgen05.ld the 128 x 256 fp32 accumulator out of TMEM (each warp
 //            its 32-lane quarter, two warps per quarter splitting the columns), add bias,
-//            apply the activation, add the residual, convert.  Each warp stages 32 rows x
-//            128 bytes of output in swizzled shared memory and writes it with one TMA
-//            store, so global writes are full lines; the residual tile arrives the same
-//            way through a TMA load.  (Shapes whose rows are not 16-byte multiples fall
-//            back to direct stores.)
+//            apply the activation, add the residual, convert and store.  A thread owns a row and
+//            moves 32 bytes per access, a whole sector, so nothing is staged: the 96 KiB that
+//            staged tiles and TMA stores took are two more stages of the ring, and the residual
+//            is fetched before the accumulator is waited for instead of after.
 // TMEM holds two accumulators (2 x 256 columns) so the epilogue of tile i overlaps the
 // mainloop of tile i+1.  Every CTA fetches its own tiles with plain TMA loads and relies on
 // L2 for reuse.  All waits are bounded (see ptx_sm100.cuh).
@@ -27,13 +28,15 @@
 //           48), the leader CTA issues one M = 256 MMA for the pair, each CTA keeps its own
 //           128 x 256 accumulator and runs its own epilogue.  Tensor-core operand reads and
 //           TMA writes compete for shared-memory bandwidth; halving the W bytes per SM is
-//           what lifts the mainloop, and the smaller stage allows a 5-deep ring.
+//           what lifts the mainloop.
+// Measured, 12-layer step of 256 x 128 tokens (hidden 768): 7.38 ms with the one-lane loops and the
+// staged epilogue on 4 stages; whole-warp loops and direct stores 7.15 (4 stages); bias out of L1
+// 6.95 (4 stages), 6.89 (5), 6.88 (6); 7 stages leave L1 too small for the residual: 7.05.
 #include <cstdlib>
 #include <type_traits>
 
-#include "activation.cuh"
+#include "gemm_common.cuh"
 #include "ops_common.h"
-#include "ptx_sm100.cuh"
 
 namespace mdc {
 
@@ -43,19 +46,13 @@ constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int TMEM_COLS = 512;
-constexpr int EPI_BUF_BYTES = 4096;  // 32 rows x 128 bytes, per warp, one for output and one for residual
 template <int CG>
 struct Cfg {
   static constexpr int B_ROWS = BN / CG;            // W rows this CTA stages per k-block
   static constexpr int B_BYTES = B_ROWS * BK * 2;   // 32 KiB (CG 1) / 16 KiB (CG 2)
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = CG == 2 ? 4 : 3;
-  // per epilogue warp: output staging (two buffers for pairs, so a chunk does not wait for
-  // the previous chunk's TMA store to drain) + one residual buffer
-  static constexpr int OUT_BUFS = CG == 2 ? 2 : 1;
-  static constexpr int EPI_WARP_BYTES = (OUT_BUFS + 1) * EPI_BUF_BYTES;
-  static constexpr size_t SMEM_BYTES =
-      static_cast<size_t>(STAGES) * STAGE_BYTES + EPI_WARPS * EPI_WARP_BYTES + 1024;  // + alignment slack
+  static constexpr int STAGES = CG == 2 ? 6 : 4;
+  static constexpr size_t SMEM_BYTES = static_cast<size_t>(STAGES) * STAGE_BYTES + 1024;  // + alignment slack
 };
 }  // namespace gemm
 
@@ -64,127 +61,25 @@ struct GemmParams {
   const float *bias;
   const void *residual;
   void *out;
-  int tma_epi;      // output (and residual) rows are 16-byte multiples: TMA-staged epilogue
-  int out_vec_ok;   // rows of out / residual can be accessed with 16-byte vectors
-  int bias_vec_ok;  // bias is 16-byte aligned
+  int vec_ok;  // rows of out / residual can be accessed in 32-byte vectors, bias in 16-byte ones
   int num_m_blocks, num_n_blocks;
   int cta_group;  // 1: one CTA per 128 x bn tile; 2: CTA pairs on 256 x bn tiles
   int bn;         // tile width in output columns: 256, 192 or 128 (accumulators stay 256 TMEM columns apart)
-  int cw;         // columns per staged output chunk: 64 (16-bit output, 128-byte rows) or 32
   uint32_t *err;
 };
-
-template <typename TOut>
-__device__ __forceinline__ void store_out8(TOut *dst, const float *v);
-template <>
-__device__ __forceinline__ void store_out8<float>(float *dst, const float *v) {
-  reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4 *>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
-template <>
-__device__ __forceinline__ void store_out8<__half>(__half *dst, const float *v) {
-  uint4 o;
-  *reinterpret_cast<__half2 *>(&o.x) = __floats2half2_rn(v[0], v[1]);
-  *reinterpret_cast<__half2 *>(&o.y) = __floats2half2_rn(v[2], v[3]);
-  *reinterpret_cast<__half2 *>(&o.z) = __floats2half2_rn(v[4], v[5]);
-  *reinterpret_cast<__half2 *>(&o.w) = __floats2half2_rn(v[6], v[7]);
-  *reinterpret_cast<uint4 *>(dst) = o;
-}
-template <>
-__device__ __forceinline__ void store_out8<__nv_bfloat16>(__nv_bfloat16 *dst, const float *v) {
-  uint4 o;
-  *reinterpret_cast<__nv_bfloat162 *>(&o.x) = __floats2bfloat162_rn(v[0], v[1]);
-  *reinterpret_cast<__nv_bfloat162 *>(&o.y) = __floats2bfloat162_rn(v[2], v[3]);
-  *reinterpret_cast<__nv_bfloat162 *>(&o.z) = __floats2bfloat162_rn(v[4], v[5]);
-  *reinterpret_cast<__nv_bfloat162 *>(&o.w) = __floats2bfloat162_rn(v[6], v[7]);
-  *reinterpret_cast<uint4 *>(dst) = o;
-}
-__device__ __forceinline__ void load_res8(const __half *src, float *v) {
-  const uint4 r = *reinterpret_cast<const uint4 *>(src);
-  const __half2 *h = reinterpret_cast<const __half2 *>(&r);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(h[i]);
-    v[2 * i] = f.x; v[2 * i + 1] = f.y;
-  }
-}
-__device__ __forceinline__ void load_res8(const __nv_bfloat16 *src, float *v) {
-  const uint4 r = *reinterpret_cast<const uint4 *>(src);
-  const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&r);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x; v[2 * i + 1] = f.y;
-  }
-}
-
-// Activation for the Gemm epilogue.  The epilogue runs beside the tensor pipe and must keep
-// up with it; its scarce resource is the special-function unit (16 results per clock and SM,
-// shared with the 16-bit conversions).  The exact-erf GELU therefore uses ONE special-function
-// operation per element:
-//   gelu(v) = max(v, 0) - 0.5 |v| erfc(|v| / sqrt 2),     erfc(t) = 2^P(t),
-// P a degree-8 polynomial fitted (minimax, t in [0, 5.7]) to log2(erfc(t)); beyond 5.7 the
-// erfc term is below 1e-15 |v| and t is clamped.  Against the double-precision erf form the
-// result is within 1e-6 absolute and 1.1e-5 relative over [-12, 12] (fp32 evaluation), 50 times
-// below the rounding of a 16-bit output.  (The rational form of Abramowitz & Stegun 7.1.26 used
-// before needs a reciprocal as well as an exponential.)
-__device__ __forceinline__ float ex2_approx(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-using ptx::F2;
-using ptx::f2;
-using ptx::f2_add;
-using ptx::f2_fma;
-using ptx::f2_get;
-using ptx::f2_mul;
-
-__device__ __forceinline__ void gelu_erf_pair(float &va, float &vb) {
-  const float aa = fabsf(va), ab = fabsf(vb);
-  const F2 T = f2(fminf(aa * 0.70710678f, 5.7f), fminf(ab * 0.70710678f, 5.7f));
-#define MDC_C2(x) f2(x, x)
-  F2 P = f2_fma(MDC_C2(1.1948015981033677e-06f), T, MDC_C2(-4.147788058617152e-05f));
-  P = f2_fma(P, T, MDC_C2(0.0006375535158440471f));
-  P = f2_fma(P, T, MDC_C2(-0.005785022862255573f));
-  P = f2_fma(P, T, MDC_C2(0.03505704924464226f));
-  P = f2_fma(P, T, MDC_C2(-0.1536988914012909f));
-  P = f2_fma(P, T, MDC_C2(-0.9163860082626343f));
-  P = f2_fma(P, T, MDC_C2(-1.628216028213501f));
-  P = f2_fma(P, T, MDC_C2(7.682551768084522e-06f));
-#undef MDC_C2
-  float pa, pb;
-  f2_get(P, pa, pb);
-  const F2 E = f2(ex2_approx(pa), ex2_approx(pb));
-  const F2 G = f2_fma(f2(-0.5f * aa, -0.5f * ab), E, f2(fmaxf(va, 0.f), fmaxf(vb, 0.f)));
-  f2_get(G, va, vb);
-}
-
-// Applies the activation to n (even) values in place.
-template <int ACT, int N>
-__device__ __forceinline__ void act_fast_n(float *v) {
-  if constexpr (ACT == kActGeluErf) {
-#pragma unroll
-    for (int j = 0; j < N; j += 2) gelu_erf_pair(v[j], v[j + 1]);
-  } else if constexpr (ACT != kActNone) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) v[j] = act_apply_t<ACT>(v[j]);
-  }
-}
 
 template <typename T16, typename TOut, int ACT, int CG>
 __global__ void __launch_bounds__(gemm::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                    const __grid_constant__ CUtensorMap tmap_b,
-                    const __grid_constant__ CUtensorMap tmap_out,
-                    const __grid_constant__ CUtensorMap tmap_res, const GemmParams p) {
+                    const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
   using namespace gemm;
   using namespace ptx;
   using C = Cfg<CG>;
   constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full_bar[2], acc_empty_bar[2];
-  __shared__ uint64_t res_bar[EPI_WARPS];
+  // bias of the columns each epilogue warp handles: kept out of L1, of which the ring leaves little
+  __shared__ __align__(16) float bias_s[EPI_WARPS][BN / 2];
   __shared__ uint32_t tmem_slot;
   __shared__ uint32_t abort_flag_s;
   volatile uint32_t *abort_flag = &abort_flag_s;
@@ -218,7 +113,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       mbar_init(&acc_full_bar[a], 1);
       mbar_init(&acc_empty_bar[a], CG * EPI_WARPS * 32);  // epilogue threads of the whole pair
     }
-    for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&res_bar[w], 1);
     mbar_init_fence();
   }
   if (warp == 1) {
@@ -242,19 +136,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   pdl_wait();  // everything above overlaps the previous kernel's tail; operands are read below
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = worker; ok && tile < num_tiles; tile += num_workers) {
-        const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
-            atomicCAS(p.err, 0u, 0x10000000u | static_cast<uint32_t>(stage));
-            ok = false;
-            break;
-          }
+    // ------------------------------ TMA producer (whole warp, elected lane issues) ------------------------------
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = worker; ok && tile < num_tiles; tile += num_workers) {
+      const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+          atomicCAS(p.err, 0u, 0x10000000u | static_cast<uint32_t>(stage));
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        if (elect_one()) {
           uint8_t *sa = tiles + stage * STAGE_BYTES;
           uint8_t *sb = sa + A_BYTES;
           if constexpr (CG == 2) {
@@ -268,15 +163,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * BK, m_blk * BM);
             tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, n_blk * bn);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer (leader CTA only) ------------------------------
-    if (lane == 0 && leader) {
+    // ---------------- MMA issuer (leader CTA only; whole warp, elected lane issues) ----------------
+    if (leader) {
       const uint32_t idesc = make_idesc_f16(BM * CG, static_cast<uint32_t>(bn),
                                             std::is_same<T16, __nv_bfloat16>::value, false, false);
+      const uint64_t desc0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -287,6 +183,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           atomicCAS(p.err, 0u, 0x30000000u | static_cast<uint32_t>(acc));
           break;
         }
+        __syncwarp();
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -295,36 +192,35 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             ok = false;
             break;
           }
+          __syncwarp();
           tc_fence_after();
-          const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
-          const uint64_t a_desc = make_smem_desc_sw128(sa, 16, 1024);
-          const uint64_t b_desc = make_smem_desc_sw128(sa + A_BYTES, 16, 1024);
+          // (descriptors hold addresses in units of 16 bytes)
+          const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
+          const uint64_t b_desc = a_desc + A_BYTES / 16;
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             // 16 k-elements = 32 bytes further along the 128-byte swizzled row
             if constexpr (CG == 2)
-              umma_f16_ss_cg2(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
-                              b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+              umma_f16_ss_cg2_warp(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
+                                   b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
             else
-              umma_f16_ss(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
-                          b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+              umma_f16_ss_warp(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
+                               b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
           }
           // the stage is reusable (in both CTAs) once these MMAs have read it
           if constexpr (CG == 2) {
-            umma_commit_cg2(smem_u32(&empty_bar[stage]));
-            umma_commit_cg2(mapa_u32(smem_u32(&empty_bar[stage]), 1));
+            umma_commit_cg2_warp(&empty_bar[stage], 3);
           } else {
-            umma_commit(&empty_bar[stage]);
+            umma_commit_warp(&empty_bar[stage]);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
         // accumulator complete: wake the epilogue warps of both CTAs
         if constexpr (CG == 2) {
-          umma_commit_cg2(smem_u32(&acc_full_bar[acc]));
-          umma_commit_cg2(mapa_u32(smem_u32(&acc_full_bar[acc]), 1));
+          umma_commit_cg2_warp(&acc_full_bar[acc], 3);
         } else {
-          umma_commit(&acc_full_bar[acc]);
+          umma_commit_warp(&acc_full_bar[acc]);
         }
         if ((acc ^= 1) == 0) acc_phase ^= 1;
       }
@@ -336,10 +232,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int half_sel = ew >> 2;   // which 128 accumulator columns this warp handles
     TOut *out = static_cast<TOut *>(p.out);
     const T16 *res = static_cast<const T16 *>(p.residual);
-    uint8_t *my_out_base = tiles + STAGES * STAGE_BYTES + ew * C::EPI_WARP_BYTES;
-    uint8_t *my_res = my_out_base + C::OUT_BUFS * EPI_BUF_BYTES;
-    int out_buf = 0;
-    uint32_t res_phase = 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     // the accumulator is handed back to the leader's MMA thread, in whichever CTA it lives
@@ -347,55 +239,51 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const uint32_t acc_empty_addr1 = mapa_u32(smem_u32(&acc_empty_bar[1]), 0);
     for (int tile = worker; tile < num_tiles; tile += num_workers) {
       const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
+      const int half_cols = bn / 2;
+      const int row = m_blk * BM + quarter * 32 + lane;
+      const bool row_ok = row < p.M;
+      const int gcol_base = n_blk * bn + half_sel * half_cols;
+      const uint32_t t_base = tmem_base + static_cast<uint32_t>(acc * BN + half_sel * half_cols) +
+                              (static_cast<uint32_t>(quarter * 32) << 16);
+      // pieces of 32 columns that hold real columns (uniform across the warp)
+      const int n_sub = gcol_base >= p.N ? 0 : min(half_cols / 32, (p.N - gcol_base + 31) / 32);
       // one lane polls, the shuffle releases the others (256 threads would otherwise spin on the
       // barrier word beside the tensor pipe for most of a mainloop)
-      if (!mbar_wait_warp(&acc_full_bar[acc], acc_phase, abort_flag)) {
-        atomicCAS(p.err, 0u, 0x40000000u | static_cast<uint32_t>(acc));
-        break;
-      }
-      tc_fence_after();
-      if (p.tma_epi) {
-        // ---- staged path.  The warp owns 32 rows x 128 accumulator columns, read from TMEM in
-        // four 32-column pieces; the load of the next piece is in flight while this one goes
-        // through bias / activation / residual.  Output leaves in chunks of CW columns
-        // (128 bytes per row): swizzled staging buffer -> one TMA store. ----
-        // chunk = cw columns; its staged rows are cw * sizeof(TOut) bytes (128, or 64 when a
-        // 16-bit tile half is not a multiple of 64 columns), residual rows cw * 2 bytes
-        const int cw = p.cw;
-        const int SUBS = cw / 32;                          // 32-column pieces per chunk
-        const int OUT_ROW_BYTES = cw * static_cast<int>(sizeof(TOut));
-        const int RES_ROW_BYTES = cw * 2;                  // residual is 16-bit
-        const int half_cols = bn / 2;
-        const int row0 = m_blk * BM + quarter * 32;
-        const int gcol_base = n_blk * bn + half_sel * half_cols;
-        const uint32_t t_base = tmem_base + static_cast<uint32_t>(acc * BN + half_sel * half_cols) +
-                                (static_cast<uint32_t>(quarter * 32) << 16);
-        // pieces that hold real columns (uniform across the warp; N is a multiple of 4 here)
-        const int n_sub = gcol_base >= p.N ? 0 : min(half_cols / 32, (p.N - gcol_base + 31) / 32);
-        // 16-byte pieces of a staged row are XOR-swizzled the way TMA expects them:
-        // 128-byte rows: piece ^ (row % 8); 64-byte rows: piece ^ ((row / 2) % 4)
-        const int swz_out = OUT_ROW_BYTES == 128 ? (lane & 7) : ((lane >> 1) & 3);
-        const int swz_res = RES_ROW_BYTES == 128 ? (lane & 7) : ((lane >> 1) & 3);
+      auto wait_acc = [&]() __attribute__((always_inline)) -> bool {
+        const bool done = mbar_wait_warp(&acc_full_bar[acc], acc_phase, abort_flag);
+        if (!done) atomicCAS(p.err, 0u, 0x40000000u | static_cast<uint32_t>(acc));
+        tc_fence_after();
+        return done;
+      };
+      if (p.vec_ok) {
+        // The warp owns 32 rows x half_cols accumulator columns, read from tensor memory in
+        // pieces of 32; the next piece's accumulator and residual loads are in flight while this
+        // one goes through bias / activation / residual.
+        // Bias and the first residual piece are fetched before the accumulator is waited for.
+        const size_t row_off = static_cast<size_t>(row) * p.N + gcol_base;
         uint32_t raw[32];
+        uint32_t rr[16];
+        auto fetch_res = [&](int sub) __attribute__((always_inline)) {
+          if (res && row_ok) {
+            ld_global_32B(res + row_off + sub * 32, rr);
+            if (gcol_base + sub * 32 + 16 < p.N) ld_global_32B(res + row_off + sub * 32 + 16, rr + 8);
+          }
+        };
+        if (n_sub > 0) fetch_res(0);
+        if (p.bias) {
+          const int c = gcol_base + lane * 4;
+          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (c < p.N) b = __ldg(reinterpret_cast<const float4 *>(p.bias + c));
+          __syncwarp();  // the previous tile's values have been read
+          *reinterpret_cast<float4 *>(&bias_s[ew][lane * 4]) = b;
+          __syncwarp();
+        }
+        if (!wait_acc()) break;
         if (n_sub > 0) tmem_ld_32x32(t_base, raw);
-        bool chunk_ok = true;
-        uint8_t *my_out = my_out_base;
 #pragma unroll 1
         for (int sub = 0; sub < n_sub; ++sub) {
           const int gcol = gcol_base + sub * 32;
-          const int sub_in_chunk = sub % SUBS;
-          const int gcol_chunk = gcol - sub_in_chunk * 32;
-          if (sub_in_chunk == 0) {
-            if (res && lane == 0) {
-              mbar_arrive_expect_tx(&res_bar[ew], 32 * RES_ROW_BYTES);
-              tma_load_2d(my_res, &tmap_res, &res_bar[ew], gcol_chunk, row0);
-            }
-            // the TMA store that last used this staging buffer must have finished reading it
-            my_out = my_out_base + out_buf * EPI_BUF_BYTES;
-            if (lane == 0) tma_store_wait_read<C::OUT_BUFS - 1>();
-            __syncwarp();
-            if constexpr (C::OUT_BUFS == 2) out_buf ^= 1;
-          }
+          const bool second = gcol + 16 < p.N;  // N is a multiple of 16: half pieces are whole
           tmem_ld_wait_regs(raw);
           float v[32];
 #pragma unroll
@@ -404,120 +292,60 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (p.bias) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-              if (gcol + j < p.N) {
-                const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
-                v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
-              }
+              const float4 b = *reinterpret_cast<const float4 *>(&bias_s[ew][sub * 32 + j]);
+              v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
             }
           }
           act_fast_n<ACT, 32>(v);
           if (res) {
-            if (sub_in_chunk == 0) {
-              if (!mbar_wait_warp(&res_bar[ew], res_phase, abort_flag)) {
-                atomicCAS(p.err, 0u, 0x50000000u | static_cast<uint32_t>(ew));
-                chunk_ok = false;
-                break;
-              }
-              res_phase ^= 1;
-            }
-            // this piece is 64 bytes (four 16-byte pieces) of the residual row
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int phys = (sub_in_chunk * 4 + j) ^ swz_res;
+            for (int j = 0; j < 32; j += 8) {
               float rv[8];
-              load_res8(reinterpret_cast<const T16 *>(my_res + lane * RES_ROW_BYTES + (phys << 4)), rv);
+              unpack_res8<T16>(rr + j / 2, rv);
 #pragma unroll
-              for (int e = 0; e < 8; ++e) v[8 * j + e] += rv[e];
+              for (int e = 0; e < 8; ++e) v[j + e] += rv[e];
             }
+            if (sub + 1 < n_sub) fetch_res(sub + 1);
           }
-          if constexpr (sizeof(TOut) == 2) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {  // 32 columns = four 16-byte pieces of the staged row
-              const int phys = (sub_in_chunk * 4 + j) ^ swz_out;
-              store_out8<TOut>(reinterpret_cast<TOut *>(my_out + lane * OUT_ROW_BYTES + (phys << 4)), v + 8 * j);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<float4 *>(my_out + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                  make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          }
-          if (sub_in_chunk == SUBS - 1 || sub + 1 == n_sub) {
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmap_out, my_out, gcol_chunk, row0);  // rows / columns past M / N are clipped
-              tma_store_commit();
-            }
+          if (row_ok) {
+            TOut *dst = out + row_off + sub * 32;
+            store_out16<TOut>(dst, v);
+            if (second) store_out16<TOut>(dst + 16, v + 16);
           }
         }
-        if (!chunk_ok) break;
       } else {
-      const int row = m_blk * BM + quarter * 32 + lane;
-      const bool row_ok = row < p.M;
+        // ragged or unaligned rows: one element at a time (static register indices)
+        if (!wait_acc()) break;
 #pragma unroll 1
-      for (int chunk = 0; chunk < bn / 2 / 32; ++chunk) {
-        const int col0 = half_sel * (bn / 2) + chunk * 32;
-        const int gcol0 = n_blk * bn + col0;
-        if (gcol0 >= p.N) break;  // uniform across the warp
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + static_cast<uint32_t>(acc * BN + col0) +
-                          (static_cast<uint32_t>(quarter * 32) << 16),
-                      r);
-        tmem_ld_wait();
-        const int ncols = min(32, p.N - gcol0);
-        if (ncols == 32 && p.out_vec_ok) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[8 * g + j]);
-            if (p.bias) {
-              if (p.bias_vec_ok) {
-                const float4 b0 = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol0 + 8 * g));
-                const float4 b1 = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol0 + 8 * g) + 1);
-                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
-              } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] += __ldg(p.bias + gcol0 + 8 * g + j);
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = act_apply_t<ACT>(v[j]);
-            if (row_ok) {
-              const size_t off = static_cast<size_t>(row) * p.N + gcol0 + 8 * g;
-              if (res) {
-                float rv[8];
-                load_res8(res + off, rv);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] += rv[j];
-              }
-              store_out8<TOut>(out + off, v);
-            }
-          }
-        } else if (row_ok) {
-          // ragged edge or unaligned rows: one element at a time (static register indices)
+        for (int sub = 0; sub < n_sub; ++sub) {
+          const int gcol = gcol_base + sub * 32;
+          uint32_t raw[32];
+          tmem_ld_32x32(t_base + sub * 32, raw);
+          tmem_ld_wait_regs(raw);
+          float v[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (j < ncols) {
-              float v = __uint_as_float(r[j]);
-              if (p.bias) v += __ldg(p.bias + gcol0 + j);
-              v = act_apply_t<ACT>(v);
-              const size_t off = static_cast<size_t>(row) * p.N + gcol0 + j;
-              if (res) v += static_cast<float>(res[off]);
-              out[off] = static_cast<TOut>(v);
+            v[j] = __uint_as_float(raw[j]);
+            if (p.bias && gcol + j < p.N) v[j] += __ldg(p.bias + gcol + j);
+          }
+          act_fast_n<ACT, 32>(v);
+          if (row_ok) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (gcol + j < p.N) {
+                const size_t off = static_cast<size_t>(row) * p.N + gcol + j;
+                if (res) v[j] += static_cast<float>(res[off]);
+                out[off] = static_cast<TOut>(v[j]);
+              }
             }
           }
         }
-      }
       }
       tc_fence_before();
       if constexpr (CG == 2) mbar_arrive_cluster(acc ? acc_empty_addr1 : acc_empty_addr0);
       else mbar_arrive(&acc_empty_bar[acc]);
       if ((acc ^= 1) == 0) acc_phase ^= 1;
     }
-    if (lane == 0) tma_store_wait<0>();  // all staged output has left shared memory
   }
   // ------------------------------ teardown ------------------------------
   if (*abort_flag) {
@@ -586,8 +414,7 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
 }
 
 template <typename T16, typename TOut, int ACT, int CG>
-static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to,
-                           const CUtensorMap &tr, const GemmParams &p, int grid, cudaStream_t s) {
+static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, cudaStream_t s) {
   auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG>;
   constexpr size_t smem = gemm::Cfg<CG>::SMEM_BYTES;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
@@ -600,7 +427,7 @@ static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const C
   }
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gemm::THREADS), smem, s, CG, ta, tb, to, tr, p),
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gemm::THREADS), smem, s, CG, ta, tb, p),
                "launch gemm");
   }
   launched("gemm_tcgen05_kernel");
@@ -608,20 +435,18 @@ static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const C
 
 // p.cta_group selects the variant; grid is CTAs (even for pairs)
 template <typename T16, typename TOut, int ACT>
-static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to,
-                        const CUtensorMap &tr, const GemmParams &p, int grid, cudaStream_t s) {
-  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2>(ta, tb, to, tr, p, grid, s);
-  else launch_gemm_cg<T16, TOut, ACT, 1>(ta, tb, to, tr, p, grid, s);
+static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, cudaStream_t s) {
+  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2>(ta, tb, p, grid, s);
+  else launch_gemm_cg<T16, TOut, ACT, 1>(ta, tb, p, grid, s);
 }
 
 template <typename T16, typename TOut>
-static void launch_gemm_act(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &to,
-                            const CUtensorMap &tr, const GemmParams &p, int grid, int act, cudaStream_t s) {
+static void launch_gemm_act(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, int act, cudaStream_t s) {
   switch (act) {
-  case MGPU_ACT_NONE: launch_gemm<T16, TOut, kActNone>(ta, tb, to, tr, p, grid, s); break;
-  case MGPU_ACT_RELU: launch_gemm<T16, TOut, kActRelu>(ta, tb, to, tr, p, grid, s); break;
-  case MGPU_ACT_GELU_ERF: launch_gemm<T16, TOut, kActGeluErf>(ta, tb, to, tr, p, grid, s); break;
-  case MGPU_ACT_GELU_TANH: launch_gemm<T16, TOut, kActGeluTanh>(ta, tb, to, tr, p, grid, s); break;
+  case MGPU_ACT_NONE: launch_gemm<T16, TOut, kActNone>(ta, tb, p, grid, s); break;
+  case MGPU_ACT_RELU: launch_gemm<T16, TOut, kActRelu>(ta, tb, p, grid, s); break;
+  case MGPU_ACT_GELU_ERF: launch_gemm<T16, TOut, kActGeluErf>(ta, tb, p, grid, s); break;
+  case MGPU_ACT_GELU_TANH: launch_gemm<T16, TOut, kActGeluTanh>(ta, tb, p, grid, s); break;
   default: fail("mgpuMatmulEx16: unknown activation");
   }
 }
@@ -716,27 +541,8 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
   p.bias = bias;
   p.residual = residual;
   p.out = out;
-  const size_t out_elem = dtype_size(out_dtype);
-  const int out_vec = static_cast<int>(16 / out_elem);
-  p.out_vec_ok = (N % out_vec == 0) && (N % 8 == 0) && !(reinterpret_cast<uintptr_t>(out) & 15u) &&
-                 (!residual || !(reinterpret_cast<uintptr_t>(residual) & 15u));
-  p.bias_vec_ok = bias && !(reinterpret_cast<uintptr_t>(bias) & 15u);
-  // staged (TMA) epilogue: rows of out / residual must be multiples of 16 bytes and the
-  // bias readable as float4
-  p.tma_epi = p.out_vec_ok && (!bias || p.bias_vec_ok);
-  CUtensorMap to = ta, tr = ta;  // placeholders when the direct-store epilogue is used
-  // staged chunks of 64 columns (128-byte rows) for 16-bit output when a tile half is a
-  // multiple of 64 columns, else 32 columns
-  const uint32_t cw = (out_elem == 2 && (bn / 2) % 64 == 0) ? 64 : 32;
-  p.cw = static_cast<int>(cw);
-  if (p.tma_epi) {
-    if (!encode_tmap_2d_ex(&to, out, out_dtype, static_cast<uint64_t>(N), static_cast<uint64_t>(M),
-                           static_cast<uint64_t>(N) * out_elem, cw, 32, static_cast<int>(cw * out_elem)))
-      return;
-    if (residual && !encode_tmap_2d_ex(&tr, residual, dtype, static_cast<uint64_t>(N), static_cast<uint64_t>(M),
-                                       static_cast<uint64_t>(N) * 2, cw, 32, static_cast<int>(cw * 2)))
-      return;
-  }
+  auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
+  p.vec_ok = N % 16 == 0 && al(out, 32) && (!residual || al(residual, 32)) && (!bias || al(bias, 16));
   p.num_m_blocks = static_cast<int>((M + gemm::BM - 1) / gemm::BM);
   p.num_n_blocks = static_cast<int>((N + bn - 1) / bn);
   p.err = err;
@@ -744,12 +550,12 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
   if (grid <= 0) { failf("too many tiles"); return; }
 
   if (dtype == MGPU_DTYPE_F16) {
-    if (out_dtype == MGPU_DTYPE_F16) launch_gemm_act<__half, __half>(ta, tb, to, tr, p, grid, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__half, float>(ta, tb, to, tr, p, grid, act, s);
+    if (out_dtype == MGPU_DTYPE_F16) launch_gemm_act<__half, __half>(ta, tb, p, grid, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__half, float>(ta, tb, p, grid, act, s);
     else failf("output type must be the operand type or F32");
   } else {
-    if (out_dtype == MGPU_DTYPE_BF16) launch_gemm_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, to, tr, p, grid, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__nv_bfloat16, float>(ta, tb, to, tr, p, grid, act, s);
+    if (out_dtype == MGPU_DTYPE_BF16) launch_gemm_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, grid, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__nv_bfloat16, float>(ta, tb, p, grid, act, s);
     else failf("output type must be the operand type or F32");
   }
 }
