@@ -50,6 +50,10 @@ struct EncoderStack {
   // all runs of a stack share one activation workspace
   cudaEvent_t done_ev = nullptr;
   bool used = false;
+  // recorded after the last layer's weights were packed; once it has been seen complete, the Gemms
+  // may read weights ahead of their dependency on the previous kernel
+  cudaEvent_t weights_ev = nullptr;
+  bool weights_complete = false;
   // CUDA graphs of whole runs, keyed by the run's pointers and shape (see run_stack_replayed)
   struct RunGraph {
     const float *x = nullptr;
@@ -144,6 +148,7 @@ static void destroy_stack(EncoderStack *st, void *stream) {
     if (st->ev_out[i]) cudaEventDestroy(st->ev_out[i]);
   }
   if (st->done_ev) cudaEventDestroy(st->done_ev);
+  if (st->weights_ev) cudaEventDestroy(st->weights_ev);
   if (st->s_in) cudaStreamDestroy(st->s_in);
   if (st->s_comp) cudaStreamDestroy(st->s_comp);
   if (st->s_out) cudaStreamDestroy(st->s_out);
@@ -153,7 +158,7 @@ static void destroy_stack(EncoderStack *st, void *stream) {
 // x_f32 != nullptr: input is fp32 and is cast first; else `cur` already holds 16-bit input.
 // y_f32 receives the fp32 result.
 static void run_stack(EncoderStack *st, const float *x_f32, const int32_t *seq_lens, float *y_f32,
-                      int64_t B, int64_t S, void *stream) {
+                      int64_t B, int64_t S, bool w_ready, void *stream) {
   const int64_t T = B * S, d = st->d, F = st->F;
   const int32_t dt = st->dtype;
   Workspace &w = st->ws;
@@ -168,22 +173,22 @@ static void run_stack(EncoderStack *st, const float *x_f32, const int32_t *seq_l
     }
     if (st->norm_first) {
       mgpuLayerNormEx(w.cur, nullptr, lw.ln1_g, lw.ln1_b, nullptr, w.n1, st->eps, T, d, dt, dt, stream);
-      mgpuMatmulEx16(w.n1, lw.wqkv, lw.bqkv, nullptr, w.qkv, T, 3 * d, d, dt, dt, MGPU_ACT_NONE, stream);
+      matmul16(w.n1, lw.wqkv, lw.bqkv, nullptr, w.qkv, T, 3 * d, d, dt, dt, MGPU_ACT_NONE, w_ready, stream);
       mgpuAttention(w.qkv, seq_lens, w.att, B, S, st->H, d / st->H, st->causal, dt, stream);
-      mgpuMatmulEx16(w.att, lw.wo, lw.bo, w.cur, w.a, T, d, d, dt, dt, MGPU_ACT_NONE, stream);
+      matmul16(w.att, lw.wo, lw.bo, w.cur, w.a, T, d, d, dt, dt, MGPU_ACT_NONE, w_ready, stream);
       mgpuLayerNormEx(w.a, nullptr, lw.ln2_g, lw.ln2_b, nullptr, w.n1, st->eps, T, d, dt, dt, stream);
-      mgpuMatmulEx16(w.n1, lw.w1, lw.b1, nullptr, w.f1, T, F, d, dt, dt, st->act, stream);
+      matmul16(w.n1, lw.w1, lw.b1, nullptr, w.f1, T, F, d, dt, dt, st->act, w_ready, stream);
       if (last)
-        mgpuMatmulEx16(w.f1, lw.w2, lw.b2, w.a, y_f32, T, d, F, dt, MGPU_DTYPE_F32, MGPU_ACT_NONE, stream);
+        matmul16(w.f1, lw.w2, lw.b2, w.a, y_f32, T, d, F, dt, MGPU_DTYPE_F32, MGPU_ACT_NONE, w_ready, stream);
       else
-        mgpuMatmulEx16(w.f1, lw.w2, lw.b2, w.a, w.cur, T, d, F, dt, dt, MGPU_ACT_NONE, stream);
+        matmul16(w.f1, lw.w2, lw.b2, w.a, w.cur, T, d, F, dt, dt, MGPU_ACT_NONE, w_ready, stream);
     } else {
-      mgpuMatmulEx16(w.cur, lw.wqkv, lw.bqkv, nullptr, w.qkv, T, 3 * d, d, dt, dt, MGPU_ACT_NONE, stream);
+      matmul16(w.cur, lw.wqkv, lw.bqkv, nullptr, w.qkv, T, 3 * d, d, dt, dt, MGPU_ACT_NONE, w_ready, stream);
       mgpuAttention(w.qkv, seq_lens, w.att, B, S, st->H, d / st->H, st->causal, dt, stream);
-      mgpuMatmulEx16(w.att, lw.wo, lw.bo, w.cur, w.a, T, d, d, dt, dt, MGPU_ACT_NONE, stream);
+      matmul16(w.att, lw.wo, lw.bo, w.cur, w.a, T, d, d, dt, dt, MGPU_ACT_NONE, w_ready, stream);
       mgpuLayerNormEx(w.a, nullptr, lw.ln1_g, lw.ln1_b, nullptr, w.n1, st->eps, T, d, dt, dt, stream);
-      mgpuMatmulEx16(w.n1, lw.w1, lw.b1, nullptr, w.f1, T, F, d, dt, dt, st->act, stream);
-      mgpuMatmulEx16(w.f1, lw.w2, lw.b2, w.n1, w.a, T, d, F, dt, dt, MGPU_ACT_NONE, stream);
+      matmul16(w.n1, lw.w1, lw.b1, nullptr, w.f1, T, F, d, dt, dt, st->act, w_ready, stream);
+      matmul16(w.f1, lw.w2, lw.b2, w.n1, w.a, T, d, F, dt, dt, MGPU_ACT_NONE, w_ready, stream);
       if (last)
         mgpuLayerNormEx(w.a, nullptr, lw.ln2_g, lw.ln2_b, nullptr, y_f32, st->eps, T, d, dt, MGPU_DTYPE_F32, stream);
       else
@@ -206,16 +211,21 @@ static bool graphs_enabled() {
 static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *lens, float *y, int64_t B, int64_t S,
                                void *stream) {
   cudaStream_t s = as_stream(stream);
-  bool eligible = graphs_enabled() && !st->graphs_off && !g_profiling && s != nullptr;
-  if (eligible) {
+  bool capturing = false;
+  if (s != nullptr) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-      (void)cudaGetLastError();
-      eligible = false;
-    }
+    capturing = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
   }
+  // (an event cannot be asked about inside a capture; what was seen before it still holds)
+  if (!st->weights_complete && !capturing && st->weights_ev) {
+    st->weights_complete = cudaEventQuery(st->weights_ev) == cudaSuccess;
+    (void)cudaGetLastError();
+  }
+  const bool w_ready = st->weights_complete;
+  const bool eligible = graphs_enabled() && !st->graphs_off && !g_profiling && s != nullptr && !capturing;
   if (!eligible) {
-    run_stack(st, x, lens, y, B, S, stream);
+    run_stack(st, x, lens, y, B, S, w_ready, stream);
     return;
   }
   EncoderStack::RunGraph *g = nullptr;
@@ -237,11 +247,11 @@ static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *
       return;
     }
     st->graphs_off = true;
-    run_stack(st, x, lens, y, B, S, stream);
+    run_stack(st, x, lens, y, B, S, w_ready, stream);
     return;
   }
   if (g->seen++ == 0 || mgpuGetLastError() != 0) {
-    run_stack(st, x, lens, y, B, S, stream);
+    run_stack(st, x, lens, y, B, S, w_ready, stream);
     return;
   }
   // second run with this key: capture it, then launch what was captured
@@ -249,11 +259,11 @@ static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     (void)cudaGetLastError();
     st->graphs_off = true;
-    run_stack(st, x, lens, y, B, S, stream);
+    run_stack(st, x, lens, y, B, S, w_ready, stream);
     return;
   }
   const uint64_t launches_before = g_launch_count.load(std::memory_order_relaxed);
-  run_stack(st, x, lens, y, B, S, stream);
+  run_stack(st, x, lens, y, B, S, w_ready, stream);
   const cudaError_t end = cudaStreamEndCapture(s, &graph);
   g_launch_count.store(launches_before, std::memory_order_relaxed);  // captured, not yet launched
   cudaGraphExec_t exec = nullptr;
@@ -262,7 +272,7 @@ static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *
     (void)cudaGetLastError();
     if (graph) cudaGraphDestroy(graph);
     st->graphs_off = true;
-    if (mgpuGetLastError() == 0) run_stack(st, x, lens, y, B, S, stream);
+    if (mgpuGetLastError() == 0) run_stack(st, x, lens, y, B, S, w_ready, stream);
     return;
   }
   cudaGraphDestroy(graph);
@@ -329,6 +339,11 @@ MDC_API void mgpuEncoderStackSetLayer(void *stack, int64_t layer, const float *q
   lw.ln1_b = dup_f32(ln1_beta, d, stream);
   lw.ln2_g = dup_f32(ln2_gamma, d, stream);
   lw.ln2_b = dup_f32(ln2_beta, d, stream);
+  st->weights_complete = false;
+  // layers may be set on different streams: each recording also covers the earlier ones
+  if (st->weights_ev) cudaStreamWaitEvent(as_stream(stream), st->weights_ev, 0);
+  if (!st->weights_ev && !check_cuda(cudaEventCreateWithFlags(&st->weights_ev, cudaEventDisableTiming), "event")) return;
+  cudaEventRecord(st->weights_ev, as_stream(stream));
 }
 
 MDC_API void mgpuEncoderStackRun(void *stack, const float *x, const int32_t *seq_lens, float *y,
@@ -521,7 +536,7 @@ MDC_API void mgpuTransformerEncoderLayer(const float *input, const float *qkv_we
   lw.ln2_g = const_cast<float *>(ln2_gamma);
   lw.ln2_b = const_cast<float *>(ln2_beta);
   if (lw.wqkv && lw.wo && lw.w1 && lw.w2) {
-    if (ensure_ws(&st, batch * seq_len, stream)) run_stack(&st, input, seq_lens, output, batch, seq_len, stream);
+    if (ensure_ws(&st, batch * seq_len, stream)) run_stack(&st, input, seq_lens, output, batch, seq_len, false, stream);
   } else {
     fail("mgpuTransformerEncoderLayer: out of device memory for the packed weights");
   }

@@ -1,0 +1,445 @@
+// Tensor-core Gemm for problems that fit the chip in one wave: the same operation as
+// gemm_tcgen05.cu (out = act(A . W^T + bias) + residual, 16-bit operands, fp32 accumulation in
+// tensor memory), one output tile per CTA (or CTA pair), and the K range of a tile optionally cut
+// over a cluster of CTAs.
+//
+// What bounds these shapes is latency, not the tensor pipe: a Gemm of a few hundred rows has too
+// few 256 x 256 tiles to use the chip, and every CTA works through its whole K range alone, at
+// 0.2 us per 64-wide k-block whatever the tile (MMA issue and barrier waits).  So
+//   * the tile is chosen small enough that about every SM has one (choose_gemm_tile), down to
+//     16 output columns;
+//   * `splits` CTAs (or pairs) of a cluster each take a slice of K; the fp32 partial tiles are
+//     exchanged through distributed shared memory, each CTA receiving the columns it finishes,
+//     and added in slice order, so the result does not depend on timing;
+//   * a ring stage holds `depth` k-blocks, fetched by one TMA instruction per operand and handed
+//     over by one barrier, and the ring is as deep as shared memory allows: a short K range is
+//     in flight as a whole and costs one memory latency;
+//   * A's box is as high as M needs; accumulator rows beyond it hold stale operands and are not
+//     stored;
+//   * W's first stages are requested before the dependency on the previous kernel is resolved
+//     when the caller knows the weights to be complete;
+//   * results go straight from registers to global memory.
+#include <cstdlib>
+#include <type_traits>
+
+#include "gemm_common.cuh"
+#include "gemm_plan.h"
+#include "ops_common.h"
+
+namespace mdc {
+
+namespace gsplit {
+constexpr int BK = 64;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + EPI_WARPS * 32;
+constexpr int MAX_STAGES = 16;
+}  // namespace gsplit
+
+struct SplitParams {
+  int M, N, num_kb;  // num_kb: 64-wide k-blocks
+  const float *bias;
+  const void *residual;
+  void *out;
+  int vec_ok;   // rows of out / residual can be accessed in 32-byte vectors, bias in 16-byte ones
+  int n_tiles;  // column tiles
+  int bn, box_m, splits, depth, stages;
+  int tmem_cols;
+  int k_in_x;   // operand maps are (k, row) instead of (64 k, row, k-block)
+  int w_ready;  // W may be read before the dependency wait
+  uint32_t *err;
+};
+
+template <typename T16, typename TOut, int ACT, int CG>
+__global__ void __launch_bounds__(gsplit::THREADS, 2)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                  const SplitParams p) {
+  using namespace gsplit;
+  using namespace ptx;
+  extern __shared__ uint8_t smem_dyn[];
+  __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ uint32_t abort_flag_s;
+  volatile uint32_t *abort_flag = &abort_flag_s;
+
+  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
+                                               ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = p.splits, cluster = CG * splits;
+  const int rank = cluster > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int half = CG == 2 ? (rank & 1) : 0;  // which 128 rows of a pair's 256
+  const int split = rank / CG;                // which slice of K
+  const bool leader = half == 0;
+  const int tile = static_cast<int>(blockIdx.x) / cluster;
+  const int m_tile = tile / p.n_tiles, n_tile = tile - m_tile * p.n_tiles;
+  const int row0 = (m_tile * CG + half) * p.box_m, col0 = n_tile * p.bn;
+  const int kb0 = p.num_kb * split / splits, kb1 = p.num_kb * (split + 1) / splits;
+  const int depth = p.depth, stages = p.stages;
+  const int a_kb_bytes = p.box_m * BK * 2, b_rows = p.bn / CG, b_kb_bytes = b_rows * BK * 2;
+  const int a_bytes = a_kb_bytes * depth;
+  const int stage_bytes = a_bytes + b_kb_bytes * depth;
+  const int steps = (kb1 - kb0 + depth - 1) / depth;
+
+  if (threadIdx.x == 0) {
+    abort_flag_s = 0;
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_bar, 1);
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    if constexpr (CG == 2) {
+      tmem_alloc_cg2(&tmem_slot, static_cast<uint32_t>(p.tmem_cols));
+      tmem_relinquish_cg2();
+    } else {
+      tmem_alloc(&tmem_slot, static_cast<uint32_t>(p.tmem_cols));
+      tmem_relinquish();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (CG == 2) cluster_sync_all();  // the peer's barriers exist before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_launch_dependents();  // after this CTA holds its tensor memory (see gemm_tcgen05.cu)
+
+  // a stage is always filled whole: k-blocks past this CTA's slice are fetched (or read as zeros
+  // past K) and not used
+  auto kx = [&](int kb) { return p.k_in_x ? kb * BK : 0; };
+  auto kz = [&](int kb) { return p.k_in_x ? 0 : kb; };
+  auto load_w = [&](int s, int kb) __attribute__((always_inline)) {
+    uint8_t *sb = tiles + s * stage_bytes + a_bytes;
+    if constexpr (CG == 2)
+      tma_load_3d_cg2(sb, &tmap_b, mapa_u32(smem_u32(&full_bar[s]), static_cast<uint32_t>(rank & ~1)), kx(kb), col0 + half * b_rows, kz(kb));
+    else
+      tma_load_3d(sb, &tmap_b, &full_bar[s], kx(kb), col0, kz(kb));
+  };
+  auto load_a = [&](int s, int kb) __attribute__((always_inline)) {
+    uint8_t *sa = tiles + s * stage_bytes;
+    if constexpr (CG == 2)
+      tma_load_3d_cg2(sa, &tmap_a, mapa_u32(smem_u32(&full_bar[s]), static_cast<uint32_t>(rank & ~1)), kx(kb), row0, kz(kb));
+    else
+      tma_load_3d(sa, &tmap_a, &full_bar[s], kx(kb), row0, kz(kb));
+  };
+  auto expect = [&](int s) __attribute__((always_inline)) {
+    if (leader) mbar_arrive_expect_tx(&full_bar[s], static_cast<uint32_t>(CG * stage_bytes));
+  };
+
+  int early = 0;  // stages whose W is already on its way
+  if (warp == 0 && p.w_ready) {
+    early = min(stages, steps);
+    if (elect_one()) {
+      for (int i = 0; i < early; ++i) {
+        expect(i);
+        load_w(i, kb0 + i * depth);
+      }
+    }
+    __syncwarp();
+  }
+  pdl_wait();  // everything above overlaps the previous kernel's tail; activations are read below
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < steps; ++i) {
+      if (i >= early && !mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x81000000u | static_cast<uint32_t>(stage));
+        break;
+      }
+      __syncwarp();
+      if (elect_one()) {
+        if (i >= early) {
+          expect(stage);
+          load_w(stage, kb0 + i * depth);
+        }
+        load_a(stage, kb0 + i * depth);
+      }
+      if (++stage == stages) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (leader of the pair) ------------------------------
+    if (leader) {
+      const uint32_t idesc = make_idesc_f16(128 * CG, static_cast<uint32_t>(p.bn), std::is_same<T16, __nv_bfloat16>::value,
+                                            false, false);
+      const uint64_t desc0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int i = 0; i < steps; ++i) {
+        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+          atomicCAS(p.err, 0u, 0x82000000u | static_cast<uint32_t>(stage));
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        tc_fence_after();
+        uint64_t a_desc = desc0 + static_cast<uint64_t>((stage * stage_bytes) >> 4);
+        uint64_t b_desc = a_desc + static_cast<uint64_t>(a_bytes >> 4);
+        const int n = min(depth, kb1 - kb0 - i * depth);
+        for (int d = 0; d < n; ++d) {
+          if constexpr (CG == 2) umma_f16_ss_kblock_cg2(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
+          else umma_f16_ss_kblock(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
+          a_desc += static_cast<uint64_t>(a_kb_bytes >> 4);
+          b_desc += static_cast<uint64_t>(b_kb_bytes >> 4);
+        }
+        if constexpr (CG == 2) umma_commit_cg2_warp(&empty_bar[stage], static_cast<uint16_t>(3u << rank));
+        else umma_commit_warp(&empty_bar[stage]);
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+      }
+      if (ok) {
+        if constexpr (CG == 2) umma_commit_cg2_warp(&acc_bar, static_cast<uint16_t>(3u << rank));
+        else umma_commit_warp(&acc_bar);
+      }
+    }
+  }
+  __syncwarp();
+
+  // ------------------------------ epilogue ------------------------------
+  const int ew = warp - 2;
+  const int quarter = warp & 3;        // tensor-memory lanes this warp may access
+  const int half_sel = ew >> 2;        // which half of the columns
+  const int own_cols = p.bn / splits;  // columns this CTA finishes
+  // in pieces of 16 (32 bytes of a 16-bit row, so that vector accesses stay aligned): the first half
+  // of the warps takes the first half of the pieces, rounded up
+  const int c_mid = (own_cols / 16 + 1) / 2 * 16;
+  const int c_begin = half_sel ? c_mid : 0, c_end = half_sel ? own_cols : c_mid;
+  const int rows_in_tile = quarter * 32 + lane;
+  const bool live_warp = warp >= 2 && quarter * 32 < p.box_m;  // box_m is a multiple of 32
+  bool ok = true;
+  if (live_warp) {
+    if (!mbar_wait_warp(&acc_bar, 0, abort_flag)) {
+      if (lane == 0) atomicCAS(p.err, 0u, 0x83000000u);
+      ok = false;
+    }
+    tc_fence_after();
+  }
+  const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+  // partial tiles received: [slot][column / 4][128 rows] of float4
+  const float4 *part = reinterpret_cast<const float4 *>(tiles);
+  if (splits > 1) {
+    // every CTA of the cluster has finished reading its ring before anyone writes into it
+    cluster_sync_all();
+    if (live_warp && ok) {
+      for (int d = 1; d < splits; ++d) {
+        const int to = split + d < splits ? split + d : split + d - splits;
+        const int slot = split < to ? split : split - 1;
+        const uint32_t dst = mapa_u32(smem_u32(tiles), static_cast<uint32_t>(to * CG + half));
+        for (int c = c_begin; c < c_end; c += 8) {
+          uint32_t r[8];
+          tmem_ld_32x8(t_lane + static_cast<uint32_t>(to * own_cols + c), r);
+          tmem_ld_wait_regs(r);
+          const uint32_t at = dst + static_cast<uint32_t>(((slot * (own_cols / 4) + c / 4) * 128 + rows_in_tile) * 16);
+          st_cluster_v4(at, r[0], r[1], r[2], r[3]);
+          st_cluster_v4(at + 128 * 16, r[4], r[5], r[6], r[7]);
+        }
+      }
+    }
+    cluster_sync_all();
+  }
+  if (live_warp && ok) {
+    TOut *out = static_cast<TOut *>(p.out);
+    const T16 *res = static_cast<const T16 *>(p.residual);
+    const int row = row0 + rows_in_tile;
+    const bool row_ok = row < p.M;
+#pragma unroll 1
+    for (int c = c_begin; c < c_end; c += 16) {
+      constexpr int NC = 16;
+      const int gcol = col0 + split * own_cols + c;
+      if (gcol >= p.N) break;  // uniform across the warp
+      uint32_t acc[NC];
+      tmem_ld_32x16(t_lane + static_cast<uint32_t>(split * own_cols + c), acc);
+      const size_t off = static_cast<size_t>(row) * p.N + gcol;
+      const bool whole = p.vec_ok && gcol + NC <= p.N;
+      float b[NC], rv[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) b[j] = rv[j] = 0.f;
+      if (p.bias) {
+        if (whole) {
+#pragma unroll
+          for (int j = 0; j < NC; j += 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
+            b[j] = q.x, b[j + 1] = q.y, b[j + 2] = q.z, b[j + 3] = q.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < NC; ++j)
+            if (gcol + j < p.N) b[j] = __ldg(p.bias + gcol + j);
+        }
+      }
+      if (res && row_ok) {
+        if (whole) {
+          uint32_t rr[NC / 2];
+          ld_global_32B(res + off, rr);
+#pragma unroll
+          for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NC; ++j)
+            if (gcol + j < p.N) rv[j] = static_cast<float>(res[off + j]);
+        }
+      }
+      tmem_ld_wait_regs(acc);
+      float v[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]);
+      if (splits > 1) {
+        // sum in slice order: slices before this CTA's, its own, the later ones
+        float s[NC];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) s[j] = split == 0 ? v[j] : 0.f;
+        for (int t = 0; t < splits; ++t) {
+          if (t == split) {
+            if (t > 0) {
+#pragma unroll
+              for (int j = 0; j < NC; ++j) s[j] += v[j];
+            }
+          } else {
+            const float4 *q = part + ((t < split ? t : t - 1) * (own_cols / 4) + c / 4) * 128 + rows_in_tile;
+#pragma unroll
+            for (int j = 0; j < NC; j += 4) {
+              const float4 f = q[(j / 4) * 128];
+              s[j] += f.x, s[j + 1] += f.y, s[j + 2] += f.z, s[j + 3] += f.w;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < NC; ++j) v[j] = s[j];
+      }
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] += b[j];
+      act_fast_n<ACT, NC>(v);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] += rv[j];
+      if (row_ok) {
+        if (whole) {
+          store_out16<TOut>(out + off, v);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NC; ++j)
+            if (gcol + j < p.N) out[off + j] = static_cast<TOut>(v[j]);
+        }
+      }
+    }
+  }
+  // ------------------------------ teardown ------------------------------
+  if (*abort_flag) {
+    // a wait gave up: give copies still in flight time to land before the CTA retires
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (CG == 2) cluster_sync_all();  // neither CTA of a pair frees tensor memory under the other
+  tc_fence_after();
+  if (warp == 1) {
+    if constexpr (CG == 2) tmem_dealloc_cg2(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+    else tmem_dealloc(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+  }
+}
+
+template <typename T16, typename TOut, int ACT, int CG>
+static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int grid, size_t smem,
+                            cudaStream_t s) {
+  auto kern = gemm_split_kernel<T16, TOut, ACT, CG>;
+  constexpr int kMaxDevices = 64;
+  static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
+  const int dev = device_info().device;
+  bool &attr_set = attr_set_on[(dev >= 0 && dev < kMaxDevices) ? dev : 0];
+  if (!attr_set) {
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitMaxSmem),
+                    "cudaFuncSetAttribute(gemm split)"))
+      return;
+    attr_set = true;
+  }
+  {
+    ProfileScope prof(kCatGemm, s);
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gsplit::THREADS), smem, s, CG * p.splits, ta, tb, p),
+               "launch gemm split");
+  }
+  launched("gemm_split_kernel");
+}
+
+template <typename T16, typename TOut>
+static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int cg, int grid,
+                             size_t smem, int act, cudaStream_t s) {
+#define MDC_SPLIT(ACT_)                                                              \
+  do {                                                                               \
+    if (cg == 2) launch_split_cg<T16, TOut, ACT_, 2>(ta, tb, p, grid, smem, s);      \
+    else launch_split_cg<T16, TOut, ACT_, 1>(ta, tb, p, grid, smem, s);              \
+  } while (0)
+  switch (act) {
+  case MGPU_ACT_NONE: MDC_SPLIT(kActNone); break;
+  case MGPU_ACT_RELU: MDC_SPLIT(kActRelu); break;
+  case MGPU_ACT_GELU_ERF: MDC_SPLIT(kActGeluErf); break;
+  case MGPU_ACT_GELU_TANH: MDC_SPLIT(kActGeluTanh); break;
+  default: fail("mgpuMatmulEx16: unknown activation");
+  }
+#undef MDC_SPLIT
+}
+
+// A [rows, Kp] row-major 16-bit matrix.  Kp a multiple of 64: as (64 k, row, k-block), so that one
+// box holds several k-blocks.  Otherwise the last k-block would run into the next row, so the map is
+// (k, row) and ends at Kp, one k-block per box.
+static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, int64_t rows, int64_t Kp, int box_rows,
+                           int depth) {
+  const bool blocked = Kp % gsplit::BK == 0;
+  const uint64_t gdim[3] = {static_cast<uint64_t>(blocked ? gsplit::BK : Kp), static_cast<uint64_t>(rows),
+                            static_cast<uint64_t>(blocked ? Kp / gsplit::BK : 1)};
+  const uint64_t gstr[2] = {static_cast<uint64_t>(Kp) * 2, gsplit::BK * 2};
+  const uint32_t box[3] = {gsplit::BK, static_cast<uint32_t>(box_rows), static_cast<uint32_t>(blocked ? depth : 1)};
+  const uint32_t estr[3] = {1, 1, 1};
+  const int before = mgpuGetLastError();
+  mgpuTensorMapEncodeTiled(map, dtype == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                           3, const_cast<void *>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return before != 0 || mgpuGetLastError() == 0;
+}
+
+void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,
+                       void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act,
+                       bool w_ready, cudaStream_t s) {
+  uint32_t *err = device_error_slot();
+  if (!err) return;
+  CUtensorMap ta, tb;
+  if (!encode_operand(&ta, a, dtype, M, Kp, t.box_m, t.depth) || !encode_operand(&tb, w_nk, dtype, N, Kp, t.bn / t.cg, t.depth))
+    return;
+  SplitParams p;
+  p.M = static_cast<int>(M), p.N = static_cast<int>(N);
+  p.num_kb = static_cast<int>((Kp + gsplit::BK - 1) / gsplit::BK);
+  p.k_in_x = Kp % gsplit::BK != 0;
+  p.bias = bias, p.residual = residual, p.out = out;
+  auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
+  p.vec_ok = N % 16 == 0 && al(out, 32) && (!residual || al(residual, 32)) && (!bias || al(bias, 16));
+  p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
+  p.bn = t.bn, p.box_m = t.box_m, p.splits = t.splits, p.stages = t.stages;
+  p.depth = p.k_in_x ? 1 : t.depth;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < t.bn) p.tmem_cols *= 2;
+  p.w_ready = w_ready ? 1 : 0;
+  p.err = err;
+  const int64_t m_tiles = (M + static_cast<int64_t>(t.box_m) * t.cg - 1) / (static_cast<int64_t>(t.box_m) * t.cg);
+  const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg * t.splits);
+  const size_t stage = static_cast<size_t>(p.depth) * (t.box_m + t.bn / t.cg) * gsplit::BK * 2;
+  const size_t partial = static_cast<size_t>(t.splits - 1) * 128 * (t.bn / t.splits) * 4;
+  // an MMA reads 128 rows of A whatever the box holds: past the last box that must still be this
+  // CTA's memory
+  const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * gsplit::BK * 2 : 0);
+  const size_t smem = (ring > partial ? ring : partial) + 1024;
+  if (dtype == MGPU_DTYPE_F16) {
+    if (out_dtype == MGPU_DTYPE_F16) launch_split_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_split_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);
+    else fail("mgpuMatmulEx16: output type must be the operand type or F32");
+  } else {
+    if (out_dtype == MGPU_DTYPE_BF16) launch_split_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_split_act<__nv_bfloat16, float>(ta, tb, p, t.cg, grid, smem, act, s);
+    else fail("mgpuMatmulEx16: output type must be the operand type or F32");
+  }
+}
+
+}  // namespace mdc

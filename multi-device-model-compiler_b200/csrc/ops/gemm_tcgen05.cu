@@ -36,6 +36,7 @@
 #include <type_traits>
 
 #include "gemm_common.cuh"
+#include "gemm_plan.h"
 #include "ops_common.h"
 
 namespace mdc {
@@ -197,16 +198,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // (descriptors hold addresses in units of 16 bytes)
           const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
           const uint64_t b_desc = a_desc + A_BYTES / 16;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            // 16 k-elements = 32 bytes further along the 128-byte swizzled row
-            if constexpr (CG == 2)
-              umma_f16_ss_cg2_warp(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
-                                   b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-            else
-              umma_f16_ss_warp(d_tmem, a_desc + static_cast<uint64_t>(2 * k),
-                               b_desc + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          if constexpr (CG == 2) umma_f16_ss_kblock_cg2(d_tmem, a_desc, b_desc, idesc, kb != 0 ? 1u : 0u);
+          else umma_f16_ss_kblock(d_tmem, a_desc, b_desc, idesc, kb != 0 ? 1u : 0u);
           // the stage is reusable (in both CTAs) once these MMAs have read it
           if constexpr (CG == 2) {
             umma_commit_cg2_warp(&empty_bar[stage], 3);
@@ -492,6 +485,99 @@ static int choose_bn(int64_t M, int64_t N, int cta_group, int sms) {
   return best;
 }
 
+// Time of a one-wave tile in microseconds, fitted to 1700 measured (shape, tile) pairs (M 32 - 4096,
+// N 768 - 4096, K 768 - 4096, weights from HBM, chained launches; 14 % rms).  The tile it picks is
+// within 3 % of the fastest measured one for 25 of the 28 shapes.  Terms: launch and drain; MMA
+// issue; operand bytes through the SM's load path; one barrier hand-over per ring stage; exchange
+// of partial tiles; epilogue columns; pairing; CTAs to place.
+static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, int sms) {
+  const int64_t m_tiles = (M + t.box_m * t.cg - 1) / (t.box_m * t.cg), n_tiles = (N + t.bn - 1) / t.bn;
+  const int64_t ctas = m_tiles * n_tiles * t.cg * t.splits;
+  if (ctas > 2 * sms) return 1e30f;
+  const float co = static_cast<float>((ctas + sms - 1) / sms);
+  const int kbs = (num_kb + t.splits - 1) / t.splits, steps = (kbs + t.depth - 1) / t.depth;
+  const int rows = M < t.box_m ? static_cast<int>(M) : t.box_m, own = t.bn / t.splits;
+  const float mma = kbs * (t.bn < 100 ? 200.f : 2.f * t.bn) / 1900.f;
+  const float bytes = kbs * static_cast<float>(rows + t.bn / t.cg) * 128.f / 1e5f;
+  float us = 2.2f + 0.33f * mma * co + 0.305f * bytes * co + 0.194f * steps + 0.0125f * own * co +
+             0.65f * static_cast<float>(ctas) / static_cast<float>(sms);
+  if (t.splits > 1) us += 0.8f + 5.7f * (t.splits - 1) * own * t.box_m * 4.f / 1e5f;
+  if (t.cg == 2) us += 1.2f;
+  return us;
+}
+
+// The fastest one-wave tile for a problem of at most one 128 x 128 tile per SM.
+static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool k_whole, int sms) {
+  GemmTile best;
+  float best_us = 1e30f;
+  for (int cg = 1; cg <= 2; ++cg)
+    for (int box_m : {32, 64, 128}) {
+      if (box_m < 128 && (cg == 2 || M > 640)) continue;  // short boxes only pay for few rows
+      if (box_m > 32 && box_m >= 2 * M) continue;
+      for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
+        if (cg == 2 && bn < 64) continue;
+        for (int splits : {1, 2, 3, 4, 6, 8}) {
+          // A slice of less than 4 k-blocks costs more to exchange than to compute; below K = 1024
+          // nothing is split, so there a row's result does not depend on the batch it is in.
+          if (splits > 1 && (num_kb < 16 || splits * 4 > num_kb || splits * cg > 8)) continue;
+          if (bn % (16 * splits) != 0) continue;
+          const int kbs = (num_kb + splits - 1) / splits;
+          for (int depth : {4, 2, 1}) {
+            if (depth > 1 && (!k_whole || depth > kbs)) continue;
+            const int steps = (kbs + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
+            // half an SM's shared memory, so that the next kernel's CTA (which may already fetch
+            // its weights) or a second CTA of this one fits beside it
+            int stages = (110 * 1024 - (128 - box_m) * 128) / stage;
+            if (stages > steps) stages = steps;
+            if (stages > 16) stages = 16;
+            if (stages < 1 || (stages < 2 && steps > 1)) continue;
+            GemmTile t;
+            t.one_wave = true, t.cg = cg, t.box_m = box_m, t.bn = bn, t.splits = splits, t.depth = depth, t.stages = stages;
+            const float us = one_wave_cost(t, M, N, num_kb, sms);
+            if (us < best_us) best_us = us, best = t;
+          }
+        }
+      }
+    }
+  return best;
+}
+
+GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
+#ifdef MDC_SWEEP
+  if (const char *e = getenv("MDC_GEMM_TILE")) {
+    GemmTile t;
+    int ow = 0;
+    if (sscanf(e, "%d,%d,%d,%d,%d,%d,%d", &ow, &t.cg, &t.box_m, &t.bn, &t.splits, &t.depth, &t.stages) == 7) {
+      t.one_wave = ow != 0;
+      return t;
+    }
+  }
+#endif
+  // the choice takes a few microseconds: kept per shape (a plan, not a result)
+  struct Entry {
+    int64_t M = -1, N = -1, K = -1;
+    int sms = 0;
+    GemmTile tile;
+  };
+  static thread_local Entry cache[64];
+  Entry &e = cache[(static_cast<uint64_t>(M) * 0x9E3779B97F4A7C15ull ^ static_cast<uint64_t>(N) * 0xC2B2AE3D27D4EB4Full ^
+                    static_cast<uint64_t>(K) * 0x165667B19E3779F9ull) >> 58];
+  if (e.M == M && e.N == N && e.K == K && e.sms == sms) return e.tile;
+  GemmTile t;
+  // One wave: up to one 128 x 128 tile per SM.  Measured either side of the line: 1024 x 2304 x 768
+  // 7.6 us one-wave, 7.9 persistent; 1024 x 3072 x 768 9.9 and 9.2; 2048 x 768 x 3072 14.1 and 15.5;
+  // 4096 x 768 x 3072 19.2 and 17.6.
+  const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
+  if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
+    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), K % 64 == 0, sms);
+  if (!t.one_wave) {
+    t.cg = choose_cta_group(M);
+    t.bn = choose_bn(M, N, t.cg, sms);
+  }
+  e.M = M, e.N = N, e.K = K, e.sms = sms, e.tile = t;
+  return t;
+}
+
 // persistent grid: one worker (CTA or CTA pair) per tile up to the number the device holds
 static int gemm_grid(const GemmParams &p, int sms) {
   const int cg = p.cta_group;
@@ -513,7 +599,7 @@ static int gemm_grid(const GemmParams &p, int sms) {
 // Shared by every entry point that ends in this Gemm; allocates nothing.
 static void matmul16_launch(const char *who, const void *a, const void *w_nk, const float *bias, const void *residual,
                             void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype,
-                            int32_t act, cudaStream_t s) {
+                            int32_t act, bool w_ready, cudaStream_t s) {
   const DeviceInfo &di = device_info();
   char msg[160];
   auto failf = [&](const char *what) {
@@ -523,8 +609,12 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
   uint32_t *err = device_error_slot();
   if (!err) return;
 
-  const int cta_group = choose_cta_group(M);
-  const int bn = choose_bn(M, N, cta_group, di.sms);
+  const GemmTile tile = choose_gemm_tile(M, N, Kp, di.sms);
+  if (tile.one_wave) {
+    gemm_split_launch(tile, a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, s);
+    return;
+  }
+  const int cta_group = tile.cg, bn = tile.bn;
   CUtensorMap ta, tb;
   if (!encode_tmap_2d(&ta, a, dtype, static_cast<uint64_t>(Kp), static_cast<uint64_t>(M),
                       static_cast<uint64_t>(Kp) * 2, gemm::BK, gemm::BM) ||
@@ -563,9 +653,9 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
 
 using namespace mdc;
 
-MDC_API void mgpuMatmulEx16(const void *a, const void *w_nk, const float *bias, const void *residual,
-                            void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype,
-                            int32_t out_dtype, int32_t act, void *stream) {
+namespace mdc {
+void matmul16(const void *a, const void *w_nk, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
+              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, bool w_ready, void *stream) {
   if (M <= 0 || N <= 0) return;
   const DeviceInfo &di = device_info();
   if (!di.ok) return;
@@ -576,7 +666,14 @@ MDC_API void mgpuMatmulEx16(const void *a, const void *w_nk, const float *bias, 
     fail("mgpuMatmulEx16: operands must be 16-byte aligned");
     return;
   }
-  matmul16_launch("mgpuMatmulEx16", a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, as_stream(stream));
+  matmul16_launch("mgpuMatmulEx16", a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, as_stream(stream));
+}
+}  // namespace mdc
+
+MDC_API void mgpuMatmulEx16(const void *a, const void *w_nk, const float *bias, const void *residual,
+                            void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype,
+                            int32_t out_dtype, int32_t act, void *stream) {
+  matmul16(a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, false, stream);
 }
 
 MDC_API uint32_t mgpuOpsCheckDeviceStatus(void *stream) {
@@ -665,5 +762,5 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   cast_rows_padded(input, a16, M, K, Kp, MGPU_DTYPE_F16, s);
   mgpuPackWeight(weight, w16, K, N, MGPU_DTYPE_F16, stream);
   matmul16_launch("mgpuMatmulNoAlloc", a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
-                  MGPU_ACT_NONE, s);
+                  MGPU_ACT_NONE, false, s);
 }

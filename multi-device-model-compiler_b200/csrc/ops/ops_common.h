@@ -118,6 +118,11 @@ struct ProfileScope {
 // fp32 [R, C] -> 16-bit [R, Cp] with zero padding of the columns C..Cp (elementwise.cu)
 void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype, cudaStream_t s);
 
+// mgpuMatmulEx16; w_ready: the weight was complete before this call (it does not come from a kernel
+// still queued), so the kernel may read it ahead of its dependency on the previous one.
+void matmul16(const void *a, const void *w_nk, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
+              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, bool w_ready, void *stream);
+
 // Packed 16-bit [N, Kp] form of an fp32 [K, N] weight, from the constant cache when the weight
 // is a copy of a registered constant (defined in ops_init.cu).
 void *packed_weight(const float *w, int64_t K, int64_t N, int32_t dtype, void *stream, bool *cached);

@@ -194,15 +194,26 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same, called by a whole warp.
-__device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                 uint32_t idesc, uint32_t accumulate) {
+// One 64-wide k-block (four MMAs, 32 bytes apart along the swizzled rows), called by a whole warp
+// and issued by its elected lane; only the first MMA may start a new accumulation.
+__device__ __forceinline__ void umma_f16_ss_kblock(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                   uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p, e;\n"
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
+      "add.s64 a1, %1, 2;\n"
+      "add.s64 b1, %2, 2;\n"
+      "add.s64 a2, %1, 4;\n"
+      "add.s64 b2, %2, 4;\n"
+      "add.s64 a3, %1, 6;\n"
+      "add.s64 b3, %2, 6;\n"
       "elect.sync _|e, 0xffffffff;\n"
       "setp.ne.b32 p, %4, 0;\n"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n"
       "}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
@@ -358,6 +369,15 @@ __device__ __forceinline__ void tma_load_2d_cg2(void *smem_dst, const CUtensorMa
       "r"(y)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_cg2(void *smem_dst, const CUtensorMap *map,
+                                                uint32_t bar_cluster_addr, int32_t x, int32_t y, int32_t z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x),
+      "r"(y), "r"(z)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_cg2(uint32_t *smem_slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                    smem_u32(smem_slot)),
@@ -371,15 +391,25 @@ __device__ __forceinline__ void tmem_dealloc_cg2(uint32_t taddr, uint32_t ncols)
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
 }
-// called by a whole warp, issued by its elected lane
-__device__ __forceinline__ void umma_f16_ss_cg2_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                     uint32_t idesc, uint32_t accumulate) {
+// the same k-block for a CTA pair
+__device__ __forceinline__ void umma_f16_ss_kblock_cg2(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                   uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p, e;\n"
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
+      "add.s64 a1, %1, 2;\n"
+      "add.s64 b1, %2, 2;\n"
+      "add.s64 a2, %1, 4;\n"
+      "add.s64 b2, %2, 4;\n"
+      "add.s64 a3, %1, 6;\n"
+      "add.s64 b3, %2, 6;\n"
       "elect.sync _|e, 0xffffffff;\n"
       "setp.ne.b32 p, %4, 0;\n"
       "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n"
       "}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");

@@ -132,6 +132,25 @@ def test_narrow_tiles_are_exact(m, M, N, K):
     assert np.array_equal(m.matmul16(a, w, bias=b, residual=r, out_dtype=m.F32), ref)
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (1, 16, 8), (33, 48, 64), (65, 2304, 768),     # rows around a box, one stage, whole K in the ring
+    (99, 768, 3072), (250, 768, 4096), (640, 192, 1024),  # K cut over a cluster
+    (641, 1000, 1032),                             # ragged K: one k-block per box
+    (1024, 2304, 768), (2048, 768, 3072), (100, 77, 2048)])
+def test_one_wave_tiles_are_exact(m, M, N, K):
+    # small integers: fp16 products and fp32 sums are exact in any order of summation, so a wrong
+    # tile, slice or partial sum is a hard mismatch (|sum| <= 4096 * 6 < 2^24)
+    rng = np.random.default_rng(11)
+    a = rng.integers(-3, 4, (M, K)).astype(np.float32)
+    w = rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    r = rng.integers(-8, 9, (M, N)).astype(np.float32)
+    ref = a @ w + b
+    for _ in range(2):  # again with the plan kept from the first call
+        assert np.array_equal(m.matmul16(a, w, bias=b, out_dtype=m.F32), ref)
+    assert np.array_equal(m.matmul16(a, w, bias=b, residual=r, out_dtype=m.F32, act=m.ACT_RELU), np.maximum(ref, 0) + r)
+
+
 @pytest.mark.parametrize("bn", ["192", "128"])
 def test_forced_tile_width(bn):
     # every shape of this file again with the tile width forced (read once per process)
