@@ -1,0 +1,670 @@
+// Convolution as an implicit Gemm on persistent CTAs: out[n, oc, oh, ow] = sum_k patch[pixel, k] *
+// filter[oc, k], fp16 operands, fp32 accumulation in tensor memory, fp32 NCHW at the boundary.
+//
+// One CTA per SM walks tiles of 128 output pixels x bn channels.  Loading patches, the MMAs and the
+// epilogue belong to different warps and TMEM holds two accumulators, so the three run side by side,
+// also across tiles; a CTA that does one tile and retires (conv_tcgen05.cu) has them one after the
+// other and spends most of its life in memory round trips.
+//
+// Two sources of patches:
+//   * kGather = false (16 or more input channels).  conv_prepare_kernel first rewrites the input as
+//     NHWC fp16 (padded to 8 channels) and the filter as [OC][channel block][tap][64].  A k-block is one
+//     tap of 64 channels, fetched by a single im2col TMA instruction: no thread touches a patch
+//     element, and the padding comes from the hardware's zero fill.  The rewrite reads and writes
+//     each input element once, the patch loads then read two bytes instead of four, from L2.
+//   * kGather = true (fewer channels, where an NHWC pixel is shorter than the 16 bytes TMA can
+//     address).  Three groups of four warps build alternate k-blocks from the NCHW input, one
+//     thread per pixel; where k lies in the window comes from a table in shared memory.
+// The filter stays in shared memory for the CTA's life when it fits there.
+//
+// Bound: bytes (input once, output once) for few channels, L2 -> shared memory bandwidth of the
+// patch loads (each input element once per tap) for many.
+// Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after:
+//   16 x 3 x 256 x 256 -> 64, 3 x 3                      220 ->  77 us (43 of HBM time)
+//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        77 ->  40 us
+//   26 x 352 x 37 x 46 -> 32, 3 x 3                      161 ->  81 us
+//   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            114 ->  34 us
+//   1 x 128 x 16 x 25 -> 64, 3 x 3                        34 ->  17 us
+// The gather was bound by instruction issue: run-time divisions and per-channel tests in the
+// epilogue, 2.7 us a tile of 128 x 64; with multiplicative division, whole-group stores and the
+// two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).
+#include <cuda_fp16.h>
+
+#include "conv_plan.h"
+#include "ops_common.h"
+#include "ptx_sm100.cuh"
+
+namespace mdc {
+bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
+                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
+
+namespace convp {
+constexpr int BM = 128, BK = 64;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int MAX_STAGES = 12;
+constexpr int EPI_WARPS = 8;
+constexpr int GATHER_GROUPS = 3, GATHER_WARPS = GATHER_GROUPS * 4;
+constexpr int kMaxGatherK = 1024;  // table entries
+constexpr int kMaxOC = 2048;       // bias kept in shared memory
+constexpr size_t kMaxSmem = 224 * 1024;
+// warps: 0-7 epilogue, 8 TMA, 9 MMA, then the gather warps
+constexpr int threads(bool gather) { return (EPI_WARPS + 2 + (gather ? GATHER_WARPS : 0)) * 32; }
+
+// Division of numbers below 2^31 by a launch constant: q = n * mul >> shift, mul = floor(2^shift / d) + 1
+// with 2^(shift - 31) >= d, so the excess of mul, at most d / 2^shift relative to 1 / d, never reaches
+// the next integer.  (A run-time integer division is some 40 instructions, two or three per thread and tile.)
+struct Divisor {
+  uint32_t mul, d;
+  int shift;
+  explicit Divisor(int64_t v = 1) : d(static_cast<uint32_t>(v)), shift(31) {
+    while ((int64_t(1) << (shift - 31)) < v) ++shift;
+    mul = static_cast<uint32_t>((uint64_t(1) << shift) / static_cast<uint64_t>(v) + 1);
+  }
+  __device__ __forceinline__ int div(int n) const {
+    return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> shift);
+  }
+  __device__ __forceinline__ int mod(int n, int q) const { return n - q * static_cast<int>(d); }
+};
+
+struct Params {
+  const float *x, *bias, *add;
+  float *out;
+  int IC, H, W, OC, KW, OH, OW, PHL, PWL, SH, SW, DH, DW, taps;
+  int M, P, K;          // output pixels, pixels per image, patch length (gather)
+  Divisor by_p, by_ow, by_ntiles;
+  int num_kb, last_k;   // k-blocks; live values of a gather tile's last block / of a partial channel block
+  int ncb;              // 64-channel blocks (im2col)
+  int bn, n_tiles, num_tiles, stages, resident, relu;
+  uint32_t tmem_cols;
+  uint32_t *err;
+};
+}  // namespace convp
+
+template <bool kGather, bool kAdd>
+__global__ void __launch_bounds__(convp::threads(kGather), 1)
+conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                       const convp::Params p) {
+  using namespace convp;
+  using namespace ptx;
+  extern __shared__ uint8_t smem_dyn[];
+  __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_full_bar[2], acc_empty_bar[2], filter_bar;
+  __shared__ uint32_t tmem_slot, abort_flag_s;
+  volatile uint32_t *abort_flag = &abort_flag_s;
+  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
+                                               ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b_bytes = p.bn * BK * 2;
+  const int stage_bytes = A_BYTES + (p.resident ? 0 : b_bytes);
+  uint8_t *filter_s = tiles + p.stages * stage_bytes;
+  float *bias_s = reinterpret_cast<float *>(filter_s + (p.resident ? p.num_kb * b_bytes : 0));
+  // 16-byte aligned: everything in front is a multiple of 1 KiB, the bias a multiple of 32 floats
+  int2 *table = reinterpret_cast<int2 *>(bias_s + (p.OC + 31) / 32 * 32);
+
+  if (threadIdx.x == 0) {
+    abort_flag_s = 0;
+    if (!kGather) tma_prefetch_desc(&tmap_x);
+    tma_prefetch_desc(&tmap_w);
+    const uint32_t loaders = kGather ? (p.resident ? 4u : 5u) : 1u;
+    for (int i = 0; i < p.stages; ++i) {
+      mbar_init(&full_bar[i], loaders);
+      mbar_init(&empty_bar[i], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full_bar[a], 1);
+      mbar_init(&acc_empty_bar[a], kGather ? EPI_WARPS / 2 : EPI_WARPS);
+    }
+    mbar_init(&filter_bar, 1);
+    mbar_init_fence();
+  }
+  if (warp == EPI_WARPS + 1) {
+    tmem_alloc(&tmem_slot, p.tmem_cols);
+    tmem_relinquish();
+  }
+  if (kGather) {
+    // k -> (offset from the window's origin, tap position); entries past K are marked -1
+    const int hw = p.H * p.W;
+    for (int k = threadIdx.x; k < p.num_kb * BK; k += threads(true)) {
+      const int ic = k / p.taps, r = k - ic * p.taps, kh = r / p.KW, kw = r - kh * p.KW;
+      table[k] = k < p.K ? make_int2(ic * hw + kh * p.DH * p.W + kw * p.DW, (kh * p.DH) << 16 | (kw * p.DW))
+                         : make_int2(-1, 0);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_launch_dependents();  // after this CTA holds its tensor memory (see the Gemm kernel)
+  pdl_wait();
+
+  if (warp < EPI_WARPS) {
+    // ---- epilogue: thread = pixel, registers = channels; a warp's 32 pixels are neighbours, so the ----
+    // ---- store of a channel is one line.  The two warps of a lane quarter take alternate groups of ----
+    // ---- channels, or alternate tiles where tiles are many and short (gather).                     ----
+    for (int i = threadIdx.x; i < (p.OC + 31) / 32 * 32; i += EPI_WARPS * 32)
+      bias_s[i] = p.bias && i < p.OC ? __ldg(p.bias + i) : 0.f;
+    asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+    constexpr int G = kGather ? 16 : 32;  // channels per group: as many as the registers allow
+    const int quarter = warp & 3, half = warp >> 2;
+    const int c_first = kGather ? 0 : half * G, c_step = kGather ? G : 2 * G;
+    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    int acc = kGather ? half : 0;
+    uint32_t acc_phase = 0;
+    for (int tile = blockIdx.x + (kGather ? half * gridDim.x : 0); tile < p.num_tiles; tile += (kGather ? 2 : 1) * gridDim.x) {
+      const int mt = p.by_ntiles.div(tile), n0 = p.by_ntiles.mod(tile, mt) * p.bn;
+      const int m = mt * BM + quarter * 32 + lane;
+      const bool live = m < p.M;
+      const int img = live ? p.by_p.div(m) : 0, pix = live ? p.by_p.mod(m, img) : 0;
+      const int64_t out_base = (static_cast<int64_t>(img) * p.OC + n0) * p.P + pix;
+      const int nc = min(p.bn, p.OC - n0);  // live channels of the tile
+      float extra[kAdd ? G : 1];
+      auto fetch = [&](int c0) __attribute__((always_inline)) {
+        if constexpr (kAdd) {
+          if (live) {
+            const float *src = p.add + out_base + static_cast<int64_t>(c0) * p.P;
+            if (c0 + G <= nc) {
+#pragma unroll
+              for (int j = 0; j < G; ++j, src += p.P) extra[j] = __ldg(src);
+            } else {
+#pragma unroll
+              for (int j = 0; j < G; ++j, src += p.P)
+                if (c0 + j < nc) extra[j] = __ldg(src);
+            }
+          }
+        }
+      };
+      if constexpr (kAdd) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) extra[j] = 0.f;
+      }
+      fetch(c_first);  // in flight while the accumulator is waited for
+      if (!mbar_wait_warp(&acc_full_bar[acc], acc_phase, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x52000000u);
+        break;
+      }
+      tc_fence_after();
+#pragma unroll 1
+      for (int c0 = c_first; c0 < nc; c0 += c_step) {
+        uint32_t a[G];
+        const uint32_t addr = tmem_base + acc * (p.tmem_cols / 2) + lane_base + static_cast<uint32_t>(c0);
+        if constexpr (G == 32) tmem_ld_32x32(addr, a);
+        else tmem_ld_32x16(addr, a);
+        tmem_ld_wait_regs(a);
+#pragma unroll
+        for (int j = 0; j < G; j += 4) {
+          float4 b = *reinterpret_cast<const float4 *>(bias_s + n0 + c0 + j);
+          if constexpr (kAdd) b.x += extra[j], b.y += extra[j + 1], b.z += extra[j + 2], b.w += extra[j + 3];
+          a[j] = __float_as_uint(__uint_as_float(a[j]) + b.x);
+          a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + b.y);
+          a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + b.z);
+          a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + b.w);
+        }
+        if (p.relu) {
+#pragma unroll
+          for (int j = 0; j < G; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
+        }
+        if (c0 + c_step < nc) fetch(c0 + c_step);
+        if (live) {
+          float *dst = p.out + out_base + static_cast<int64_t>(c0) * p.P;
+          if (c0 + G <= nc) {
+#pragma unroll
+            for (int j = 0; j < G; ++j, dst += p.P) *dst = __uint_as_float(a[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < G; ++j, dst += p.P)
+              if (c0 + j < nc) *dst = __uint_as_float(a[j]);
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
+      if (kGather || (acc ^= 1) == 0) acc_phase ^= 1;
+    }
+  } else if (warp == EPI_WARPS) {
+    // ---------------- TMA: filter blocks, and the patches when they are not gathered ----------------
+    if (p.resident) {
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&filter_bar, static_cast<uint32_t>(p.num_kb * b_bytes));
+        for (int kb = 0; kb < p.num_kb; ++kb) tma_load_2d(filter_s + kb * b_bytes, &tmap_w, &filter_bar, kb * BK, 0);
+      }
+      __syncwarp();
+    }
+    if (!kGather || !p.resident) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
+        const int mt = tile / p.n_tiles, n0 = (tile - mt * p.n_tiles) * p.bn;
+        const int m0 = mt * BM, img = m0 / p.P, pix = m0 - img * p.P, oh = pix / p.OW;
+        const int h0 = oh * p.SH - p.PHL, w0 = (pix - oh * p.OW) * p.SW - p.PWL;
+        int c0 = 0, kh = 0, kw = 0;  // k-blocks run over the taps of 64 channels, then the next 64
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+            atomicCAS(p.err, 0u, 0x51000000u | static_cast<uint32_t>(stage));
+            ok = false;
+            break;
+          }
+          __syncwarp();
+          if (elect_one()) {
+            uint8_t *sa = tiles + stage * stage_bytes;
+            mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>((kGather ? 0 : A_BYTES) + (p.resident ? 0 : b_bytes)));
+            if (!kGather)
+              tma_load_im2col_4d(sa, &tmap_x, &full_bar[stage], c0, w0, h0, img, static_cast<uint16_t>(kw * p.DW),
+                                 static_cast<uint16_t>(kh * p.DH));
+            if (!p.resident) tma_load_2d(sa + A_BYTES, &tmap_w, &full_bar[stage], kb * BK, n0);
+          }
+          if (++kw == p.KW) {
+            kw = 0;
+            if (++kh * p.KW == p.taps) kh = 0, c0 += BK;
+          }
+          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == EPI_WARPS + 1) {
+    // ---------------- MMA issuer (whole warp, elected lane issues) ----------------
+    const uint32_t idesc = make_idesc_f16(BM, static_cast<uint32_t>(p.bn), false, false, false);
+    const uint64_t a0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
+    const uint64_t f0 = make_smem_desc_sw128(smem_u32(filter_s), 16, 1024);
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    if (p.resident && !mbar_wait(&filter_bar, 0, abort_flag)) {
+      atomicCAS(p.err, 0u, 0x55000000u);
+      ok = false;
+    }
+    // the blocks that may be partial: the last one of a gathered patch, all taps of the last 64 channels
+    const int partial_from = p.last_k == BK ? p.num_kb : p.num_kb - (kGather ? 1 : p.taps);
+    const int partial_steps = (p.last_k + 15) / 16;
+    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
+      if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x54000000u);
+        break;
+      }
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t d = tmem_base + acc * (p.tmem_cols / 2);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+          atomicCAS(p.err, 0u, 0x53000000u | static_cast<uint32_t>(stage));
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        tc_fence_after();
+        const uint64_t ad = a0 + static_cast<uint64_t>(stage * (stage_bytes / 16));
+        const uint64_t bd = p.resident ? f0 + static_cast<uint64_t>(kb * (b_bytes / 16)) : ad + A_BYTES / 16;
+        if (kb < partial_from) {
+          umma_f16_ss_kblock(d, ad, bd, idesc, kb != 0 ? 1u : 0u);
+        } else {
+          for (int k = 0; k < partial_steps; ++k)
+            umma_f16_ss_warp(d, ad + static_cast<uint64_t>(2 * k), bd + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+        }
+        umma_commit_warp(&empty_bar[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      umma_commit_warp(&acc_full_bar[acc]);
+      if ((acc ^= 1) == 0) acc_phase ^= 1;
+    }
+  } else if constexpr (kGather) {
+    // ---------------- gather: one thread per pixel, groups of four warps take alternate k-blocks ----------------
+    const int group = (warp - EPI_WARPS - 2) >> 2;
+    const int row = ((warp - EPI_WARPS - 2) & 3) * 32 + lane;
+    const uint32_t row_off = static_cast<uint32_t>(row) * 128u, swz = static_cast<uint32_t>(row & 7);
+    const int max_dh = (p.taps / p.KW - 1) * p.DH, max_dw = (p.KW - 1) * p.DW;
+    int turn = 0, stage = 0;  // turn: which group's k-block this is
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
+      const int m = p.by_ntiles.div(tile) * BM + row;
+      const bool live = m < p.M;
+      int h0 = 0, w0 = 0;
+      const float *origin = p.x;  // of the window; may lie outside the image, then only live taps are read
+      if (live) {
+        const int img = p.by_p.div(m), pix = p.by_p.mod(m, img), oh = p.by_ow.div(pix);
+        h0 = oh * p.SH - p.PHL;
+        w0 = p.by_ow.mod(pix, oh) * p.SW - p.PWL;
+        origin += static_cast<int64_t>(img) * p.IC * p.H * p.W + h0 * p.W + w0;
+      }
+      // windows of the whole warp inside the image: no bounds tests
+      const bool interior = __all_sync(0xffffffffu, live && h0 >= 0 && w0 >= 0 && h0 + max_dh < p.H && w0 + max_dw < p.W);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (turn == group) {
+          const int pieces = kb == p.num_kb - 1 ? (p.last_k + 31) / 32 : 2;  // of 32 values
+          uint8_t *sa = tiles + stage * stage_bytes + row_off;
+          for (int h = 0; h < pieces; ++h) {
+            const int4 *t4 = reinterpret_cast<const int4 *>(table + kb * BK + h * 32);
+            float v[32];
+            if (interior) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int4 t = t4[j];
+                v[2 * j] = t.x >= 0 ? __ldg(origin + t.x) : 0.f;
+                v[2 * j + 1] = t.z >= 0 ? __ldg(origin + t.z) : 0.f;
+              }
+            } else {
+              auto tap = [&](int off, int pos) __attribute__((always_inline)) {
+                const bool in = live && off >= 0 && static_cast<unsigned>(h0 + (pos >> 16)) < static_cast<unsigned>(p.H) &&
+                                static_cast<unsigned>(w0 + (pos & 0xffff)) < static_cast<unsigned>(p.W);
+                return in ? __ldg(origin + off) : 0.f;
+              };
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int4 t = t4[j];
+                v[2 * j] = tap(t.x, t.y);
+                v[2 * j + 1] = tap(t.z, t.w);
+              }
+            }
+            // the loads are in flight; only now does the stage have to be free
+            if (h == 0 && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
+              atomicCAS(p.err, 0u, 0x50000000u | static_cast<uint32_t>(stage));
+              ok = false;
+              break;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const __half2 h0_ = __floats2half2_rn(v[c * 8 + 0], v[c * 8 + 1]), h1_ = __floats2half2_rn(v[c * 8 + 2], v[c * 8 + 3]);
+              const __half2 h2_ = __floats2half2_rn(v[c * 8 + 4], v[c * 8 + 5]), h3_ = __floats2half2_rn(v[c * 8 + 6], v[c * 8 + 7]);
+              uint4 q;
+              q.x = *reinterpret_cast<const uint32_t *>(&h0_);
+              q.y = *reinterpret_cast<const uint32_t *>(&h1_);
+              q.z = *reinterpret_cast<const uint32_t *>(&h2_);
+              q.w = *reinterpret_cast<const uint32_t *>(&h3_);
+              // 128-byte swizzle: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
+              *reinterpret_cast<uint4 *>(sa + ((static_cast<uint32_t>(h * 4 + c) ^ swz) << 4)) = q;
+            }
+          }
+          if (!ok) break;
+          fence_proxy_async_smem();  // the tensor core reads these rows through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full_bar[stage]);
+        }
+        if (++turn == GATHER_GROUPS) turn = 0;
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+  }
+
+  if (*abort_flag) {
+    // a wait gave up: give copies still in flight time to land before the CTA retires
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == EPI_WARPS + 1) tmem_dealloc(tmem_base, p.tmem_cols);
+}
+
+// Operands of the persistent kernels in one launch: blocks below `input_blocks` rewrite the input
+// (NCHW fp32 -> NHWC fp16, channels zero-padded to Cp) in tiles of 64 pixels x 64 channels of one
+// image, the others one (output channel, block of 64 input channels) of the filter each:
+// OIHW fp32 -> [OC][channel block][tap][64] fp16, or for the gather kernel its own order padded to Kp.
+// Bound by bytes: 6 per input element.
+struct ConvPrepareParams {
+  const float *x, *w;
+  __half *x16, *w16;
+  int IC, HW, Cp, pixel_tiles, channel_tiles, taps, ncb;
+  int K, Kp;        // gather order (ncb == 0): patch length and row pitch
+  int vec_ok;       // the image planes can be read in 16-byte vectors
+  int sampled, H, W, SH, SW, PHL, PWL;  // sampled: pixel (h, w) of the copy is (h*SH - PHL, w*SW - PWL) of the input
+  convp::Divisor by_w;
+  int64_t input_blocks;
+};
+__global__ void __launch_bounds__(256) conv_prepare_kernel(const ConvPrepareParams p) {
+  __shared__ float tile[64][65];
+  pdl_launch_dependents();
+  pdl_wait();
+  int64_t b = blockIdx.x;
+  if (b < p.input_blocks) {
+    const int ct = static_cast<int>(b % p.channel_tiles);
+    b /= p.channel_tiles;
+    const int pt = static_cast<int>(b % p.pixel_tiles);
+    const int64_t n = b / p.pixel_tiles;
+    const int p0 = pt * 64, c0 = ct * 64;
+    const int plane = p.sampled ? p.H * p.W : p.HW;
+    const float *src = p.x + (n * p.IC + c0) * static_cast<int64_t>(plane);
+    int at[4];  // where this thread's four pixels lie in a plane; -1: outside
+    const int px = (threadIdx.x & 15) * 4, cr = threadIdx.x >> 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int q = p0 + px + e;
+      at[e] = q < p.HW ? q : -1;
+      if (p.sampled && q < p.HW) {
+        const int oh = p.by_w.div(q), h = oh * p.SH - p.PHL, w = p.by_w.mod(q, oh) * p.SW - p.PWL;
+        at[e] = static_cast<unsigned>(h) < static_cast<unsigned>(p.H) && static_cast<unsigned>(w) < static_cast<unsigned>(p.W)
+                    ? h * p.W + w : -1;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = cr + 16 * i;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c0 + c < p.IC) {
+        const float *s = src + static_cast<int64_t>(c) * plane;
+        if (p.vec_ok && at[3] >= 0) {
+          v = __ldcs(reinterpret_cast<const float4 *>(s + at[0]));
+        } else {
+          if (at[0] >= 0) v.x = s[at[0]];
+          if (at[1] >= 0) v.y = s[at[1]];
+          if (at[2] >= 0) v.z = s[at[2]];
+          if (at[3] >= 0) v.w = s[at[3]];
+        }
+      }
+      tile[c][px] = v.x, tile[c][px + 1] = v.y, tile[c][px + 2] = v.z, tile[c][px + 3] = v.w;
+    }
+    __syncthreads();
+    const int chunk = (threadIdx.x & 7) * 8, pr = threadIdx.x >> 3;
+    if (c0 + chunk < p.Cp) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int q = pr + 32 * i;
+        if (p0 + q < p.HW) {
+          __align__(16) __half h[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(tile[chunk + e][q]);
+          *reinterpret_cast<uint4 *>(p.x16 + (n * p.HW + p0 + q) * static_cast<int64_t>(p.Cp) + c0 + chunk) =
+              *reinterpret_cast<const uint4 *>(h);
+        }
+      }
+    }
+    return;
+  }
+  b -= p.input_blocks;
+  if (p.ncb == 0) {
+    const float *w = p.w + b * p.K;
+    __half *out = p.w16 + b * p.Kp;
+    for (int i = threadIdx.x; i < p.Kp; i += 256) out[i] = __float2half_rn(i < p.K ? __ldg(w + i) : 0.f);
+    return;
+  }
+  // the block's 64 x taps weights are contiguous in w: strided reads, served by L1 after the first touch
+  const int cb = static_cast<int>(b % p.ncb);
+  const int64_t oc = b / p.ncb;
+  const float *w = p.w + (oc * p.IC + cb * 64) * static_cast<int64_t>(p.taps);
+  __half *out = p.w16 + (oc * p.ncb + cb) * static_cast<int64_t>(p.taps) * 64;
+  for (int i = threadIdx.x; i < p.taps * 64; i += 256) {
+    const int ic = i & 63, tap = i >> 6;
+    out[i] = __float2half_rn(cb * 64 + ic < p.IC ? __ldg(w + ic * p.taps + tap) : 0.f);
+  }
+}
+
+namespace {
+using EncodeIm2col = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const int *, const int *, cuuint32_t, cuuint32_t,
+                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeIm2col encode_im2col() {
+  static const EncodeIm2col fn = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      (void)cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<EncodeIm2col>(f);
+  }();
+  return fn;
+}
+
+// Tile width, by the cycles of the busiest CTA: rounds x the slowest of a tile's three engines.
+// Loads: about 64 bytes per cycle and SM out of L2 (a gathered k-block about 400 cycles with three
+// groups at work); MMAs: 2 cycles per column and k-block, at least what reading A takes; epilogue:
+// about 24 bytes per cycle and SM of HBM.  E.g. 6272 pixels x 256 channels: 147 tiles of 96 columns
+// in one round (224 units of load) beat 98 of 128 in one (256) and 49 of 256 (384).
+int choose_conv_bn(int64_t m_tiles, int64_t OC, int num_kb, bool gather, bool add, int sms) {
+  int best = 32;
+  double best_cost = 1e300;
+  for (int bn = 256; bn >= 32; bn -= 32) {
+    if (bn > 32 && bn >= OC + 32) continue;
+    const int64_t n_tiles = (OC + bn - 1) / bn;
+    const int64_t rounds = (m_tiles * n_tiles + sms - 1) / sms;
+    const double load = num_kb * ((gather ? 400.0 : 256.0) + bn * 2.0);
+    const double mma = num_kb * (bn < 64 ? 160.0 : bn < 96 ? 192.0 : 2.0 * bn);
+    const double epi = bn * (add ? 1024.0 : 512.0) / 24.0;
+    double tile = load > mma ? load : mma;
+    if (epi > tile) tile = epi;
+    const double cost = static_cast<double>(rounds) * tile + epi;
+    if (cost < best_cost * 0.97) best_cost = cost, best = bn;
+  }
+  return best;
+}
+
+template <bool kGather, bool kAdd>
+void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp::Params &p, size_t smem, int sms,
+                       cudaStream_t s) {
+  auto kern = conv_persistent_kernel<kGather, kAdd>;
+  static bool set_on[64] = {false};  // the attribute is per device
+  const int dev = device_info().device;
+  bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
+  if (!set) {
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(convp::kMaxSmem)),
+                    "cudaFuncSetAttribute(conv)"))
+      return;
+    set = true;
+  }
+  // the fewest CTAs that finish in the same number of rounds
+  const int rounds = (p.num_tiles + sms - 1) / sms, grid = (p.num_tiles + rounds - 1) / rounds;
+  {
+    ProfileScope prof(kCatGemm, s);
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convp::threads(kGather)), smem, s, 1, tx, tw, p),
+               "launch conv_persistent_kernel");
+  }
+  launched("conv_persistent_kernel");
+}
+}  // namespace
+
+bool conv_persistent(const ConvShape &call, cudaStream_t s) {
+  using namespace convp;
+  // A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels
+  // only, and the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56,
+  // stride 2: 108 us with the whole input rewritten, 65 sampled.)
+  ConvShape c = call;
+  const bool sampled = c.IC >= 16 && c.KH * c.KW == 1 && (c.SH > 1 || c.SW > 1);
+  if (sampled) c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
+  const DeviceInfo &di = device_info();
+  const int64_t taps = c.KH * c.KW, K = c.IC * taps, M = c.N * c.OH * c.OW;
+  if (c.OC > kMaxOC || taps > 4096 || M * c.OC > (int64_t(1) << 40)) return false;
+  // 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks
+  const bool gather = c.IC < 16;
+  const int64_t span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
+  // im2col: first and last window origin relative to the first and last column / row of the image
+  const int64_t up_w = (c.OW - 1) * c.SW - c.PWL - (c.W - 1), up_h = (c.OH - 1) * c.SH - c.PHL - (c.H - 1);
+  if (gather) {
+    if (K > kMaxGatherK || span_h > 32767 || span_w > 32767) return false;
+  } else {
+    // limits of the im2col tensor map: strides, corners and tap offsets
+    if (c.SW > 8 || c.SH > 8 || c.PWL > 127 || c.PHL > 127 || up_w < -128 || up_w > 127 || up_h < -128 || up_h > 127 ||
+        span_w > 255 || span_h > 255 || !encode_im2col())
+      return false;
+  }
+  const int64_t Cp = (c.IC + 7) / 8 * 8, ncb = (c.IC + 63) / 64;
+  const int64_t num_kb = gather ? (K + BK - 1) / BK : ncb * taps;
+  const int64_t Kp = gather ? (K + 7) / 8 * 8 : num_kb * BK;
+  const int64_t m_tiles = (M + BM - 1) / BM;
+  if (num_kb > (1 << 20)) return false;
+
+  Params p;
+  p.x = c.x, p.bias = c.bias, p.add = c.add, p.out = c.out;
+  p.IC = int(c.IC), p.H = int(c.H), p.W = int(c.W), p.OC = int(c.OC), p.KW = int(c.KW), p.OH = int(c.OH), p.OW = int(c.OW);
+  p.PHL = int(c.PHL), p.PWL = int(c.PWL), p.SH = int(c.SH), p.SW = int(c.SW), p.DH = int(c.DH), p.DW = int(c.DW);
+  p.taps = int(taps), p.M = int(M), p.P = int(c.OH * c.OW), p.K = int(K), p.num_kb = int(num_kb), p.ncb = int(ncb);
+  p.last_k = int(gather ? K - (num_kb - 1) * BK : c.IC - (ncb - 1) * BK);
+  p.relu = c.relu ? 1 : 0;
+  p.bn = choose_conv_bn(m_tiles, c.OC, p.num_kb, gather, c.add != nullptr, di.sms);
+  p.n_tiles = int((c.OC + p.bn - 1) / p.bn);
+  if (m_tiles * p.n_tiles > INT32_MAX) return false;
+  p.num_tiles = int(m_tiles * p.n_tiles);
+  p.by_p = Divisor(p.P), p.by_ow = Divisor(p.OW), p.by_ntiles = Divisor(p.n_tiles);
+  p.tmem_cols = 32;
+  while (p.tmem_cols < 2u * p.bn) p.tmem_cols *= 2;
+  // the filter stays when it is one tile wide, there is a second tile to use it, and it leaves the ring room
+  const int64_t filter_bytes = num_kb * p.bn * BK * 2;
+  p.resident = p.n_tiles == 1 && p.num_tiles > di.sms && filter_bytes <= 100 * 1024;
+  const int64_t stage_bytes = A_BYTES + (p.resident ? 0 : p.bn * BK * 2);
+  const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128 + (gather ? num_kb * BK * 8 : 0);
+  int64_t stages = (static_cast<int64_t>(kMaxSmem) - 4096 - fixed) / stage_bytes;
+  // gathered patches are read nine-fold through L1: leave it most of the memory
+  const int64_t cap = gather ? 4 : MAX_STAGES;
+  p.stages = int(stages < cap ? stages : cap);
+  if (p.stages < 2) return false;
+  const size_t smem = static_cast<size_t>(fixed + p.stages * stage_bytes);
+  p.err = device_error_slot();
+  if (!p.err) return true;
+
+  // one block for both operands; without memory for it the caller's other kernel takes over
+  const uint64_t w_bytes = (static_cast<uint64_t>(c.OC) * Kp * 2 + 255) / 256 * 256;
+  const uint64_t x_bytes = gather ? 0 : static_cast<uint64_t>(c.N) * c.H * c.W * Cp * 2;
+  const int before = mgpuGetLastError();
+  char *ws = static_cast<char *>(mgpuMemAllocAsync(w_bytes + x_bytes, s));
+  if (!ws) {
+    if (before == 0 && x_bytes) {
+      mgpuClearLastError();
+      return false;
+    }
+    return true;
+  }
+  ConvPrepareParams q = {};
+  q.x = c.x, q.w = c.w, q.w16 = reinterpret_cast<__half *>(ws), q.x16 = reinterpret_cast<__half *>(ws + w_bytes);
+  q.IC = int(c.IC), q.HW = int(c.H * c.W), q.Cp = int(Cp), q.taps = int(taps), q.ncb = gather ? 0 : int(ncb);
+  q.K = int(K), q.Kp = int(Kp);
+  q.sampled = sampled ? 1 : 0;
+  q.H = int(call.H), q.W = int(call.W), q.SH = int(call.SH), q.SW = int(call.SW), q.PHL = int(call.PHL), q.PWL = int(call.PWL);
+  q.by_w = Divisor(c.W);
+  q.pixel_tiles = int((c.H * c.W + 63) / 64), q.channel_tiles = int(ncb);
+  q.vec_ok = !sampled && (c.H * c.W) % 4 == 0 && (reinterpret_cast<uintptr_t>(c.x) & 15u) == 0;
+  q.input_blocks = gather ? 0 : c.N * q.pixel_tiles * q.channel_tiles;
+  const int64_t blocks = q.input_blocks + c.OC * (gather ? 1 : ncb);
+
+  CUtensorMap tx = {}, tw;
+  bool ok = blocks <= INT32_MAX &&
+            encode_tmap_2d(&tw, ws, MGPU_DTYPE_F16, static_cast<uint64_t>(Kp), static_cast<uint64_t>(c.OC),
+                           static_cast<uint64_t>(Kp) * 2, BK, static_cast<uint32_t>(p.bn));
+  if (ok && !gather) {
+    const cuuint64_t gdim[4] = {cuuint64_t(Cp), cuuint64_t(c.W), cuuint64_t(c.H), cuuint64_t(c.N)};
+    const cuuint64_t gstr[3] = {cuuint64_t(Cp) * 2, cuuint64_t(Cp) * 2 * c.W, cuuint64_t(Cp) * 2 * c.W * c.H};
+    const int lower[2] = {-int(c.PWL), -int(c.PHL)}, upper[2] = {int(up_w), int(up_h)};
+    const cuuint32_t estr[4] = {1, cuuint32_t(c.SW), cuuint32_t(c.SH), 1};
+    ok = encode_im2col()(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, ws + w_bytes, gdim, gstr, lower, upper, BK, BM, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
+  if (ok) {
+    {
+      ProfileScope prof(kCatElementwise, s);
+      check_cuda(launch_chain(conv_prepare_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, 1, q),
+                 "launch conv_prepare_kernel");
+    }
+    launched("conv_prepare_kernel");
+    if (gather && p.add) launch_persistent<true, true>(tx, tw, p, smem, di.sms, s);
+    else if (gather) launch_persistent<true, false>(tx, tw, p, smem, di.sms, s);
+    else if (p.add) launch_persistent<false, true>(tx, tw, p, smem, di.sms, s);
+    else launch_persistent<false, false>(tx, tw, p, smem, di.sms, s);
+  }
+  mgpuMemFreeAsync(ws, s);
+  return ok;
+}
+
+}  // namespace mdc

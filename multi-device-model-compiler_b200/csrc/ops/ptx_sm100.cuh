@@ -134,6 +134,19 @@ __device__ __forceinline__ void tma_load_3d(void *smem_dst, const CUtensorMap *m
       "r"(y), "r"(z)
       : "memory");
 }
+// 128-pixel x 64-channel patch tile of an NHWC tensor through an im2col map: (c, w, h, n) is the
+// window origin of the first pixel (inside the map's pixel box), (off_w, off_h) the filter tap; the
+// hardware walks the following pixels of the box, image after image, and fills what lies outside the
+// image (the padding) with zeros.
+__device__ __forceinline__ void tma_load_im2col_4d(void *smem_dst, const CUtensorMap *map, uint64_t *bar, int32_t c,
+                                                   int32_t w, int32_t h, int32_t n, uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h),
+      "r"(n), "h"(off_w), "h"(off_h)
+      : "memory");
+}
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, const void *smem_src,
                                              int32_t x, int32_t y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -214,6 +227,19 @@ __device__ __forceinline__ void umma_f16_ss_kblock(uint32_t d_tmem, uint64_t a_d
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n"
+      "}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// One K = 16 step, called by a whole warp and issued by its elected lane.
+__device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");

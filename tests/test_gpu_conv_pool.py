@@ -122,6 +122,53 @@ def test_conv_exact_on_small_integers(m):
     assert np.array_equal(got, ref)
 
 
+@pytest.mark.parametrize("shape", [
+    # N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
+    (1, 16, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),      # one partial tile, im2col's fewest channels
+    (1, 15, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),      # the gather kernel's most channels
+    (5, 24, 9, 5, 33, 3, 2, (2, 1), (0, 1, 2, 0), (1, 2), True, True),        # asymmetric in every respect
+    (3, 20, 11, 13, 40, 5, 3, (1, 3), (2, 0, 1, 2), (2, 1), True, False),     # channels padded to 24
+    (2, 96, 10, 6, 65, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),      # a half-full block of 64 channels
+    (300, 72, 8, 8, 48, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, False),     # tiles of two images, one round and a bit
+    (60, 64, 20, 21, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True),     # filter kept, several tiles per CTA
+    (40, 128, 20, 20, 96, 3, 3, (2, 2), (1, 1, 1, 1), (1, 1), False, False),  # filter streamed
+    (1, 256, 4, 4, 300, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False),     # many k-blocks, few pixels
+    (90, 3, 17, 19, 40, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),     # one k-block, 32 of 64 values
+    (40, 5, 31, 30, 24, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), True, False),     # four k-blocks, gather groups out of step
+    (2, 14, 12, 12, 260, 7, 7, (1, 1), (3, 3, 3, 3), (1, 1), False, False),   # gathered, filter streamed, two channel tiles
+    (3, 33, 11, 14, 20, 1, 1, (2, 3), (1, 0, 0, 2), (1, 1), True, False),     # strided 1 x 1, padded: sampled copy
+    (70, 64, 20, 20, 32, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), False, True),
+    (2, 16, 30, 30, 8, 2, 2, (9, 1), (0, 0, 0, 0), (1, 1), False, False),     # stride outside the im2col map: direct kernel
+])
+def test_conv_persistent_edges(m, shape):
+    """Small integers (see test_conv_exact_on_small_integers): equal bit for bit."""
+    N, IC, H, W, OC, KH, KW, stride, pad, dil, has_add, relu = shape
+    rng = np.random.default_rng(IC * 1000 + OC)
+    x = rng.integers(-4, 5, size=(N, IC, H, W)).astype(np.float32)
+    w = rng.integers(-3, 4, size=(OC, IC, KH, KW)).astype(np.float32)
+    b = rng.integers(-8, 9, size=OC).astype(np.float32)
+    OH = (H + pad[0] + pad[2] - (KH - 1) * dil[0] - 1) // stride[0] + 1
+    OW = (W + pad[1] + pad[3] - (KW - 1) * dil[1] - 1) // stride[1] + 1
+    add = rng.integers(-8, 9, size=(N, OC, OH, OW)).astype(np.float32) if has_add else None
+    kw = dict(post_add=add, stride=stride, pad=pad, dilation=dil, relu=relu)
+    assert np.array_equal(m.conv2d(x, w, b, **kw), oracle.conv2d(x, w, b, **kw))
+
+
+def test_conv_output_smaller_than_the_geometry(m):
+    """The caller may ask for fewer output rows and columns than the padded input would give."""
+    rng = np.random.default_rng(3)
+    N, IC, H, W, OC, OH, OW = 4, 32, 12, 11, 24, 7, 8
+    x = rng.integers(-4, 5, size=(N, IC, H, W)).astype(np.float32)
+    w = rng.integers(-3, 4, size=(OC, IC, 3, 3)).astype(np.float32)
+    dx, dw, out = m.to_device(x), m.to_device(w), m.DeviceBuffer(N * OC * OH * OW * 4)
+    m.ops().mgpuConv2d(dx.ptr, dw.ptr, None, out.ptr, None, N, IC, H, W, OC, 3, 3, OH, OW, 1, 1, 1, 1, 1, 1, 1, 1,
+                       False, False, None)
+    m.check("conv")
+    got = m.to_host(out, (N, OC, OH, OW), np.float32)
+    ref = oracle.conv2d(x, w, None, pad=(1, 1, 1, 1))[:, :, :OH, :OW]
+    assert np.array_equal(got, ref)
+
+
 def test_conv_reference_test_layer_full_size(m):
     """test/End2End/GPU/conv.mlir: 16x3x256x256 -> 16x64x256x256, 3x3, padding 1."""
     rng = np.random.default_rng(11)
