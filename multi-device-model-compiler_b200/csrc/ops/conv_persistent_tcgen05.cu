@@ -31,6 +31,7 @@
 #include <cuda_fp16.h>
 
 #include "conv_plan.h"
+#include "fast_div.h"
 #include "ops_common.h"
 #include "ptx_sm100.cuh"
 
@@ -49,22 +50,6 @@ constexpr int kMaxOC = 2048;       // bias kept in shared memory
 constexpr size_t kMaxSmem = 224 * 1024;
 // warps: 0-7 epilogue, 8 TMA, 9 MMA, then the gather warps
 constexpr int threads(bool gather) { return (EPI_WARPS + 2 + (gather ? GATHER_WARPS : 0)) * 32; }
-
-// Division of numbers below 2^31 by a launch constant: q = n * mul >> shift, mul = floor(2^shift / d) + 1
-// with 2^(shift - 31) >= d, so the excess of mul, at most d / 2^shift relative to 1 / d, never reaches
-// the next integer.  (A run-time integer division is some 40 instructions, two or three per thread and tile.)
-struct Divisor {
-  uint32_t mul, d;
-  int shift;
-  explicit Divisor(int64_t v = 1) : d(static_cast<uint32_t>(v)), shift(31) {
-    while ((int64_t(1) << (shift - 31)) < v) ++shift;
-    mul = static_cast<uint32_t>((uint64_t(1) << shift) / static_cast<uint64_t>(v) + 1);
-  }
-  __device__ __forceinline__ int div(int n) const {
-    return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> shift);
-  }
-  __device__ __forceinline__ int mod(int n, int q) const { return n - q * static_cast<int>(d); }
-};
 
 struct Params {
   const float *x, *bias, *add;
@@ -410,7 +395,7 @@ struct ConvPrepareParams {
   int K, Kp;        // gather order (ncb == 0): patch length and row pitch
   int vec_ok;       // the image planes can be read in 16-byte vectors
   int sampled, H, W, SH, SW, PHL, PWL;  // sampled: pixel (h, w) of the copy is (h*SH - PHL, w*SW - PWL) of the input
-  convp::Divisor by_w;
+  Divisor by_w;
   int64_t input_blocks;
 };
 __global__ void __launch_bounds__(256) conv_prepare_kernel(const ConvPrepareParams p) {
@@ -626,7 +611,7 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
     }
     return true;
   }
-  ConvPrepareParams q = {};
+  ConvPrepareParams q;
   q.x = c.x, q.w = c.w, q.w16 = reinterpret_cast<__half *>(ws), q.x16 = reinterpret_cast<__half *>(ws + w_bytes);
   q.IC = int(c.IC), q.HW = int(c.H * c.W), q.Cp = int(Cp), q.taps = int(taps), q.ncb = gather ? 0 : int(ncb);
   q.K = int(K), q.Kp = int(Kp);
