@@ -120,10 +120,10 @@ static float *dup_f32(const float *src, int64_t n, void *stream) {
   return dst;
 }
 
-static void *pack(const float *w, int64_t K, int64_t N, int32_t dtype, void *stream) {
+static void *pack(const float *w, int64_t K, int64_t N, OperandList *list, void *stream) {
   if (!w) return nullptr;
   void *dst = mgpuMemAllocAsync(static_cast<uint64_t>(N) * K * 2, stream);
-  if (dst) mgpuPackWeight(w, dst, K, N, dtype, stream);
+  if (dst) list->pack(w, dst, K, N);
   return dst;
 }
 
@@ -155,14 +155,14 @@ static void destroy_stack(EncoderStack *st, void *stream) {
   delete st;
 }
 
-// x_f32 != nullptr: input is fp32 and is cast first; else `cur` already holds 16-bit input.
+// x_f32 != nullptr: input is fp32 and is cast first; else the workspace already holds it in 16 bits.
 // y_f32 receives the fp32 result.
 static void run_stack(EncoderStack *st, const float *x_f32, const int32_t *seq_lens, float *y_f32,
                       int64_t B, int64_t S, bool w_ready, void *stream) {
   const int64_t T = B * S, d = st->d, F = st->F;
   const int32_t dt = st->dtype;
   Workspace &w = st->ws;
-  mgpuCast(x_f32, MGPU_DTYPE_F32, w.cur, dt, T * d, stream);
+  if (x_f32) mgpuCast(x_f32, MGPU_DTYPE_F32, w.cur, dt, T * d, stream);
   const int64_t L = st->layers_n;
   for (int64_t l = 0; l < L; ++l) {
     const LayerWeights &lw = st->layers[l];
@@ -327,10 +327,12 @@ MDC_API void mgpuEncoderStackSetLayer(void *stack, int64_t layer, const float *q
   drop_graphs(st);  // captured runs hold the old weights' addresses
   free_layer(lw, stream);
   const int64_t d = st->d, F = st->F;
-  lw.wqkv = pack(qkv_weight, d, 3 * d, st->dtype, stream);
-  lw.wo = pack(proj_weight, d, d, st->dtype, stream);
-  lw.w1 = pack(ffn1_weight, d, F, st->dtype, stream);
-  lw.w2 = pack(ffn2_weight, F, d, st->dtype, stream);
+  OperandList list;
+  lw.wqkv = pack(qkv_weight, d, 3 * d, &list, stream);
+  lw.wo = pack(proj_weight, d, d, &list, stream);
+  lw.w1 = pack(ffn1_weight, d, F, &list, stream);
+  lw.w2 = pack(ffn2_weight, F, d, &list, stream);
+  list.launch(st->dtype, stream);
   lw.bqkv = dup_f32(qkv_bias, 3 * d, stream);
   lw.bo = dup_f32(proj_bias, d, stream);
   lw.b1 = dup_f32(ffn1_bias, F, stream);
@@ -523,10 +525,11 @@ MDC_API void mgpuTransformerEncoderLayer(const float *input, const float *qkv_we
   LayerWeights &lw = st.layers[0];
   const int64_t d = d_model, F = feed_forward_dim;
   bool cached[4] = {false, false, false, false};
-  lw.wqkv = packed_weight(qkv_weight, d, 3 * d, dtype, stream, &cached[0]);
-  lw.wo = packed_weight(proj_weight, d, d, dtype, stream, &cached[1]);
-  lw.w1 = packed_weight(ffn1_weight, d, F, dtype, stream, &cached[2]);
-  lw.w2 = packed_weight(ffn2_weight, F, d, dtype, stream, &cached[3]);
+  OperandList list;
+  lw.wqkv = packed_weight(qkv_weight, d, 3 * d, dtype, stream, &cached[0], &list);
+  lw.wo = packed_weight(proj_weight, d, d, dtype, stream, &cached[1], &list);
+  lw.w1 = packed_weight(ffn1_weight, d, F, dtype, stream, &cached[2], &list);
+  lw.w2 = packed_weight(ffn2_weight, F, d, dtype, stream, &cached[3], &list);
   lw.bqkv = const_cast<float *>(qkv_bias);
   lw.bo = const_cast<float *>(proj_bias);
   lw.b1 = const_cast<float *>(ffn1_bias);
@@ -536,7 +539,11 @@ MDC_API void mgpuTransformerEncoderLayer(const float *input, const float *qkv_we
   lw.ln2_g = const_cast<float *>(ln2_gamma);
   lw.ln2_b = const_cast<float *>(ln2_beta);
   if (lw.wqkv && lw.wo && lw.w1 && lw.w2) {
-    if (ensure_ws(&st, batch * seq_len, stream)) run_stack(&st, input, seq_lens, output, batch, seq_len, false, stream);
+    if (ensure_ws(&st, batch * seq_len, stream)) {
+      list.cast(input, st.ws.cur, batch * seq_len, d, d);
+      list.launch(dtype, stream);
+      run_stack(&st, nullptr, seq_lens, output, batch, seq_len, false, stream);
+    }
   } else {
     fail("mgpuTransformerEncoderLayer: out of device memory for the packed weights");
   }

@@ -724,9 +724,6 @@ constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 // host-side cache of the array's device address, per device ordinal
 static unsigned char *g_noalloc_ptr[kMaxDevices] = {nullptr};
-
-void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype,
-                      cudaStream_t s);
 }  // namespace mdc
 
 MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *output, int64_t M,
@@ -759,8 +756,10 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   void *a16 = base;
   void *w16 = base + a_bytes;
   cudaStream_t s = as_stream(stream);
-  cast_rows_padded(input, a16, M, K, Kp, MGPU_DTYPE_F16, s);
-  mgpuPackWeight(weight, w16, K, N, MGPU_DTYPE_F16, stream);
+  OperandList list;
+  list.pack(weight, w16, K, N);
+  list.cast(input, a16, M, K, Kp);
+  list.launch(MGPU_DTYPE_F16, stream);
   matmul16_launch("mgpuMatmulNoAlloc", a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
                   MGPU_ACT_NONE, false, s);
 }

@@ -3,16 +3,11 @@
 #include "ops_common.h"
 
 namespace mdc {
-void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype,
-                      cudaStream_t s);
-}
-
-namespace mdc {
 // The packed ([N, Kp], 16-bit) form of the fp32 weight w [K, N] on `stream`.  *cached = true:
 // the buffer belongs to the constant cache (w is a copy of a registered constant; packed at
 // the first use, reused afterwards) and must not be freed; false: a pool block the caller
-// frees after its last use.  nullptr when out of memory.
-void *packed_weight(const float *w, int64_t K, int64_t N, int32_t dtype, void *stream, bool *cached) {
+// frees after its last use, and the packing is left to `list`.  nullptr when out of memory.
+void *packed_weight(const float *w, int64_t K, int64_t N, int32_t dtype, void *stream, bool *cached, OperandList *list) {
   *cached = false;
   const int64_t Kp = (K + 7) / 8 * 8;
   const uint64_t bytes = static_cast<uint64_t>(N) * Kp * 2;
@@ -31,7 +26,7 @@ void *packed_weight(const float *w, int64_t K, int64_t N, int32_t dtype, void *s
     }
   }
   void *buf = mgpuMemAllocAsync(bytes, stream);
-  if (buf) mgpuPackWeight(w, buf, K, N, dtype, stream);
+  if (buf) list->pack(w, buf, K, N);
   return buf;
 }
 }  // namespace mdc
@@ -71,9 +66,12 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   const int64_t Kp = (K + 7) / 8 * 8;
   void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
   bool w_cached = false;
-  void *w16 = packed_weight(weight, K, N, MGPU_DTYPE_F16, stream, &w_cached);
+  OperandList list;
+  void *w16 = packed_weight(weight, K, N, MGPU_DTYPE_F16, stream, &w_cached, &list);
   if (a16 && w16) {
-    cast_rows_padded(input, a16, M, K, Kp, MGPU_DTYPE_F16, as_stream(stream));
+    list.launch(MGPU_DTYPE_F16, stream);  // on its own: callers count on a cached weight saving a launch
+    list.cast(input, a16, M, K, Kp);
+    list.launch(MGPU_DTYPE_F16, stream);
     mgpuMatmulEx16(a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
                    MGPU_ACT_NONE, stream);
   }

@@ -79,12 +79,14 @@ static void matmul_ex(T *input, T *weight, T *bias, T *output, T *residual, int6
   // operands in the Gemm's form: A 16-bit [M, Kp], W 16-bit [N, Kp], bias fp32, residual 16-bit
   float *w32 = is16 ? to_f32(weight, K * N, s) : reinterpret_cast<float *>(weight);
   bool w_cached = false;
-  void *w16 = w32 ? packed_weight(w32, K, N, MGPU_DTYPE_F16, s, &w_cached) : nullptr;
+  OperandList list;
+  void *w16 = w32 ? packed_weight(w32, K, N, MGPU_DTYPE_F16, s, &w_cached, &list) : nullptr;
   void *a16 = input;
   if (!is16) {
     a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, s);
-    if (a16) cast_rows_padded(reinterpret_cast<const float *>(input), a16, M, K, Kp, MGPU_DTYPE_F16, stream);
+    if (a16) list.cast(reinterpret_cast<const float *>(input), a16, M, K, Kp);
   }
+  list.launch(MGPU_DTYPE_F16, s);
   float *b32 = nullptr;
   if (hasBias) b32 = is16 ? to_f32(bias, N, s) : reinterpret_cast<float *>(bias);
   void *r16 = nullptr;
