@@ -195,7 +195,7 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 // job is filled by the next and the launch gaps go: a 1024-wide
 // context layer with 2048 tokens (five operands) 130 -> 118 us a call; 35 x 3086 x 3392 Gemm, whose rows
 // need padding, 50 -> 38 us (with the one-wave Gemm).
-constexpr int64_t kCastItems = kEwBlock * 32, kPadItems = kEwBlock * 4;
+constexpr int64_t kCastItems = kEwBlock * 16, kPadItems = kEwBlock * 4;
 struct OperandJobs {
   OperandList::Job j[OperandList::kMax];
   int n;
@@ -217,14 +217,14 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
     const int64_t n = job.rows * job.pitch, base = b * (job.vec_ok ? kCastItems : kPadItems);
     if (job.vec_ok) {
       const float4 *s4 = reinterpret_cast<const float4 *>(job.src);
-      float4 v[8];
+      float4 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 2; ++u) {
         const int64_t i = base + (u * kEwBlock + threadIdx.x) * 8;
         if (i + 7 < n) v[2 * u] = __ldcs(s4 + i / 4), v[2 * u + 1] = __ldcs(s4 + i / 4 + 1);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 2; ++u) {
         const int64_t i = base + (u * kEwBlock + threadIdx.x) * 8;
         if (i + 7 < n) {
           Vec8<T16> o;
@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
   }
   const float *w = job.src;
   const int64_t K = job.rows, N = job.cols, Kp = job.pitch;
-  const int64_t tk = b / job.tiles_n, k0 = tk * 64, n0 = (b - tk * job.tiles_n) * 64;
+  const uint32_t b32 = static_cast<uint32_t>(b), tk = b32 / static_cast<uint32_t>(job.tiles_n);
+  const int64_t k0 = static_cast<int64_t>(tk) * 64, n0 = static_cast<int64_t>(b32 - tk * job.tiles_n) * 64;
   {
     const int c4 = (threadIdx.x & 15) * 4, r0 = threadIdx.x >> 4;  // 16 threads per k-row, 16 rows per pass
 #pragma unroll
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (k < K) {
         if (job.vec_ok && n + 3 < N) {
-          v = __ldcs(reinterpret_cast<const float4 *>(w + k * N + n));
+          v = __ldg(reinterpret_cast<const float4 *>(w + k * N + n));
         } else {
           if (n < N) v.x = w[k * N + n];
           if (n + 1 < N) v.y = w[k * N + n + 1];
