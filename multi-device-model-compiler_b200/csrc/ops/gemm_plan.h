@@ -13,7 +13,6 @@ struct GemmTile {
   int cg = 2;             // CTAs per tile (2 = tcgen05 CTA pair)
   int box_m = 128;        // rows of A per CTA
   int bn = 256;           // output columns per tile
-  int splits = 1;         // CTAs (pairs) of a cluster that share a tile's K range
   int depth = 1;          // 64-wide k-blocks per ring stage
   int stages = 4;
 };

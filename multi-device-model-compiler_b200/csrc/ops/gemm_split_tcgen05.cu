@@ -1,16 +1,15 @@
 // Tensor-core Gemm for problems that fit the chip in one wave: the same operation as
 // gemm_tcgen05.cu (out = act(A . W^T + bias) + residual, 16-bit operands, fp32 accumulation in
-// tensor memory), one output tile per CTA (or CTA pair), and the K range of a tile optionally cut
-// over a cluster of CTAs.
+// tensor memory), one output tile per CTA (or CTA pair).
 //
 // What bounds these shapes is latency, not the tensor pipe: a Gemm of a few hundred rows has too
 // few 256 x 256 tiles to use the chip, and every CTA works through its whole K range alone, at
 // 0.2 us per 64-wide k-block whatever the tile (MMA issue and barrier waits).  So
 //   * the tile is chosen small enough that about every SM has one (choose_gemm_tile), down to
 //     16 output columns;
-//   * `splits` CTAs (or pairs) of a cluster each take a slice of K; the fp32 partial tiles are
-//     exchanged through distributed shared memory, each CTA receiving the columns it finishes,
-//     and added in slice order, so the result does not depend on timing;
+//   * K is never cut: an element is one sum over K in order, as in gemm_tcgen05.cu, whatever the
+//     tile.  The tile follows from M, so anything else would let a row's bits depend on the batch
+//     that it is in (a sequence run alone, in a host chunk or on another GPU gives the same bits);
 //   * a ring stage holds `depth` k-blocks, fetched by one TMA instruction per operand and handed
 //     over by one barrier, and the ring is as deep as shared memory allows: a short K range is
 //     in flight as a whole and costs one memory latency;
@@ -42,7 +41,7 @@ struct SplitParams {
   void *out;
   int vec_ok;   // rows of out / residual can be accessed in 32-byte vectors, bias in 16-byte ones
   int n_tiles;  // column tiles
-  int bn, box_m, splits, depth, stages;
+  int bn, box_m, depth, stages;
   int tmem_cols;
   int k_in_x;   // operand maps are (k, row) instead of (64 k, row, k-block)
   int w_ready;  // W may be read before the dependency wait
@@ -64,20 +63,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int splits = p.splits, cluster = CG * splits;
-  const int rank = cluster > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  const int half = CG == 2 ? (rank & 1) : 0;  // which 128 rows of a pair's 256
-  const int split = rank / CG;                // which slice of K
+  const int half = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;  // which 128 rows of a pair's 256
   const bool leader = half == 0;
-  const int tile = static_cast<int>(blockIdx.x) / cluster;
+  const int tile = static_cast<int>(blockIdx.x) / CG;
   const int m_tile = tile / p.n_tiles, n_tile = tile - m_tile * p.n_tiles;
   const int row0 = (m_tile * CG + half) * p.box_m, col0 = n_tile * p.bn;
-  const int kb0 = p.num_kb * split / splits, kb1 = p.num_kb * (split + 1) / splits;
   const int depth = p.depth, stages = p.stages;
   const int a_kb_bytes = p.box_m * BK * 2, b_rows = p.bn / CG, b_kb_bytes = b_rows * BK * 2;
   const int a_bytes = a_kb_bytes * depth;
   const int stage_bytes = a_bytes + b_kb_bytes * depth;
-  const int steps = (kb1 - kb0 + depth - 1) / depth;
+  const int steps = (p.num_kb + depth - 1) / depth;
 
   if (threadIdx.x == 0) {
     abort_flag_s = 0;
@@ -106,21 +101,20 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t tmem_base = tmem_slot;
   pdl_launch_dependents();  // after this CTA holds its tensor memory (see gemm_tcgen05.cu)
 
-  // a stage is always filled whole: k-blocks past this CTA's slice are fetched (or read as zeros
-  // past K) and not used
+  // a stage is always filled whole: k-blocks past the last one read as zeros and are not used
   auto kx = [&](int kb) { return p.k_in_x ? kb * BK : 0; };
   auto kz = [&](int kb) { return p.k_in_x ? 0 : kb; };
   auto load_w = [&](int s, int kb) __attribute__((always_inline)) {
     uint8_t *sb = tiles + s * stage_bytes + a_bytes;
     if constexpr (CG == 2)
-      tma_load_3d_cg2(sb, &tmap_b, mapa_u32(smem_u32(&full_bar[s]), static_cast<uint32_t>(rank & ~1)), kx(kb), col0 + half * b_rows, kz(kb));
+      tma_load_3d_cg2(sb, &tmap_b, mapa_u32(smem_u32(&full_bar[s]), 0), kx(kb), col0 + half * b_rows, kz(kb));
     else
       tma_load_3d(sb, &tmap_b, &full_bar[s], kx(kb), col0, kz(kb));
   };
   auto load_a = [&](int s, int kb) __attribute__((always_inline)) {
     uint8_t *sa = tiles + s * stage_bytes;
     if constexpr (CG == 2)
-      tma_load_3d_cg2(sa, &tmap_a, mapa_u32(smem_u32(&full_bar[s]), static_cast<uint32_t>(rank & ~1)), kx(kb), row0, kz(kb));
+      tma_load_3d_cg2(sa, &tmap_a, mapa_u32(smem_u32(&full_bar[s]), 0), kx(kb), row0, kz(kb));
     else
       tma_load_3d(sa, &tmap_a, &full_bar[s], kx(kb), row0, kz(kb));
   };
@@ -134,7 +128,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (elect_one()) {
       for (int i = 0; i < early; ++i) {
         expect(i);
-        load_w(i, kb0 + i * depth);
+        load_w(i, i * depth);
       }
     }
     __syncwarp();
@@ -154,9 +148,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (elect_one()) {
         if (i >= early) {
           expect(stage);
-          load_w(stage, kb0 + i * depth);
+          load_w(stage, i * depth);
         }
-        load_a(stage, kb0 + i * depth);
+        load_a(stage, i * depth);
       }
       if (++stage == stages) { stage = 0; phase ^= 1; }
     }
@@ -179,19 +173,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         tc_fence_after();
         uint64_t a_desc = desc0 + static_cast<uint64_t>((stage * stage_bytes) >> 4);
         uint64_t b_desc = a_desc + static_cast<uint64_t>(a_bytes >> 4);
-        const int n = min(depth, kb1 - kb0 - i * depth);
+        const int n = min(depth, p.num_kb - i * depth);
         for (int d = 0; d < n; ++d) {
           if constexpr (CG == 2) umma_f16_ss_kblock_cg2(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
           else umma_f16_ss_kblock(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
           a_desc += static_cast<uint64_t>(a_kb_bytes >> 4);
           b_desc += static_cast<uint64_t>(b_kb_bytes >> 4);
         }
-        if constexpr (CG == 2) umma_commit_cg2_warp(&empty_bar[stage], static_cast<uint16_t>(3u << rank));
+        if constexpr (CG == 2) umma_commit_cg2_warp(&empty_bar[stage], 3);
         else umma_commit_warp(&empty_bar[stage]);
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (ok) {
-        if constexpr (CG == 2) umma_commit_cg2_warp(&acc_bar, static_cast<uint16_t>(3u << rank));
+        if constexpr (CG == 2) umma_commit_cg2_warp(&acc_bar, 3);
         else umma_commit_warp(&acc_bar);
       }
     }
@@ -202,11 +196,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int ew = warp - 2;
   const int quarter = warp & 3;        // tensor-memory lanes this warp may access
   const int half_sel = ew >> 2;        // which half of the columns
-  const int own_cols = p.bn / splits;  // columns this CTA finishes
-  // in pieces of 16 (32 bytes of a 16-bit row, so that vector accesses stay aligned): the first half
-  // of the warps takes the first half of the pieces, rounded up
-  const int c_mid = (own_cols / 16 + 1) / 2 * 16;
-  const int c_begin = half_sel ? c_mid : 0, c_end = half_sel ? own_cols : c_mid;
+  // columns in pieces of 16 (32 bytes of a 16-bit row, so that vector accesses stay aligned): the first
+  // half of the warps takes the first half of the pieces, rounded up
+  const int c_mid = (p.bn / 16 + 1) / 2 * 16;
+  const int c_begin = half_sel ? c_mid : 0, c_end = half_sel ? p.bn : c_mid;
   const int rows_in_tile = quarter * 32 + lane;
   const bool live_warp = warp >= 2 && quarter * 32 < p.box_m;  // box_m is a multiple of 32
   bool ok = true;
@@ -218,28 +211,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tc_fence_after();
   }
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-  // partial tiles received: [slot][column / 4][128 rows] of float4
-  const float4 *part = reinterpret_cast<const float4 *>(tiles);
-  if (splits > 1) {
-    // every CTA of the cluster has finished reading its ring before anyone writes into it
-    cluster_sync_all();
-    if (live_warp && ok) {
-      for (int d = 1; d < splits; ++d) {
-        const int to = split + d < splits ? split + d : split + d - splits;
-        const int slot = split < to ? split : split - 1;
-        const uint32_t dst = mapa_u32(smem_u32(tiles), static_cast<uint32_t>(to * CG + half));
-        for (int c = c_begin; c < c_end; c += 8) {
-          uint32_t r[8];
-          tmem_ld_32x8(t_lane + static_cast<uint32_t>(to * own_cols + c), r);
-          tmem_ld_wait_regs(r);
-          const uint32_t at = dst + static_cast<uint32_t>(((slot * (own_cols / 4) + c / 4) * 128 + rows_in_tile) * 16);
-          st_cluster_v4(at, r[0], r[1], r[2], r[3]);
-          st_cluster_v4(at + 128 * 16, r[4], r[5], r[6], r[7]);
-        }
-      }
-    }
-    cluster_sync_all();
-  }
   if (live_warp && ok) {
     TOut *out = static_cast<TOut *>(p.out);
     const T16 *res = static_cast<const T16 *>(p.residual);
@@ -248,10 +219,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll 1
     for (int c = c_begin; c < c_end; c += 16) {
       constexpr int NC = 16;
-      const int gcol = col0 + split * own_cols + c;
+      const int gcol = col0 + c;
       if (gcol >= p.N) break;  // uniform across the warp
       uint32_t acc[NC];
-      tmem_ld_32x16(t_lane + static_cast<uint32_t>(split * own_cols + c), acc);
+      tmem_ld_32x16(t_lane + static_cast<uint32_t>(c), acc);
       const size_t off = static_cast<size_t>(row) * p.N + gcol;
       const bool whole = p.vec_ok && gcol + NC <= p.N;
       float b[NC], rv[NC];
@@ -286,29 +257,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       float v[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]);
-      if (splits > 1) {
-        // sum in slice order: slices before this CTA's, its own, the later ones
-        float s[NC];
-#pragma unroll
-        for (int j = 0; j < NC; ++j) s[j] = split == 0 ? v[j] : 0.f;
-        for (int t = 0; t < splits; ++t) {
-          if (t == split) {
-            if (t > 0) {
-#pragma unroll
-              for (int j = 0; j < NC; ++j) s[j] += v[j];
-            }
-          } else {
-            const float4 *q = part + ((t < split ? t : t - 1) * (own_cols / 4) + c / 4) * 128 + rows_in_tile;
-#pragma unroll
-            for (int j = 0; j < NC; j += 4) {
-              const float4 f = q[(j / 4) * 128];
-              s[j] += f.x, s[j + 1] += f.y, s[j + 2] += f.z, s[j + 3] += f.w;
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < NC; ++j) v[j] = s[j];
-      }
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] += b[j];
       act_fast_n<ACT, NC>(v);
@@ -358,7 +306,7 @@ static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const 
   }
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gsplit::THREADS), smem, s, CG * p.splits, ta, tb, p),
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gsplit::THREADS), smem, s, CG, ta, tb, p),
                "launch gemm split");
   }
   launched("gemm_split_kernel");
@@ -417,20 +365,19 @@ void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const
   auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
   p.vec_ok = N % 16 == 0 && al(out, 32) && (!residual || al(residual, 32)) && (!bias || al(bias, 16));
   p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
-  p.bn = t.bn, p.box_m = t.box_m, p.splits = t.splits, p.stages = t.stages;
+  p.bn = t.bn, p.box_m = t.box_m, p.stages = t.stages;
   p.depth = p.k_in_x ? 1 : t.depth;
   p.tmem_cols = 32;
   while (p.tmem_cols < t.bn) p.tmem_cols *= 2;
   p.w_ready = w_ready ? 1 : 0;
   p.err = err;
   const int64_t m_tiles = (M + static_cast<int64_t>(t.box_m) * t.cg - 1) / (static_cast<int64_t>(t.box_m) * t.cg);
-  const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg * t.splits);
+  const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg);
   const size_t stage = static_cast<size_t>(p.depth) * (t.box_m + t.bn / t.cg) * gsplit::BK * 2;
-  const size_t partial = static_cast<size_t>(t.splits - 1) * 128 * (t.bn / t.splits) * 4;
   // an MMA reads 128 rows of A whatever the box holds: past the last box that must still be this
   // CTA's memory
   const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * gsplit::BK * 2 : 0);
-  const size_t smem = (ring > partial ? ring : partial) + 1024;
+  const size_t smem = ring + 1024;
   if (dtype == MGPU_DTYPE_F16) {
     if (out_dtype == MGPU_DTYPE_F16) launch_split_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
     else if (out_dtype == MGPU_DTYPE_F32) launch_split_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);

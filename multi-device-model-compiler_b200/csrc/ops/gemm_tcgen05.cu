@@ -487,22 +487,21 @@ static int choose_bn(int64_t M, int64_t N, int cta_group, int sms) {
 
 // Time of a one-wave tile in microseconds, fitted to 1700 measured (shape, tile) pairs (M 32 - 4096,
 // N 768 - 4096, K 768 - 4096, weights from HBM, chained launches; 14 % rms).  Terms: launch and drain;
-// MMA issue; operand bytes through the SM's load path; one barrier hand-over per ring stage; exchange
-// of partial tiles; epilogue columns; pairing; CTAs to place.  At most one CTA per SM: the tile it
+// MMA issue; operand bytes through the SM's load path; one barrier hand-over per ring stage; epilogue
+// columns; pairing; CTAs to place.  At most one CTA per SM: the tile it
 // picks is then within 4 % (geometric mean; at most 11 %) of the fastest of all measured ones over 13
 // shapes from 16 x 1024 x 2048 to 2048 x 1024 x 4096.  (With two CTAs per SM allowed, each on half the
 // shared memory, it was 27 % off: see the ring below.)
 static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, int sms) {
   const int64_t m_tiles = (M + t.box_m * t.cg - 1) / (t.box_m * t.cg), n_tiles = (N + t.bn - 1) / t.bn;
-  const int64_t ctas = m_tiles * n_tiles * t.cg * t.splits;
+  const int64_t ctas = m_tiles * n_tiles * t.cg;
   if (ctas > sms) return 1e30f;
-  const int kbs = (num_kb + t.splits - 1) / t.splits, steps = (kbs + t.depth - 1) / t.depth;
-  const int rows = M < t.box_m ? static_cast<int>(M) : t.box_m, own = t.bn / t.splits;
-  const float mma = kbs * (t.bn < 100 ? 200.f : 2.f * t.bn) / 1900.f;
-  const float bytes = kbs * static_cast<float>(rows + t.bn / t.cg) * 128.f / 1e5f;
-  float us = 2.2f + 0.33f * mma + 0.305f * bytes + 0.194f * steps + 0.0125f * own +
+  const int steps = (num_kb + t.depth - 1) / t.depth;
+  const int rows = M < t.box_m ? static_cast<int>(M) : t.box_m;
+  const float mma = num_kb * (t.bn < 100 ? 200.f : 2.f * t.bn) / 1900.f;
+  const float bytes = num_kb * static_cast<float>(rows + t.bn / t.cg) * 128.f / 1e5f;
+  float us = 2.2f + 0.33f * mma + 0.305f * bytes + 0.194f * steps + 0.0125f * t.bn +
              0.65f * static_cast<float>(ctas) / static_cast<float>(sms);
-  if (t.splits > 1) us += 0.8f + 5.7f * (t.splits - 1) * own * t.box_m * 4.f / 1e5f;
   if (t.cg == 2) us += 1.2f;
   return us;
 }
@@ -517,29 +516,22 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool k_whole, 
       if (box_m > 32 && box_m >= 2 * M) continue;
       for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
         if (cg == 2 && bn < 64) continue;
-        for (int splits : {1, 2, 3, 4, 6, 8}) {
-          // A slice of less than 4 k-blocks costs more to exchange than to compute; below K = 1024
-          // nothing is split, so there a row's result does not depend on the batch it is in.
-          if (splits > 1 && (num_kb < 16 || splits * 4 > num_kb || splits * cg > 8)) continue;
-          if (bn % (16 * splits) != 0) continue;
-          const int kbs = (num_kb + splits - 1) / splits;
-          for (int depth : {4, 2, 1}) {
-            if (depth > 1 && (!k_whole || depth > kbs)) continue;
-            const int steps = (kbs + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
-            // all of an SM's shared memory: the ring has to cover the latency of operands that come out
-            // of L2 at 60 - 100 bytes per cycle.  Half of it, so that the next kernel's CTA fits beside
-            // this one, loses more than that overlap wins: 2048 x 1024 x 4096 29.1 -> 19.6 us,
-            // 1000 x 1024 x 4096 18.6 -> 15.2, 99 x 768 x 3072 7.9 -> 7.2; a 12-layer pass over 99 tokens,
-            // where every kernel is of this kind, 468 -> 432 us.
-            int stages = (220 * 1024 - (128 - box_m) * 128) / stage;
-            if (stages > steps) stages = steps;
-            if (stages > 16) stages = 16;
-            if (stages < 1 || (stages < 2 && steps > 1)) continue;
-            GemmTile t;
-            t.one_wave = true, t.cg = cg, t.box_m = box_m, t.bn = bn, t.splits = splits, t.depth = depth, t.stages = stages;
-            const float us = one_wave_cost(t, M, N, num_kb, sms);
-            if (us < best_us) best_us = us, best = t;
-          }
+        for (int depth : {4, 2, 1}) {
+          if (depth > 1 && (!k_whole || depth > num_kb)) continue;
+          const int steps = (num_kb + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
+          // all of an SM's shared memory: the ring has to cover the latency of operands that come out
+          // of L2 at 60 - 100 bytes per cycle.  Half of it, so that the next kernel's CTA fits beside
+          // this one, loses more than that overlap wins: 2048 x 1024 x 4096 29.1 -> 19.6 us,
+          // 1000 x 1024 x 4096 18.6 -> 15.2, 99 x 768 x 3072 7.9 -> 7.2; a 12-layer pass over 99 tokens,
+          // where every kernel is of this kind, 468 -> 432 us.
+          int stages = (220 * 1024 - (128 - box_m) * 128) / stage;
+          if (stages > steps) stages = steps;
+          if (stages > 16) stages = 16;
+          if (stages < 1 || (stages < 2 && steps > 1)) continue;
+          GemmTile t;
+          t.one_wave = true, t.cg = cg, t.box_m = box_m, t.bn = bn, t.depth = depth, t.stages = stages;
+          const float us = one_wave_cost(t, M, N, num_kb, sms);
+          if (us < best_us) best_us = us, best = t;
         }
       }
     }
@@ -551,7 +543,7 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   if (const char *e = getenv("MDC_GEMM_TILE")) {
     GemmTile t;
     int ow = 0;
-    if (sscanf(e, "%d,%d,%d,%d,%d,%d,%d", &ow, &t.cg, &t.box_m, &t.bn, &t.splits, &t.depth, &t.stages) == 7) {
+    if (sscanf(e, "%d,%d,%d,%d,%d,%d", &ow, &t.cg, &t.box_m, &t.bn, &t.depth, &t.stages) == 6) {
       t.one_wave = ow != 0;
       return t;
     }

@@ -321,3 +321,25 @@ def test_graph_replay_follows_inputs_lengths_and_weights(m):
     ops.mgpuEncoderStackRun(st.h, dx.ptr, dl.ptr, dy2.ptr, B, S, stream)
     assert np.array_equal(m.to_host(dy2, (B, S, d), np.float32, stream), got)
     st.close()
+
+
+@pytest.mark.parametrize("dtype_name,norm_first", [("bf16", True), ("f16", False)])
+def test_small_batches_reproduce_the_same_bits(m, dtype_name, norm_first):
+    # the same property where the Gemm's tile changes with the number of tokens (2048 down to 48) and
+    # K = 3072 is long: an element is one sum over K in one order, whatever the tile, so a sequence
+    # gives the same bits in a full batch, alone, and in the chunks of the host pipeline
+    rng = np.random.default_rng(51)
+    L, B, S, d, F, H = 2, 16, 128, 768, 3072, 12
+    layers = [make_layer(rng, d, F, bias_std=0.02) for _ in range(L)]
+    x = rng.standard_normal((B, S, d)).astype(np.float32)
+    st = m.EncoderStack(layers, H, norm_first=norm_first, causal=norm_first, dtype=m.BF16 if dtype_name == "bf16" else m.F16)
+    y = st.run(x, None)
+    for lo, hi in ((0, 1), (3, 5), (8, 12), (5, 13)):
+        assert np.array_equal(st.run(x[lo:hi], None), y[lo:hi]), (lo, hi)
+    y2 = np.empty_like(x)
+    st.run_host(x, y2, None, chunks=4)
+    assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+    assert np.array_equal(y2, y)
+    if norm_first:  # causal: the first rows of a sequence are those of a shorter one (48 tokens)
+        assert np.array_equal(st.run(np.ascontiguousarray(x[2:3, :48]), None), y[2:3, :48])
+    st.close()

@@ -162,3 +162,15 @@ def test_forced_tile_width(bn):
                         "-k", "small_integers or ragged or epilogues or narrow"],
                        env=env, capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("N,K", [(768, 3072), (1000, 1000), (1024, 4096)])
+def test_a_row_does_not_depend_on_the_number_of_rows(m, N, K):
+    # from 1 row (narrow one-wave tiles) to 6000 (persistent CTA pairs): the same sum over K in the
+    # same order, so equal bit for bit
+    rng = np.random.default_rng(13)
+    a = rng.standard_normal((6000, K)).astype(np.float32)
+    w = (0.02 * rng.standard_normal((K, N))).astype(np.float32)
+    whole = m.matmul16(a, w, out_dtype=m.F32)
+    for M in (1, 16, 99, 128, 250, 512, 1000, 1024, 2048, 4096):
+        assert np.array_equal(m.matmul16(a[:M], w, out_dtype=m.F32), whole[:M]), M
