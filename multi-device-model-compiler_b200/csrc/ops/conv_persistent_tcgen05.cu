@@ -224,12 +224,11 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         const int h0 = oh * p.SH - p.PHL, w0 = (pix - oh * p.OW) * p.SW - p.PWL;
         int c0 = 0, kh = 0, kw = 0;  // k-blocks run over the taps of 64 channels, then the next 64
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+          if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
             atomicCAS(p.err, 0u, 0x51000000u | static_cast<uint32_t>(stage));
             ok = false;
             break;
           }
-          __syncwarp();
           if (elect_one()) {
             uint8_t *sa = tiles + stage * stage_bytes;
             mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>((kGather ? 0 : A_BYTES) + (p.resident ? 0 : b_bytes)));
@@ -254,7 +253,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool ok = true;
-    if (p.resident && !mbar_wait(&filter_bar, 0, abort_flag)) {
+    if (p.resident && !mbar_wait_all(&filter_bar, 0, abort_flag)) {
       atomicCAS(p.err, 0u, 0x55000000u);
       ok = false;
     }
@@ -262,20 +261,18 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     const int partial_from = p.last_k == BK ? p.num_kb : p.num_kb - (kGather ? 1 : p.taps);
     const int partial_steps = (p.last_k + 15) / 16;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
-      if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
+      if (!mbar_wait_all(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
         atomicCAS(p.err, 0u, 0x54000000u);
         break;
       }
-      __syncwarp();
       tc_fence_after();
       const uint32_t d = tmem_base + acc * (p.tmem_cols / 2);
       for (int kb = 0; kb < p.num_kb; ++kb) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x53000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
-        __syncwarp();
         tc_fence_after();
         const uint64_t ad = a0 + static_cast<uint64_t>(stage * (stage_bytes / 16));
         const uint64_t bd = p.resident ? f0 + static_cast<uint64_t>(kb * (b_bytes / 16)) : ad + A_BYTES / 16;

@@ -140,11 +140,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     int stage = 0;
     uint32_t phase = 0;
     for (int i = 0; i < steps; ++i) {
-      if (i >= early && !mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+      if (i >= early && !mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
         atomicCAS(p.err, 0u, 0x81000000u | static_cast<uint32_t>(stage));
         break;
       }
-      __syncwarp();
       if (elect_one()) {
         if (i >= early) {
           expect(stage);
@@ -164,12 +163,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t phase = 0;
       bool ok = true;
       for (int i = 0; i < steps; ++i) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x82000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
-        __syncwarp();
         tc_fence_after();
         uint64_t a_desc = desc0 + static_cast<uint64_t>((stage * stage_bytes) >> 4);
         uint64_t b_desc = a_desc + static_cast<uint64_t>(a_bytes >> 4);

@@ -144,12 +144,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int tile = worker; ok && tile < num_tiles; tile += num_workers) {
       const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
           atomicCAS(p.err, 0u, 0x10000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
-        __syncwarp();
         if (elect_one()) {
           uint8_t *sa = tiles + stage * STAGE_BYTES;
           uint8_t *sb = sa + A_BYTES;
@@ -180,20 +179,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = worker; ok && tile < num_tiles; tile += num_workers) {
-        if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
+        if (!mbar_wait_all(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
           atomicCAS(p.err, 0u, 0x30000000u | static_cast<uint32_t>(acc));
           break;
         }
-        __syncwarp();
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+          if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
             atomicCAS(p.err, 0u, 0x20000000u | static_cast<uint32_t>(stage));
             ok = false;
             break;
           }
-          __syncwarp();
           tc_fence_after();
           // (descriptors hold addresses in units of 16 bytes)
           const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));

@@ -110,6 +110,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity,
   return ok != 0;
 }
 
+// The wait of a loop that a whole converged warp runs.  Every lane polls for itself and sees the
+// barrier with its own acquire; the vote gives all of them one verdict.  (A lane's own verdict mixes
+// the barrier, the abort flag and the timer, so when a wait gives up the lanes need not agree, and a
+// loop that some of them leave strands the others at its next warp-wide instruction.)
+__device__ __forceinline__ bool mbar_wait_all(uint64_t *bar, uint32_t parity,
+                                              volatile uint32_t *abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // ---------------- TMA (cp.async.bulk.tensor), plain tile copies only ----------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");

@@ -1,0 +1,45 @@
+"""Source check of the device-side waits (no GPU): a bounded wait that gives up must not leave a warp
+divided, which no run on a GPU may provoke."""
+import os
+import re
+
+import pytest
+
+OPS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "multi-device-model-compiler_b200", "csrc", "ops")
+
+
+def _code(name):
+    with open(os.path.join(OPS, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def _enclosing(code, position):
+    """What opens each block that holds `position`, outermost first."""
+    stack, start = [], 0
+    for i, c in enumerate(code[:position]):
+        if c == "{":
+            stack.append(code[start:i].strip())
+        elif c == "}":
+            stack.pop()
+        if c in "{};":
+            start = i + 1
+    return stack
+
+
+@pytest.mark.parametrize("name", ["gemm_tcgen05.cu", "gemm_split_tcgen05.cu", "conv_persistent_tcgen05.cu", "conv_tcgen05.cu"])
+def test_warps_wait_with_one_verdict(name):
+    """mbar_wait is one thread's wait: its verdict mixes the barrier, the abort flag and the timer, and
+    lanes that each ask for themselves can get different ones.  It may stand only where a single
+    lane runs; whole warps use mbar_wait_all or mbar_wait_warp."""
+    code = _code(name)
+    for call in re.finditer(r"\bmbar_wait\(", code):
+        assert any("lane == 0" in opener for opener in _enclosing(code, call.start())), code[call.start() - 80:call.end() + 60]
+
+
+def test_the_warp_waits_are_uniform():
+    code = _code("ptx_sm100.cuh")
+
+    def body(function):
+        return code[code.index("bool " + function):].split("\n}\n")[0]
+    assert "__all_sync(0xffffffffu, mbar_wait(" in body("mbar_wait_all")
+    assert "__shfl_sync(0xffffffffu, ok, 0)" in body("mbar_wait_warp")
