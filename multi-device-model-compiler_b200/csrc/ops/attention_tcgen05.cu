@@ -317,7 +317,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
       // m_run is the reference point of the exponent (in score units), l_run the row sum
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < it.n_kv && ok; ++j, ++t) {
-        if (!mbar_wait(&s_full, t & 1, abort_flag)) {
+        if (!mbar_wait_all(&s_full, t & 1, abort_flag)) {
           atomicCAS(p.err, 0u, 0x61000000u | (t & 0xffff));
           ok = false;
           break;
@@ -418,7 +418,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
       ++qn;
     }
     if (ok && pending) {
-      if (!mbar_wait(&all_done, 0, abort_flag)) {
+      if (!mbar_wait_all(&all_done, 0, abort_flag)) {
         atomicCAS(p.err, 0u, 0x62000000u);
       } else {
         tc_fence_after();
@@ -638,7 +638,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < it.n_kv && ok; ++j, ++t) {
         const uint32_t ph = t & 1;
-        if (!mbar_wait(&bar_s_full, ph, abort_flag)) {
+        if (!mbar_wait_all(&bar_s_full, ph, abort_flag)) {
           atomicCAS(p.err, 0u, 0x61000000u | (t & 0xffff));
           ok = false;
           break;
@@ -742,7 +742,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         tc_fence_before();
         mbar_arrive(&bar_p_ready);
         // O_t = P.V of this tile: fold it into the running output, then hand the columns back
-        if (!mbar_wait(&bar_o_full, ph, abort_flag)) {
+        if (!mbar_wait_all(&bar_o_full, ph, abort_flag)) {
           atomicCAS(p.err, 0u, 0x62000000u | (t & 0xffff));
           ok = false;
           break;

@@ -26,7 +26,7 @@ def _enclosing(code, position):
     return stack
 
 
-@pytest.mark.parametrize("name", ["gemm_tcgen05.cu", "gemm_split_tcgen05.cu", "conv_persistent_tcgen05.cu", "conv_tcgen05.cu"])
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(OPS) if f.endswith(".cu")))
 def test_warps_wait_with_one_verdict(name):
     """mbar_wait is one thread's wait: its verdict mixes the barrier, the abort flag and the timer, and
     lanes that each ask for themselves can get different ones.  It may stand only where a single
