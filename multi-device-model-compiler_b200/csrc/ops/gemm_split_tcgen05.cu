@@ -257,7 +257,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]);
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] += b[j];
-      act_fast_n<ACT, NC>(v);
+      if (p.vec_ok) {
+        act_fast_n<ACT, NC>(v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) v[j] = act_apply_t<ACT>(v[j]);
+      }
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] += rv[j];
       if (row_ok) {

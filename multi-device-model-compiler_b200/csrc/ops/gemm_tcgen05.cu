@@ -317,8 +317,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int j = 0; j < 32; ++j) {
             v[j] = __uint_as_float(raw[j]);
             if (p.bias && gcol + j < p.N) v[j] += __ldg(p.bias + gcol + j);
+            v[j] = act_apply_t<ACT>(v[j]);
           }
-          act_fast_n<ACT, 32>(v);
           if (row_ok) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
