@@ -12,7 +12,22 @@
 
 namespace mdc {
 
-// The epilogue's thread owns one row: it moves 32 bytes (one DRAM sector) per access.
+// How the rows of a call can be accessed, decided on the host.
+struct RowAccess {
+  bool vec;   // rows of out and residual are multiples of 16 bytes, their columns of 8
+  bool fast;  // and the bias can be read in 16-byte vectors
+  bool wide;  // and rows can be moved 32 bytes, a whole DRAM sector, per access and thread
+};
+inline RowAccess row_access(int64_t N, const void *out, size_t out_elem, const void *residual, const void *bias) {
+  auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
+  RowAccess r;
+  r.vec = N % 8 == 0 && al(out, 16) && al(residual, 16);
+  r.fast = r.vec && al(bias, 16);
+  r.wide = r.fast && N * static_cast<int64_t>(out_elem) % 32 == 0 && al(out, 32) &&
+           (!residual || (N % 16 == 0 && al(residual, 32)));
+  return r;
+}
+
 __device__ __forceinline__ void ld_global_32B(const void *src, uint32_t *r) {
   asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -22,6 +37,9 @@ __device__ __forceinline__ void st_global_32B(void *dst, const uint32_t *r) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]),
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
+}
+__device__ __forceinline__ void ld_global_16B(const void *src, uint32_t *r) {
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(src));
 }
 template <typename T16>
 __device__ __forceinline__ uint32_t pack_pair(float a, float b);
@@ -35,19 +53,31 @@ __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
-// 16 values of a row as TOut; dst is 32-byte aligned
+// 16 values of a row as TOut; dst is 32-byte aligned.  `second`: the last eight lie inside the row (a
+// 16-bit row that is a multiple of 32 bytes always holds both).
 template <typename TOut>
-__device__ __forceinline__ void store_out16(TOut *dst, const float *v) {
+__device__ __forceinline__ void store_out16(TOut *dst, const float *v, bool second) {
   uint32_t q[16];
   if constexpr (sizeof(TOut) == 4) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) q[i] = __float_as_uint(v[i]);
     st_global_32B(dst, q);
-    st_global_32B(dst + 8, q + 8);
+    if (second) st_global_32B(dst + 8, q + 8);
   } else {
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = pack_pair<TOut>(v[2 * i], v[2 * i + 1]);
     st_global_32B(dst, q);
+  }
+}
+// 8 values of a row as TOut; dst is 16-byte aligned
+template <typename TOut>
+__device__ __forceinline__ void store_out8(TOut *dst, const float *v) {
+  if constexpr (sizeof(TOut) == 4) {
+    reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(pack_pair<TOut>(v[0], v[1]), pack_pair<TOut>(v[2], v[3]),
+                                                 pack_pair<TOut>(v[4], v[5]), pack_pair<TOut>(v[6], v[7]));
   }
 }
 // eight 16-bit residual values (four registers) as fp32
@@ -61,6 +91,36 @@ __device__ __forceinline__ void unpack_res8(const uint32_t *r, float *v) {
     else
       f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(r + i));
     v[2 * i] = f.x, v[2 * i + 1] = f.y;
+  }
+}
+
+// Residual and store of NC finished values of a row, `cols` of which lie inside it: eight at a time where
+// rows allow it, else one by one (static register indices).
+template <typename T16, typename TOut, int NC>
+__device__ __forceinline__ void store_row(TOut *out, const T16 *res, float *v, int cols, bool vec) {
+  if (vec) {
+#pragma unroll
+    for (int g = 0; g < NC; g += 8) {
+      if (g < cols) {
+        if (res) {
+          uint32_t r[4];
+          float rv[8];
+          ld_global_16B(res + g, r);
+          unpack_res8<T16>(r, rv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[g + j] += rv[j];
+        }
+        store_out8<TOut>(out + g, v + g);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      if (j < cols) {
+        if (res) v[j] += static_cast<float>(res[j]);
+        out[j] = static_cast<TOut>(v[j]);
+      }
+    }
   }
 }
 

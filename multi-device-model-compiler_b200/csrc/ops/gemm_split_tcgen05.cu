@@ -17,7 +17,9 @@
 //     stored;
 //   * W's first stages are requested before the dependency on the previous kernel is resolved
 //     when the caller knows the weights to be complete;
-//   * results go straight from registers to global memory.
+//   * results go straight from registers to global memory: 32 bytes per access (kWide), or for rows
+//     that are not aligned to that 16 bytes or one element, a variant of its own so that the common
+//     one stays short (as run-time branches they took 2 % of a 12-layer pass over 99 tokens).
 #include <cstdlib>
 #include <type_traits>
 
@@ -39,7 +41,7 @@ struct SplitParams {
   const float *bias;
   const void *residual;
   void *out;
-  int vec_ok;   // rows of out / residual can be accessed in 32-byte vectors, bias in 16-byte ones
+  RowAccess rows;
   int n_tiles;  // column tiles
   int bn, box_m, depth, stages;
   int tmem_cols;
@@ -48,7 +50,7 @@ struct SplitParams {
   uint32_t *err;
 };
 
-template <typename T16, typename TOut, int ACT, int CG>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 __global__ void __launch_bounds__(gsplit::THREADS, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const SplitParams p) {
@@ -222,57 +224,49 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t acc[NC];
       tmem_ld_32x16(t_lane + static_cast<uint32_t>(c), acc);
       const size_t off = static_cast<size_t>(row) * p.N + gcol;
-      const bool whole = p.vec_ok && gcol + NC <= p.N;
-      float b[NC], rv[NC];
+      const int cols = p.N - gcol;
+      float v[NC];
+      if (kWide || p.rows.fast) {
+        float b[NC], rv[NC];
 #pragma unroll
-      for (int j = 0; j < NC; ++j) b[j] = rv[j] = 0.f;
-      if (p.bias) {
-        if (whole) {
+        for (int j = 0; j < NC; ++j) b[j] = rv[j] = 0.f;
+        if (p.bias) {
 #pragma unroll
           for (int j = 0; j < NC; j += 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
-            b[j] = q.x, b[j + 1] = q.y, b[j + 2] = q.z, b[j + 3] = q.w;
+            if (j < cols) {
+              const float4 q = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
+              b[j] = q.x, b[j + 1] = q.y, b[j + 2] = q.z, b[j + 3] = q.w;
+            }
           }
-        } else {
-#pragma unroll
-          for (int j = 0; j < NC; ++j)
-            if (gcol + j < p.N) b[j] = __ldg(p.bias + gcol + j);
         }
-      }
-      if (res && row_ok) {
-        if (whole) {
-          uint32_t rr[NC / 2];
-          ld_global_32B(res + off, rr);
+        if constexpr (kWide) {
+          if (res && row_ok) {
+            uint32_t rr[NC / 2];
+            ld_global_32B(res + off, rr);
 #pragma unroll
-          for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
-        } else {
-#pragma unroll
-          for (int j = 0; j < NC; ++j)
-            if (gcol + j < p.N) rv[j] = static_cast<float>(res[off + j]);
+            for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
+          }
         }
-      }
-      tmem_ld_wait_regs(acc);
-      float v[NC];
+        tmem_ld_wait_regs(acc);
 #pragma unroll
-      for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]);
-#pragma unroll
-      for (int j = 0; j < NC; ++j) v[j] += b[j];
-      if (p.vec_ok) {
+        for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]) + b[j];
         act_fast_n<ACT, NC>(v);
-      } else {
+        if constexpr (kWide) {
 #pragma unroll
-        for (int j = 0; j < NC; ++j) v[j] = act_apply_t<ACT>(v[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < NC; ++j) v[j] += rv[j];
-      if (row_ok) {
-        if (whole) {
-          store_out16<TOut>(out + off, v);
-        } else {
-#pragma unroll
-          for (int j = 0; j < NC; ++j)
-            if (gcol + j < p.N) out[off + j] = static_cast<TOut>(v[j]);
+          for (int j = 0; j < NC; ++j) v[j] += rv[j];
         }
+      } else {
+        tmem_ld_wait_regs(acc);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          v[j] = __uint_as_float(acc[j]);
+          if (p.bias && j < cols) v[j] += __ldg(p.bias + gcol + j);
+          v[j] = act_apply_t<ACT>(v[j]);
+        }
+      }
+      if (row_ok) {
+        if constexpr (kWide) store_out16<TOut>(out + off, v, cols > 8);
+        else store_row<T16, TOut, NC>(out + off, res ? res + off : nullptr, v, cols, p.rows.vec);
       }
     }
   }
@@ -293,10 +287,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
 }
 
-template <typename T16, typename TOut, int ACT, int CG>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int grid, size_t smem,
                             cudaStream_t s) {
-  auto kern = gemm_split_kernel<T16, TOut, ACT, CG>;
+  auto kern = gemm_split_kernel<T16, TOut, ACT, CG, kWide>;
   constexpr int kMaxDevices = 64;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   const int dev = device_info().device;
@@ -318,10 +312,12 @@ static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const 
 template <typename T16, typename TOut>
 static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int cg, int grid,
                              size_t smem, int act, cudaStream_t s) {
-#define MDC_SPLIT(ACT_)                                                              \
-  do {                                                                               \
-    if (cg == 2) launch_split_cg<T16, TOut, ACT_, 2>(ta, tb, p, grid, smem, s);      \
-    else launch_split_cg<T16, TOut, ACT_, 1>(ta, tb, p, grid, smem, s);              \
+#define MDC_SPLIT(ACT_)                                                                                  \
+  do {                                                                                                   \
+    if (cg == 2 && p.rows.wide) launch_split_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s);     \
+    else if (cg == 2) launch_split_cg<T16, TOut, ACT_, 2, false>(ta, tb, p, grid, smem, s);              \
+    else if (p.rows.wide) launch_split_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);           \
+    else launch_split_cg<T16, TOut, ACT_, 1, false>(ta, tb, p, grid, smem, s);                           \
   } while (0)
   switch (act) {
   case MGPU_ACT_NONE: MDC_SPLIT(kActNone); break;
@@ -365,8 +361,7 @@ void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const
   p.num_kb = static_cast<int>((Kp + gsplit::BK - 1) / gsplit::BK);
   p.k_in_x = Kp % gsplit::BK != 0;
   p.bias = bias, p.residual = residual, p.out = out;
-  auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
-  p.vec_ok = N % 16 == 0 && al(out, 32) && (!residual || al(residual, 32)) && (!bias || al(bias, 16));
+  p.rows = row_access(N, out, dtype_size(out_dtype), residual, bias);
   p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
   p.bn = t.bn, p.box_m = t.box_m, p.stages = t.stages;
   p.depth = p.k_in_x ? 1 : t.depth;

@@ -13,10 +13,16 @@
 //            bound by instruction issue, 590 cycles per k-block where the MMAs need 512).
 //   warps 2-9 epilogue: tcgen05.ld the 128 x 256 fp32 accumulator out of TMEM (each warp
 //            its 32-lane quarter, two warps per quarter splitting the columns), add bias,
-//            apply the activation, add the residual, convert and store.  A thread owns a row and
-//            moves 32 bytes per access, a whole sector, so nothing is staged: the 96 KiB that
-//            staged tiles and TMA stores took are two more stages of the ring, and the residual
-//            is fetched before the accumulator is waited for instead of after.
+//            apply the activation, add the residual, convert and store.  Two forms (kWide):
+//            Rows that can be moved 32 bytes at a time: a thread owns a row and moves a whole
+//            sector per access, so nothing is staged.  The ring has two more stages, and the
+//            residual is fetched before the accumulator is waited for instead of after.
+//            Rows of other multiples of 16 bytes (N = 8 mod 16, or a pointer off its 32-byte
+//            boundary): each warp stages 32 rows x 128 bytes in swizzled shared memory and moves
+//            it with one TMA store, the residual arrives by a TMA load, and 96 KiB of the ring go
+//            to that.  32768 x 1000 x 768: 51 us, with residual 66; with 16-byte accesses from
+//            registers, half a sector each, 57 and 84; one element at a time 351 and 516.
+//            Ragged rows, and a bias off its boundary, are stored from registers.
 // TMEM holds two accumulators (2 x 256 columns) so the epilogue of tile i overlaps the
 // mainloop of tile i+1.  Every CTA fetches its own tiles with plain TMA loads and relies on
 // L2 for reuse.  All waits are bounded (see ptx_sm100.cuh).
@@ -47,13 +53,19 @@ constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int TMEM_COLS = 512;
-template <int CG>
+constexpr int EPI_BUF_BYTES = 4096;  // staged rows: 32 x 128 bytes, per warp
+template <int CG, bool kWide>
 struct Cfg {
   static constexpr int B_ROWS = BN / CG;            // W rows this CTA stages per k-block
   static constexpr int B_BYTES = B_ROWS * BK * 2;   // 32 KiB (CG 1) / 16 KiB (CG 2)
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = CG == 2 ? 6 : 4;
-  static constexpr size_t SMEM_BYTES = static_cast<size_t>(STAGES) * STAGE_BYTES + 1024;  // + alignment slack
+  static constexpr int STAGES = kWide ? (CG == 2 ? 6 : 4) : (CG == 2 ? 4 : 3);
+  // staged rows: output (two buffers for pairs, so that a chunk does not wait for the previous one's
+  // TMA store to drain) and residual
+  static constexpr int OUT_BUFS = CG == 2 ? 2 : 1;
+  static constexpr int EPI_WARP_BYTES = kWide ? 0 : (OUT_BUFS + 1) * EPI_BUF_BYTES;
+  static constexpr size_t SMEM_BYTES =
+      static_cast<size_t>(STAGES) * STAGE_BYTES + EPI_WARPS * EPI_WARP_BYTES + 1024;  // + alignment slack
 };
 }  // namespace gemm
 
@@ -62,25 +74,34 @@ struct GemmParams {
   const float *bias;
   const void *residual;
   void *out;
-  int vec_ok;  // rows of out / residual can be accessed in 32-byte vectors, bias in 16-byte ones
+  RowAccess rows;
   int num_m_blocks, num_n_blocks;
   int cta_group;  // 1: one CTA per 128 x bn tile; 2: CTA pairs on 256 x bn tiles
   int bn;         // tile width in output columns: 256, 192 or 128 (accumulators stay 256 TMEM columns apart)
+  int cw;         // staged rows: columns per chunk, 64 (16-bit output, 128-byte rows) or 32
   uint32_t *err;
 };
+// tensor maps of the staged rows
+template <bool kWide>
+struct RowMaps {
+  CUtensorMap out, res;
+};
+template <>
+struct RowMaps<true> {};
 
-template <typename T16, typename TOut, int ACT, int CG>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 __global__ void __launch_bounds__(gemm::THREADS, 1)
-gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                    const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                    const __grid_constant__ RowMaps<kWide> rows, const GemmParams p) {
   using namespace gemm;
   using namespace ptx;
-  using C = Cfg<CG>;
+  using C = Cfg<CG, kWide>;
   constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full_bar[2], acc_empty_bar[2];
   // bias of the columns each epilogue warp handles: kept out of L1, of which the ring leaves little
-  __shared__ __align__(16) float bias_s[EPI_WARPS][BN / 2];
+  __shared__ __align__(16) float bias_s[kWide ? EPI_WARPS : 1][kWide ? BN / 2 : 4];
+  __shared__ uint64_t res_bar[kWide ? 1 : EPI_WARPS];
   __shared__ uint32_t tmem_slot;
   __shared__ uint32_t abort_flag_s;
   volatile uint32_t *abort_flag = &abort_flag_s;
@@ -114,6 +135,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       mbar_init(&acc_full_bar[a], 1);
       mbar_init(&acc_empty_bar[a], CG * EPI_WARPS * 32);  // epilogue threads of the whole pair
     }
+    if constexpr (!kWide)
+      for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&res_bar[w], 1);
     mbar_init_fence();
   }
   if (warp == 1) {
@@ -222,6 +245,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int half_sel = ew >> 2;   // which 128 accumulator columns this warp handles
     TOut *out = static_cast<TOut *>(p.out);
     const T16 *res = static_cast<const T16 *>(p.residual);
+    [[maybe_unused]] uint8_t *my_out_base = tiles + STAGES * STAGE_BYTES + ew * C::EPI_WARP_BYTES;
+    [[maybe_unused]] uint8_t *my_res = my_out_base + C::OUT_BUFS * EPI_BUF_BYTES;
+    [[maybe_unused]] int out_buf = 0;
+    [[maybe_unused]] uint32_t res_phase = 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     // the accumulator is handed back to the leader's MMA thread, in whichever CTA it lives
@@ -245,7 +272,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tc_fence_after();
         return done;
       };
-      if (p.vec_ok) {
+      if constexpr (kWide) {
         // The warp owns 32 rows x half_cols accumulator columns, read from tensor memory in
         // pieces of 32; the next piece's accumulator and residual loads are in flight while this
         // one goes through bias / activation / residual.
@@ -273,7 +300,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll 1
         for (int sub = 0; sub < n_sub; ++sub) {
           const int gcol = gcol_base + sub * 32;
-          const bool second = gcol + 16 < p.N;  // N is a multiple of 16: half pieces are whole
+          const bool second = gcol + 16 < p.N;
           tmem_ld_wait_regs(raw);
           float v[32];
 #pragma unroll
@@ -299,35 +326,130 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           if (row_ok) {
             TOut *dst = out + row_off + sub * 32;
-            store_out16<TOut>(dst, v);
-            if (second) store_out16<TOut>(dst + 16, v + 16);
+            store_out16<TOut>(dst, v, gcol + 8 < p.N);
+            if (second) store_out16<TOut>(dst + 16, v + 16, gcol + 24 < p.N);
           }
         }
-      } else {
-        // ragged or unaligned rows: one element at a time (static register indices)
+      } else if (p.rows.fast) {
+        // ---- staged rows.  Output leaves in chunks of cw columns: swizzled buffer -> one TMA store ----
         if (!wait_acc()) break;
+        const int cw = p.cw;
+        const int SUBS = cw / 32;                          // 32-column pieces per chunk
+        const int OUT_ROW_BYTES = cw * static_cast<int>(sizeof(TOut));
+        const int RES_ROW_BYTES = cw * 2;                  // residual is 16-bit
+        const int row0 = m_blk * BM + quarter * 32;
+        // 16-byte pieces of a staged row are XOR-swizzled the way TMA expects them:
+        // 128-byte rows: piece ^ (row % 8); 64-byte rows: piece ^ ((row / 2) % 4)
+        const int swz_out = OUT_ROW_BYTES == 128 ? (lane & 7) : ((lane >> 1) & 3);
+        const int swz_res = RES_ROW_BYTES == 128 ? (lane & 7) : ((lane >> 1) & 3);
+        uint32_t raw[32];
+        if (n_sub > 0) tmem_ld_32x32(t_base, raw);
+        bool chunk_ok = true;
+        uint8_t *my_out = my_out_base;
 #pragma unroll 1
         for (int sub = 0; sub < n_sub; ++sub) {
           const int gcol = gcol_base + sub * 32;
-          uint32_t raw[32];
-          tmem_ld_32x32(t_base + sub * 32, raw);
+          const int sub_in_chunk = sub % SUBS;
+          const int gcol_chunk = gcol - sub_in_chunk * 32;
+          if (sub_in_chunk == 0) {
+            if (res && lane == 0) {
+              mbar_arrive_expect_tx(&res_bar[ew], 32 * RES_ROW_BYTES);
+              tma_load_2d(my_res, &rows.res, &res_bar[ew], gcol_chunk, row0);
+            }
+            // the TMA store that last used this buffer must have finished reading it
+            my_out = my_out_base + out_buf * EPI_BUF_BYTES;
+            if (lane == 0) tma_store_wait_read<C::OUT_BUFS - 1>();
+            __syncwarp();
+            if constexpr (C::OUT_BUFS == 2) out_buf ^= 1;
+          }
           tmem_ld_wait_regs(raw);
           float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            v[j] = __uint_as_float(raw[j]);
-            if (p.bias && gcol + j < p.N) v[j] += __ldg(p.bias + gcol + j);
-            v[j] = act_apply_t<ACT>(v[j]);
-          }
-          if (row_ok) {
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
+          if (sub + 1 < n_sub) tmem_ld_32x32(t_base + (sub + 1) * 32, raw);  // overlaps the math below
+          if (p.bias) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
+            for (int j = 0; j < 32; j += 4) {
               if (gcol + j < p.N) {
-                const size_t off = static_cast<size_t>(row) * p.N + gcol + j;
-                if (res) v[j] += static_cast<float>(res[off]);
-                out[off] = static_cast<TOut>(v[j]);
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
+                v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
               }
             }
+          }
+          act_fast_n<ACT, 32>(v);
+          if (res) {
+            if (sub_in_chunk == 0) {
+              if (!mbar_wait_warp(&res_bar[ew], res_phase, abort_flag)) {
+                atomicCAS(p.err, 0u, 0x50000000u | static_cast<uint32_t>(ew));
+                chunk_ok = false;
+                break;
+              }
+              res_phase ^= 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // this piece is 64 bytes of the residual row
+              const int phys = (sub_in_chunk * 4 + j) ^ swz_res;
+              const uint4 q = *reinterpret_cast<const uint4 *>(my_res + lane * RES_ROW_BYTES + (phys << 4));
+              const uint32_t r[4] = {q.x, q.y, q.z, q.w};
+              float rv[8];
+              unpack_res8<T16>(r, rv);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[8 * j + e] += rv[e];
+            }
+          }
+          if constexpr (sizeof(TOut) == 2) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // 32 columns = four 16-byte pieces of the staged row
+              const int phys = (sub_in_chunk * 4 + j) ^ swz_out;
+              store_out8<TOut>(reinterpret_cast<TOut *>(my_out + lane * OUT_ROW_BYTES + (phys << 4)), v + 8 * j);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4 *>(my_out + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                  make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          }
+          if (sub_in_chunk == SUBS - 1 || sub + 1 == n_sub) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&rows.out, my_out, gcol_chunk, row0);  // rows / columns past M / N are clipped
+              tma_store_commit();
+            }
+          }
+        }
+        if (!chunk_ok) break;
+      } else {
+        // ---- ragged rows, or a bias off its boundary ----
+        if (!wait_acc()) break;
+#pragma unroll 1
+        for (int sub = 0; sub < n_sub; ++sub) {
+          const int gcol = gcol_base + sub * 32, cols = p.N - gcol;
+          uint32_t raw[32];
+          tmem_ld_32x32(t_base + sub * 32, raw);
+          tmem_ld_wait_regs(raw);
+          const size_t off = static_cast<size_t>(row) * p.N + gcol;
+          if (p.rows.vec && cols >= 32) {
+#pragma unroll
+            for (int g = 0; g < 32; g += 8) {
+              float v[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                v[j] = __uint_as_float(raw[g + j]);
+                if (p.bias) v[j] += __ldg(p.bias + gcol + g + j);
+                v[j] = act_apply_t<ACT>(v[j]);
+              }
+              if (row_ok) store_row<T16, TOut, 8>(out + off + g, res ? res + off + g : nullptr, v, 8, true);
+            }
+          } else {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              v[j] = __uint_as_float(raw[j]);
+              if (p.bias && j < cols) v[j] += __ldg(p.bias + gcol + j);
+              v[j] = act_apply_t<ACT>(v[j]);
+            }
+            if (row_ok) store_row<T16, TOut, 32>(out + off, res ? res + off : nullptr, v, cols, false);
           }
         }
       }
@@ -335,6 +457,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if constexpr (CG == 2) mbar_arrive_cluster(acc ? acc_empty_addr1 : acc_empty_addr0);
       else mbar_arrive(&acc_empty_bar[acc]);
       if ((acc ^= 1) == 0) acc_phase ^= 1;
+    }
+    if constexpr (!kWide) {
+      if (lane == 0) tma_store_wait<0>();  // all staged output has left shared memory
     }
   }
   // ------------------------------ teardown ------------------------------
@@ -403,10 +528,11 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
   return encode_tmap_2d_ex(map, base, dtype, inner, outer, row_stride_bytes, box_inner, box_outer, 128);
 }
 
-template <typename T16, typename TOut, int ACT, int CG>
-static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, cudaStream_t s) {
-  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG>;
-  constexpr size_t smem = gemm::Cfg<CG>::SMEM_BYTES;
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
+static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p,
+                           int grid, cudaStream_t s) {
+  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG, kWide>;
+  constexpr size_t smem = gemm::Cfg<CG, kWide>::SMEM_BYTES;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   bool &attr_set = attr_set_on[current_device_index()];
   if (!attr_set) {
@@ -417,28 +543,50 @@ static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const G
   }
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gemm::THREADS), smem, s, CG, ta, tb, p),
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gemm::THREADS), smem, s, CG, ta, tb, rows, p),
                "launch gemm");
   }
   launched("gemm_tcgen05_kernel");
 }
 
 // p.cta_group selects the variant; grid is CTAs (even for pairs)
-template <typename T16, typename TOut, int ACT>
-static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, cudaStream_t s) {
-  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2>(ta, tb, p, grid, s);
-  else launch_gemm_cg<T16, TOut, ACT, 1>(ta, tb, p, grid, s);
+template <typename T16, typename TOut, int ACT, bool kWide>
+static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p, int grid,
+                        cudaStream_t s) {
+  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, kWide>(ta, tb, rows, p, grid, s);
+  else launch_gemm_cg<T16, TOut, ACT, 1, kWide>(ta, tb, rows, p, grid, s);
+}
+
+template <typename T16, typename TOut, bool kWide>
+static void launch_gemm_act(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p,
+                            int grid, int act, cudaStream_t s) {
+  switch (act) {
+  case MGPU_ACT_NONE: launch_gemm<T16, TOut, kActNone>(ta, tb, rows, p, grid, s); break;
+  case MGPU_ACT_RELU: launch_gemm<T16, TOut, kActRelu>(ta, tb, rows, p, grid, s); break;
+  case MGPU_ACT_GELU_ERF: launch_gemm<T16, TOut, kActGeluErf>(ta, tb, rows, p, grid, s); break;
+  case MGPU_ACT_GELU_TANH: launch_gemm<T16, TOut, kActGeluTanh>(ta, tb, rows, p, grid, s); break;
+  default: fail("mgpuMatmulEx16: unknown activation");
+  }
 }
 
 template <typename T16, typename TOut>
-static void launch_gemm_act(const CUtensorMap &ta, const CUtensorMap &tb, const GemmParams &p, int grid, int act, cudaStream_t s) {
-  switch (act) {
-  case MGPU_ACT_NONE: launch_gemm<T16, TOut, kActNone>(ta, tb, p, grid, s); break;
-  case MGPU_ACT_RELU: launch_gemm<T16, TOut, kActRelu>(ta, tb, p, grid, s); break;
-  case MGPU_ACT_GELU_ERF: launch_gemm<T16, TOut, kActGeluErf>(ta, tb, p, grid, s); break;
-  case MGPU_ACT_GELU_TANH: launch_gemm<T16, TOut, kActGeluTanh>(ta, tb, p, grid, s); break;
-  default: fail("mgpuMatmulEx16: unknown activation");
+static void launch_gemm_rows(const CUtensorMap &ta, const CUtensorMap &tb, GemmParams &p, int32_t dtype, int32_t out_dtype,
+                             int grid, int act, cudaStream_t s) {
+  if (p.rows.wide) {
+    launch_gemm_act<T16, TOut, true>(ta, tb, RowMaps<true>{}, p, grid, act, s);
+    return;
   }
+  RowMaps<false> rows{ta, ta};  // placeholders for rows that are not staged
+  // staged chunks of 64 columns (128-byte rows) for 16-bit output when a tile half is a multiple of
+  // that, else of 32
+  p.cw = sizeof(TOut) == 2 && (p.bn / 2) % 64 == 0 ? 64 : 32;
+  const uint64_t N = static_cast<uint64_t>(p.N), M = static_cast<uint64_t>(p.M);
+  const uint32_t cw = static_cast<uint32_t>(p.cw);
+  if (p.rows.fast) {
+    if (!encode_tmap_2d_ex(&rows.out, p.out, out_dtype, N, M, N * sizeof(TOut), cw, 32, static_cast<int>(cw * sizeof(TOut)))) return;
+    if (p.residual && !encode_tmap_2d_ex(&rows.res, p.residual, dtype, N, M, N * 2, cw, 32, static_cast<int>(cw * 2))) return;
+  }
+  launch_gemm_act<T16, TOut, false>(ta, tb, rows, p, grid, act, s);
 }
 
 // CTA pairs whenever there are at least two 128-row blocks; MDC_GEMM_CTA_GROUP=1|2 overrides
@@ -624,8 +772,7 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
   p.bias = bias;
   p.residual = residual;
   p.out = out;
-  auto al = [](const void *q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
-  p.vec_ok = N % 16 == 0 && al(out, 32) && (!residual || al(residual, 32)) && (!bias || al(bias, 16));
+  p.rows = row_access(N, out, dtype_size(out_dtype), residual, bias);
   p.num_m_blocks = static_cast<int>((M + gemm::BM - 1) / gemm::BM);
   p.num_n_blocks = static_cast<int>((N + bn - 1) / bn);
   p.err = err;
@@ -633,12 +780,12 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
   if (grid <= 0) { failf("too many tiles"); return; }
 
   if (dtype == MGPU_DTYPE_F16) {
-    if (out_dtype == MGPU_DTYPE_F16) launch_gemm_act<__half, __half>(ta, tb, p, grid, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__half, float>(ta, tb, p, grid, act, s);
+    if (out_dtype == MGPU_DTYPE_F16) launch_gemm_rows<__half, __half>(ta, tb, p, dtype, out_dtype, grid, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_rows<__half, float>(ta, tb, p, dtype, out_dtype, grid, act, s);
     else failf("output type must be the operand type or F32");
   } else {
-    if (out_dtype == MGPU_DTYPE_BF16) launch_gemm_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, grid, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_act<__nv_bfloat16, float>(ta, tb, p, grid, act, s);
+    if (out_dtype == MGPU_DTYPE_BF16) launch_gemm_rows<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, dtype, out_dtype, grid, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_gemm_rows<__nv_bfloat16, float>(ta, tb, p, dtype, out_dtype, grid, act, s);
     else failf("output type must be the operand type or F32");
   }
 }

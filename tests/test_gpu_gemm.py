@@ -205,3 +205,73 @@ def test_gelu_of_ragged_rows_is_exact_to_fp32(m, M, N, bias_offset):
     ref = np.repeat(_gelu64(v)[:, None], N - 1, axis=1)
     assert np.linalg.norm(got[:, :-1] - ref) <= 1.5e-7 * np.linalg.norm(ref)
     assert np.all(np.isposinf(got[:, -1]))
+
+
+def _matmul16_at(m, a, w, b, r, out_dtype, act=0, out_off=0, res_off=0, bias_off=0, repeat=0):
+    """mgpuMatmulEx16 with out / residual / bias that many bytes off their allocation; repeat > 0: the
+    median time of that many calls in microseconds instead of the result."""
+    M, K = a.shape
+    N = w.shape[1]
+    item = 4 if out_dtype == m.F32 else 2
+
+    def at(arr, nbytes):
+        return m.to_device(np.concatenate([np.zeros(nbytes, np.uint8), np.ascontiguousarray(arr).view(np.uint8).ravel()]))
+    da, dw, db, dr = m.to_device(a.astype(np.float16)), m.to_device(w), at(b, bias_off), at(r.astype(np.float16), res_off)
+    dwp, do = m.DeviceBuffer(N * K * 2), m.DeviceBuffer(M * N * item + 64)
+    m.ops().mgpuPackWeight(dw.ptr, dwp.ptr, K, N, m.F16, None)
+
+    def call(stream=None):
+        m.ops().mgpuMatmulEx16(da.ptr, dwp.ptr, db.ptr + bias_off, dr.ptr + res_off, do.ptr + out_off, M, N, K, m.F16, out_dtype, act, stream)
+    if repeat:
+        import torch
+        s = torch.cuda.Stream()
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(repeat + 4)]
+        m.runtime().mgpuStreamSynchronize(None)
+        for e in ev:
+            e.record(s)
+            call(s.cuda_stream)
+        s.synchronize()
+        return float(np.median([x.elapsed_time(y) * 1e3 for x, y in zip(ev[3:-1], ev[4:])]))
+    rt = m.runtime()
+    rt.mgpuMemset32(do.ptr, 0x7fc00000, (M * N * item + 64) // 4, None)
+    call()
+    raw = m.to_host(do, (M * N * item + 64,), np.uint8)
+    assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+    m.check("mgpuMatmulEx16")
+    fill = np.full(16 + M * N * item // 4 + 1, 0x7fc00000, np.uint32).view(np.uint8)
+    end = out_off + M * N * item  # nothing beside the result was written
+    assert np.array_equal(raw[:out_off], fill[:out_off]) and np.array_equal(raw[end:], fill[end:len(raw)])
+    got = raw[out_off:end].view(np.float32 if out_dtype == m.F32 else np.float16).reshape(M, N)
+    return got.astype(np.float32)
+
+
+@pytest.mark.parametrize("offsets", [(0, 0, 0), (16, 0, 0), (0, 16, 0), (16, 16, 0), (0, 0, 4), (4, 2, 0)])
+@pytest.mark.parametrize("M,N", [(70, 8), (70, 40), (200, 1000), (20000, 24), (19300, 128), (2500, 2056)])
+def test_row_alignments_are_exact(m, M, N, offsets):
+    # 32-byte, 16-byte and element-wise rows of both Gemm kernels (one-wave up to 200 rows here,
+    # persistent above), with the tail columns of N = 8 mod 16; small integers, so equal bit for bit
+    rng = np.random.default_rng(19)
+    K = 64
+    a = rng.integers(-3, 4, (M, K)).astype(np.float32)
+    w = rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    r = rng.integers(-8, 9, (M, N)).astype(np.float32)
+    ref = np.maximum(a @ w + b, 0) + r
+    oo, ro, bo = offsets
+    for out_dtype in (m.F16, m.F32):
+        assert np.array_equal(_matmul16_at(m, a, w, b, r, out_dtype, m.ACT_RELU, oo, ro, bo), ref)
+
+
+@pytest.mark.parametrize("N,offsets", [(1000, (0, 0, 0)), (768, (16, 0, 0)), (768, (0, 16, 0))])
+def test_rows_of_16_byte_multiples_are_not_slow(m, N, offsets):
+    # against the next width of whole sectors: up to 1.3 times its time, 4 to 10 times when such rows
+    # went one element at a time
+    rng = np.random.default_rng(23)
+    M, K, wide = 32768, 768, (N + 15) // 16 * 16
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    for out_dtype in (m.F16, m.F32):
+        t = []
+        for n, off in ((N, offsets), (wide, (0, 0, 0))):
+            w = (0.02 * rng.standard_normal((K, n))).astype(np.float32)
+            t.append(_matmul16_at(m, a, w, np.zeros(n, np.float32), np.zeros((M, n), np.float32), out_dtype, 0, *off, repeat=20))
+        assert t[0] <= 2.5 * t[1], t
