@@ -109,6 +109,54 @@ def test_conv_gather_modes_agree(m):
         assert np.array_equal(staged, direct)
 
 
+@pytest.mark.parametrize("IC,taps", [(32, (3, 3)), (32, (1, 1)), (96, (3, 2)), (160, (1, 3)), (64, (3, 3))])
+def test_conv_direct_k_order(m, IC, taps):
+    """The direct kernel's dense k order (groups of 32 channels of one tap; two taps share a k-block in
+    a last block of 32 channels): exact on small integers, and bit for bit the im2col kernel's sums
+    on real ones."""
+    import os
+    rng = np.random.default_rng(IC)
+    kw = dict(stride=(2, 1), pad=(1, 0, 1, 1))
+    for x, w in ((rng.integers(-4, 5, size=(3, IC, 13, 11)), rng.integers(-3, 4, size=(70, IC) + taps)),
+                 (rng.standard_normal((3, IC, 13, 11)), rng.standard_normal((70, IC) + taps) / np.sqrt(IC * 9))):
+        x, w, b = x.astype(np.float32), w.astype(np.float32), rng.integers(-8, 9, size=70).astype(np.float32)
+        persistent = m.conv2d(x, w, b, **kw)
+        os.environ["MDC_CONV_DIRECT"] = "1"
+        try:
+            direct = m.conv2d(x, w, b, **kw)
+        finally:
+            del os.environ["MDC_CONV_DIRECT"]
+        assert np.array_equal(direct, persistent)
+        if float(x.flat[0]).is_integer():
+            assert np.array_equal(direct, oracle.conv2d(x, w, b, **kw))
+
+
+def test_conv_direct_has_no_empty_half_blocks(m):
+    """32 input channels cost the direct kernel half of what 64 do: two taps share a k-block.  (0.58 of
+    the time measured; 0.9 when every tap was padded to 64 channels.)"""
+    import os
+    import torch
+    s = torch.cuda.Stream()
+    times = []
+    for IC in (32, 64):
+        x, w, b = torch.randn(64, IC, 56, 56, device="cuda"), torch.randn(64, IC, 3, 3, device="cuda"), torch.randn(64, device="cuda")
+        out = torch.empty(64, 64, 56, 56, device="cuda")
+        torch.cuda.synchronize()
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(24)]
+        os.environ["MDC_CONV_DIRECT"] = "1"
+        try:
+            for e in ev:
+                e.record(s)
+                m.ops().mgpuConv2d(x.data_ptr(), w.data_ptr(), b.data_ptr(), out.data_ptr(), None, 64, IC, 56, 56, 64, 3, 3, 56, 56,
+                                   1, 1, 1, 1, 1, 1, 1, 1, False, False, s.cuda_stream)
+        finally:
+            del os.environ["MDC_CONV_DIRECT"]
+        s.synchronize()
+        m.check("conv")
+        times.append(float(np.median([a.elapsed_time(b) for a, b in zip(ev[3:-1], ev[4:])])))
+    assert times[0] <= 0.75 * times[1], times
+
+
 def test_conv_exact_on_small_integers(m):
     """Integer-valued operands are exact in fp16 and every partial sum is exact in fp32, so the
     result must equal the oracle bit for bit: this isolates the gather / scatter indexing."""
