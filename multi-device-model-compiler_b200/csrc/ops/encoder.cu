@@ -73,6 +73,18 @@ static void drop_graphs(EncoderStack *st) {
   st->graphs.clear();
 }
 
+// Whether the weights have been packed.  An event query is one of the calls that a capture in global
+// mode forbids to every thread, whatever stream it captures; refused, it would also invalidate that
+// capture.  This event belongs to no capture, so the thread asks in relaxed mode.
+static void see_weights(EncoderStack *st) {
+  if (st->weights_complete || !st->weights_ev) return;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+  st->weights_complete = cudaEventQuery(st->weights_ev) == cudaSuccess;
+  if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
+  (void)cudaGetLastError();
+}
+
 static void order_after_previous(EncoderStack *st, void *stream) {
   if (!st->done_ev) check_cuda(cudaEventCreateWithFlags(&st->done_ev, cudaEventDisableTiming), "event");
   if (st->used && st->done_ev) cudaStreamWaitEvent(as_stream(stream), st->done_ev, 0);
@@ -218,10 +230,7 @@ static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *
     (void)cudaGetLastError();
   }
   // (an event cannot be asked about inside a capture; what was seen before it still holds)
-  if (!st->weights_complete && !capturing && st->weights_ev) {
-    st->weights_complete = cudaEventQuery(st->weights_ev) == cudaSuccess;
-    (void)cudaGetLastError();
-  }
+  if (!capturing) see_weights(st);
   const bool w_ready = st->weights_complete;
   const bool eligible = graphs_enabled() && !st->graphs_off && !g_profiling && s != nullptr && !capturing;
   if (!eligible) {

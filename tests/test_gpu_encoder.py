@@ -343,3 +343,52 @@ def test_small_batches_reproduce_the_same_bits(m, dtype_name, norm_first):
     if norm_first:  # causal: the first rows of a sequence are those of a shorter one (48 tokens)
         assert np.array_equal(st.run(np.ascontiguousarray(x[2:3, :48]), None), y[2:3, :48])
     st.close()
+
+
+def _set_layers(m, st, layers, stream):
+    """SetLayer for every layer, without waiting; returns the weight buffers, to be kept until it ran."""
+    keep = []
+    for i, lw in enumerate(layers):
+        bufs = [m.to_device(np.ascontiguousarray(lw[k], dtype=np.float32), stream) if lw[k] is not None else None for k in
+                ("wqkv", "bqkv", "wo", "bo", "w1", "b1", "w2", "b2", "ln1_g", "ln1_b", "ln2_g", "ln2_b")]
+        keep.append(bufs)
+    for i, bufs in enumerate(keep):
+        m.ops().mgpuEncoderStackSetLayer(st.h, i, *[b.ptr if b else None for b in bufs], stream)
+    return keep
+
+
+def test_run_leaves_a_capture_on_another_stream_alone(m):
+    """A run on one stream while another one is being captured in global mode, after new weights: it
+    may not make a call that such a capture forbids, which would also invalidate the capture."""
+    import torch
+    rt, ops = m.runtime(), m.ops()
+    rng = np.random.default_rng(61)
+    B, S, d, F, H = 2, 64, 128, 256, 2
+    layers = [make_layer(rng, d, F, std=0.05)]
+    st = m.EncoderStack(layers, H)
+    stream = rt.mgpuStreamCreate()
+    x = rng.standard_normal((B, S, d)).astype(np.float32)
+    dx, dy = m.to_device(x, stream), m.DeviceBuffer(x.nbytes, stream)
+    ops.mgpuEncoderStackRun(st.h, dx.ptr, None, dy.ptr, B, S, stream)  # workspace and kernels are set up
+    expect = m.to_host(dy, x.shape, np.float32, stream)
+    keep = _set_layers(m, st, layers, stream)  # the same weights again
+    rt.mgpuStreamSynchronize(stream)
+    rt.mgpuMemset32(dy.ptr, 0, x.size, stream)
+    rt.mgpuStreamSynchronize(stream)
+    a = torch.zeros(1024, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="global")
+        a.add_(1.0)
+        ops.mgpuEncoderStackRun(st.h, dx.ptr, None, dy.ptr, B, S, stream)
+        a.add_(1.0)
+        graph.capture_end()  # raises when the capture was invalidated
+    m.check("run beside a capture")
+    assert np.array_equal(m.to_host(dy, x.shape, np.float32, stream), expect)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(a[0]) == 2.0
+    del graph, keep
+    st.close()
