@@ -54,6 +54,7 @@ struct EncoderStack {
   // may read weights ahead of their dependency on the previous kernel
   cudaEvent_t weights_ev = nullptr;
   bool weights_complete = false;
+  bool early_weights = true;  // false for good once the event does not cover every layer (see note_weights)
   // CUDA graphs of whole runs, keyed by the run's pointers and shape (see run_stack_replayed)
   struct RunGraph {
     const float *x = nullptr;
@@ -77,12 +78,35 @@ static void drop_graphs(EncoderStack *st) {
 // mode forbids to every thread, whatever stream it captures; refused, it would also invalidate that
 // capture.  This event belongs to no capture, so the thread asks in relaxed mode.
 static void see_weights(EncoderStack *st) {
-  if (st->weights_complete || !st->weights_ev) return;
+  if (st->weights_complete || !st->weights_ev || !st->early_weights) return;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
   st->weights_complete = cudaEventQuery(st->weights_ev) == cudaSuccess;
   if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
   (void)cudaGetLastError();
+}
+
+static bool is_capturing(cudaStream_t s) {
+  if (s == nullptr) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool yes = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return yes;
+}
+
+// Records that a layer's weights are packed once `s` has come this far.  Layers may be set on
+// different streams: each recording also covers the earlier ones.  Weights whose packing is captured
+// are packed whenever that graph runs, and an event that was not recorded would query as complete:
+// such a stack waits for its dependencies before it reads weights.
+static void note_weights(EncoderStack *st, cudaStream_t s) {
+  st->weights_complete = false;
+  if (is_capturing(s)) st->early_weights = false;
+  if (!st->early_weights) return;
+  if (!st->weights_ev)
+    st->early_weights = check_cuda(cudaEventCreateWithFlags(&st->weights_ev, cudaEventDisableTiming), "event");
+  else
+    st->early_weights = check_cuda(cudaStreamWaitEvent(s, st->weights_ev, 0), "order after the other layers' weights");
+  if (st->early_weights) st->early_weights = check_cuda(cudaEventRecord(st->weights_ev, s), "record the weights' event");
 }
 
 static void order_after_previous(EncoderStack *st, void *stream) {
@@ -223,12 +247,7 @@ static bool graphs_enabled() {
 static void run_stack_replayed(EncoderStack *st, const float *x, const int32_t *lens, float *y, int64_t B, int64_t S,
                                void *stream) {
   cudaStream_t s = as_stream(stream);
-  bool capturing = false;
-  if (s != nullptr) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    capturing = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
-    (void)cudaGetLastError();
-  }
+  const bool capturing = is_capturing(s);
   // (an event cannot be asked about inside a capture; what was seen before it still holds)
   if (!capturing) see_weights(st);
   const bool w_ready = st->weights_complete;
@@ -350,11 +369,7 @@ MDC_API void mgpuEncoderStackSetLayer(void *stack, int64_t layer, const float *q
   lw.ln1_b = dup_f32(ln1_beta, d, stream);
   lw.ln2_g = dup_f32(ln2_gamma, d, stream);
   lw.ln2_b = dup_f32(ln2_beta, d, stream);
-  st->weights_complete = false;
-  // layers may be set on different streams: each recording also covers the earlier ones
-  if (st->weights_ev) cudaStreamWaitEvent(as_stream(stream), st->weights_ev, 0);
-  if (!st->weights_ev && !check_cuda(cudaEventCreateWithFlags(&st->weights_ev, cudaEventDisableTiming), "event")) return;
-  cudaEventRecord(st->weights_ev, as_stream(stream));
+  note_weights(st, as_stream(stream));
 }
 
 MDC_API void mgpuEncoderStackRun(void *stack, const float *x, const int32_t *seq_lens, float *y,

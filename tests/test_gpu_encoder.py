@@ -392,3 +392,78 @@ def test_run_leaves_a_capture_on_another_stream_alone(m):
     assert float(a[0]) == 2.0
     del graph, keep
     st.close()
+
+
+def test_layers_can_be_set_inside_a_capture(m):
+    """SetLayer is a sequence of stream operations and can be captured, also after layers were set
+    eagerly; the weights are then packed whenever the graph runs, so a later run must not read them
+    ahead of its dependencies."""
+    import torch
+    rt, ops = m.runtime(), m.ops()
+    rng = np.random.default_rng(71)
+    B, S, d, F, H = 2, 64, 128, 256, 2
+    old, new = [make_layer(rng, d, F, std=0.05)], [make_layer(rng, d, F, std=0.05)]
+    st, st_new = m.EncoderStack(old, H), m.EncoderStack(new, H)
+    torch_stream = torch.cuda.Stream()
+    stream = torch_stream.cuda_stream
+    x = rng.standard_normal((B, S, d)).astype(np.float32)
+    dx, dy = m.to_device(x, stream), m.DeviceBuffer(x.nbytes, stream)
+
+    def run(handle):
+        ops.mgpuEncoderStackRun(handle.h, dx.ptr, None, dy.ptr, B, S, stream)
+        y = m.to_host(dy, x.shape, np.float32, stream)
+        assert ops.mgpuOpsCheckDeviceStatus(stream) == 0
+        m.check("run")
+        return y
+    expect = run(st_new)
+    assert not np.array_equal(run(st), expect)
+    keep = _set_layers(m, st, old, stream)
+    rt.mgpuStreamSynchronize(stream)
+    weights = [[m.to_device(np.ascontiguousarray(lw[k], dtype=np.float32), stream) if lw[k] is not None else None for k in
+                ("wqkv", "bqkv", "wo", "bo", "w1", "b1", "w2", "b2", "ln1_g", "ln1_b", "ln2_g", "ln2_b")] for lw in new]
+    torch.cuda.synchronize()
+    rt.mgpuPoolTrim()  # a block last used on another stream would have to be waited for
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch_stream):
+        graph.capture_begin(capture_error_mode="relaxed")
+        for i, bufs in enumerate(weights):
+            ops.mgpuEncoderStackSetLayer(st.h, i, *[b.ptr if b else None for b in bufs], stream)
+        graph.capture_end()
+    m.check("SetLayer inside a capture")
+    for _ in range(4):  # eager, captured and replayed runs
+        graph.replay()
+        assert np.array_equal(run(st), expect)
+    del graph, keep
+    st.close()
+    st_new.close()
+    torch.cuda.synchronize()
+    rt.mgpuPoolTrim()  # nor may a block that was freed inside the capture be handed to another stream
+    rt.mgpuClearLastError()
+
+
+def test_run_right_after_the_layers_were_set(m):
+    """Nothing between SetLayer and Run: the weights are still being
+    packed when the first Gemm could read them ahead of its dependencies, which it must not."""
+    rt, ops = m.runtime(), m.ops()
+    rng = np.random.default_rng(81)
+    B, S, d, F, H = 1, 48, 768, 3072, 12
+    weights = [[make_layer(rng, d, F) for _ in range(2)] for _ in range(3)]
+    x = rng.standard_normal((B, S, d)).astype(np.float32)
+    expect = []
+    for layers in weights:
+        st = m.EncoderStack(layers, H)
+        expect.append(st.run(x, None))
+        st.close()
+    stream = rt.mgpuStreamCreate()
+    st = m.EncoderStack(weights[0], H)
+    dx, dy = m.to_device(x, stream), m.DeviceBuffer(x.nbytes, stream)
+    for turn in range(6):  # in between, replays of a captured run with weights known to be complete
+        which = turn % 3
+        keep = _set_layers(m, st, weights[which], stream)
+        for _ in range(1 + turn % 3):
+            ops.mgpuEncoderStackRun(st.h, dx.ptr, None, dy.ptr, B, S, stream)
+        assert np.array_equal(m.to_host(dy, x.shape, np.float32, stream), expect[which]), turn
+        del keep
+    assert ops.mgpuOpsCheckDeviceStatus(stream) == 0
+    m.check("set and run")
+    st.close()
