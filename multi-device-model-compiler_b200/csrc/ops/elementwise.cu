@@ -186,8 +186,7 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 }
 
 // All operands of a call in one launch; a block belongs to one job.
-//   cast: kCastItems elements of a contiguous array, or kPadItems of rows that are padded (element by
-//         element: shorter, so that a few odd rows still spread over the SMs).
+//   cast: kCastItems elements of a contiguous array, or kPadItems of rows that are padded.
 //   pack: weight fp32 [K, N] (N contiguous) -> 16-bit [N, Kp] (K contiguous), zero padded to Kp, in
 //         64 x 64 tiles through shared memory: reads are 16-byte vectors along n (whole lines of w),
 //         writes are 16-byte vectors of eight 16-bit values along k (whole lines of out).
@@ -195,7 +194,7 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 // job is filled by the next and the launch gaps go: a 1024-wide
 // context layer with 2048 tokens (five operands) 130 -> 118 us a call; 35 x 3086 x 3392 Gemm, whose rows
 // need padding, 50 -> 38 us (with the one-wave Gemm).
-constexpr int64_t kCastItems = kEwBlock * 16, kPadItems = kEwBlock * 4;
+constexpr int64_t kCastItems = OperandList::kCastItems, kPadItems = OperandList::kPadItems;
 struct OperandJobs {
   OperandList::Job j[OperandList::kMax];
   int n;
@@ -203,7 +202,7 @@ struct OperandJobs {
 
 template <typename T16>
 __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const OperandJobs jobs) {
-  static_assert(kEwBlock == 256, "the 64 x 64 tiles are walked by 256 threads");
+  static_assert(kEwBlock == OperandList::kThreads, "the 64 x 64 tiles are walked by 256 threads");
   __shared__ float tile[64][65];
   pdl_launch_dependents();
   pdl_wait();
@@ -288,27 +287,13 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
   }
 }
 
-void OperandList::cast(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp) {
-  if (n == kMax || R <= 0 || Cp <= 0) return;
-  Job &j = jobs[n++];
-  j.src = src, j.dst = dst, j.rows = R, j.cols = C, j.pitch = Cp, j.first_block = blocks, j.tiles_n = 0;
-  j.vec_ok = C == Cp && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-  const int64_t items = j.vec_ok ? kCastItems : kPadItems;
-  blocks += (R * Cp + items - 1) / items;
-}
-
-void OperandList::pack(const float *w, void *dst, int64_t K, int64_t N) {
-  if (n == kMax || K <= 0 || N <= 0) return;
-  Job &j = jobs[n++];
-  j.src = w, j.dst = dst, j.rows = K, j.cols = N, j.pitch = (K + 7) / 8 * 8, j.first_block = blocks;
-  j.tiles_n = static_cast<int>((N + 63) / 64);
-  j.vec_ok = (N % 4 == 0) && !(reinterpret_cast<uintptr_t>(w) & 15u);
-  blocks += j.tiles_n * ((j.pitch + 63) / 64);
-}
-
 void OperandList::launch(int32_t dtype, void *stream) {
   if (n == 0) return;
-  if (blocks > 0x7fffffff) { fail("operand conversion: shape too large"); return; }
+  if (overflow || blocks > 0x7fffffff) {
+    fail(overflow ? "operand conversion: more operands than a call may have" : "operand conversion: shape too large");
+    clear();
+    return;
+  }
   OperandJobs a;
   for (int i = 0; i < kMax; ++i) a.j[i] = jobs[i < n ? i : 0];
   a.n = n;
@@ -320,10 +305,8 @@ void OperandList::launch(int32_t dtype, void *stream) {
   else
     check_cuda(launch_chain(prepare_operands_kernel<__nv_bfloat16>, grid, dim3(kEwBlock), 0, s, 1, a), "launch prepare_operands");
   launched("mdc_prepare_operands");
-  n = 0;
-  blocks = 0;
+  clear();
 }
-
 
 }  // namespace mdc
 

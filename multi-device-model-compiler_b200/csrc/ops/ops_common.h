@@ -13,6 +13,7 @@
 
 #include "mdc_gpu_ops.h"
 #include "mdc_gpu_runtime.h"
+#include "operand_list.h"
 
 #define MDC_API extern "C" __attribute__((visibility("default")))
 #define MDC_CXX_API __attribute__((visibility("default")))
@@ -117,26 +118,6 @@ struct ProfileScope {
 
 // fp32 [R, C] -> 16-bit [R, Cp] with zero padding of the columns C..Cp (elementwise.cu)
 void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype, cudaStream_t s);
-
-// Operands that one call has to bring into 16 bits, collected and then converted by ONE launch
-// (elementwise.cu): casts of activations and packings of weights.
-struct OperandList {
-  static constexpr int kMax = 5;  // a transformer layer: its input and four weights
-  struct Job {
-    const float *src;
-    void *dst;
-    int64_t rows, cols, pitch;  // cast: [rows, cols] -> [rows, pitch]; pack: [rows = K, cols = N] -> [N, pitch]
-    int64_t first_block;
-    int tiles_n;                // pack: 64-column tiles; 0 marks a cast
-    int vec_ok;
-  };
-  Job jobs[kMax];
-  int n = 0;
-  int64_t blocks = 0;
-  void cast(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp);
-  void pack(const float *w, void *dst, int64_t K, int64_t N);
-  void launch(int32_t dtype, void *stream);  // nothing when empty
-};
 
 // mgpuMatmulEx16; w_ready: the weight was complete before this call (it does not come from a kernel
 // still queued), so the kernel may read it ahead of its dependency on the previous one.
