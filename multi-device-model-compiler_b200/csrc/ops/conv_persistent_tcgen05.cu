@@ -602,11 +602,9 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   const int before = mgpuGetLastError();
   char *ws = static_cast<char *>(mgpuMemAllocAsync(w_bytes + x_bytes, s));
   if (!ws) {
-    if (before == 0 && x_bytes) {
-      mgpuClearLastError();
-      return false;
-    }
-    return true;
+    if (!x_bytes) return true;
+    if (before == 0) mgpuClearLastError();  // an earlier failure's status stays
+    return false;
   }
   ConvPrepareParams q;
   q.x = c.x, q.w = c.w, q.w16 = reinterpret_cast<__half *>(ws), q.x16 = reinterpret_cast<__half *>(ws + w_bytes);

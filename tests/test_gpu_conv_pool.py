@@ -202,6 +202,45 @@ def test_conv_persistent_edges(m, shape):
     assert np.array_equal(m.conv2d(x, w, b, **kw), oracle.conv2d(x, w, b, **kw))
 
 
+@pytest.mark.parametrize("earlier_failure", [False, True])
+def test_conv_without_memory_for_the_copy(m, earlier_failure):
+    """With no device memory left for the NHWC copy of the input the direct kernel takes over, whether
+    or not an earlier call has left a status; that status stays."""
+    import torch
+    rt, ops = m.runtime(), m.ops()
+    N, IC, H, W, OC, OH, OW = 12, 32, 2048, 2048, 16, 256, 256  # 6.4 GB in, a copy of 3.2 GB
+    x = torch.randint(-4, 5, (N, IC, H, W), device="cuda", dtype=torch.int8).float()
+    w = torch.randint(-3, 4, (OC, IC, 1, 2), device="cuda", dtype=torch.int8).float()
+    out = torch.empty(N, OC, OH, OW, device="cuda")
+
+    def call():
+        out.zero_()
+        torch.cuda.synchronize()
+        ops.mgpuConv2d(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), None, N, IC, H, W, OC, 1, 2, OH, OW, 0, 0, 0, 0, 8, 8, 1, 1,
+                       False, False, None)
+        rt.mgpuStreamSynchronize(None)
+        return out.clone()
+    expect = call()
+    m.check("conv")
+    assert float(expect.abs().max()) > 0
+    torch.cuda.empty_cache()
+    rt.mgpuPoolTrim()
+    hog = torch.empty(max(torch.cuda.mem_get_info()[0] - (2 << 30), 0), device="cuda", dtype=torch.uint8)
+    try:
+        if earlier_failure:
+            ops.mgpuConv2d(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), None, -1, 0, H, W, OC, 1, 2, 1, 1, 0, 0, 0, 0, 1, 1, 1, 1,
+                           False, False, None)
+            ops.mgpuPool2d(None, None, 1, 1, 4, 4, 3, 3, 2, 2, 0, 0, 0, 0, 2, 2, 0, None)  # bad geometry: sets the status
+            assert rt.mgpuGetLastError() != 0
+        got = call()
+        assert torch.equal(got, expect)
+        assert (rt.mgpuGetLastError() != 0) == earlier_failure
+    finally:
+        rt.mgpuClearLastError()
+        del hog
+        torch.cuda.empty_cache()
+
+
 def test_conv_output_smaller_than_the_geometry(m):
     """The caller may ask for fewer output rows and columns than the padded input would give."""
     rng = np.random.default_rng(3)
