@@ -94,33 +94,33 @@ __device__ __forceinline__ void unpack_res8(const uint32_t *r, float *v) {
   }
 }
 
-// Residual and store of NC finished values of a row, `cols` of which lie inside it: eight at a time where
-// rows allow it, else one by one (static register indices).
-template <typename T16, typename TOut, int NC>
-__device__ __forceinline__ void store_row(TOut *out, const T16 *res, float *v, int cols, bool vec) {
+// Rows that the 32-byte form does not take, NC values of which `cols` lie inside: eight at a time where
+// rows allow it (vec), else one by one (static register indices).  Residuals are loaded ahead of the
+// activation and of every store: loads between the stores would wait one after the other.
+template <typename T16, int NC>
+__device__ __forceinline__ void load_row(const T16 *res, float *rv, int cols, bool vec) {
   if (vec) {
+    uint32_t r[NC / 2] = {};
 #pragma unroll
-    for (int g = 0; g < NC; g += 8) {
-      if (g < cols) {
-        if (res) {
-          uint32_t r[4];
-          float rv[8];
-          ld_global_16B(res + g, r);
-          unpack_res8<T16>(r, rv);
+    for (int g = 0; g < NC; g += 8)
+      if (g < cols) ld_global_16B(res + g, r + g / 2);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[g + j] += rv[j];
-        }
-        store_out8<TOut>(out + g, v + g);
-      }
-    }
+    for (int g = 0; g < NC; g += 8) unpack_res8<T16>(r + g / 2, rv + g);
   } else {
 #pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      if (j < cols) {
-        if (res) v[j] += static_cast<float>(res[j]);
-        out[j] = static_cast<TOut>(v[j]);
-      }
-    }
+    for (int j = 0; j < NC; ++j) rv[j] = j < cols ? static_cast<float>(res[j]) : 0.f;
+  }
+}
+template <typename TOut, int NC>
+__device__ __forceinline__ void store_row(TOut *out, const float *v, int cols, bool vec) {
+  if (vec) {
+#pragma unroll
+    for (int g = 0; g < NC; g += 8)
+      if (g < cols) store_out8<TOut>(out + g, v + g);
+  } else {
+#pragma unroll
+    for (int j = 0; j < NC; ++j)
+      if (j < cols) out[j] = static_cast<TOut>(v[j]);
   }
 }
 

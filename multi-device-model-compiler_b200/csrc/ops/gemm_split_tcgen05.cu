@@ -225,48 +225,48 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       tmem_ld_32x16(t_lane + static_cast<uint32_t>(c), acc);
       const size_t off = static_cast<size_t>(row) * p.N + gcol;
       const int cols = p.N - gcol;
-      float v[NC];
-      if (kWide || p.rows.fast) {
-        float b[NC], rv[NC];
+      float v[NC], rv[NC];  // bias, then the result; residual
 #pragma unroll
-        for (int j = 0; j < NC; ++j) b[j] = rv[j] = 0.f;
-        if (p.bias) {
+      for (int j = 0; j < NC; ++j) v[j] = rv[j] = 0.f;
+      if (p.bias) {
+        if (kWide || p.rows.fast) {
 #pragma unroll
           for (int j = 0; j < NC; j += 4) {
             if (j < cols) {
               const float4 q = __ldg(reinterpret_cast<const float4 *>(p.bias + gcol + j));
-              b[j] = q.x, b[j + 1] = q.y, b[j + 2] = q.z, b[j + 3] = q.w;
+              v[j] = q.x, v[j + 1] = q.y, v[j + 2] = q.z, v[j + 3] = q.w;
             }
           }
-        }
-        if constexpr (kWide) {
-          if (res && row_ok) {
-            uint32_t rr[NC / 2];
-            ld_global_32B(res + off, rr);
+        } else {
 #pragma unroll
-            for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
-          }
-        }
-        tmem_ld_wait_regs(acc);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) v[j] = __uint_as_float(acc[j]) + b[j];
-        act_fast_n<ACT, NC>(v);
-        if constexpr (kWide) {
-#pragma unroll
-          for (int j = 0; j < NC; ++j) v[j] += rv[j];
-        }
-      } else {
-        tmem_ld_wait_regs(acc);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-          v[j] = __uint_as_float(acc[j]);
-          if (p.bias && j < cols) v[j] += __ldg(p.bias + gcol + j);
-          v[j] = act_apply_t<ACT>(v[j]);
+          for (int j = 0; j < NC; ++j)
+            if (j < cols) v[j] = __ldg(p.bias + gcol + j);
         }
       }
+      if (res && row_ok) {
+        if constexpr (kWide) {
+          uint32_t rr[NC / 2];
+          ld_global_32B(res + off, rr);
+#pragma unroll
+          for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
+        } else {
+          load_row<T16, NC>(res + off, rv, cols, p.rows.vec);
+        }
+      }
+      tmem_ld_wait_regs(acc);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] += __uint_as_float(acc[j]);
+      if (kWide || p.rows.fast) {
+        act_fast_n<ACT, NC>(v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) v[j] = act_apply_t<ACT>(v[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] += rv[j];
       if (row_ok) {
         if constexpr (kWide) store_out16<TOut>(out + off, v, cols > 8);
-        else store_row<T16, TOut, NC>(out + off, res ? res + off : nullptr, v, cols, p.rows.vec);
+        else store_row<TOut, NC>(out + off, v, cols, p.rows.vec);
       }
     }
   }

@@ -427,29 +427,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const int gcol = gcol_base + sub * 32, cols = p.N - gcol;
           uint32_t raw[32];
           tmem_ld_32x32(t_base + sub * 32, raw);
-          tmem_ld_wait_regs(raw);
           const size_t off = static_cast<size_t>(row) * p.N + gcol;
-          if (p.rows.vec && cols >= 32) {
+          float v[32], rv[32];
+          if (res && row_ok) load_row<T16, 32>(res + off, rv, cols, p.rows.vec);
 #pragma unroll
-            for (int g = 0; g < 32; g += 8) {
-              float v[8];
+          for (int j = 0; j < 32; ++j) v[j] = p.bias && j < cols ? __ldg(p.bias + gcol + j) : 0.f;
+          tmem_ld_wait_regs(raw);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                v[j] = __uint_as_float(raw[g + j]);
-                if (p.bias) v[j] += __ldg(p.bias + gcol + g + j);
-                v[j] = act_apply_t<ACT>(v[j]);
-              }
-              if (row_ok) store_row<T16, TOut, 8>(out + off + g, res ? res + off + g : nullptr, v, 8, true);
+          for (int j = 0; j < 32; ++j) v[j] = act_apply_t<ACT>(__uint_as_float(raw[j]) + v[j]);
+          if (row_ok) {
+            if (res) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += rv[j];
             }
-          } else {
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] = __uint_as_float(raw[j]);
-              if (p.bias && j < cols) v[j] += __ldg(p.bias + gcol + j);
-              v[j] = act_apply_t<ACT>(v[j]);
-            }
-            if (row_ok) store_row<T16, TOut, 32>(out + off, res ? res + off : nullptr, v, cols, false);
+            store_row<TOut, 32>(out + off, v, cols, p.rows.vec);
           }
         }
       }
