@@ -10,16 +10,16 @@
 //   * K is never cut: an element is one sum over K in order, as in gemm_tcgen05.cu, whatever the
 //     tile.  The tile follows from M, so anything else would let a row's bits depend on the batch
 //     that it is in (a sequence run alone, in a host chunk or on another GPU gives the same bits);
-//   * a ring stage holds `depth` k-blocks, fetched by one TMA instruction per operand and handed
-//     over by one barrier, and the ring is as deep as shared memory allows: a short K range is
-//     in flight as a whole and costs one memory latency;
+//   * a ring stage holds `depth` k-blocks, handed over by one barrier (and fetched by one TMA
+//     instruction per operand where K is a multiple of 64), and the ring is as deep as shared memory
+//     allows: a short K range is in flight as a whole and costs one memory latency;
 //   * A's box is as high as M needs; accumulator rows beyond it hold stale operands and are not
 //     stored;
 //   * W's first stages are requested before the dependency on the previous kernel is resolved
 //     when the caller knows the weights to be complete;
-//   * results go straight from registers to global memory: 32 bytes per access (kWide), or for rows
-//     that are not aligned to that 16 bytes or one element, a variant of its own so that the common
-//     one stays short (as run-time branches they took 2 % of a 12-layer pass over 99 tokens).
+//   * results go straight from registers to global memory, 32 bytes per access.  Rows that are not
+//     aligned to that, and a K that is no multiple of 64, are left to a variant of their own (kWide =
+//     false): as run-time branches they took 2 to 3 % of a 12-layer pass over 99 tokens.
 #include <cstdlib>
 #include <type_traits>
 
@@ -104,21 +104,24 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   pdl_launch_dependents();  // after this CTA holds its tensor memory (see gemm_tcgen05.cu)
 
   // a stage is always filled whole: k-blocks past the last one read as zeros and are not used
-  auto kx = [&](int kb) { return p.k_in_x ? kb * BK : 0; };
-  auto kz = [&](int kb) { return p.k_in_x ? 0 : kb; };
+  auto fetch = [&](uint8_t *dst, const CUtensorMap *map, int s, int row, int kb, int kb_bytes) __attribute__((always_inline)) {
+    auto box = [&](uint8_t *to, int x, int z) __attribute__((always_inline)) {
+      if constexpr (CG == 2) tma_load_3d_cg2(to, map, mapa_u32(smem_u32(&full_bar[s]), 0), x, row, z);
+      else tma_load_3d(to, map, &full_bar[s], x, row, z);
+    };
+    if constexpr (!kWide) {
+      if (p.k_in_x) {  // see encode_operand
+        for (int d = 0; d < depth; ++d) box(dst + d * kb_bytes, (kb + d) * BK, 0);
+        return;
+      }
+    }
+    box(dst, 0, kb);
+  };
   auto load_w = [&](int s, int kb) __attribute__((always_inline)) {
-    uint8_t *sb = tiles + s * stage_bytes + a_bytes;
-    if constexpr (CG == 2)
-      tma_load_3d_cg2(sb, &tmap_b, mapa_u32(smem_u32(&full_bar[s]), 0), kx(kb), col0 + half * b_rows, kz(kb));
-    else
-      tma_load_3d(sb, &tmap_b, &full_bar[s], kx(kb), col0, kz(kb));
+    fetch(tiles + s * stage_bytes + a_bytes, &tmap_b, s, col0 + half * b_rows, kb, b_kb_bytes);
   };
   auto load_a = [&](int s, int kb) __attribute__((always_inline)) {
-    uint8_t *sa = tiles + s * stage_bytes;
-    if constexpr (CG == 2)
-      tma_load_3d_cg2(sa, &tmap_a, mapa_u32(smem_u32(&full_bar[s]), 0), kx(kb), row0, kz(kb));
-    else
-      tma_load_3d(sa, &tmap_a, &full_bar[s], kx(kb), row0, kz(kb));
+    fetch(tiles + s * stage_bytes, &tmap_a, s, row0, kb, a_kb_bytes);
   };
   auto expect = [&](int s) __attribute__((always_inline)) {
     if (leader) mbar_arrive_expect_tx(&full_bar[s], static_cast<uint32_t>(CG * stage_bytes));
@@ -312,11 +315,12 @@ static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const 
 template <typename T16, typename TOut>
 static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int cg, int grid,
                              size_t smem, int act, cudaStream_t s) {
+  const bool wide = p.rows.wide && !p.k_in_x;
 #define MDC_SPLIT(ACT_)                                                                                  \
   do {                                                                                                   \
-    if (cg == 2 && p.rows.wide) launch_split_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s);     \
+    if (cg == 2 && wide) launch_split_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s);            \
     else if (cg == 2) launch_split_cg<T16, TOut, ACT_, 2, false>(ta, tb, p, grid, smem, s);              \
-    else if (p.rows.wide) launch_split_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);           \
+    else if (wide) launch_split_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);                  \
     else launch_split_cg<T16, TOut, ACT_, 1, false>(ta, tb, p, grid, smem, s);                           \
   } while (0)
   switch (act) {
@@ -331,7 +335,8 @@ static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const
 
 // A [rows, Kp] row-major 16-bit matrix.  Kp a multiple of 64: as (64 k, row, k-block), so that one
 // box holds several k-blocks.  Otherwise the last k-block would run into the next row, so the map is
-// (k, row) and ends at Kp, one k-block per box.
+// (k, row) and ends at Kp, one k-block per box and `depth` boxes per stage: the hand-over of a stage
+// costs 0.2 us however it is filled (69 x 141 x 3720: 20.3 us with one k-block a stage, 11.6 with four).
 static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, int64_t rows, int64_t Kp, int box_rows,
                            int depth) {
   const bool blocked = Kp % gsplit::BK == 0;
@@ -364,7 +369,7 @@ void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const
   p.rows = row_access(N, out, dtype_size(out_dtype), residual, bias);
   p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
   p.bn = t.bn, p.box_m = t.box_m, p.stages = t.stages;
-  p.depth = p.k_in_x ? 1 : t.depth;
+  p.depth = t.depth;
   p.tmem_cols = 32;
   while (p.tmem_cols < t.bn) p.tmem_cols *= 2;
   p.w_ready = w_ready ? 1 : 0;

@@ -643,7 +643,7 @@ static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, 
 }
 
 // The fastest one-wave tile for a problem of at most one 128 x 128 tile per SM.
-static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool k_whole, int sms) {
+static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
   GemmTile best;
   float best_us = 1e30f;
   for (int cg = 1; cg <= 2; ++cg)
@@ -653,7 +653,7 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool k_whole, 
       for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
         if (cg == 2 && bn < 64) continue;
         for (int depth : {4, 2, 1}) {
-          if (depth > 1 && (!k_whole || depth > num_kb)) continue;
+          if (depth > num_kb) continue;
           const int steps = (num_kb + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
           // all of an SM's shared memory: the ring has to cover the latency of operands that come out
           // of L2 at 60 - 100 bytes per cycle.  Half of it, so that the next kernel's CTA fits beside
@@ -701,7 +701,7 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   // 4096 x 768 x 3072 19.2 and 17.6.
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
-    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), K % 64 == 0, sms);
+    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), sms);
   if (!t.one_wave) {
     t.cg = choose_cta_group(M);
     t.bn = choose_bn(M, N, t.cg, sms);
