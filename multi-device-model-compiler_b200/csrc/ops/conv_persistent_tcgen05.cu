@@ -538,30 +538,41 @@ void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp
 }
 }  // namespace
 
+// 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks.
+static bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
+
+// A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels only, and
+// the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56, stride 2: 108 us
+// with the whole input rewritten, 65 sampled.)
+static bool conv_sampled(ConvShape &c) {
+  if (conv_gathers(c) || c.KH * c.KW != 1 || (c.SH == 1 && c.SW == 1)) return false;
+  c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
+  return true;
+}
+
+// im2col: first and last window origin relative to the first and last column / row of the image.
+static int64_t conv_upper_w(const ConvShape &c) { return (c.OW - 1) * c.SW - c.PWL - (c.W - 1); }
+static int64_t conv_upper_h(const ConvShape &c) { return (c.OH - 1) * c.SH - c.PHL - (c.H - 1); }
+
+bool conv_persistent_takes(const ConvShape &call) {
+  ConvShape c = call;
+  conv_sampled(c);
+  const int64_t taps = c.KH * c.KW, span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
+  if (c.OC > convp::kMaxOC || taps > 4096 || c.N * c.OH * c.OW * c.OC > (int64_t(1) << 40)) return false;
+  if (conv_gathers(c)) return c.IC * taps <= convp::kMaxGatherK && span_h <= 32767 && span_w <= 32767;
+  // limits of the im2col tensor map: strides, corners and tap offsets
+  const int64_t up_w = conv_upper_w(c), up_h = conv_upper_h(c);
+  return c.SW <= 8 && c.SH <= 8 && c.PWL <= 127 && c.PHL <= 127 && up_w >= -128 && up_w <= 127 && up_h >= -128 &&
+         up_h <= 127 && span_w <= 255 && span_h <= 255 && encode_im2col() != nullptr;
+}
+
 bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   using namespace convp;
-  // A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels
-  // only, and the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56,
-  // stride 2: 108 us with the whole input rewritten, 65 sampled.)
+  if (!conv_persistent_takes(call)) return false;
   ConvShape c = call;
-  const bool sampled = c.IC >= 16 && c.KH * c.KW == 1 && (c.SH > 1 || c.SW > 1);
-  if (sampled) c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
+  const bool sampled = conv_sampled(c), gather = conv_gathers(c);
   const DeviceInfo &di = device_info();
   const int64_t taps = c.KH * c.KW, K = c.IC * taps, M = c.N * c.OH * c.OW;
-  if (c.OC > kMaxOC || taps > 4096 || M * c.OC > (int64_t(1) << 40)) return false;
-  // 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks
-  const bool gather = c.IC < 16;
-  const int64_t span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
-  // im2col: first and last window origin relative to the first and last column / row of the image
-  const int64_t up_w = (c.OW - 1) * c.SW - c.PWL - (c.W - 1), up_h = (c.OH - 1) * c.SH - c.PHL - (c.H - 1);
-  if (gather) {
-    if (K > kMaxGatherK || span_h > 32767 || span_w > 32767) return false;
-  } else {
-    // limits of the im2col tensor map: strides, corners and tap offsets
-    if (c.SW > 8 || c.SH > 8 || c.PWL > 127 || c.PHL > 127 || up_w < -128 || up_w > 127 || up_h < -128 || up_h > 127 ||
-        span_w > 255 || span_h > 255 || !encode_im2col())
-      return false;
-  }
   const int64_t Cp = (c.IC + 7) / 8 * 8, ncb = (c.IC + 63) / 64;
   const int64_t num_kb = gather ? (K + BK - 1) / BK : ncb * taps;
   const int64_t Kp = gather ? (K + 7) / 8 * 8 : num_kb * BK;
@@ -625,7 +636,7 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   if (ok && !gather) {
     const cuuint64_t gdim[4] = {cuuint64_t(Cp), cuuint64_t(c.W), cuuint64_t(c.H), cuuint64_t(c.N)};
     const cuuint64_t gstr[3] = {cuuint64_t(Cp) * 2, cuuint64_t(Cp) * 2 * c.W, cuuint64_t(Cp) * 2 * c.W * c.H};
-    const int lower[2] = {-int(c.PWL), -int(c.PHL)}, upper[2] = {int(up_w), int(up_h)};
+    const int lower[2] = {-int(c.PWL), -int(c.PHL)}, upper[2] = {int(conv_upper_w(c)), int(conv_upper_h(c))};
     const cuuint32_t estr[4] = {1, cuuint32_t(c.SW), cuuint32_t(c.SH), 1};
     ok = encode_im2col()(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, ws + w_bytes, gdim, gstr, lower, upper, BK, BM, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -15,6 +15,9 @@ struct ConvShape {
   bool relu;
 };
 
+// Whether the shape is one that the persistent kernels take.
+bool conv_persistent_takes(const ConvShape &c);
+
 // Runs the convolution on the persistent kernels; false (and nothing launched) when the shape is one
 // that they do not take or there is no memory for their operands.
 bool conv_persistent(const ConvShape &c, cudaStream_t s);

@@ -41,15 +41,16 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
                     uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
 namespace conv {
-// Where the 32 values of group q (k / 32) of a TAP_MAJOR patch come from.
+// Where the 32 values of group q (k / 32) of a TAP_MAJOR patch come from; blocks64: blocks of 64 channels
+// ahead of those of 32.
 struct Group {
   int ic0, tap;
 };
-__host__ __device__ __forceinline__ Group group_at(int q, int IC, int taps) {
-  const int whole = IC / 64 * taps * 2;  // groups of the 64-channel blocks
-  if (q >= whole) return {IC / 64 * 64, q - whole};
-  const int cb = q / (2 * taps), r = q - cb * 2 * taps;
-  return {cb * 64 + (r & 1) * 32, r >> 1};
+__host__ __device__ __forceinline__ Group group_at(int q, int taps, int blocks64) {
+  const int r = q - blocks64 * taps * 2;
+  if (r >= 0) return {blocks64 * 64 + r / taps * 32, r % taps};
+  const int cb = q / (2 * taps), g = q - cb * 2 * taps;
+  return {cb * 64 + (g & 1) * 32, g >> 1};
 }
 
 constexpr int BM = 128;          // output pixels per CTA
@@ -65,6 +66,7 @@ struct Params {
   int IC, H, W, OC, KH, KW, OH, OW, PHL, PWL, SH, SW, DH, DW;
   int M, P, K, num_kb;  // pixels in total, pixels per image, IC*KH*KW, k-blocks
   int bn;               // channels per CTA: 32, 64, 128 or 256
+  int blocks64;         // TAP_MAJOR: see group_at
   int relu;
   uint32_t *err;
 };
@@ -74,11 +76,12 @@ constexpr size_t kMaxSmem = 226 * 1024;  // dynamic part; the static part (barri
 }  // namespace conv
 
 // TAP_MAJOR (IC a multiple of 32): k runs in groups of 32 channels of one filter tap (one bounds test
-// per thread, 32 loads a channel plane apart): the taps of the first 64 channels, two groups each, then
-// those of the next 64, whose input lines are thus re-served by L1 instead of L2, and a last block
-// of 32 channels one group a tap, so a k-block there is two taps and none is half empty (padded to 64
-// channels, 32 x 32 x 56 x 56 -> 64 took 50 us instead of 42).  The additions happen in the
-// order of the persistent im2col kernel.
+// per thread, 32 loads a channel plane apart), the taps of the same channels after one another, whose
+// input lines are thus re-served by L1 instead of L2: all taps of 32 channels, then the next 32.  No
+// k-block holds padding (padded to 64 channels, 32 x 32 x 56 x 56 -> 64 took 50 us instead of 38).
+// A shape that the persistent im2col kernel also takes keeps that kernel's order of additions, blocks of
+// 64 channels as far as they go, so that a call gives the same bits when it ends up here for want of
+// memory; blocks of 32 need less of L1 (37 x 64 x 54 x 175 -> 8, stride 9: 71 us; 64-channel blocks 83).
 // Otherwise k = (ic*KH + kh)*KW + kw (the filter's own order) and every element carries its
 // own tap arithmetic.
 template <bool TAP_MAJOR>
@@ -147,7 +150,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
     auto gather = [&](int kb, float (&v)[32]) __attribute__((always_inline)) {
       const int k0 = kb * BK + half * 32;
       if constexpr (TAP_MAJOR) {
-        const Group g = group_at(kb * 2 + half, p.IC, khw);
+        const Group g = group_at(kb * 2 + half, khw, p.blocks64);
         const int kh = g.tap / p.KW, kw = g.tap - kh * p.KW;
         const int ih = ih0 + kh * p.DH, iw = iw0 + kw * p.DW;
         if (live && k0 < p.K && static_cast<unsigned>(ih) < static_cast<unsigned>(p.H) &&
@@ -324,14 +327,14 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
 
 // OIHW fp32 filter -> fp16 [OC][K] in the k order of the TAP_MAJOR kernel
 __global__ void __launch_bounds__(256) pack_filter_tap_major(const float *__restrict__ w, __half *__restrict__ out,
-                                                             int OC, int IC, int taps) {
+                                                             int OC, int IC, int taps, int blocks64) {
   const int K = IC * taps;
   const int64_t total = static_cast<int64_t>(OC) * K;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t oc = i / K;
     const int k = static_cast<int>(i - oc * K);
-    const conv::Group g = conv::group_at(k >> 5, IC, taps);
+    const conv::Group g = conv::group_at(k >> 5, taps, blocks64);
     out[i] = __float2half_rn(__ldg(w + (oc * IC + g.ic0 + (k & 31)) * taps + g.tap));
   }
 }
@@ -366,12 +369,11 @@ MDC_API void mgpuConv2d(float *input, float *weight, float *bias, float *output,
   if (!device_info().ok) return;
   cudaStream_t s = as_stream(stream);
   // MDC_CONV_DIRECT selects the direct gather for every shape (for comparisons)
-  if (getenv("MDC_CONV_DIRECT") == nullptr) {
-    const ConvShape c{input, weight, bias, hasPostAdd ? postAdd : nullptr, output, N, IC, H, W, OC, KH, KW, OH, OW,
-                      PHL, PWL, SH, SW, DH, DW, hasContainRelu};
-    if (conv_persistent(c, s)) return;
-  }
+  const ConvShape c{input, weight, bias, hasPostAdd ? postAdd : nullptr, output, N, IC, H, W, OC, KH, KW, OH, OW,
+                    PHL, PWL, SH, SW, DH, DW, hasContainRelu};
+  if (getenv("MDC_CONV_DIRECT") == nullptr && conv_persistent(c, s)) return;
   const bool tap_major = IC % 32 == 0;
+  const int blocks64 = conv_persistent_takes(c) ? int(IC / 64) : 0;
   const int64_t Kp = (K + 7) / 8 * 8;  // filter rows padded to 16-byte multiples for TMA
   void *w16 = mgpuMemAllocAsync(static_cast<uint64_t>(OC) * Kp * 2, stream);
   if (!w16) return;
@@ -379,7 +381,7 @@ MDC_API void mgpuConv2d(float *input, float *weight, float *bias, float *output,
     const int64_t total = OC * K;
     const int64_t blocks = (total + 255) / 256;
     pack_filter_tap_major<<<static_cast<unsigned>(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(
-        weight, static_cast<__half *>(w16), int(OC), int(IC), int(KH * KW));
+        weight, static_cast<__half *>(w16), int(OC), int(IC), int(KH * KW), blocks64);
     check_cuda(cudaGetLastError(), "launch pack_filter_tap_major");
     launched("mdc_pack_filter");
   } else {
@@ -398,6 +400,7 @@ MDC_API void mgpuConv2d(float *input, float *weight, float *bias, float *output,
   const int64_t m_tiles = (M + conv::BM - 1) / conv::BM;
   while (p.bn > 64 && m_tiles * ((OC + p.bn - 1) / p.bn) < device_info().sms) p.bn /= 2;
   p.relu = hasContainRelu ? 1 : 0;
+  p.blocks64 = blocks64;
   p.err = device_error_slot();
   CUtensorMap tw;
   // rows beyond OC and k beyond Kp read as zero

@@ -187,6 +187,7 @@ def test_conv_exact_on_small_integers(m):
     (3, 33, 11, 14, 20, 1, 1, (2, 3), (1, 0, 0, 2), (1, 1), True, False),     # strided 1 x 1, padded: sampled copy
     (70, 64, 20, 20, 32, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), False, True),
     (2, 16, 30, 30, 8, 2, 2, (9, 1), (0, 0, 0, 0), (1, 1), False, False),     # stride outside the im2col map: direct kernel
+    (2, 160, 30, 30, 8, 3, 2, (9, 1), (1, 0, 0, 1), (1, 1), True, False),     # the same, 32 channels a block
 ])
 def test_conv_persistent_edges(m, shape):
     """Small integers (see test_conv_exact_on_small_integers): equal bit for bit."""
