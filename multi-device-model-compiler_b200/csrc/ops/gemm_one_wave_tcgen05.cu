@@ -29,14 +29,14 @@
 
 namespace mdc {
 
-namespace gsplit {
+namespace onewave {
 constexpr int BK = 64;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int MAX_STAGES = 16;
-}  // namespace gsplit
+}  // namespace onewave
 
-struct SplitParams {
+struct OneWaveParams {
   int M, N, num_kb;  // num_kb: 64-wide k-blocks
   const float *bias;
   const void *residual;
@@ -51,10 +51,10 @@ struct SplitParams {
 };
 
 template <typename T16, typename TOut, int ACT, int CG, bool kWide>
-__global__ void __launch_bounds__(gsplit::THREADS, 2)
-gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const SplitParams p) {
-  using namespace gsplit;
+__global__ void __launch_bounds__(onewave::THREADS, 1)
+gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                  const OneWaveParams p) {
+  using namespace onewave;
   using namespace ptx;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_bar;
@@ -291,46 +291,46 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 template <typename T16, typename TOut, int ACT, int CG, bool kWide>
-static void launch_split_cg(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int grid, size_t smem,
+static void launch_one_wave_cg(const CUtensorMap &ta, const CUtensorMap &tb, const OneWaveParams &p, int grid, size_t smem,
                             cudaStream_t s) {
-  auto kern = gemm_split_kernel<T16, TOut, ACT, CG, kWide>;
+  auto kern = gemm_one_wave_kernel<T16, TOut, ACT, CG, kWide>;
   constexpr int kMaxDevices = 64;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   const int dev = device_info().device;
   bool &attr_set = attr_set_on[(dev >= 0 && dev < kMaxDevices) ? dev : 0];
   if (!attr_set) {
-    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitMaxSmem),
-                    "cudaFuncSetAttribute(gemm split)"))
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneWaveMaxSmem),
+                    "cudaFuncSetAttribute(gemm one-wave)"))
       return;
     attr_set = true;
   }
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(gsplit::THREADS), smem, s, CG, ta, tb, p),
-               "launch gemm split");
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(onewave::THREADS), smem, s, CG, ta, tb, p),
+               "launch gemm one-wave");
   }
-  launched("gemm_split_kernel");
+  launched("gemm_one_wave_kernel");
 }
 
 template <typename T16, typename TOut>
-static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const SplitParams &p, int cg, int grid,
-                             size_t smem, int act, cudaStream_t s) {
+static void launch_one_wave_act(const CUtensorMap &ta, const CUtensorMap &tb, const OneWaveParams &p, int cg, int grid,
+                                size_t smem, int act, cudaStream_t s) {
   const bool wide = p.rows.wide && !p.k_in_x;
-#define MDC_SPLIT(ACT_)                                                                                  \
-  do {                                                                                                   \
-    if (cg == 2 && wide) launch_split_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s);            \
-    else if (cg == 2) launch_split_cg<T16, TOut, ACT_, 2, false>(ta, tb, p, grid, smem, s);              \
-    else if (wide) launch_split_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);                  \
-    else launch_split_cg<T16, TOut, ACT_, 1, false>(ta, tb, p, grid, smem, s);                           \
+#define MDC_ONE_WAVE(ACT_)                                                                      \
+  do {                                                                                          \
+    if (cg == 2 && wide) launch_one_wave_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s); \
+    else if (cg == 2) launch_one_wave_cg<T16, TOut, ACT_, 2, false>(ta, tb, p, grid, smem, s);   \
+    else if (wide) launch_one_wave_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);       \
+    else launch_one_wave_cg<T16, TOut, ACT_, 1, false>(ta, tb, p, grid, smem, s);                \
   } while (0)
   switch (act) {
-  case MGPU_ACT_NONE: MDC_SPLIT(kActNone); break;
-  case MGPU_ACT_RELU: MDC_SPLIT(kActRelu); break;
-  case MGPU_ACT_GELU_ERF: MDC_SPLIT(kActGeluErf); break;
-  case MGPU_ACT_GELU_TANH: MDC_SPLIT(kActGeluTanh); break;
+  case MGPU_ACT_NONE: MDC_ONE_WAVE(kActNone); break;
+  case MGPU_ACT_RELU: MDC_ONE_WAVE(kActRelu); break;
+  case MGPU_ACT_GELU_ERF: MDC_ONE_WAVE(kActGeluErf); break;
+  case MGPU_ACT_GELU_TANH: MDC_ONE_WAVE(kActGeluTanh); break;
   default: fail("mgpuMatmulEx16: unknown activation");
   }
-#undef MDC_SPLIT
+#undef MDC_ONE_WAVE
 }
 
 // A [rows, Kp] row-major 16-bit matrix.  Kp a multiple of 64: as (64 k, row, k-block), so that one
@@ -339,11 +339,11 @@ static void launch_split_act(const CUtensorMap &ta, const CUtensorMap &tb, const
 // costs 0.2 us however it is filled (69 x 141 x 3720: 20.3 us with one k-block a stage, 11.6 with four).
 static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, int64_t rows, int64_t Kp, int box_rows,
                            int depth) {
-  const bool blocked = Kp % gsplit::BK == 0;
-  const uint64_t gdim[3] = {static_cast<uint64_t>(blocked ? gsplit::BK : Kp), static_cast<uint64_t>(rows),
-                            static_cast<uint64_t>(blocked ? Kp / gsplit::BK : 1)};
-  const uint64_t gstr[2] = {static_cast<uint64_t>(Kp) * 2, gsplit::BK * 2};
-  const uint32_t box[3] = {gsplit::BK, static_cast<uint32_t>(box_rows), static_cast<uint32_t>(blocked ? depth : 1)};
+  const bool blocked = Kp % onewave::BK == 0;
+  const uint64_t gdim[3] = {static_cast<uint64_t>(blocked ? onewave::BK : Kp), static_cast<uint64_t>(rows),
+                            static_cast<uint64_t>(blocked ? Kp / onewave::BK : 1)};
+  const uint64_t gstr[2] = {static_cast<uint64_t>(Kp) * 2, onewave::BK * 2};
+  const uint32_t box[3] = {onewave::BK, static_cast<uint32_t>(box_rows), static_cast<uint32_t>(blocked ? depth : 1)};
   const uint32_t estr[3] = {1, 1, 1};
   const int before = mgpuGetLastError();
   mgpuTensorMapEncodeTiled(map, dtype == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
@@ -353,7 +353,7 @@ static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, in
   return before != 0 || mgpuGetLastError() == 0;
 }
 
-void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,
+void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,
                        void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act,
                        bool w_ready, cudaStream_t s) {
   uint32_t *err = device_error_slot();
@@ -361,10 +361,10 @@ void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const
   CUtensorMap ta, tb;
   if (!encode_operand(&ta, a, dtype, M, Kp, t.box_m, t.depth) || !encode_operand(&tb, w_nk, dtype, N, Kp, t.bn / t.cg, t.depth))
     return;
-  SplitParams p;
+  OneWaveParams p;
   p.M = static_cast<int>(M), p.N = static_cast<int>(N);
-  p.num_kb = static_cast<int>((Kp + gsplit::BK - 1) / gsplit::BK);
-  p.k_in_x = Kp % gsplit::BK != 0;
+  p.num_kb = static_cast<int>((Kp + onewave::BK - 1) / onewave::BK);
+  p.k_in_x = Kp % onewave::BK != 0;
   p.bias = bias, p.residual = residual, p.out = out;
   p.rows = row_access(N, out, dtype_size(out_dtype), residual, bias);
   p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
@@ -376,18 +376,18 @@ void gemm_split_launch(const GemmTile &t, const void *a, const void *w_nk, const
   p.err = err;
   const int64_t m_tiles = (M + static_cast<int64_t>(t.box_m) * t.cg - 1) / (static_cast<int64_t>(t.box_m) * t.cg);
   const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg);
-  const size_t stage = static_cast<size_t>(p.depth) * (t.box_m + t.bn / t.cg) * gsplit::BK * 2;
+  const size_t stage = static_cast<size_t>(p.depth) * (t.box_m + t.bn / t.cg) * onewave::BK * 2;
   // an MMA reads 128 rows of A whatever the box holds: past the last box that must still be this
   // CTA's memory
-  const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * gsplit::BK * 2 : 0);
+  const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * onewave::BK * 2 : 0);
   const size_t smem = ring + 1024;
   if (dtype == MGPU_DTYPE_F16) {
-    if (out_dtype == MGPU_DTYPE_F16) launch_split_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_split_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);
+    if (out_dtype == MGPU_DTYPE_F16) launch_one_wave_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);
     else fail("mgpuMatmulEx16: output type must be the operand type or F32");
   } else {
-    if (out_dtype == MGPU_DTYPE_BF16) launch_split_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, t.cg, grid, smem, act, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_split_act<__nv_bfloat16, float>(ta, tb, p, t.cg, grid, smem, act, s);
+    if (out_dtype == MGPU_DTYPE_BF16) launch_one_wave_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__nv_bfloat16, float>(ta, tb, p, t.cg, grid, smem, act, s);
     else fail("mgpuMatmulEx16: output type must be the operand type or F32");
   }
 }

@@ -621,13 +621,11 @@ static int choose_bn(int64_t M, int64_t N, int cta_group, int sms) {
   return best;
 }
 
-// Time of a one-wave tile in microseconds, fitted to 1700 measured (shape, tile) pairs (M 32 - 4096,
-// N 768 - 4096, K 768 - 4096, weights from HBM, chained launches; 14 % rms).  Terms: launch and drain;
-// MMA issue; operand bytes through the SM's load path; one barrier hand-over per ring stage; epilogue
-// columns; pairing; CTAs to place.  At most one CTA per SM: the tile it
-// picks is then within 4 % (geometric mean; at most 11 %) of the fastest of all measured ones over 13
-// shapes from 16 x 1024 x 2048 to 2048 x 1024 x 4096.  (With two CTAs per SM allowed, each on half the
-// shared memory, it was 27 % off: see the ring below.)
+// Time of a one-wave tile in microseconds, at most one CTA per SM.  Terms: launch and drain; MMA issue;
+// operand bytes through the SM's load path; one barrier hand-over per ring stage; epilogue columns;
+// pairing; CTAs to place.  Fitted to 1700 measured (shape, tile) pairs (M 32 - 4096, N 768 - 4096, K 768
+// - 4096, weights from HBM, chained launches; 14 % rms), an extrapolation elsewhere: over 140 random
+// calls (M 1 - 40000, N and K 8 - 5000) none was slower than with the persistent kernel for every shape.
 static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, int sms) {
   const int64_t m_tiles = (M + t.box_m * t.cg - 1) / (t.box_m * t.cg), n_tiles = (N + t.bn - 1) / t.bn;
   const int64_t ctas = m_tiles * n_tiles * t.cg;
@@ -657,9 +655,9 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
           const int steps = (num_kb + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
           // all of an SM's shared memory: the ring has to cover the latency of operands that come out
           // of L2 at 60 - 100 bytes per cycle.  Half of it, so that the next kernel's CTA fits beside
-          // this one, loses more than that overlap wins: 2048 x 1024 x 4096 29.1 -> 19.6 us,
-          // 1000 x 1024 x 4096 18.6 -> 15.2, 99 x 768 x 3072 7.9 -> 7.2; a 12-layer pass over 99 tokens,
-          // where every kernel is of this kind, 468 -> 432 us.
+          // this one, loses more than that overlap wins: 2048 x 1024 x 4096 31.7 -> 22.0 us,
+          // 1000 x 1024 x 4096 25.8 -> 18.0, 99 x 768 x 3072 11.7 -> 10.5; a 12-layer pass over 99 tokens,
+          // where every kernel is of this kind, 501 -> 450 us.
           int stages = (220 * 1024 - (128 - box_m) * 128) / stage;
           if (stages > steps) stages = steps;
           if (stages > 16) stages = 16;
@@ -675,16 +673,6 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
 }
 
 GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
-#ifdef MDC_SWEEP
-  if (const char *e = getenv("MDC_GEMM_TILE")) {
-    GemmTile t;
-    int ow = 0;
-    if (sscanf(e, "%d,%d,%d,%d,%d,%d", &ow, &t.cg, &t.box_m, &t.bn, &t.depth, &t.stages) == 6) {
-      t.one_wave = ow != 0;
-      return t;
-    }
-  }
-#endif
   // the choice takes a few microseconds: kept per shape (a plan, not a result)
   struct Entry {
     int64_t M = -1, N = -1, K = -1;
@@ -743,7 +731,7 @@ static void matmul16_launch(const char *who, const void *a, const void *w_nk, co
 
   const GemmTile tile = choose_gemm_tile(M, N, Kp, di.sms);
   if (tile.one_wave) {
-    gemm_split_launch(tile, a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, s);
+    gemm_one_wave_launch(tile, a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, s);
     return;
   }
   const int cta_group = tile.cg, bn = tile.bn;

@@ -280,9 +280,6 @@ __device__ __forceinline__ void umma_commit_warp(uint64_t *bar) {
       "}\n" ::"r"(smem_u32(bar))
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 // Same wait, but naming the destination registers of the load it completes: the compiler
 // must then keep every use of them after this point (the load fills them asynchronously).
 __device__ __forceinline__ void tmem_ld_wait_regs(uint32_t (&r)[32]) {

@@ -88,9 +88,9 @@ def test_conv_wide_channel_tiles(m, OC):
 
 
 def test_conv_gather_modes_agree(m):
-    """Channel counts that are multiples of 32 are served either by the direct gather or by the
-    shared-memory staged one; both feed the tensor core the same operands in the same order, so
-    the results are bit-identical."""
+    """Channel counts that are multiples of 32 are served by the im2col kernel or, without memory for
+    its copy of the input, by the direct gather; both feed the tensor core the same operands in the
+    same order, so the results are bit-identical."""
     import os
     rng = np.random.default_rng(21)
     cases = [((4, 64, 14, 14), (96, 64, 3, 3), dict(pad=(1, 1, 1, 1))),

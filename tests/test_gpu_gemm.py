@@ -134,12 +134,12 @@ def test_narrow_tiles_are_exact(m, M, N, K):
 
 @pytest.mark.parametrize("M,N,K", [
     (1, 16, 8), (33, 48, 64), (65, 2304, 768),     # rows around a box, one stage, whole K in the ring
-    (99, 768, 3072), (250, 768, 4096), (640, 192, 1024),  # K cut over a cluster
-    (641, 1000, 1032),                             # ragged K: one k-block per box
+    (99, 768, 3072), (250, 768, 4096), (640, 192, 1024),  # long K: the ring goes round
+    (641, 1000, 1032), (5, 24, 72), (70, 40, 200), # ragged K: a box per k-block, the last stage partly past K
     (1024, 2304, 768), (2048, 768, 3072), (100, 77, 2048)])
 def test_one_wave_tiles_are_exact(m, M, N, K):
     # small integers: fp16 products and fp32 sums are exact in any order of summation, so a wrong
-    # tile, slice or partial sum is a hard mismatch (|sum| <= 4096 * 6 < 2^24)
+    # tile or stage is a hard mismatch (|sum| <= 4096 * 6 < 2^24)
     rng = np.random.default_rng(11)
     a = rng.integers(-3, 4, (M, K)).astype(np.float32)
     w = rng.integers(-2, 3, (K, N)).astype(np.float32)
