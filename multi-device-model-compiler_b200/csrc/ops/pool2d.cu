@@ -14,6 +14,7 @@
 
 #include "fast_div.h"
 #include "ops_common.h"
+#include "pool_slices.h"
 
 namespace mdc {
 namespace {
@@ -138,21 +139,15 @@ MDC_API void mgpuPool2d(float *input, float *output, int64_t N, int64_t C, int64
   const bool tiled = PHL == 0 && PWL == 0 && KW == SW && (KW == 4 || KW == 2) && W % KW == 0 &&
                      (OH - 1) * SH + KH <= H && OW * KW <= W &&
                      reinterpret_cast<uintptr_t>(input) % (KW * 4) == 0;
-  // Output indices are 31 bits: larger tensors go in slices, of whole planes or, for a plane of more
-  // than 2^30 outputs, of its rows.
-  const int64_t planes = N * C, per = OH * OW, limit = int64_t(1) << 30;
-  const int64_t plane_step = per <= limit ? limit / per : 1;
-  const int64_t row_step = per <= limit ? OH : (OW < limit ? limit / OW : 1);
-  for (int64_t p0 = 0; p0 < planes; p0 += plane_step)
-    for (int64_t r0 = 0; r0 < OH; r0 += row_step) {
-      const int64_t rows = OH - r0 < row_step ? OH - r0 : row_step;
-      g.oh0 = int(r0), g.by_oh = Divisor(rows);
-      g.total = int((planes - p0 < plane_step ? planes - p0 : plane_step) * rows * OW);
-      const float *x = input + p0 * H * W;
-      float *y = output + p0 * per + r0 * OW;
-      if (method == 1) launch_pool<true>(x, y, g, tiled, s);
-      else launch_pool<false>(x, y, g, tiled, s);
-    }
+  // output indices are 31 bits
+  for_each_pool_slice(N * C, OH, OW, int64_t(1) << 30, [&](const PoolSlice &p) {
+    g.oh0 = int(p.row0), g.by_oh = Divisor(p.rows);
+    g.total = int(p.planes * p.rows * OW);
+    const float *x = input + p.plane0 * H * W;
+    float *y = output + p.plane0 * OH * OW + p.row0 * OW;
+    if (method == 1) launch_pool<true>(x, y, g, tiled, s);
+    else launch_pool<false>(x, y, g, tiled, s);
+  });
   check_cuda(cudaGetLastError(), "launch pool2d");
   launched("mdc_pool2d");
 }

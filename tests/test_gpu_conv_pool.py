@@ -306,6 +306,38 @@ def test_pool_against_oracle(m, case, method):
         assert np.max(np.abs(got - ref)) <= 1e-6 * max(1.0, kernel[0] * kernel[1] / 9)
 
 
+@pytest.mark.parametrize("case", [
+    # H, W, kernel, stride, pad(t,l,b,r)
+    (9, 11, (2, 2), (2, 2), (0, 0, 0, 0)),    # odd width: compiled 2 x 2 instead of row vectors
+    (8, 10, (2, 2), (1, 1), (0, 0, 0, 0)),
+    (8, 10, (2, 2), (2, 2), (1, 0, 0, 1)),    # windows cut by the padding on one side
+    (13, 18, (4, 4), (2, 2), (0, 0, 0, 0)),   # overlapping 4 x 4
+    (14, 15, (4, 4), (4, 4), (2, 1, 0, 3)),
+    (9, 12, (3, 2), (2, 2), (0, 0, 0, 0)),    # row vectors under a window of another height
+    (15, 16, (3, 4), (1, 4), (0, 0, 0, 0)),
+    (12, 12, (5, 3), (2, 3), (1, 2, 3, 0)),   # run-time window
+    (4, 4, (4, 4), (4, 4), (0, 0, 0, 0)),     # one output a plane
+])
+@pytest.mark.parametrize("method", [0, 1])
+@pytest.mark.parametrize("offset", [0, 1])    # floats that the input lies off its allocation
+def test_pool_kernel_forms(m, case, method, offset):
+    H, W, kernel, stride, pad = case
+    rng = np.random.default_rng(H * W + kernel[0])
+    planes = 7
+    x = rng.standard_normal((1, planes, H, W)).astype(np.float32)
+    ref = oracle.pool2d(x, kernel, stride, pad=pad, method=method)
+    OH, OW = ref.shape[2:]
+    dx = m.to_device(np.concatenate([np.zeros(offset, np.float32), x.ravel()]))
+    dy = m.DeviceBuffer(ref.nbytes)
+    m.ops().mgpuPool2d(dx.ptr + 4 * offset, dy.ptr, 1, planes, H, W, OH, OW, kernel[0], kernel[1], *pad, stride[0], stride[1], method, None)
+    got = m.to_host(dy, ref.shape, np.float32)
+    m.check("pool")
+    if method == 0:
+        assert np.array_equal(got, ref)
+    else:
+        assert np.max(np.abs(got - ref)) <= 1e-6 * max(1.0, kernel[0] * kernel[1] / 9)
+
+
 def test_pool_special_values(m):
     x = np.zeros((1, 1, 4, 4), np.float32)
     x[0, 0, 0, 0] = -np.inf
