@@ -62,9 +62,9 @@ def bytes_touched_per_step(batch):
 # residual, output) scaled and the weights kept.
 GEMM_DRAM_TRAFFIC = {
     # tokens: {shape: bytes}
-    32768: {"gemm_qkv": 53925888 + 96961536, "gemm_proj": 51560192 + 10394880,
-            "gemm_ffn1": 55139072 + 143000064, "gemm_ffn2": 206767872 + 37095936},
-    4096: {"gemm_qkv": 9883904, "gemm_proj": 7518208, "gemm_ffn1": 11096832, "gemm_ffn2": 29931520 + 1280},
+    32768: {"gemm_qkv": 53904640 + 99526400, "gemm_proj": 51540224 + 11512576,
+            "gemm_ffn1": 55092992 + 148391424, "gemm_ffn2": 206821632 + 36534272},
+    4096: {"gemm_qkv": 9863168, "gemm_proj": 7498240, "gemm_ffn1": 11051264, "gemm_ffn2": 29911296},
 }
 
 

@@ -33,7 +33,9 @@ enum { MGPU_ACT_NONE = 0, MGPU_ACT_RELU = 1, MGPU_ACT_GELU_ERF = 2, MGPU_ACT_GEL
 /* include/multi-device-model-compiler/Kernels/GPU/Ops.h:23-25, lib/Kernels/GPU/Ops.cu:59-120.
  * output[M,N] = input[M,K] . weight[K,N] + bias[N]; all row-major fp32.  Operands are
  * rounded to fp16 for the tensor cores, accumulation is fp32 (the reference asks cuBLASLt
- * for CUBLAS_COMPUTE_32F_FAST_16F, Ops.cu:74-75); bias and output stay fp32. */
+ * for CUBLAS_COMPUTE_32F_FAST_16F, Ops.cu:74-75); bias and output stay fp32.  Every element is
+ * one sum over K in one order, whatever M and N are: a row's result is the same, bit for bit, in a
+ * batch of any size. */
 void mgpuMatmul(float *input, float *weight, float *bias, float *output, int64_t M, int64_t N,
                 int64_t K, mgpu_cuda_stream_t stream);
 
@@ -116,7 +118,10 @@ void mgpuPackWeight(const float *weight_kn, void *packed_nk, int64_t K, int64_t 
  * out[M,N] = act(a[M,Kp] . w[N,Kp]^T + bias[N]) + residual[M,N].
  * a and w are `dtype` (F16 or BF16) with Kp (a multiple of 8) contiguous; bias is fp32 or
  * NULL; residual is `dtype` or NULL; out is `out_dtype`.  Generalises mgpuMatmulEx<half>
- * (Ops.h:51-55, lib/Kernels/GPU/Ops.cu:136-234), which accumulated in fp16. */
+ * (Ops.h:51-55, lib/Kernels/GPU/Ops.cu:136-234), which accumulated in fp16.  A row's result does
+ * not depend on M, as in mgpuMatmul.  Any alignment and width is taken; rows of out and residual that
+ * are multiples of 16 bytes (N % 8 == 0) on 16-byte boundaries, with the bias on one too, are the fast
+ * ones. */
 void mgpuMatmulEx16(const void *a, const void *w_nk, const float *bias, const void *residual,
                     void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype,
                     int32_t act, mgpu_cuda_stream_t stream);

@@ -19,11 +19,13 @@
 //
 // Bound: bytes (input once, output once) for few channels, L2 -> shared memory bandwidth of the
 // patch loads (each input element once per tap) for many.
-// Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after:
-//   16 x 3 x 256 x 256 -> 64, 3 x 3                      220 ->  77 us (43 of HBM time)
-//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        77 ->  40 us
-//   26 x 352 x 37 x 46 -> 32, 3 x 3                      161 ->  81 us
-//   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            114 ->  34 us
+// Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
+// changing from call to call:
+//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  73 us (43 of HBM time)
+//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        74 ->  34 us
+// L2 flushed between calls:
+//   26 x 352 x 37 x 46 -> 32, 3 x 3                      155 ->  81 us
+//   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            116 ->  34 us
 //   1 x 128 x 16 x 25 -> 64, 3 x 3                        34 ->  17 us
 // The gather was bound by instruction issue: run-time divisions and per-channel tests in the
 // epilogue, 2.7 us a tile of 128 x 64; with multiplicative division, whole-group stores and the
