@@ -81,7 +81,7 @@ constexpr size_t kMaxSmem = 226 * 1024;  // dynamic part; the static part (barri
 // k-block holds padding (padded to 64 channels, 32 x 32 x 56 x 56 -> 64 took 50 us instead of 38).
 // A shape that the persistent im2col kernel also takes keeps that kernel's order of additions, blocks of
 // 64 channels as far as they go, so that a call gives the same bits when it ends up here for want of
-// memory; blocks of 32 need less of L1 (37 x 64 x 54 x 175 -> 8, stride 9: 71 us; 64-channel blocks 83).
+// memory; blocks of 32 need less of L1 (37 x 64 x 54 x 175 -> 8, stride 9: 69 us; 64-channel blocks 81).
 // Otherwise k = (ic*KH + kh)*KW + kw (the filter's own order) and every element carries its
 // own tap arithmetic.
 template <bool TAP_MAJOR>
