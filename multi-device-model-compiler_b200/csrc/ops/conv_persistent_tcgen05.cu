@@ -279,7 +279,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         const uint64_t ad = a0 + static_cast<uint64_t>(stage * (stage_bytes / 16));
         const uint64_t bd = p.resident ? f0 + static_cast<uint64_t>(kb * (b_bytes / 16)) : ad + A_BYTES / 16;
         if (kb < partial_from) {
-          umma_f16_ss_kblock(d, ad, bd, idesc, kb != 0 ? 1u : 0u);
+          umma_f16_ss_kblocks<1, 1>(d, kblock_desc(ad, bd), idesc, kb != 0 ? 1u : 0u);
         } else {
           for (int k = 0; k < partial_steps; ++k)
             umma_f16_ss_warp(d, ad + static_cast<uint64_t>(2 * k), bd + static_cast<uint64_t>(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);

@@ -163,7 +163,9 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (leader) {
       const uint32_t idesc = make_idesc_f16(128 * CG, static_cast<uint32_t>(p.bn), std::is_same<T16, __nv_bfloat16>::value,
                                             false, false);
-      const uint64_t desc0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
+      const KblockDesc desc0 = kblock_desc(make_smem_desc_sw128(smem_u32(tiles), 16, 1024),
+                                           make_smem_desc_sw128(smem_u32(tiles) + static_cast<uint32_t>(a_bytes), 16, 1024));
+      const uint32_t a_kb16 = static_cast<uint32_t>(a_kb_bytes) >> 4, b_kb16 = static_cast<uint32_t>(b_kb_bytes) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -174,14 +176,17 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           break;
         }
         tc_fence_after();
-        uint64_t a_desc = desc0 + static_cast<uint64_t>((stage * stage_bytes) >> 4);
-        uint64_t b_desc = a_desc + static_cast<uint64_t>(a_bytes >> 4);
+        KblockDesc kd = desc0;
+        kd.a_lo += static_cast<uint32_t>(stage * stage_bytes) >> 4;
+        kd.b_lo += static_cast<uint32_t>(stage * stage_bytes) >> 4;
         const int n = min(depth, p.num_kb - i * depth);
-        for (int d = 0; d < n; ++d) {
-          if constexpr (CG == 2) umma_f16_ss_kblock_cg2(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
-          else umma_f16_ss_kblock(tmem_base, a_desc, b_desc, idesc, (i | d) != 0 ? 1u : 0u);
-          a_desc += static_cast<uint64_t>(a_kb_bytes >> 4);
-          b_desc += static_cast<uint64_t>(b_kb_bytes >> 4);
+        if (n == 4) {
+          umma_f16_ss_kblocks<CG, 4>(tmem_base, kd, idesc, i != 0 ? 1u : 0u, a_kb16, b_kb16);
+        } else {
+          for (int d = 0; d < n; ++d) {
+            umma_f16_ss_kblocks<CG, 1>(tmem_base, kd, idesc, (i | d) != 0 ? 1u : 0u);
+            kd.a_lo += a_kb16, kd.b_lo += b_kb16;
+          }
         }
         if constexpr (CG == 2) umma_commit_cg2_warp(&empty_bar[stage], 3);
         else umma_commit_warp(&empty_bar[stage]);

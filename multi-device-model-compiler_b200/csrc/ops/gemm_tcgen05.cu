@@ -218,8 +218,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           // (descriptors hold addresses in units of 16 bytes)
           const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
           const uint64_t b_desc = a_desc + A_BYTES / 16;
-          if constexpr (CG == 2) umma_f16_ss_kblock_cg2(d_tmem, a_desc, b_desc, idesc, kb != 0 ? 1u : 0u);
-          else umma_f16_ss_kblock(d_tmem, a_desc, b_desc, idesc, kb != 0 ? 1u : 0u);
+          umma_f16_ss_kblocks<CG, 1>(d_tmem, kblock_desc(a_desc, b_desc), idesc, kb != 0 ? 1u : 0u);
           // the stage is reusable (in both CTAs) once these MMAs have read it
           if constexpr (CG == 2) {
             umma_commit_cg2_warp(&empty_bar[stage], 3);

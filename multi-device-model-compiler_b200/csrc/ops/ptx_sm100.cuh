@@ -216,30 +216,73 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One 64-wide k-block (four MMAs, 32 bytes apart along the swizzled rows), called by a whole warp
-// and issued by its elected lane; only the first MMA may start a new accumulation.
-__device__ __forceinline__ void umma_f16_ss_kblock(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                   uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, e;\n"
-      ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
-      "add.s64 a1, %1, 2;\n"
-      "add.s64 b1, %2, 2;\n"
-      "add.s64 a2, %1, 4;\n"
-      "add.s64 b2, %2, 4;\n"
-      "add.s64 a3, %1, 6;\n"
-      "add.s64 b3, %2, 6;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n"
-      "}\n"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// Two operand descriptors of 64-wide k-blocks: their low words move, the high ones are constant.
+struct KblockDesc {
+  uint32_t a_lo, a_hi, b_lo, b_hi;
+};
+__device__ __forceinline__ KblockDesc kblock_desc(uint64_t a, uint64_t b) {
+  return {static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), static_cast<uint32_t>(b), static_cast<uint32_t>(b >> 32)};
 }
+// NKB (one or four) k-blocks of 64, four MMAs each, called by a whole warp and issued by its elected lane;
+// only the first MMA may start a new accumulation.  Along a k-block the operands advance by two units of
+// 16 bytes (32 bytes of a swizzled row), from one k-block to the next by a_kb / b_kb units.
+// A tile of few columns is bound by this warp's instructions, not by the tensor pipe: 32-bit address
+// arithmetic and four k-blocks per election instead of 64-bit adds and an election each.
+#define MDC_KBLOCK(CGS, A, B, P)                                             \
+  "add.u32 x1, " A ", 2;\n"                                                  \
+  "add.u32 y1, " B ", 2;\n"                                                  \
+  "add.u32 x2, " A ", 4;\n"                                                  \
+  "add.u32 y2, " B ", 4;\n"                                                  \
+  "add.u32 x3, " A ", 6;\n"                                                  \
+  "add.u32 y3, " B ", 6;\n"                                                  \
+  "mov.b64 da, {" A ", %2};\n"                                               \
+  "mov.b64 db, {" B ", %4};\n"                                               \
+  "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, " P ";\n"   \
+  "mov.b64 da, {x1, %2};\n"                                                  \
+  "mov.b64 db, {y1, %4};\n"                                                  \
+  "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, 1;\n"       \
+  "mov.b64 da, {x2, %2};\n"                                                  \
+  "mov.b64 db, {y2, %4};\n"                                                  \
+  "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, 1;\n"       \
+  "mov.b64 da, {x3, %2};\n"                                                  \
+  "mov.b64 db, {y3, %4};\n"                                                  \
+  "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, 1;\n"
+#define MDC_KBLOCKS_1(CGS)                                                   \
+  "{\n"                                                                      \
+  ".reg .pred p, e;\n"                                                       \
+  ".reg .b32 x1, x2, x3, y1, y2, y3;\n"                                      \
+  ".reg .b64 da, db;\n"                                                      \
+  "elect.sync _|e, 0xffffffff;\n"                                            \
+  "setp.ne.b32 p, %6, 0;\n" MDC_KBLOCK(CGS, "%1", "%3", "p") "}\n"
+#define MDC_KBLOCKS_4(CGS)                                                   \
+  "{\n"                                                                      \
+  ".reg .pred p, e;\n"                                                       \
+  ".reg .b32 x1, x2, x3, y1, y2, y3, ka1, ka2, ka3, kb1, kb2, kb3;\n"        \
+  ".reg .b64 da, db;\n"                                                      \
+  "elect.sync _|e, 0xffffffff;\n"                                            \
+  "setp.ne.b32 p, %6, 0;\n"                                                  \
+  "add.u32 ka1, %1, %7;\n"                                                   \
+  "add.u32 kb1, %3, %8;\n"                                                   \
+  "add.u32 ka2, ka1, %7;\n"                                                  \
+  "add.u32 kb2, kb1, %8;\n"                                                  \
+  "add.u32 ka3, ka2, %7;\n"                                                  \
+  "add.u32 kb3, kb2, %8;\n" MDC_KBLOCK(CGS, "%1", "%3", "p")                 \
+  MDC_KBLOCK(CGS, "ka1", "kb1", "1") MDC_KBLOCK(CGS, "ka2", "kb2", "1") MDC_KBLOCK(CGS, "ka3", "kb3", "1") "}\n"
+template <int CG, int NKB>
+__device__ __forceinline__ void umma_f16_ss_kblocks(uint32_t d_tmem, const KblockDesc &d, uint32_t idesc, uint32_t accumulate,
+                                                    uint32_t a_kb = 0, uint32_t b_kb = 0) {
+  static_assert((CG == 1 || CG == 2) && (NKB == 1 || NKB == 4), "");
+#define MDC_KBLOCK_ARGS \
+  "r"(d_tmem), "r"(d.a_lo), "r"(d.a_hi), "r"(d.b_lo), "r"(d.b_hi), "r"(idesc), "r"(accumulate), "r"(a_kb), "r"(b_kb) : "memory"
+  if constexpr (CG == 1 && NKB == 1) asm volatile(MDC_KBLOCKS_1("1")::MDC_KBLOCK_ARGS);
+  else if constexpr (CG == 1) asm volatile(MDC_KBLOCKS_4("1")::MDC_KBLOCK_ARGS);
+  else if constexpr (NKB == 1) asm volatile(MDC_KBLOCKS_1("2")::MDC_KBLOCK_ARGS);
+  else asm volatile(MDC_KBLOCKS_4("2")::MDC_KBLOCK_ARGS);
+#undef MDC_KBLOCK_ARGS
+}
+#undef MDC_KBLOCK
+#undef MDC_KBLOCKS_1
+#undef MDC_KBLOCKS_4
 // One K = 16 step, called by a whole warp and issued by its elected lane.
 __device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate) {
@@ -405,29 +448,6 @@ __device__ __forceinline__ void tmem_relinquish_cg2() {
 __device__ __forceinline__ void tmem_dealloc_cg2(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
-}
-// the same k-block for a CTA pair
-__device__ __forceinline__ void umma_f16_ss_kblock_cg2(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                   uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, e;\n"
-      ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
-      "add.s64 a1, %1, 2;\n"
-      "add.s64 b1, %2, 2;\n"
-      "add.s64 a2, %1, 4;\n"
-      "add.s64 b2, %2, 4;\n"
-      "add.s64 a3, %1, 6;\n"
-      "add.s64 b3, %2, 6;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n"
-      "}\n"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 // arrives on the barrier at this shared-memory offset in every CTA of `cta_mask` once the pair's
 // MMAs issued so far have completed; called by a whole warp
