@@ -197,15 +197,16 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 constexpr int64_t kCastItems = OperandList::kCastItems, kPadItems = OperandList::kPadItems;
 struct OperandJobs {
   OperandList::Job j[OperandList::kMax];
-  int n;
+  int n, late;
 };
 
 template <typename T16>
 __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const OperandJobs jobs) {
   static_assert(kEwBlock == OperandList::kThreads, "the 64 x 64 tiles are walked by 256 threads");
   __shared__ float tile[64][65];
-  pdl_launch_dependents();
+  if (!jobs.late) pdl_launch_dependents();
   pdl_wait();
+  if (jobs.late) pdl_launch_dependents();
   OperandList::Job job = jobs.j[0];
 #pragma unroll
   for (int i = 1; i < OperandList::kMax; ++i)
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
   }
 }
 
-void OperandList::launch(int32_t dtype, void *stream) {
+void OperandList::launch(int32_t dtype, void *stream, bool late) {
   if (n == 0) return;
   if (overflow || blocks > 0x7fffffff) {
     fail(overflow ? "operand conversion: more operands than a call may have" : "operand conversion: shape too large");
@@ -296,7 +297,7 @@ void OperandList::launch(int32_t dtype, void *stream) {
   }
   OperandJobs a;
   for (int i = 0; i < kMax; ++i) a.j[i] = jobs[i < n ? i : 0];
-  a.n = n;
+  a.n = n, a.late = late ? 1 : 0;
   cudaStream_t s = as_stream(stream);
   ProfileScope prof(kCatElementwise, s);
   const dim3 grid(static_cast<unsigned>(blocks));

@@ -1,0 +1,277 @@
+// Tensor-core Gemm for a few rows against an fp32 weight as the caller has it: out[M, N] = A[M, Kp] . W[K, N]
+// + bias[N], M <= 64, A fp16, W fp32 rounded to fp16 on its way into shared memory, fp32 accumulation.
+//
+// With few rows every weight is used once, by one CTA, so a 16-bit copy in memory would only be written
+// to be read back, and this kernel is bound by the bytes of W (4 K N) or, where those are few, by
+// latency.  Eight warps read W straight into registers, 16 vector loads of a thread in flight (64 KB an
+// SM); a warp fills a ring stage of 128 k x 16 columns or 64 k x 32 by itself, converting to core
+// matrices of 8 columns x 8 k.  A comes by TMA.  W does not wait for the kernel that converts A: that
+// kernel lets this one start after its own wait, so what is older than it is complete.
+//
+// Whole call, before (conversion of W, of A, one-wave Gemm) and after: 16 x 1000 x 2048 14.2 -> 9.3 us one
+// after another; cold inputs: 16 x 4096 x 4096 44 -> 27.6 (2.4 TB/s), 48 x 1408 x 577 19.5 -> 13.3, 16 x 768 x 320
+// 13.4 -> 9.2.  Sixteen loading warps instead of eight: 10.9 for the first.
+//
+// K order: one sum over K in steps of 16, as in the other Gemm kernels; a row's bits do not depend on
+// which of them takes a call.
+#include "gemm_common.cuh"
+#include "gemm_plan.h"
+#include "ops_common.h"
+
+namespace mdc {
+bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
+                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
+
+namespace fewrows {
+constexpr int LOAD_WARPS = 8;
+constexpr int THREADS = 64 + LOAD_WARPS * 32;
+constexpr int MAX_STAGES = 24;
+// Columns in groups of eight, k in groups of eight: 128-byte core matrices.  They lie 144 bytes apart along the
+// columns, which puts the eight 16-byte stores of a quarter-warp on different banks.
+constexpr int SBO = 144;
+template <int BN>
+struct Cfg {
+  static constexpr int STAGE_K = 2048 / BN;                      // a warp's 16 loads of 4 values per lane
+  static constexpr int LBO = BN == 16 ? 288 : 4 * SBO;           // bytes from one group of eight k to the next
+  static constexpr int B_BYTES = STAGE_K / 8 * LBO;              // 4608
+};
+}  // namespace fewrows
+
+struct FewRowsParams {
+  const float *w, *bias;
+  float *out;
+  int M, N, K;
+  int box_m, stages, steps;  // steps: stages' worth of K
+  int w_vec, out_vec;        // rows of W / of out and the bias in 16-byte vectors
+  uint32_t *err;
+};
+
+template <int BN>
+__global__ void __launch_bounds__(fewrows::THREADS, 1)
+gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsParams p) {
+  using namespace fewrows;
+  using namespace ptx;
+  using C = Cfg<BN>;
+  constexpr int KBS = C::STAGE_K / 64;  // 64-wide k-blocks of A per stage
+  extern __shared__ uint8_t smem_dyn[];
+  __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_bar;
+  __shared__ uint32_t tmem_slot, abort_flag_s;
+  volatile uint32_t *abort_flag = &abort_flag_s;
+  uint8_t *a_s = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int a_kb = p.box_m * 128, a_bytes = KBS * a_kb;
+  // an MMA reads 128 rows of A whatever the box holds: what follows the last stage's A is W's part
+  uint8_t *b_s = a_s + p.stages * a_bytes + (128 - p.box_m) * 128;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col0 = blockIdx.x * BN;
+
+  if (threadIdx.x == 0) {
+    abort_flag_s = 0;
+    tma_prefetch_desc(&tmap_a);
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full_bar[s], 2);  // A's bytes, and the warp that brings W
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_bar, 1);
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, 32);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_launch_dependents();  // after this CTA holds its tensor memory (see gemm_tcgen05.cu)
+
+  if (warp == 0) {
+    // ------------------------------ A ------------------------------
+    pdl_wait();
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < p.steps; ++i) {
+      if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x91000000u | static_cast<uint32_t>(stage));
+        break;
+      }
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(a_bytes));
+#pragma unroll
+        for (int kb = 0; kb < KBS; ++kb)
+          tma_load_2d(a_s + stage * a_bytes + kb * a_kb, &tmap_a, &full_bar[stage], (i * KBS + kb) * 64, 0);
+      }
+      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer ------------------------------
+    const uint32_t idesc = make_idesc_f16(128, BN, false, false, false);
+    const uint64_t a0 = make_smem_desc_sw128(smem_u32(a_s), 16, 1024);
+    // no swizzle (see make_smem_desc_sw128 for the fields)
+    const uint64_t b0 = static_cast<uint64_t>(smem_u32(b_s) >> 4) | static_cast<uint64_t>(C::LBO / 16) << 16 |
+                        static_cast<uint64_t>(SBO / 16) << 32 | static_cast<uint64_t>(1) << 46;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int i = 0; i < p.steps; ++i) {
+      if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x92000000u | static_cast<uint32_t>(stage));
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const uint64_t ad = a0 + static_cast<uint64_t>(stage * (a_bytes >> 4)), bd = b0 + static_cast<uint64_t>(stage * (C::B_BYTES >> 4));
+#pragma unroll
+      for (int kb = 0; kb < KBS; ++kb)
+        umma_f16_ss_kblocks<1, 1, 2 * C::LBO / 16>(tmem_base, kblock_desc(ad + static_cast<uint64_t>(kb * (a_kb >> 4)),
+                                                                         bd + static_cast<uint64_t>(kb * (8 * C::LBO >> 4))),
+                                                  idesc, (i | kb) != 0 ? 1u : 0u);
+      umma_commit_warp(&empty_bar[stage]);
+      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+    }
+    if (ok) umma_commit_warp(&acc_bar);
+  } else {
+    // ------------------------------ W, then the epilogue ------------------------------
+    const int lw = warp - 2;
+    constexpr int LANES_N = BN / 4;                 // lanes side by side in a row of W
+    constexpr int OCTETS = 32 / LANES_N;            // groups of eight k that a warp covers per pass of eight loads
+    const int n = (lane % LANES_N) * 4, octet = lane / LANES_N;
+    const int gcol = col0 + n;
+    bool ok = true;
+    for (int i = lw; i < p.steps; i += LOAD_WARPS) {
+      float4 v[2][8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int k = i * C::STAGE_K + (h * OCTETS + octet) * 8 + e;
+          float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+          const float *src = p.w + static_cast<int64_t>(k) * p.N + gcol;
+          if (k < p.K) {
+            if (p.w_vec) {
+              if (gcol < p.N) q = __ldcs(reinterpret_cast<const float4 *>(src));
+            } else {
+              if (gcol < p.N) q.x = __ldcs(src);
+              if (gcol + 1 < p.N) q.y = __ldcs(src + 1);
+              if (gcol + 2 < p.N) q.z = __ldcs(src + 2);
+              if (gcol + 3 < p.N) q.w = __ldcs(src + 3);
+            }
+          }
+          v[h][e] = q;
+        }
+      const int stage = i % p.stages;
+      const uint32_t phase = static_cast<uint32_t>(i / p.stages) & 1u;
+      if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        atomicCAS(p.err, 0u, 0x90000000u | static_cast<uint32_t>(stage));
+        ok = false;
+        break;
+      }
+      uint8_t *dst = b_s + stage * C::B_BYTES;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = j == 0 ? v[h][e].x : j == 1 ? v[h][e].y : j == 2 ? v[h][e].z : v[h][e].w;
+          const uint4 q = make_uint4(pack_pair<__half>(f[0], f[1]), pack_pair<__half>(f[2], f[3]),
+                                     pack_pair<__half>(f[4], f[5]), pack_pair<__half>(f[6], f[7]));
+          *reinterpret_cast<uint4 *>(dst + (h * OCTETS + octet) * C::LBO + ((n + j) >> 3) * SBO + ((n + j) & 7) * 16) = q;
+        }
+      fence_proxy_async_smem();  // the tensor core reads the stage through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[stage]);
+    }
+    const int quarter = warp & 3;
+    if (ok && quarter * 32 < p.M) {
+      // the two warps of a lane quarter take 16 columns each; 16 columns in all are the first one's
+      const int c0 = (lw >> 2) * 16;
+      const int row = quarter * 32 + lane, cols = p.N - (col0 + c0);
+      if (c0 < BN && cols > 0) {
+        float b[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) b[j] = p.bias && j < cols ? __ldg(p.bias + col0 + c0 + j) : 0.f;
+        if (!mbar_wait_warp(&acc_bar, 0, abort_flag)) {
+          atomicCAS(p.err, 0u, 0x93000000u);
+        } else {
+          tc_fence_after();
+          uint32_t acc[16];
+          tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c0), acc);
+          tmem_ld_wait_regs(acc);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) b[j] += __uint_as_float(acc[j]);
+          if (row < p.M) {
+            float *dst = p.out + static_cast<int64_t>(row) * p.N + col0 + c0;
+            if (p.out_vec) {
+#pragma unroll
+              for (int j = 0; j < 16; j += 4)
+                if (j < cols) *reinterpret_cast<float4 *>(dst + j) = make_float4(b[j], b[j + 1], b[j + 2], b[j + 3]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (j < cols) dst[j] = b[j];
+            }
+          }
+        }
+      }
+    }
+  }
+  // ------------------------------ teardown ------------------------------
+  if (*abort_flag) {
+    // a wait gave up: give copies still in flight time to land before the CTA retires
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem_base, 32);
+}
+
+template <int BN>
+static void launch_few_rows(const CUtensorMap &ta, FewRowsParams &p, cudaStream_t s) {
+  using C = fewrows::Cfg<BN>;
+  auto kern = gemm_few_rows_kernel<BN>;
+  constexpr int kMaxSmem = 224 * 1024;
+  static bool set_on[64] = {false};  // the attribute is per device
+  const int dev = device_info().device;
+  bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
+  if (!set) {
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "cudaFuncSetAttribute(gemm few rows)"))
+      return;
+    set = true;
+  }
+  p.steps = (p.K + C::STAGE_K - 1) / C::STAGE_K;
+  const int stage = C::STAGE_K / 64 * p.box_m * 128 + C::B_BYTES, fixed = 1024 + (128 - p.box_m) * 128;
+  p.stages = (kMaxSmem - fixed) / stage;
+  if (p.stages > fewrows::MAX_STAGES) p.stages = fewrows::MAX_STAGES;
+  if (p.stages > p.steps) p.stages = p.steps;
+  const size_t smem = static_cast<size_t>(fixed) + static_cast<size_t>(p.stages) * stage;
+  {
+    ProfileScope prof(kCatGemm, s);
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>((p.N + BN - 1) / BN)), dim3(fewrows::THREADS), smem, s, 1, ta, p),
+               "launch gemm few rows");
+  }
+  launched("gemm_few_rows_kernel");
+}
+
+void gemm_few_rows(const void *a16, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K, cudaStream_t s) {
+  const DeviceInfo &di = device_info();
+  uint32_t *err = device_error_slot();
+  if (!err) return;
+  const uint64_t Kp = static_cast<uint64_t>((K + 7) / 8 * 8);
+  FewRowsParams p;
+  p.w = w, p.bias = bias, p.out = out;
+  p.M = static_cast<int>(M), p.N = static_cast<int>(N), p.K = static_cast<int>(K);
+  p.box_m = M <= 32 ? 32 : 64;
+  p.w_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
+  p.out_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.err = err;
+  CUtensorMap ta;
+  if (!encode_tmap_2d(&ta, a16, MGPU_DTYPE_F16, Kp, static_cast<uint64_t>(M), Kp * 2, 64, static_cast<uint32_t>(p.box_m))) return;
+  // 16 columns spread a narrow weight over more SMs; 32 read whole lines of a wide one
+  if ((N + 15) / 16 <= di.sms) launch_few_rows<16>(ta, p, s);
+  else launch_few_rows<32>(ta, p, s);
+}
+
+}  // namespace mdc

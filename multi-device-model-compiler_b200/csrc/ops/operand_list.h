@@ -45,7 +45,9 @@ struct OperandList {
     blocks += j->tiles_n * ((j->pitch + 63) / 64);
   }
   void clear() { n = 0, blocks = 0, overflow = false; }
-  void launch(int32_t dtype, void *stream);  // nothing when empty; the list is empty afterwards
+  // Nothing when empty; the list is empty afterwards.  late: the next kernel may start once this one's own
+  // dependency is resolved, instead of at once: what is older than this launch is then complete for it.
+  void launch(int32_t dtype, void *stream, bool late = false);
 
  private:
   Job *add(const float *src, void *dst, int64_t rows, int64_t cols, int64_t pitch) {

@@ -1,5 +1,6 @@
 // Library lifetime (gpuOpsInit / gpuOpsDeinit), the reference's mgpuMatmul entry point on
 // top of the tensor-core Gemm.
+#include "gemm_plan.h"
 #include "ops_common.h"
 
 namespace mdc {
@@ -64,6 +65,16 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   if (K <= 0) { fail("mgpuMatmul: K must be positive"); return; }
   if (!device_info().ok) return;
   const int64_t Kp = (K + 7) / 8 * 8;
+  if (gemm_takes_few_rows(M, N, K) && !mgpuConstantSourceOf(weight)) {
+    void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
+    if (!a16) return;
+    OperandList list;
+    list.cast(input, a16, M, K, Kp);
+    list.launch(MGPU_DTYPE_F16, stream, true);
+    gemm_few_rows(a16, weight, bias, output, M, N, K, as_stream(stream));
+    mgpuMemFreeAsync(a16, stream);
+    return;
+  }
   void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
   bool w_cached = false;
   OperandList list;

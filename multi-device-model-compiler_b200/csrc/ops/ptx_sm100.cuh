@@ -216,6 +216,7 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+constexpr int kStepKMajor = 2;
 // Two operand descriptors of 64-wide k-blocks: their low words move, the high ones are constant.
 struct KblockDesc {
   uint32_t a_lo, a_hi, b_lo, b_hi;
@@ -225,16 +226,17 @@ __device__ __forceinline__ KblockDesc kblock_desc(uint64_t a, uint64_t b) {
 }
 // NKB (one or four) k-blocks of 64, four MMAs each, called by a whole warp and issued by its elected lane;
 // only the first MMA may start a new accumulation.  Along a k-block the operands advance by two units of
-// 16 bytes (32 bytes of a swizzled row), from one k-block to the next by a_kb / b_kb units.
+// 16 bytes (32 bytes of a swizzled row; B by B_STEP where it is laid out otherwise), from one k-block to the
+// next by a_kb / b_kb units.
 // A tile of few columns is bound by this warp's instructions, not by the tensor pipe: 32-bit address
 // arithmetic and four k-blocks per election instead of 64-bit adds and an election each.
 #define MDC_KBLOCK(CGS, A, B, P)                                             \
   "add.u32 x1, " A ", 2;\n"                                                  \
-  "add.u32 y1, " B ", 2;\n"                                                  \
+  "add.u32 y1, " B ", %9;\n"                                                  \
   "add.u32 x2, " A ", 4;\n"                                                  \
-  "add.u32 y2, " B ", 4;\n"                                                  \
+  "add.u32 y2, " B ", %10;\n"                                                  \
   "add.u32 x3, " A ", 6;\n"                                                  \
-  "add.u32 y3, " B ", 6;\n"                                                  \
+  "add.u32 y3, " B ", %11;\n"                                                  \
   "mov.b64 da, {" A ", %2};\n"                                               \
   "mov.b64 db, {" B ", %4};\n"                                               \
   "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, " P ";\n"   \
@@ -268,12 +270,13 @@ __device__ __forceinline__ KblockDesc kblock_desc(uint64_t a, uint64_t b) {
   "add.u32 ka3, ka2, %7;\n"                                                  \
   "add.u32 kb3, kb2, %8;\n" MDC_KBLOCK(CGS, "%1", "%3", "p")                 \
   MDC_KBLOCK(CGS, "ka1", "kb1", "1") MDC_KBLOCK(CGS, "ka2", "kb2", "1") MDC_KBLOCK(CGS, "ka3", "kb3", "1") "}\n"
-template <int CG, int NKB>
+template <int CG, int NKB, int B_STEP = kStepKMajor>
 __device__ __forceinline__ void umma_f16_ss_kblocks(uint32_t d_tmem, const KblockDesc &d, uint32_t idesc, uint32_t accumulate,
                                                     uint32_t a_kb = 0, uint32_t b_kb = 0) {
   static_assert((CG == 1 || CG == 2) && (NKB == 1 || NKB == 4), "");
 #define MDC_KBLOCK_ARGS \
-  "r"(d_tmem), "r"(d.a_lo), "r"(d.a_hi), "r"(d.b_lo), "r"(d.b_hi), "r"(idesc), "r"(accumulate), "r"(a_kb), "r"(b_kb) : "memory"
+  "r"(d_tmem), "r"(d.a_lo), "r"(d.a_hi), "r"(d.b_lo), "r"(d.b_hi), "r"(idesc), "r"(accumulate), "r"(a_kb), "r"(b_kb), \
+      "n"(B_STEP), "n"(2 * B_STEP), "n"(3 * B_STEP) : "memory"
   if constexpr (CG == 1 && NKB == 1) asm volatile(MDC_KBLOCKS_1("1")::MDC_KBLOCK_ARGS);
   else if constexpr (CG == 1) asm volatile(MDC_KBLOCKS_4("1")::MDC_KBLOCK_ARGS);
   else if constexpr (NKB == 1) asm volatile(MDC_KBLOCKS_1("2")::MDC_KBLOCK_ARGS);

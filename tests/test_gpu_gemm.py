@@ -275,3 +275,62 @@ def test_rows_of_16_byte_multiples_are_not_slow(m, N, offsets):
             w = (0.02 * rng.standard_normal((K, n))).astype(np.float32)
             t.append(_matmul16_at(m, a, w, np.zeros(n, np.float32), np.zeros((M, n), np.float32), out_dtype, 0, *off, repeat=20))
         assert t[0] <= 2.5 * t[1], t
+
+
+def _exact_matmul(m, M, N, K, seed):
+    # small integers, so any order of summation is exact and a wrong tile, stage or padding is a hard mismatch
+    rng = np.random.default_rng(seed)
+    a = rng.integers(-3, 4, (M, K)).astype(np.float32)
+    w = rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    assert np.array_equal(m.matmul(a, w, b), a @ w + b)
+    assert np.array_equal(m.matmul(a, w, None), a @ w)
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 8), (1, 1, 1), (5, 17, 24), (32, 16, 128), (33, 15, 129),    # a stage, its edges, one column tile
+    (16, 1000, 2048), (64, 2368, 200), (64, 2369, 200), (3, 4100, 63),  # 16 columns a CTA, 32, odd widths
+    (7, 1100, 3210), (40, 2400, 3333), (7, 48, 6001)])                  # the ring goes round; a long K that it leaves
+def test_few_rows_are_exact(m, M, N, K):
+    """Up to 64 rows the weight is read in fp32 by the Gemm itself."""
+    _exact_matmul(m, M, N, K, 23)
+
+
+@pytest.mark.parametrize("offset", [4, 8])
+def test_few_rows_off_their_boundaries(m, offset):
+    M, N, K = 20, 64, 96
+    rng = np.random.default_rng(29)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    pad = np.zeros(offset // 4, np.float32)
+    da, dw, db = (m.to_device(np.concatenate([pad, t.ravel()])) for t in (a, w, b))
+    do = m.DeviceBuffer(M * N * 4 + 64)
+    m.ops().mgpuMatmul(da.ptr + offset, dw.ptr + offset, db.ptr + offset, do.ptr + offset, M, N, K, None)
+    got = m.to_host(do, (M * N + 16,), np.float32)[offset // 4:][:M * N].reshape(M, N)
+    m.check("mgpuMatmul")
+    assert np.array_equal(got, a @ w + b)
+
+
+def test_few_rows_keep_infinities_to_themselves(m):
+    # a row or column with an infinity leaves the others alone
+    rng = np.random.default_rng(31)
+    a, w = rng.standard_normal((9, 300)).astype(np.float32), rng.standard_normal((300, 40)).astype(np.float32)
+    clean = m.matmul(a, w, None)
+    a2, w2 = a.copy(), w.copy()
+    a2[4, 7], w2[200, 13] = np.inf, np.nan
+    got = m.matmul(a2, w2, None)
+    keep = np.ones_like(clean, bool)
+    keep[4, :], keep[:, 13] = False, False
+    assert np.array_equal(got[keep], clean[keep])
+    assert not np.isfinite(got[4]).any() and np.isnan(got[:, 13]).all()
+
+
+@pytest.mark.parametrize("N,K", [(768, 3072), (1000, 1000), (72, 333)])
+def test_matmul_rows_do_not_depend_on_their_number(m, N, K):
+    # few rows, one wave, CTA pairs: the same sum over K in the same order
+    rng = np.random.default_rng(37)
+    a = rng.standard_normal((6000, K)).astype(np.float32)
+    w = (0.02 * rng.standard_normal((K, N))).astype(np.float32)
+    whole = m.matmul(a, w, None)
+    for M in (1, 16, 33, 64, 65, 128, 250, 1000, 2048):
+        assert np.array_equal(m.matmul(a[:M], w, None), whole[:M]), M
