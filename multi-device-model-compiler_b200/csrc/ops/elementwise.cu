@@ -368,7 +368,7 @@ MDC_API void mgpuAdd(const float *a, const float *b, float *c, int64_t n, void *
   const DeviceInfo &di = device_info();
   if (!di.ok) return;
   ProfileScope prof(kCatElementwise, as_stream(stream));
-  mdc_add_f32<<<ew_grid((n + 3) / 4, di.sms), kEwBlock, 0, as_stream(stream)>>>(a, b, c, n);
+  check_cuda(launch_chain(mdc_add_f32, dim3(ew_grid((n + 3) / 4, di.sms)), dim3(kEwBlock), 0, as_stream(stream), 1, a, b, c, n), "launch add");
   launched("mdc_add_f32");
 }
 
@@ -377,8 +377,8 @@ MDC_API void mgpuBiasAdd(const float *x, const float *bias, float *y, int64_t ro
   if (rows <= 0 || cols <= 0) return;
   const DeviceInfo &di = device_info();
   if (!di.ok) return;
-  mdc_bias_add_f32<<<ew_grid((rows * cols + 3) / 4, di.sms), kEwBlock, 0, as_stream(stream)>>>(
-      x, bias, y, rows, cols);
+  check_cuda(launch_chain(mdc_bias_add_f32, dim3(ew_grid((rows * cols + 3) / 4, di.sms)), dim3(kEwBlock), 0, as_stream(stream), 1,
+                          x, bias, y, rows, cols), "launch bias add");
   launched("mdc_bias_add_f32");
 }
 
@@ -390,13 +390,13 @@ MDC_API void mgpuActivation(const float *x, float *y, int64_t n, int32_t act, vo
   cudaStream_t s = as_stream(stream);
   switch (act) {
   case MGPU_ACT_RELU:
-    mdc_relu_f32<<<grid, kEwBlock, 0, s>>>(x, y, n);
+    check_cuda(launch_chain(mdc_relu_f32, dim3(grid), dim3(kEwBlock), 0, s, 1, x, y, n), "launch activation");
     break;
   case MGPU_ACT_GELU_ERF:
-    mdc_gelu_erf_f32<<<grid, kEwBlock, 0, s>>>(x, y, n);
+    check_cuda(launch_chain(mdc_gelu_erf_f32, dim3(grid), dim3(kEwBlock), 0, s, 1, x, y, n), "launch activation");
     break;
   case MGPU_ACT_GELU_TANH:
-    mdc_gelu_tanh_f32<<<grid, kEwBlock, 0, s>>>(x, y, n);
+    check_cuda(launch_chain(mdc_gelu_tanh_f32, dim3(grid), dim3(kEwBlock), 0, s, 1, x, y, n), "launch activation");
     break;
   case MGPU_ACT_NONE:
     if (x != y) check_cuda(cudaMemcpyAsync(y, x, n * sizeof(float), cudaMemcpyDeviceToDevice, s), "copy");

@@ -14,6 +14,9 @@
 #include "mdc_gpu_ops.h"
 #include "mdc_gpu_runtime.h"
 #include "operand_list.h"
+#ifdef __CUDACC__
+#include "pdl.cuh"
+#endif
 
 #define MDC_API extern "C" __attribute__((visibility("default")))
 #define MDC_CXX_API __attribute__((visibility("default")))
@@ -57,7 +60,7 @@ inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 // Launch helper for the kernels of the layer chain.  With programmatic dependent launch the
 // front end may set the next kernel up (and start its CTAs on SMs the previous kernel has
 // already left) while the previous kernel drains; each such kernel calls pdl_wait() (device,
-// ptx_sm100.cuh / below) before it touches global memory, which orders it after the whole
+// pdl.cuh) before it touches global memory, which orders it after the whole
 // previous grid.  MDC_PDL=0 turns the attribute off (plain stream order).
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
@@ -86,18 +89,6 @@ inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, s
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
-#ifdef __CUDACC__
-// Blocks until the grid this one was made dependent on has completed and its writes are
-// visible; returns at once for a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets the NEXT kernel of the chain be set up now: once every CTA of this grid has executed
-// this (or exited), the dependent grid's CTAs are placed on whatever SM resources are free
-// and run their prologue (barrier init, tensor-memory allocation, descriptor prefetch) up to
-// their own pdl_wait(), which still holds them until this whole grid has finished and its
-// writes are visible.  Called first thing in every chain kernel, so nothing of the next
-// kernel's launch and set-up latency is left exposed between two kernels.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-#endif
 
 // Optional per-launch timing: while profiling is on (mgpuOpsProfileBegin), every launch
 // site brackets its kernel with two CUDA events on the launching stream; mgpuOpsProfileEnd
