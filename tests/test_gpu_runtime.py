@@ -413,3 +413,22 @@ def test_pool_guard_bands_catch_a_write_past_the_end():
     env = dict(os.environ, MDC_POOL_GUARD="1")
     res = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300, env=env, cwd=root)
     assert res.returncode == 0 and "GUARD_OK" in res.stdout, res.stdout[-1500:] + res.stderr[-1500:]
+
+
+@pytest.mark.parametrize("nbytes,offset", [((1 << 20) + 3, 1), (9 << 20, 4095), ((17 << 20) + 5, 64)])
+def test_download_into_unmapped_pages(m, nbytes, offset):
+    """A large download brings the pages of its destination in beforehand: a fresh mapping, off its page
+    boundaries, gets the bytes and its neighbours keep theirs; so does memory that is in use."""
+    import ctypes
+    import mmap
+    rt = m.runtime()
+    src = np.random.default_rng(nbytes).integers(0, 256, nbytes, dtype=np.uint8)
+    dev = m.to_device(src)
+    fresh = mmap.mmap(-1, nbytes + 2 * 4096)
+    used = np.full(nbytes + 2 * 4096, 0x5a, np.uint8)
+    for buf, keep in ((np.frombuffer(fresh, np.uint8), 0), (used, 0x5a)):
+        rt.mgpuMemcpy(ctypes.c_void_p(buf.ctypes.data + offset), dev.ptr, nbytes, None)
+        rt.mgpuStreamSynchronize(None)
+        m.check("download")
+        assert np.array_equal(buf[offset:offset + nbytes], src)
+        assert (buf[:offset] == keep).all() and (buf[offset + nbytes:] == keep).all()
