@@ -22,7 +22,7 @@
 // Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
 // changing from call to call:
 //   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  73 us (43 of HBM time)
-//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        74 ->  34 us
+//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        74 ->  32 us
 // L2 flushed between calls:
 //   26 x 352 x 37 x 46 -> 32, 3 x 3                      155 ->  81 us
 //   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            116 ->  34 us
@@ -34,6 +34,7 @@
 
 #include "conv_plan.h"
 #include "fast_div.h"
+#include "gemm_common.cuh"
 #include "ops_common.h"
 #include "ptx_sm100.cuh"
 
@@ -386,19 +387,19 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
 // (NCHW fp32 -> NHWC fp16, channels zero-padded to Cp) in tiles of 64 pixels x 64 channels of one
 // image, the others one (output channel, block of 64 input channels) of the filter each:
 // OIHW fp32 -> [OC][channel block][tap][64] fp16, or for the gather kernel its own order padded to Kp.
-// Bound by bytes: 6 per input element.
+// Bound by bytes: 6 per input element.  A lane reads 16 channels of its pixel, all in flight, a line per warp and
+// channel, and writes one whole sector: nothing goes through shared memory (a 64 x 64 transposition there had
+// twice the instructions).  32 x 64 x 56 x 56 in a whole call 34.1 -> 31.9 us; cold, 9 x 32 x 239 x 207 56.3 -> 46.0.
 struct ConvPrepareParams {
   const float *x, *w;
   __half *x16, *w16;
   int IC, HW, Cp, pixel_tiles, channel_tiles, taps, ncb;
   int K, Kp;        // gather order (ncb == 0): patch length and row pitch
-  int vec_ok;       // the image planes can be read in 16-byte vectors
   int sampled, H, W, SH, SW, PHL, PWL;  // sampled: pixel (h, w) of the copy is (h*SH - PHL, w*SW - PWL) of the input
   Divisor by_w;
   int64_t input_blocks;
 };
 __global__ void __launch_bounds__(256) conv_prepare_kernel(const ConvPrepareParams p) {
-  __shared__ float tile[64][65];
   pdl_launch_dependents();
   pdl_wait();
   int64_t b = blockIdx.x;
@@ -406,53 +407,41 @@ __global__ void __launch_bounds__(256) conv_prepare_kernel(const ConvPreparePara
     const int ct = static_cast<int>(b % p.channel_tiles);
     b /= p.channel_tiles;
     const int pt = static_cast<int>(b % p.pixel_tiles);
-    const int64_t n = b / p.pixel_tiles;
-    const int p0 = pt * 64, c0 = ct * 64;
+    // warp: 32 pixels x 16 channels, a lane's channels one 32-byte sector of its pixel's row
+    const int q = pt * 64 + (threadIdx.x >> 5 & 1) * 32 + (threadIdx.x & 31), c0 = ct * 64 + (threadIdx.x >> 6) * 16;
+    if (q >= p.HW || c0 >= p.Cp) return;
     const int plane = p.sampled ? p.H * p.W : p.HW;
-    const float *src = p.x + (n * p.IC + c0) * static_cast<int64_t>(plane);
-    int at[4];  // where this thread's four pixels lie in a plane; -1: outside
-    const int px = (threadIdx.x & 15) * 4, cr = threadIdx.x >> 4;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int q = p0 + px + e;
-      at[e] = q < p.HW ? q : -1;
-      if (p.sampled && q < p.HW) {
-        const int oh = p.by_w.div(q), h = oh * p.SH - p.PHL, w = p.by_w.mod(q, oh) * p.SW - p.PWL;
-        at[e] = static_cast<unsigned>(h) < static_cast<unsigned>(p.H) && static_cast<unsigned>(w) < static_cast<unsigned>(p.W)
-                    ? h * p.W + w : -1;
-      }
+    int at = q;  // where the pixel lies in a plane
+    bool in = true;
+    if (p.sampled) {
+      const int oh = p.by_w.div(q), h = oh * p.SH - p.PHL, w = p.by_w.mod(q, oh) * p.SW - p.PWL;
+      in = static_cast<unsigned>(h) < static_cast<unsigned>(p.H) && static_cast<unsigned>(w) < static_cast<unsigned>(p.W);
+      at = h * p.W + w;
     }
+    const int n = min(16, p.IC - c0);  // live channels; what is left of Cp is zeros
+    // pixels outside read an element that is there and drop it: no branch per load
+    const char *src = reinterpret_cast<const char *>(p.x + (b / p.pixel_tiles * p.IC + c0) * static_cast<int64_t>(plane) + (in ? at : 0));
+    float v[16];
+    if (n == 16) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = cr + 16 * i;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c0 + c < p.IC) {
-        const float *s = src + static_cast<int64_t>(c) * plane;
-        if (p.vec_ok && at[3] >= 0) {
-          v = __ldcs(reinterpret_cast<const float4 *>(s + at[0]));
-        } else {
-          if (at[0] >= 0) v.x = s[at[0]];
-          if (at[1] >= 0) v.y = s[at[1]];
-          if (at[2] >= 0) v.z = s[at[2]];
-          if (at[3] >= 0) v.w = s[at[3]];
-        }
-      }
-      tile[c][px] = v.x, tile[c][px + 1] = v.y, tile[c][px + 2] = v.z, tile[c][px + 3] = v.w;
+      for (int j = 0; j < 16; ++j) v[j] = __ldcs(reinterpret_cast<const float *>(src + static_cast<uint64_t>(static_cast<uint32_t>(plane)) * (4u * j)));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        v[j] = j < n ? __ldcs(reinterpret_cast<const float *>(src + static_cast<uint64_t>(static_cast<uint32_t>(plane)) * (4u * j))) : 0.f;
     }
-    __syncthreads();
-    const int chunk = (threadIdx.x & 7) * 8, pr = threadIdx.x >> 3;
-    if (c0 + chunk < p.Cp) {
+    uint32_t o[8];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int q = pr + 32 * i;
-        if (p0 + q < p.HW) {
-          __align__(16) __half h[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(tile[chunk + e][q]);
-          *reinterpret_cast<uint4 *>(p.x16 + (n * p.HW + p0 + q) * static_cast<int64_t>(p.Cp) + c0 + chunk) =
-              *reinterpret_cast<const uint4 *>(h);
-        }
-      }
+    for (int e = 0; e < 8; ++e) {
+      const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+      o[e] = in ? *reinterpret_cast<const uint32_t *>(&h) : 0u;
+    }
+    __half *dst = p.x16 + (b / p.pixel_tiles * p.HW + q) * static_cast<int64_t>(p.Cp) + c0;
+    if (p.Cp % 16 == 0) {
+      st_global_32B(dst, o);
+    } else {
+      *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (c0 + 8 < p.Cp) *reinterpret_cast<uint4 *>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
     }
     return;
   }
@@ -627,7 +616,6 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   q.H = int(call.H), q.W = int(call.W), q.SH = int(call.SH), q.SW = int(call.SW), q.PHL = int(call.PHL), q.PWL = int(call.PWL);
   q.by_w = Divisor(c.W);
   q.pixel_tiles = int((c.H * c.W + 63) / 64), q.channel_tiles = int(ncb);
-  q.vec_ok = !sampled && (c.H * c.W) % 4 == 0 && (reinterpret_cast<uintptr_t>(c.x) & 15u) == 0;
   q.input_blocks = gather ? 0 : c.N * q.pixel_tiles * q.channel_tiles;
   const int64_t blocks = q.input_blocks + c.OC * (gather ? 1 : ncb);
 
