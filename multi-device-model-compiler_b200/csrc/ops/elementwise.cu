@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "elementwise_kernels.cuh"
+#include "gemm_common.cuh"
 #include "ops_common.h"
 
 namespace mdc {
@@ -187,9 +188,10 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 
 // All operands of a call in one launch; a block belongs to one job.
 //   cast: kCastItems elements of a contiguous array, or kPadItems of rows that are padded.
-//   pack: weight fp32 [K, N] (N contiguous) -> 16-bit [N, Kp] (K contiguous), zero padded to Kp, in
-//         64 x 64 tiles through shared memory: reads are 16-byte vectors along n (whole lines of w),
-//         writes are 16-byte vectors of eight 16-bit values along k (whole lines of out).
+//   pack: weight fp32 [K, N] (N contiguous) -> 16-bit [N, Kp] (K contiguous), zero padded to Kp, in tiles of
+//         64 x 64.  A lane reads 16 values of its column, all in flight, a line per warp and k whatever N is, and
+//         writes one whole sector; through shared memory (16-byte reads, 16-byte writes of eight values)
+//         the five operands of an 8 x 256 token layer, 1024 wide, took 2.9 us longer (98.6 -> 95.7 us a call).
 // Bound by HBM bytes (6 per element).  One launch instead of one per operand: the tail of one
 // job is filled by the next and the launch gaps go: a 1024-wide
 // context layer with 2048 tokens (five operands) 130 -> 118 us a call; 35 x 3086 x 3392 Gemm, whose rows
@@ -203,7 +205,6 @@ struct OperandJobs {
 template <typename T16>
 __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const OperandJobs jobs) {
   static_assert(kEwBlock == OperandList::kThreads, "the 64 x 64 tiles are walked by 256 threads");
-  __shared__ float tile[64][65];
   if (!jobs.late) pdl_launch_dependents();
   pdl_wait();
   if (jobs.late) pdl_launch_dependents();
@@ -249,42 +250,31 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
     }
     return;
   }
-  const float *w = job.src;
+  // warp: 32 columns x 16 k, a lane's values one 32-byte sector of its column's packed row
   const int64_t K = job.rows, N = job.cols, Kp = job.pitch;
   const uint32_t b32 = static_cast<uint32_t>(b), tk = b32 / static_cast<uint32_t>(job.tiles_n);
-  const int64_t k0 = static_cast<int64_t>(tk) * 64, n0 = static_cast<int64_t>(b32 - tk * job.tiles_n) * 64;
-  {
-    const int c4 = (threadIdx.x & 15) * 4, r0 = threadIdx.x >> 4;  // 16 threads per k-row, 16 rows per pass
+  const int64_t k0 = static_cast<int64_t>(tk) * 64 + (threadIdx.x >> 6) * 16;
+  const int64_t n = static_cast<int64_t>(b32 - tk * job.tiles_n) * 64 + (threadIdx.x & 63);
+  if (n >= N || k0 >= Kp) return;
+  const float *w = job.src + k0 * N + n;
+  const int live = K - k0 < 16 ? static_cast<int>(K - k0) : 16;  // at most 0 in the padding
+  float v[16];
+  if (live == 16) {
 #pragma unroll
-    for (int r = r0; r < 64; r += 16) {
-      const int64_t k = k0 + r, n = n0 + c4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k < K) {
-        if (job.vec_ok && n + 3 < N) {
-          v = __ldg(reinterpret_cast<const float4 *>(w + k * N + n));
-        } else {
-          if (n < N) v.x = w[k * N + n];
-          if (n + 1 < N) v.y = w[k * N + n + 1];
-          if (n + 2 < N) v.z = w[k * N + n + 2];
-          if (n + 3 < N) v.w = w[k * N + n + 3];
-        }
-      }
-      tile[r][c4] = v.x, tile[r][c4 + 1] = v.y, tile[r][c4 + 2] = v.z, tile[r][c4 + 3] = v.w;
-    }
+    for (int j = 0; j < 16; ++j) v[j] = __ldcs(w + j * N);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = j < live ? __ldcs(w + j * N) : 0.f;
   }
-  __syncthreads();
-  {
-    const int kg = (threadIdx.x & 7) * 8, r0 = threadIdx.x >> 3;  // 8 threads per n-row, 32 rows per pass
+  uint32_t o[8];
 #pragma unroll
-    for (int r = r0; r < 64; r += 32) {
-      const int64_t n = n0 + r, k = k0 + kg;
-      if (n < N && k < Kp) {  // Kp is a multiple of 8: a group of eight is inside or outside as a whole
-        __align__(16) T16 h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = from_f32<T16>(tile[kg + e][r]);
-        *reinterpret_cast<uint4 *>(out + n * Kp + k) = *reinterpret_cast<const uint4 *>(h);
-      }
-    }
+  for (int e = 0; e < 8; ++e) o[e] = pack_pair<T16>(v[2 * e], v[2 * e + 1]);
+  T16 *dst = out + n * Kp + k0;
+  if (job.vec_ok) {
+    st_global_32B(dst, o);
+  } else {
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (k0 + 8 < Kp) *reinterpret_cast<uint4 *>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
   }
 }
 

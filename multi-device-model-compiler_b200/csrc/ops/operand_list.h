@@ -18,7 +18,7 @@ struct OperandList {
     int64_t rows, cols, pitch;  // cast: [rows, cols] -> [rows, pitch]; pack: [rows = K, cols = N] -> [N, pitch]
     int64_t first_block;
     int tiles_n;                // pack: 64-column tiles; 0 marks a cast
-    int vec_ok;
+    int vec_ok;                 // cast: 16-byte accesses; pack: stores of whole sectors
   };
   Job jobs[kMax];
   int n = 0;
@@ -41,7 +41,7 @@ struct OperandList {
     Job *j = add(w, dst, K, N, (K + 7) / 8 * 8);
     if (!j) return;
     j->tiles_n = static_cast<int>((N + 63) / 64);
-    j->vec_ok = N % 4 == 0 && !(reinterpret_cast<uintptr_t>(w) & 15u);
+    j->vec_ok = j->pitch % 16 == 0 && !(reinterpret_cast<uintptr_t>(dst) & 31u);
     blocks += j->tiles_n * ((j->pitch + 63) / 64);
   }
   // weight fp32 [K, N] -> 16 bits in its own order, the rows padded to a multiple of 8, or packed
