@@ -50,7 +50,7 @@ struct OneWaveParams {
   uint32_t *err;
 };
 
-template <typename T16, typename TOut, int ACT, int CG, bool kWide, bool kRows>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 __global__ void __launch_bounds__(onewave::THREADS, 1)
 gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const OneWaveParams p) {
@@ -118,15 +118,6 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     box(dst, 0, kb);
   };
   auto load_w = [&](int s, int kb) __attribute__((always_inline)) {
-    if constexpr (kRows) {
-      // boxes of 64 columns and a stage's K range, one behind the other
-      for (int c = 0; c < b_rows; c += 64) {
-        uint8_t *dst = tiles + s * stage_bytes + a_bytes + c * depth * BK * 2;
-        if constexpr (CG == 2) tma_load_2d_cg2(dst, &tmap_b, mapa_u32(smem_u32(&full_bar[s]), 0), col0 + half * b_rows + c, kb * BK);
-        else tma_load_2d(dst, &tmap_b, &full_bar[s], col0 + c, kb * BK);
-      }
-      return;
-    }
     fetch(tiles + s * stage_bytes + a_bytes, &tmap_b, s, col0 + half * b_rows, kb, b_kb_bytes);
   };
   auto load_a = [&](int s, int kb) __attribute__((always_inline)) {
@@ -171,12 +162,10 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     // ------------------------------ MMA issuer (leader of the pair) ------------------------------
     if (leader) {
       const uint32_t idesc = make_idesc_f16(128 * CG, static_cast<uint32_t>(p.bn), std::is_same<T16, __nv_bfloat16>::value,
-                                            false, kRows);
+                                            false, false);
       const KblockDesc desc0 = kblock_desc(make_smem_desc_sw128(smem_u32(tiles), 16, 1024),
-                                           make_smem_desc_sw128(smem_u32(tiles) + static_cast<uint32_t>(a_bytes),
-                                                                kRows ? static_cast<uint32_t>(depth * 64 * BK * 2) : 16, 1024));
-      const uint32_t a_kb16 = static_cast<uint32_t>(a_kb_bytes) >> 4, b_kb16 = static_cast<uint32_t>(kRows ? 64 * BK * 2 : b_kb_bytes) >> 4;
-      constexpr int B_STEP = kRows ? kStepMnMajor : kStepKMajor;
+                                           make_smem_desc_sw128(smem_u32(tiles) + static_cast<uint32_t>(a_bytes), 16, 1024));
+      const uint32_t a_kb16 = static_cast<uint32_t>(a_kb_bytes) >> 4, b_kb16 = static_cast<uint32_t>(b_kb_bytes) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -192,10 +181,10 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         kd.b_lo += static_cast<uint32_t>(stage * stage_bytes) >> 4;
         const int n = min(depth, p.num_kb - i * depth);
         if (n == 4) {
-          umma_f16_ss_kblocks<CG, 4, B_STEP>(tmem_base, kd, idesc, i != 0 ? 1u : 0u, a_kb16, b_kb16);
+          umma_f16_ss_kblocks<CG, 4>(tmem_base, kd, idesc, i != 0 ? 1u : 0u, a_kb16, b_kb16);
         } else {
           for (int d = 0; d < n; ++d) {
-            umma_f16_ss_kblocks<CG, 1, B_STEP>(tmem_base, kd, idesc, (i | d) != 0 ? 1u : 0u);
+            umma_f16_ss_kblocks<CG, 1>(tmem_base, kd, idesc, (i | d) != 0 ? 1u : 0u);
             kd.a_lo += a_kb16, kd.b_lo += b_kb16;
           }
         }
@@ -306,10 +295,10 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   }
 }
 
-template <typename T16, typename TOut, int ACT, int CG, bool kWide, bool kRows>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 static void launch_one_wave_cg(const CUtensorMap &ta, const CUtensorMap &tb, const OneWaveParams &p, int grid, size_t smem,
                             cudaStream_t s) {
-  auto kern = gemm_one_wave_kernel<T16, TOut, ACT, CG, kWide, kRows>;
+  auto kern = gemm_one_wave_kernel<T16, TOut, ACT, CG, kWide>;
   constexpr int kMaxDevices = 64;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   const int dev = device_info().device;
@@ -330,19 +319,14 @@ static void launch_one_wave_cg(const CUtensorMap &ta, const CUtensorMap &tb, con
 
 template <typename T16, typename TOut>
 static void launch_one_wave_act(const CUtensorMap &ta, const CUtensorMap &tb, const OneWaveParams &p, int cg, int grid,
-                                size_t smem, int act, bool w_rows, cudaStream_t s) {
+                                size_t smem, int act, cudaStream_t s) {
   const bool wide = p.rows.wide && !p.k_in_x;
-#define MDC_ONE_WAVE_CG(ACT_, CG_, WIDE_)                                                            \
-  do {                                                                                             \
-    if (w_rows) launch_one_wave_cg<T16, TOut, ACT_, CG_, WIDE_, true>(ta, tb, p, grid, smem, s);   \
-    else launch_one_wave_cg<T16, TOut, ACT_, CG_, WIDE_, false>(ta, tb, p, grid, smem, s);         \
-  } while (0)
-#define MDC_ONE_WAVE(ACT_)                          \
-  do {                                              \
-    if (cg == 2 && wide) MDC_ONE_WAVE_CG(ACT_, 2, true); \
-    else if (cg == 2) MDC_ONE_WAVE_CG(ACT_, 2, false);   \
-    else if (wide) MDC_ONE_WAVE_CG(ACT_, 1, true);       \
-    else MDC_ONE_WAVE_CG(ACT_, 1, false);                \
+#define MDC_ONE_WAVE(ACT_)                                                                      \
+  do {                                                                                          \
+    if (cg == 2 && wide) launch_one_wave_cg<T16, TOut, ACT_, 2, true>(ta, tb, p, grid, smem, s); \
+    else if (cg == 2) launch_one_wave_cg<T16, TOut, ACT_, 2, false>(ta, tb, p, grid, smem, s);   \
+    else if (wide) launch_one_wave_cg<T16, TOut, ACT_, 1, true>(ta, tb, p, grid, smem, s);       \
+    else launch_one_wave_cg<T16, TOut, ACT_, 1, false>(ta, tb, p, grid, smem, s);                \
   } while (0)
   switch (act) {
   case MGPU_ACT_NONE: MDC_ONE_WAVE(kActNone); break;
@@ -352,7 +336,6 @@ static void launch_one_wave_act(const CUtensorMap &ta, const CUtensorMap &tb, co
   default: fail("mgpuMatmulEx16: unknown activation");
   }
 #undef MDC_ONE_WAVE
-#undef MDC_ONE_WAVE_CG
 }
 
 // A [rows, Kp] row-major 16-bit matrix.  Kp a multiple of 64: as (64 k, row, k-block), so that one
@@ -375,15 +358,13 @@ static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, in
   return before != 0 || mgpuGetLastError() == 0;
 }
 
-void gemm_one_wave_launch(const GemmTile &t, const void *a, const Weight16 &w, const float *bias, const void *residual,
+void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,
                        void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act,
-                       cudaStream_t s) {
+                       bool w_ready, cudaStream_t s) {
   uint32_t *err = device_error_slot();
   if (!err) return;
   CUtensorMap ta, tb;
-  if (!encode_operand(&ta, a, dtype, M, Kp, t.box_m, t.depth)) return;
-  if (w.rows ? !encode_weight_rows(&tb, w, dtype, N, t.depth * onewave::BK)
-             : !encode_operand(&tb, w.data, dtype, N, Kp, t.bn / t.cg, t.depth))
+  if (!encode_operand(&ta, a, dtype, M, Kp, t.box_m, t.depth) || !encode_operand(&tb, w_nk, dtype, N, Kp, t.bn / t.cg, t.depth))
     return;
   OneWaveParams p;
   p.M = static_cast<int>(M), p.N = static_cast<int>(N);
@@ -396,7 +377,7 @@ void gemm_one_wave_launch(const GemmTile &t, const void *a, const Weight16 &w, c
   p.depth = t.depth;
   p.tmem_cols = 32;
   while (p.tmem_cols < t.bn) p.tmem_cols *= 2;
-  p.w_ready = w.ready ? 1 : 0;
+  p.w_ready = w_ready ? 1 : 0;
   p.err = err;
   const int64_t m_tiles = (M + static_cast<int64_t>(t.box_m) * t.cg - 1) / (static_cast<int64_t>(t.box_m) * t.cg);
   const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg);
@@ -406,12 +387,12 @@ void gemm_one_wave_launch(const GemmTile &t, const void *a, const Weight16 &w, c
   const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * onewave::BK * 2 : 0);
   const size_t smem = ring + 1024;
   if (dtype == MGPU_DTYPE_F16) {
-    if (out_dtype == MGPU_DTYPE_F16) launch_one_wave_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, w.rows, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, w.rows, s);
+    if (out_dtype == MGPU_DTYPE_F16) launch_one_wave_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);
     else fail("mgpuMatmulEx16: output type must be the operand type or F32");
   } else {
-    if (out_dtype == MGPU_DTYPE_BF16) launch_one_wave_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, t.cg, grid, smem, act, w.rows, s);
-    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__nv_bfloat16, float>(ta, tb, p, t.cg, grid, smem, act, w.rows, s);
+    if (out_dtype == MGPU_DTYPE_BF16) launch_one_wave_act<__nv_bfloat16, __nv_bfloat16>(ta, tb, p, t.cg, grid, smem, act, s);
+    else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__nv_bfloat16, float>(ta, tb, p, t.cg, grid, smem, act, s);
     else fail("mgpuMatmulEx16: output type must be the operand type or F32");
   }
 }

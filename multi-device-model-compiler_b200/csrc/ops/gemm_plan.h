@@ -6,8 +6,6 @@
 
 #include <cuda_runtime.h>
 
-#include "ops_common.h"
-
 namespace mdc {
 
 struct GemmTile {
@@ -21,16 +19,14 @@ struct GemmTile {
 
 constexpr int kOneWaveMaxSmem = 226 * 1024;  // the rest of the 227 KiB is the kernel's static part
 
-// w_rows: W is [K, N] and a CTA's columns come in boxes of 64.
-GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, bool w_rows, int sms);
+GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms);
 
 // Whether gemm_few_rows takes a call whose fp32 weight would have to be converted first.  A CTA of it walks K
 // alone, at about 0.07 us per 16 values, so K is to be short or the columns many: 16 x 1000 x 2048 14.2 -> 10.5
 // us, 16 x 4096 x 4096 44 -> 28 (inputs out of memory), but 16 x 1000 x 4096 25.6 -> 27.6, 16 x 491 x 2136 19.4
-// -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.  Rows that are not
-// loaded in vectors take a shorter K still: 16 x 906 x 1751 21.5 -> 15.4, but 32 x 1221 x 3008 23.6 -> 25.6.
+// -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.
 inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K) {
-  return M <= 64 && N <= (1 << 30) && (K <= 1536 || K <= (N % 4 == 0 ? 3 : 2) * N) && K <= (1 << 30);
+  return M <= 64 && N <= (1 << 30) && (K <= 1536 || K <= 3 * N) && K <= (1 << 30);
 }
 
 // out[M, N] = a16[M, Kp] . w[K, N] + bias, fp16 operands, the weight as the caller has it
@@ -38,12 +34,10 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K) {
 // wait (OperandList::launch with `late`): the weight is read ahead of that launch's end.
 void gemm_few_rows(const void *a16, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K, cudaStream_t s);
 
-// Tensor map of a weight in [K, N] order: boxes of 64 columns (128 bytes) x k_rows, zeros past either end.
-bool encode_weight_rows(CUtensorMap *map, const Weight16 &w, int32_t dtype, int64_t N, int k_rows);
-
-// One call of the one-wave kernel.
-void gemm_one_wave_launch(const GemmTile &t, const void *a, const Weight16 &w, const float *bias, const void *residual,
+// One call of the one-wave kernel.  w_ready: W was complete before this launch was issued (it does
+// not come from a kernel still queued), so it may be read ahead of the dependency wait.
+void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,
                        void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act,
-                       cudaStream_t s);
+                       bool w_ready, cudaStream_t s);
 
 }  // namespace mdc

@@ -78,7 +78,6 @@ struct GemmParams {
   int num_m_blocks, num_n_blocks;
   int cta_group;  // 1: one CTA per 128 x bn tile; 2: CTA pairs on 256 x bn tiles
   int bn;         // tile width in output columns: 256, 192 or 128 (accumulators stay 256 TMEM columns apart)
-  bool w_rows;    // W is [K, N]
   int cw;         // staged rows: columns per chunk, 64 (16-bit output, 128-byte rows) or 32
   uint32_t *err;
 };
@@ -90,7 +89,7 @@ struct RowMaps {
 template <>
 struct RowMaps<true> {};
 
-template <typename T16, typename TOut, int ACT, int CG, bool kWide, bool kRows>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 __global__ void __launch_bounds__(gemm::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ RowMaps<kWide> rows, const GemmParams p) {
@@ -181,20 +180,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), 0);
             if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * stage_tx_bytes);
             tma_load_2d_cg2(sa, &tmap_a, bar, kb * BK, m_blk * BM);
-            if constexpr (kRows) {
-              for (int c = 0; c < bn / 2; c += 64)
-                tma_load_2d_cg2(sb + c * BK * 2, &tmap_b, bar, n_blk * bn + cta_rank * (bn / 2) + c, kb * BK);
-            } else {
-              tma_load_2d_cg2(sb, &tmap_b, bar, kb * BK, n_blk * bn + cta_rank * (bn / 2));
-            }
+            tma_load_2d_cg2(sb, &tmap_b, bar, kb * BK, n_blk * bn + cta_rank * (bn / 2));
           } else {
             mbar_arrive_expect_tx(&full_bar[stage], stage_tx_bytes);
             tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * BK, m_blk * BM);
-            if constexpr (kRows) {
-              for (int c = 0; c < bn; c += 64) tma_load_2d(sb + c * BK * 2, &tmap_b, &full_bar[stage], n_blk * bn + c, kb * BK);
-            } else {
-              tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, n_blk * bn);
-            }
+            tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, n_blk * bn);
           }
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -204,11 +194,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // ---------------- MMA issuer (leader CTA only; whole warp, elected lane issues) ----------------
     if (leader) {
       const uint32_t idesc = make_idesc_f16(BM * CG, static_cast<uint32_t>(bn),
-                                            std::is_same<T16, __nv_bfloat16>::value, false, kRows);
+                                            std::is_same<T16, __nv_bfloat16>::value, false, false);
       const uint64_t desc0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
-      // W in rows: 64-column blocks of 64 k x 128 bytes one behind the other
-      const uint64_t desc0_b = make_smem_desc_sw128(smem_u32(tiles) + A_BYTES, kRows ? 64 * BK * 2 : 16, 1024);
-      constexpr int B_STEP = kRows ? kStepMnMajor : kStepKMajor;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -230,8 +217,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           tc_fence_after();
           // (descriptors hold addresses in units of 16 bytes)
           const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
-          const uint64_t b_desc = desc0_b + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
-          umma_f16_ss_kblocks<CG, 1, B_STEP>(d_tmem, kblock_desc(a_desc, b_desc), idesc, kb != 0 ? 1u : 0u);
+          const uint64_t b_desc = a_desc + A_BYTES / 16;
+          umma_f16_ss_kblocks<CG, 1>(d_tmem, kblock_desc(a_desc, b_desc), idesc, kb != 0 ? 1u : 0u);
           // the stage is reusable (in both CTAs) once these MMAs have read it
           if constexpr (CG == 2) {
             umma_commit_cg2_warp(&empty_bar[stage], 3);
@@ -531,15 +518,10 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
   return encode_tmap_2d_ex(map, base, dtype, inner, outer, row_stride_bytes, box_inner, box_outer, 128);
 }
 
-bool encode_weight_rows(CUtensorMap *map, const Weight16 &w, int32_t dtype, int64_t N, int k_rows) {
-  return encode_tmap_2d(map, w.data, dtype, static_cast<uint64_t>(N), static_cast<uint64_t>(w.K),
-                        static_cast<uint64_t>((N + 7) / 8 * 8) * 2, 64, static_cast<uint32_t>(k_rows));
-}
-
-template <typename T16, typename TOut, int ACT, int CG, bool kWide, bool kRows>
+template <typename T16, typename TOut, int ACT, int CG, bool kWide>
 static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p,
                            int grid, cudaStream_t s) {
-  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG, kWide, kRows>;
+  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG, kWide>;
   constexpr size_t smem = gemm::Cfg<CG, kWide>::SMEM_BYTES;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   bool &attr_set = attr_set_on[current_device_index()];
@@ -561,10 +543,8 @@ static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const R
 template <typename T16, typename TOut, int ACT, bool kWide>
 static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p, int grid,
                         cudaStream_t s) {
-  if (p.cta_group == 2 && p.w_rows) launch_gemm_cg<T16, TOut, ACT, 2, kWide, true>(ta, tb, rows, p, grid, s);
-  else if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, kWide, false>(ta, tb, rows, p, grid, s);
-  else if (p.w_rows) launch_gemm_cg<T16, TOut, ACT, 1, kWide, true>(ta, tb, rows, p, grid, s);
-  else launch_gemm_cg<T16, TOut, ACT, 1, kWide, false>(ta, tb, rows, p, grid, s);
+  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, kWide>(ta, tb, rows, p, grid, s);
+  else launch_gemm_cg<T16, TOut, ACT, 1, kWide>(ta, tb, rows, p, grid, s);
 }
 
 template <typename T16, typename TOut, bool kWide>
@@ -615,18 +595,17 @@ static int choose_cta_group(int64_t M) {
 // tiles) wastes less: e.g. M = 32768, N = 768 on 74 CTA pairs is 6 waves of 256-wide tiles
 // (5.2 needed) but 7 waves of 192-wide ones (6.9 needed) at 3/4 of the cost each.
 // MDC_GEMM_BN=256|192|128 overrides (for measurements).
-static int choose_bn(int64_t M, int64_t N, int cta_group, bool w_rows, int sms) {
+static int choose_bn(int64_t M, int64_t N, int cta_group, int sms) {
   static const int forced = [] {
     const char *e = getenv("MDC_GEMM_BN");
     return e ? atoi(e) : 0;
   }();
-  if (forced == 256 || (forced == 192 && !(w_rows && cta_group == 2)) || forced == 128) return forced;
+  if (forced == 256 || forced == 192 || forced == 128) return forced;
   const int64_t workers = sms / cta_group > 0 ? sms / cta_group : 1;
   const int64_t m_units = (M + gemm::BM * cta_group - 1) / (gemm::BM * cta_group);
   int best = 256;
   double best_cost = 1e300;
   for (int bn : {256, 192, 128}) {
-    if (w_rows && (bn / cta_group) % 64 != 0) continue;
     const int64_t tiles = m_units * ((N + bn - 1) / bn);
     const int64_t waves = (tiles + workers - 1) / workers;
     // per-tile cost: measured, a 192-wide tile takes about 0.95 of the time of a 256-wide one
@@ -661,7 +640,7 @@ static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, 
 }
 
 // The fastest one-wave tile for a problem of at most one 128 x 128 tile per SM.
-static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool w_rows, int sms) {
+static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
   GemmTile best;
   float best_us = 1e30f;
   for (int cg = 1; cg <= 2; ++cg)
@@ -670,7 +649,6 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool w_rows, i
       if (box_m > 32 && box_m >= 2 * M) continue;
       for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
         if (cg == 2 && bn < 64) continue;
-        if (w_rows && bn % (64 * cg) != 0) continue;
         for (int depth : {4, 2, 1}) {
           if (depth > num_kb) continue;
           const int steps = (num_kb + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
@@ -693,48 +671,30 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, bool w_rows, i
   return best;
 }
 
-GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, bool w_rows, int sms) {
+GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   // the choice takes a few microseconds: kept per shape (a plan, not a result)
   struct Entry {
     int64_t M = -1, N = -1, K = -1;
     int sms = 0;
-    bool w_rows = false;
     GemmTile tile;
   };
   static thread_local Entry cache[64];
   Entry &e = cache[(static_cast<uint64_t>(M) * 0x9E3779B97F4A7C15ull ^ static_cast<uint64_t>(N) * 0xC2B2AE3D27D4EB4Full ^
-                    static_cast<uint64_t>(K) * 0x165667B19E3779F9ull ^ (w_rows ? 0x27D4EB2F165667C5ull : 0)) >> 58];
-  if (e.M == M && e.N == N && e.K == K && e.sms == sms && e.w_rows == w_rows) return e.tile;
+                    static_cast<uint64_t>(K) * 0x165667B19E3779F9ull) >> 58];
+  if (e.M == M && e.N == N && e.K == K && e.sms == sms) return e.tile;
   GemmTile t;
   // One wave: up to one 128 x 128 tile per SM.  Measured either side of the line: 1024 x 2304 x 768
   // 7.6 us one-wave, 7.9 persistent; 1024 x 3072 x 768 9.9 and 9.2; 2048 x 768 x 3072 14.1 and 15.5;
   // 4096 x 768 x 3072 19.2 and 17.6.
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
-    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), w_rows, sms);
+    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), sms);
   if (!t.one_wave) {
     t.cg = choose_cta_group(M);
-    t.bn = choose_bn(M, N, t.cg, w_rows, sms);
+    t.bn = choose_bn(M, N, t.cg, sms);
   }
-  e.M = M, e.N = N, e.K = K, e.sms = sms, e.w_rows = w_rows, e.tile = t;
+  e.M = M, e.N = N, e.K = K, e.sms = sms, e.tile = t;
   return t;
-}
-
-// A weight in its own order saves its transposition: 30 -> 20 us for 4096 x 4096, 0.8 us per million
-// values.  Against that stand tiles that it does not come in, of a width that is no multiple of 64 per CTA
-// (2048 x 3072 x 1024: 18.5 us in 192 columns, 20.5 in 256), and rows that would have to be padded, which
-// are cast value by value (1376 x 3834 x 1024, whole call: 62 us transposed, 71 padded).
-bool gemm_reads_rows(int64_t M, int64_t N, int64_t K) {
-  const int sms = device_info().sms;
-  if (N % 8 != 0 || N < 64 || sms <= 0) return false;
-  const int num_kb = static_cast<int>((K + 63) / 64);
-  auto us = [&](const GemmTile &t) {
-    if (t.one_wave) return one_wave_cost(t, M, N, num_kb, sms);
-    const int64_t tiles = (M + 128 * t.cg - 1) / (128 * t.cg) * ((N + t.bn - 1) / t.bn), workers = sms / t.cg > 0 ? sms / t.cg : 1;
-    return static_cast<float>((tiles + workers - 1) / workers) * num_kb * (t.bn == 256 ? 0.4f : t.bn == 192 ? 0.38f : 0.32f);
-  };
-  return us(choose_gemm_tile(M, N, K, true, sms)) <=
-         us(choose_gemm_tile(M, N, K, false, sms)) + 0.8e-6f * static_cast<float>(K) * static_cast<float>(N);
 }
 
 // persistent grid: one worker (CTA or CTA pair) per tile up to the number the device holds
@@ -756,9 +716,9 @@ static int gemm_grid(const GemmParams &p, int sms) {
 
 // The whole of mgpuMatmulEx16 after the argument checks: tile choice, tensor maps, launch.
 // Shared by every entry point that ends in this Gemm; allocates nothing.
-static void matmul16_launch(const char *who, const void *a, const Weight16 &w, const float *bias, const void *residual,
+static void matmul16_launch(const char *who, const void *a, const void *w_nk, const float *bias, const void *residual,
                             void *out, int64_t M, int64_t N, int64_t Kp, int32_t dtype, int32_t out_dtype,
-                            int32_t act, cudaStream_t s) {
+                            int32_t act, bool w_ready, cudaStream_t s) {
   const DeviceInfo &di = device_info();
   char msg[160];
   auto failf = [&](const char *what) {
@@ -768,25 +728,22 @@ static void matmul16_launch(const char *who, const void *a, const Weight16 &w, c
   uint32_t *err = device_error_slot();
   if (!err) return;
 
-  const GemmTile tile = choose_gemm_tile(M, N, Kp, w.rows, di.sms);
+  const GemmTile tile = choose_gemm_tile(M, N, Kp, di.sms);
   if (tile.one_wave) {
-    gemm_one_wave_launch(tile, a, w, bias, residual, out, M, N, Kp, dtype, out_dtype, act, s);
+    gemm_one_wave_launch(tile, a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, s);
     return;
   }
   const int cta_group = tile.cg, bn = tile.bn;
   CUtensorMap ta, tb;
   if (!encode_tmap_2d(&ta, a, dtype, static_cast<uint64_t>(Kp), static_cast<uint64_t>(M),
-                      static_cast<uint64_t>(Kp) * 2, gemm::BK, gemm::BM))
-    return;
-  if (w.rows ? !encode_weight_rows(&tb, w, dtype, N, gemm::BK)
-             : !encode_tmap_2d(&tb, w.data, dtype, static_cast<uint64_t>(Kp), static_cast<uint64_t>(N),
-                               static_cast<uint64_t>(Kp) * 2, gemm::BK, bn / cta_group))
+                      static_cast<uint64_t>(Kp) * 2, gemm::BK, gemm::BM) ||
+      !encode_tmap_2d(&tb, w_nk, dtype, static_cast<uint64_t>(Kp), static_cast<uint64_t>(N),
+                      static_cast<uint64_t>(Kp) * 2, gemm::BK, bn / cta_group))
     return;
 
   GemmParams p;
   p.cta_group = cta_group;
   p.bn = bn;
-  p.w_rows = w.rows;
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
   p.K = static_cast<int>(Kp);
@@ -815,19 +772,19 @@ static void matmul16_launch(const char *who, const void *a, const Weight16 &w, c
 using namespace mdc;
 
 namespace mdc {
-void matmul16(const void *a, const Weight16 &w, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
-              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, void *stream) {
+void matmul16(const void *a, const void *w_nk, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
+              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, bool w_ready, void *stream) {
   if (M <= 0 || N <= 0) return;
   const DeviceInfo &di = device_info();
   if (!di.ok) return;
   if (!dtype_is16(dtype)) { fail("mgpuMatmulEx16: dtype must be F16 or BF16"); return; }
   if (Kp <= 0 || (Kp & 7)) { fail("mgpuMatmulEx16: K must be a positive multiple of 8"); return; }
   if (M > 0x7fffffff || N > 0x7fffffff || Kp > 0x7fffffff) { fail("mgpuMatmulEx16: shape too large"); return; }
-  if ((reinterpret_cast<uintptr_t>(a) & 15u) || (reinterpret_cast<uintptr_t>(w.data) & 15u)) {
+  if ((reinterpret_cast<uintptr_t>(a) & 15u) || (reinterpret_cast<uintptr_t>(w_nk) & 15u)) {
     fail("mgpuMatmulEx16: operands must be 16-byte aligned");
     return;
   }
-  matmul16_launch("mgpuMatmulEx16", a, w, bias, residual, out, M, N, Kp, dtype, out_dtype, act, as_stream(stream));
+  matmul16_launch("mgpuMatmulEx16", a, w_nk, bias, residual, out, M, N, Kp, dtype, out_dtype, act, w_ready, as_stream(stream));
 }
 }  // namespace mdc
 
@@ -896,8 +853,7 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   if (M > 0x7fffffff || N > 0x7fffffff || K > 0x7fffffff) { fail("mgpuMatmulNoAlloc: shape too large"); return; }
   const int64_t Kp = (K + 7) / 8 * 8;
   auto up256 = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t a_bytes = up256(static_cast<size_t>(M) * Kp * 2), w_bytes = up256(weight16_bytes(K, N, false));
-  const bool rows = gemm_reads_rows(M, N, K) && a_bytes + weight16_bytes(K, N, true) <= kNoAllocScratchBytes;
+  const size_t a_bytes = up256(static_cast<size_t>(M) * Kp * 2), w_bytes = up256(static_cast<size_t>(N) * Kp * 2);
   if (a_bytes + w_bytes > kNoAllocScratchBytes) {
     char msg[200];
     snprintf(msg, sizeof(msg),
@@ -925,9 +881,9 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
     gemm_few_rows(a16, weight, bias, output, M, N, K, s);
     return;
   }
-  list.weight(weight, w16, K, N, rows);
+  list.pack(weight, w16, K, N);
   list.cast(input, a16, M, K, Kp);
   list.launch(MGPU_DTYPE_F16, stream);
-  matmul16_launch("mgpuMatmulNoAlloc", a16, Weight16{w16, false, rows, K}, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
-                  MGPU_ACT_NONE, s);
+  matmul16_launch("mgpuMatmulNoAlloc", a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
+                  MGPU_ACT_NONE, false, s);
 }

@@ -44,11 +44,6 @@ struct OperandList {
     j->vec_ok = j->pitch % 16 == 0 && !(reinterpret_cast<uintptr_t>(dst) & 31u);
     blocks += j->tiles_n * ((j->pitch + 63) / 64);
   }
-  // weight fp32 [K, N] -> 16 bits in its own order, the rows padded to a multiple of 8, or packed
-  void weight(const float *w, void *dst, int64_t K, int64_t N, bool rows) {
-    if (rows) cast(w, dst, K, N, (N + 7) / 8 * 8);
-    else pack(w, dst, K, N);
-  }
   void clear() { n = 0, blocks = 0, overflow = false; }
   // Nothing when empty; the list is empty afterwards.  late: the next kernel may start once this one's own
   // dependency is resolved, instead of at once: what is older than this launch is then complete for it.

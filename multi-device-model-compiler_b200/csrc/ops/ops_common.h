@@ -110,28 +110,10 @@ struct ProfileScope {
 // fp32 [R, C] -> 16-bit [R, Cp] with zero padding of the columns C..Cp (elementwise.cu)
 void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype, cudaStream_t s);
 
-// A 16-bit weight as a Gemm reads it.
-struct Weight16 {
-  const void *data;
-  bool ready = false;  // complete before the call was issued (it does not come from a kernel still queued): the
-                       // kernel may read it ahead of its dependency on the previous one
-  bool rows = false;   // [K, pitch] as in the fp32 weight, the pitch N rounded up to 8; else packed, [N, Kp]
-  int64_t K = 0;       // rows: how many
-};
-// mgpuMatmulEx16 on such a weight
-void matmul16(const void *a, const Weight16 &w, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
-              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, void *stream);
-inline void matmul16(const void *a, const void *w_nk, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
-                     int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, bool w_ready, void *stream) {
-  matmul16(a, Weight16{w_nk, w_ready}, bias, residual, out, M, N, Kp, dtype, out_dtype, act, stream);
-}
-
-// Whether a weight that a call of M rows converts itself keeps its [K, N] order: the conversion is then a plain
-// cast (defined beside the tile choice, gemm_tcgen05.cu).
-bool gemm_reads_rows(int64_t M, int64_t N, int64_t K);
-inline uint64_t weight16_bytes(int64_t K, int64_t N, bool rows) {
-  return static_cast<uint64_t>(rows ? K * ((N + 7) / 8 * 8) : N * ((K + 7) / 8 * 8)) * 2;
-}
+// mgpuMatmulEx16; w_ready: the weight was complete before this call (it does not come from a kernel
+// still queued), so the kernel may read it ahead of its dependency on the previous one.
+void matmul16(const void *a, const void *w_nk, const float *bias, const void *residual, void *out, int64_t M, int64_t N,
+              int64_t Kp, int32_t dtype, int32_t out_dtype, int32_t act, bool w_ready, void *stream);
 
 // Packed 16-bit [N, Kp] form of an fp32 [K, N] weight, from the constant cache when the weight
 // is a copy of a registered constant (defined in ops_init.cu).  A weight that is not is added to

@@ -54,9 +54,8 @@ MDC_CXX_API void checkCudaStatus(cudaError_t status) { check_cuda(status, "check
 
 // ---- mgpuMatmul: fp32 at the boundary, fp16 tensor-core math, fp32 accumulate ----
 // input [M,K] and weight [K,N] are converted on every call (the caller may have rewritten
-// them since the last one): input by a cast, the weight by one too, which the Gemm then reads as an
-// MN-major operand, or by the cast + transpose of a packed weight (gemm_reads_rows), or inside the Gemm
-// (gemm_takes_few_rows).  Scratch comes from the runtime's device pool.
+// them since the last one): input by a cast, weight by the cast + transpose that gives the
+// Gemm its K-contiguous operand.  Scratch comes from the runtime's device pool.
 // Exception: a weight buffer that the runtime knows to be an unmodified copy of a registered
 // constant (mgpuRegisterConstant + mgpuMemcpy, what a lowered graph does with its weights on
 // every call) is packed once; the packed copy lives with the registration.
@@ -79,23 +78,16 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
   bool w_cached = false;
   OperandList list;
-  void *w16;
-  const bool rows = gemm_reads_rows(M, N, K) && !mgpuConstantSourceOf(weight);
-  if (rows) {
-    w16 = mgpuMemAllocAsync(weight16_bytes(K, N, true), stream);
-    if (w16) list.weight(weight, w16, K, N, true);
-  } else {
-    w16 = packed_weight(weight, K, N, MGPU_DTYPE_F16, stream, &w_cached, &list);
-  }
+  void *w16 = packed_weight(weight, K, N, MGPU_DTYPE_F16, stream, &w_cached, &list);
   if (a16 && w16) {
-    // A small weight's conversion is a launch of its own, so a weight that the constant cache holds saves
-    // one (that is how a caller can see the cache at work, mgpuOpsLaunchCount).  From a million values on both
-    // operands share a launch: 2048 x 4096 x 4096 88.6 -> 87.1 us.
-    if (K * N < (int64_t(1) << 20)) list.launch(MGPU_DTYPE_F16, stream);
+    // The pack is a launch of its own, so a weight that the constant cache holds saves one (that is how
+    // a caller can see the cache at work, mgpuOpsLaunchCount).  One launch for both operands would
+    // save a dependent launch, about 2 us, in calls with other weights.
+    list.launch(MGPU_DTYPE_F16, stream);
     list.cast(input, a16, M, K, Kp);
     list.launch(MGPU_DTYPE_F16, stream);
-    matmul16(a16, Weight16{w16, false, rows, K}, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
-             MGPU_ACT_NONE, stream);
+    mgpuMatmulEx16(a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,
+                   MGPU_ACT_NONE, stream);
   }
   if (a16) mgpuMemFreeAsync(a16, stream);
   if (w16 && !w_cached) mgpuMemFreeAsync(w16, stream);

@@ -216,9 +216,7 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// How far apart (units of 16 bytes) the operands of a k-block's MMAs lie: 32 bytes along the swizzled rows of a
-// K-major tile, sixteen 128-byte rows of an MN-major one.
-constexpr int kStepKMajor = 2, kStepMnMajor = 128;
+constexpr int kStepKMajor = 2;
 // Two operand descriptors of 64-wide k-blocks: their low words move, the high ones are constant.
 struct KblockDesc {
   uint32_t a_lo, a_hi, b_lo, b_hi;

@@ -288,16 +288,6 @@ def _exact_matmul(m, M, N, K, seed):
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (65, 64, 8), (65, 63, 40), (130, 72, 129), (200, 1000, 136),   # one-wave, a ragged K; 63 columns: packed
-    (128, 4104, 200), (641, 192, 1032), (1024, 2304, 768),         # CTA pairs, several k-blocks a stage
-    (700, 1000, 1100), (3000, 712, 1500),                          # both operands in one launch
-    (5000, 264, 72), (20000, 328, 64), (9000, 136, 203)])          # persistent: tails of M, N and K
-def test_weight_in_its_own_order(m, M, N, K):
-    """mgpuMatmul converts a weight without transposing it; the Gemm reads it as an MN-major operand."""
-    _exact_matmul(m, M, N, K, 19)
-
-
-@pytest.mark.parametrize("M,N,K", [
     (1, 8, 8), (1, 1, 1), (5, 17, 24), (32, 16, 128), (33, 15, 129),    # a stage, its edges, one column tile
     (16, 1000, 2048), (64, 2368, 200), (64, 2369, 200), (3, 4100, 63),  # 16 columns a CTA, 32, odd widths
     (7, 1100, 3210), (40, 2400, 3333), (7, 48, 6001)])                  # the ring goes round; a long K that it leaves
