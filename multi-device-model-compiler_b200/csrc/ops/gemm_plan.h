@@ -24,9 +24,10 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms);
 // Whether gemm_few_rows takes a call whose fp32 weight would have to be converted first.  A CTA of it walks K
 // alone, at about 0.07 us per 16 values, so K is to be short or the columns many: 16 x 1000 x 2048 14.2 -> 10.5
 // us, 16 x 4096 x 4096 44 -> 28 (inputs out of memory), but 16 x 1000 x 4096 25.6 -> 27.6, 16 x 491 x 2136 19.4
-// -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.
+// -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.  Rows that are not
+// loaded in vectors take a shorter K still: 16 x 906 x 1751 21.5 -> 15.4, but 32 x 1221 x 3008 23.6 -> 25.6.
 inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K) {
-  return M <= 64 && N <= (1 << 30) && (K <= 1536 || K <= 3 * N) && K <= (1 << 30);
+  return M <= 64 && N <= (1 << 30) && (K <= 1536 || K <= (N % 4 == 0 ? 3 : 2) * N) && K <= (1 << 30);
 }
 
 // out[M, N] = a16[M, Kp] . w[K, N] + bias, fp16 operands, the weight as the caller has it

@@ -80,10 +80,10 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   OperandList list;
   void *w16 = packed_weight(weight, K, N, MGPU_DTYPE_F16, stream, &w_cached, &list);
   if (a16 && w16) {
-    // The pack is a launch of its own, so a weight that the constant cache holds saves one (that is how
-    // a caller can see the cache at work, mgpuOpsLaunchCount).  One launch for both operands would
-    // save a dependent launch, about 2 us, in calls with other weights.
-    list.launch(MGPU_DTYPE_F16, stream);
+    // A small weight's pack is a launch of its own, so a weight that the constant cache holds saves one (that
+    // is how a caller can see the cache at work, mgpuOpsLaunchCount).  From a million values on both operands
+    // share a launch: 2048 x 4096 x 4096 90.5 -> 89.3 us.
+    if (K * N < (int64_t(1) << 20)) list.launch(MGPU_DTYPE_F16, stream);
     list.cast(input, a16, M, K, Kp);
     list.launch(MGPU_DTYPE_F16, stream);
     mgpuMatmulEx16(a16, w16, bias, nullptr, output, M, N, Kp, MGPU_DTYPE_F16, MGPU_DTYPE_F32,

@@ -288,6 +288,15 @@ def _exact_matmul(m, M, N, K, seed):
 
 
 @pytest.mark.parametrize("M,N,K", [
+    (65, 64, 8), (66, 63, 41), (130, 72, 129), (200, 1000, 136),   # packed rows of 16 k values, and of 8 more
+    (128, 4104, 200), (641, 193, 1032), (5000, 264, 72),
+    (700, 1000, 1100), (3000, 711, 1500)])                         # both operands in one launch
+def test_packed_weights_are_exact(m, M, N, K):
+    """Edges of the packing's tiles: 64 columns, 64 k in groups of 16, sectors and half sectors."""
+    _exact_matmul(m, M, N, K, 19)
+
+
+@pytest.mark.parametrize("M,N,K", [
     (1, 8, 8), (1, 1, 1), (5, 17, 24), (32, 16, 128), (33, 15, 129),    # a stage, its edges, one column tile
     (16, 1000, 2048), (64, 2368, 200), (64, 2369, 200), (3, 4100, 63),  # 16 columns a CTA, 32, odd widths
     (7, 1100, 3210), (40, 2400, 3333), (7, 48, 6001)])                  # the ring goes round; a long K that it leaves
