@@ -119,3 +119,18 @@ def test_large_scores_do_not_overflow(m, D):
     ref = oracle.attention(qkv, None, B, S, H, D, round_mode=oracle.ROUND_F16)
     assert np.all(np.isfinite(got))
     assert oracle.max_rel_err(ref, got, floor_frac=1.0) <= TOL
+
+
+@pytest.mark.parametrize("heads,head_dim,batch,padded", [(12, 64, 20, False), (12, 64, 20, True), (8, 128, 16, False), (8, 128, 9, True)])
+def test_causal_item_order(m, heads, head_dim, batch, padded):
+    """A CTA takes several items: causal query tiles run slowest, the longest first.  The same sequences one at a
+    time (a single item per CTA, tiles fastest) give the same bits."""
+    rng = np.random.default_rng(heads + batch)
+    S = 300  # three query tiles, the last one partial
+    qkv = rng.standard_normal((batch * S, 3, heads, head_dim)).astype(np.float32)
+    lens = rng.integers(1, S + 1, batch).astype(np.int32) if padded else None
+    got = m.attention(qkv, lens, batch, S, heads, head_dim, causal=True)
+    for b in (0, 1, batch // 2, batch - 1):
+        one = m.attention(qkv[b * S:(b + 1) * S], None if lens is None else lens[b:b + 1], 1, S, heads, head_dim, causal=True)
+        n = S if lens is None else lens[b]
+        assert np.array_equal(got.reshape(batch, S, -1)[b, :n], one.reshape(S, -1)[:n]), b
