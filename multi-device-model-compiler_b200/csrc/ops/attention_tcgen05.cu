@@ -95,17 +95,13 @@ __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
 // Query tile of a work item, and the rest of the index.  Persistent CTAs take every 148th (or 444th) item; with
 // the tile fastest, a sequence of two or four of them gives a CTA, and an SM, the same tile every time: one key
 // tile for some and four for others under a causal mask.  Where a CTA takes more than one item, causal tiles
-// therefore run slowest, the longest first: 32 x 512 tokens, 12 x 64, 59.8 -> 46.3 us; 16 x 512, 8 x 128, 46.7 -> 33.9;
-// with padding 48 x 512 68.0 -> 58.5.  Padding alone does not gain (32 x 384 37.6 us, 39.3 in this order), nor does
+// therefore run slowest, the longest first: 32 x 512 tokens, 12 x 64, 59.8 -> 46.3 us; 16 x 512, 8 x 128, 46.5 -> 33.2;
+// with padding 48 x 512 67.5 -> 59.0.  Padding alone does not gain (32 x 384 37.6 us, 39.3 in this order), nor does
 // one item per CTA (3 x 300 11.9, 12.3).
 __device__ __forceinline__ int attn_tile(const AttnParams &p, int item, int q_tiles, int &rest) {
-  if (p.tiles_outer) {
-    const int per_tile = p.heads * p.batch, qt = item / per_tile;
-    rest = item - qt * per_tile;
-    return q_tiles - 1 - qt;
-  }
-  rest = item / q_tiles;
-  return item - rest * q_tiles;
+  const int d = p.tiles_outer ? p.heads * p.batch : q_tiles, quot = item / d, r = item - quot * d;
+  rest = p.tiles_outer ? r : quot;
+  return p.tiles_outer ? q_tiles - 1 - quot : r;
 }
 
 struct AttnItem {
@@ -487,10 +483,12 @@ constexpr size_t SMEM_BYTES = 3 * TILE_BYTES + 4 * 4096 + 1024;
 struct AttnItem64 {
   int q0, head, b, kv_end, n_kv;
 };
+// kOuter: p.tiles_outer, compiled in (as a run-time choice it cost the short items of this kernel 2 to 6 %)
+template <bool kOuter>
 __device__ __forceinline__ AttnItem64 attn_item64(const AttnParams &p, int item, int q_tiles) {
   AttnItem64 it;
-  int rest;
-  const int qt = attn_tile(p, item, q_tiles, rest);
+  const int d = kOuter ? p.heads * p.batch : q_tiles;
+  const int rest = kOuter ? item % d : item / d, qt = kOuter ? q_tiles - 1 - item / d : item % d;
   it.head = rest % p.heads;
   it.b = rest / p.heads;
   it.q0 = qt * attn64::BQ;
@@ -506,7 +504,7 @@ __device__ __forceinline__ AttnItem64 attn_item64(const AttnParams &p, int item,
 // per step (parity t & 1), so loads for step t+1 (of the same or of the next item) are issued
 // while step t is still in its softmax: K (and the next item's Q) as soon as S = Q.K^T of
 // step t has been computed, V as soon as P.V of step t has.
-template <typename T16>
+template <typename T16, bool kOuter>
 __global__ void __launch_bounds__(attn64::THREADS, attn64::CTAS_PER_SM)
 attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
                      const __grid_constant__ CUtensorMap tmap_out, const AttnParams p) {
@@ -573,7 +571,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
       // first item with at least one visible key
       int item = blockIdx.x;
       AttnItem64 cur{};
-      while (item < n_items && (cur = attn_item64(p, item, q_tiles)).n_kv == 0) item += gridDim.x;
+      while (item < n_items && (cur = attn_item64<kOuter>(p, item, q_tiles)).n_kv == 0) item += gridDim.x;
       uint32_t code = 0, t = 0, q_cnt = 0;
       if (item < n_items) {
         load_q(cur);
@@ -589,7 +587,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         if (n_j >= cur.n_kv) {
           n_j = 0;
           n_item = item + gridDim.x;
-          while (n_item < n_items && (nxt = attn_item64(p, n_item, q_tiles)).n_kv == 0) n_item += gridDim.x;
+          while (n_item < n_items && (nxt = attn_item64<kOuter>(p, n_item, q_tiles)).n_kv == 0) n_item += gridDim.x;
         }
         const bool has_next = n_item < n_items;
         if (j == 0) {
@@ -647,7 +645,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
     uint32_t t = 0;  // key tiles processed so far by this CTA (same count as the control thread)
     bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const AttnItem64 it = attn_item64(p, item, q_tiles);
+      const AttnItem64 it = attn_item64<kOuter>(p, item, q_tiles);
       const int q_local = it.q0 + r;  // query index inside the sequence
       float o_acc[D];
 #pragma unroll
@@ -815,10 +813,10 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
   if (warp == 4) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-template <typename T16>
-static void launch_attention64(const CUtensorMap &tm, const CUtensorMap &tmo, AttnParams p, int64_t n_items,
+template <typename T16, bool kOuter>
+static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &tmo, AttnParams p, int64_t n_items,
                                const DeviceInfo &di, cudaStream_t s) {
-  auto kern = attention_d64_kernel<T16>;
+  auto kern = attention_d64_kernel<T16, kOuter>;
   static bool set_on[64] = {false};  // the attribute is per device
   bool &set = set_on[(di.device >= 0 && di.device < 64) ? di.device : 0];
   if (!set) {
@@ -828,9 +826,16 @@ static void launch_attention64(const CUtensorMap &tm, const CUtensorMap &tmo, At
     set = true;
   }
   const int64_t slots = static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM;
-  p.tiles_outer = p.causal && n_items > slots;
+  p.tiles_outer = kOuter;
   dim3 grid(static_cast<unsigned>(n_items < slots ? n_items : slots));
   check_cuda(launch_chain(kern, grid, dim3(attn64::THREADS), attn64::SMEM_BYTES, s, 1, tm, tmo, p), "launch attention");
+}
+
+template <typename T16>
+static void launch_attention64(const CUtensorMap &tm, const CUtensorMap &tmo, const AttnParams &p, int64_t n_items,
+                               const DeviceInfo &di, cudaStream_t s) {
+  if (p.causal && n_items > static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM) launch_attention64_order<T16, true>(tm, tmo, p, n_items, di, s);
+  else launch_attention64_order<T16, false>(tm, tmo, p, n_items, di, s);
 }
 
 template <typename T16, int HD>
