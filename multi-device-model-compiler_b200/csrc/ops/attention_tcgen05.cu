@@ -90,8 +90,6 @@ __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
   return *reinterpret_cast<uint32_t *>(&h);
 }
 
-// One unit of work: 128 queries of one (sequence, head).  Decoded identically by all three
-// roles, so they walk the same sequence of key tiles.
 // Query tile of a work item, and the rest of the index.  Persistent CTAs take every 148th (or 444th) item; with
 // the tile fastest, a sequence of two or four of them gives a CTA, and an SM, the same tile every time: one key
 // tile for some and four for others under a causal mask.  Where a CTA takes more than one item, causal tiles
@@ -104,6 +102,8 @@ __device__ __forceinline__ int attn_tile(const AttnParams &p, int item, int q_ti
   return p.tiles_outer ? q_tiles - 1 - quot : r;
 }
 
+// One unit of work: 128 queries of one (sequence, head).  Decoded identically by all three
+// roles, so they walk the same sequence of key tiles.
 struct AttnItem {
   int q0, head, b, kv_end, n_kv;
 };
