@@ -35,7 +35,7 @@ enum { MGPU_ACT_NONE = 0, MGPU_ACT_RELU = 1, MGPU_ACT_GELU_ERF = 2, MGPU_ACT_GEL
  * rounded to fp16 for the tensor cores, accumulation is fp32 (the reference asks cuBLASLt
  * for CUBLAS_COMPUTE_32F_FAST_16F, Ops.cu:74-75); bias and output stay fp32.  Every element is
  * one sum over K in one order, whatever M and N are: a row's result is the same, bit for bit, in a
- * batch of any size. */
+ * batch of any size.  output may overlap input or weight (both are read before the first store). */
 void mgpuMatmul(float *input, float *weight, float *bias, float *output, int64_t M, int64_t N,
                 int64_t K, mgpu_cuda_stream_t stream);
 

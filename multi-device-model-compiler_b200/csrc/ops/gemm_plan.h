@@ -26,8 +26,12 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms);
 // us, 16 x 4096 x 4096 44 -> 28 (inputs out of memory), but 16 x 1000 x 4096 25.6 -> 27.6, 16 x 491 x 2136 19.4
 // -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.  Rows that are not
 // loaded in vectors take a shorter K still: 16 x 906 x 1751 21.5 -> 15.4, but 32 x 1221 x 3008 23.6 -> 25.6.
-inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K) {
-  return M <= 64 && N <= (1 << 30) && (K <= 1536 || K <= (N % 4 == 0 ? 3 : 2) * N) && K <= (1 << 30);
+// An output that overlaps the weight stays with the conversion too: it has read the whole weight before the
+// first store, while here CTAs still read columns of it that others have finished and stored over.
+inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w, const float *out) {
+  if (M > 64 || N > (1 << 30) || K > (1 << 30) || (K > 1536 && K > (N % 4 == 0 ? 3 : 2) * N)) return false;
+  const uintptr_t w0 = reinterpret_cast<uintptr_t>(w), o0 = reinterpret_cast<uintptr_t>(out);
+  return o0 >= w0 + static_cast<uintptr_t>(K) * N * 4 || w0 >= o0 + static_cast<uintptr_t>(M) * N * 4;
 }
 
 // out[M, N] = a16[M, Kp] . w[K, N] + bias, fp16 operands, the weight as the caller has it

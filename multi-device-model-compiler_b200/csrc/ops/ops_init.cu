@@ -65,7 +65,7 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   if (K <= 0) { fail("mgpuMatmul: K must be positive"); return; }
   if (!device_info().ok) return;
   const int64_t Kp = (K + 7) / 8 * 8;
-  if (gemm_takes_few_rows(M, N, K) && !mgpuConstantSourceOf(weight)) {
+  if (gemm_takes_few_rows(M, N, K, weight, output) && !mgpuConstantSourceOf(weight)) {
     void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
     if (!a16) return;
     OperandList list;

@@ -320,6 +320,24 @@ def test_few_rows_off_their_boundaries(m, offset):
     assert np.array_equal(got, a @ w + b)
 
 
+@pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
+@pytest.mark.parametrize("M,N,K", [(16, 1000, 1024), (40, 2400, 500)])
+def test_output_may_overlap_the_weight(m, entry, M, N, K):
+    """The whole weight is read before the first store, with few rows too."""
+    rng = np.random.default_rng(41)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    da, db, pad = m.to_device(a), m.to_device(b), M * N
+    for at in (0, 1, K * N // 2, K * N - 4, -M * N + 4):  # of the output, in floats from the weight
+        mem = m.to_device(np.concatenate([np.zeros(pad, np.float32), w.ravel(), np.zeros(pad, np.float32)]))
+        first = mem.ptr + 4 * pad
+        getattr(m.ops(), entry)(da.ptr, first, db.ptr, first + 4 * at, M, N, K, None)
+        got = m.to_host(mem, (M, N), np.float32, offset_bytes=4 * (pad + at))
+        assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+        m.check(entry)
+        assert np.array_equal(got, a @ w + b), at
+
+
 def test_few_rows_keep_infinities_to_themselves(m):
     # a row or column with an infinity leaves the others alone
     rng = np.random.default_rng(31)
