@@ -202,8 +202,10 @@ struct OperandJobs {
   int n, late;
 };
 
-template <typename T16>
-__global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const OperandJobs jobs) {
+// kOdd: there is a weight among them whose packed rows are an odd multiple of 16 bytes (compiled apart: it
+// costs registers, and 5 % of a 4096 x 1001 weight's time).
+template <typename T16, bool kOdd>
+__global__ void __launch_bounds__(kEwBlock, 8) prepare_operands_kernel(const OperandJobs jobs) {
   static_assert(kEwBlock == OperandList::kThreads, "the 64 x 64 tiles are walked by 256 threads");
   if (!jobs.late) pdl_launch_dependents();
   pdl_wait();
@@ -255,9 +257,12 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
   const uint32_t b32 = static_cast<uint32_t>(b), tk = b32 / static_cast<uint32_t>(job.tiles_n);
   const int64_t k0 = static_cast<int64_t>(tk) * 64 + (threadIdx.x >> 6) * 16;
   const int64_t n = static_cast<int64_t>(b32 - tk * job.tiles_n) * 64 + (threadIdx.x & 63);
-  if (n >= N || k0 >= Kp) return;
+  const bool odd_pitch = kOdd && Kp % 16 != 0;
+  if (!odd_pitch && (n >= N || k0 >= Kp)) return;
   const float *w = job.src + k0 * N + n;
-  const int live = K - k0 < 16 ? static_cast<int>(K - k0) : 16;  // at most 0 in the padding
+  int live = K - k0 < 16 ? static_cast<int>(K - k0) : 16;  // at most 0 in the padding
+  const int room = !kOdd ? 16 : n >= N ? 0 : Kp - k0 < 16 ? static_cast<int>(Kp - k0) : 16;  // of an odd row: 16, 8 or none
+  if (kOdd && room <= 0) live = 0;
   float v[16];
   if (live == 16) {
 #pragma unroll
@@ -270,12 +275,40 @@ __global__ void __launch_bounds__(kEwBlock) prepare_operands_kernel(const Operan
 #pragma unroll
   for (int e = 0; e < 8; ++e) o[e] = pack_pair<T16>(v[2 * e], v[2 * e + 1]);
   T16 *dst = out + n * Kp + k0;
-  if (job.vec_ok) {
-    st_global_32B(dst, o);
-  } else {
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-    if (k0 + 8 < Kp) *reinterpret_cast<uint4 *>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+  const uint4 lo = make_uint4(o[0], o[1], o[2], o[3]), hi = make_uint4(o[4], o[5], o[6], o[7]);
+  if (!odd_pitch) {
+    if (job.vec_ok) {
+      st_global_32B(dst, o);
+    } else {
+      *reinterpret_cast<uint4 *>(dst) = lo;
+      *reinterpret_cast<uint4 *>(dst + 8) = hi;
+    }
+    return;
   }
+  // Every second row starts inside a sector.  Its groups hand their upper halves on, so that these rows too are
+  // written in whole sectors but for the ends of the tile.  With half sectors throughout 2048 x 1024 x 1000 took
+  // 22.1 us a call (20.4 now) and 3000 x 3000 x 3000 72.8 (71.9), the latter's conversion by itself 23.0 (21.0).
+  // Lanes of such rows reading 8 k further down instead: the weight alone as fast, but the calls 21.0 and 78 us one
+  // after another, as lines that two lanes share did not stay in what L1 the Gemm ahead left.
+  __shared__ uint4 upper[4][32];  // of two neighbouring columns one has such a row
+  uint4 *mine = &upper[threadIdx.x >> 6][(threadIdx.x & 63) >> 1];
+  const bool in_sector = (reinterpret_cast<uintptr_t>(dst) & 31u) != 0;
+  if (in_sector) *mine = hi;
+  __syncthreads();
+  if (room <= 0) return;
+  if (!in_sector) {
+    if (room == 16) st_global_32B(dst, o);
+    else *reinterpret_cast<uint4 *>(dst) = lo;
+    return;
+  }
+  if (threadIdx.x >= 64) {
+    const uint4 before = *(mine - 32);
+    const uint32_t q[8] = {before.x, before.y, before.z, before.w, lo.x, lo.y, lo.z, lo.w};
+    st_global_32B(dst - 8, q);
+  } else {
+    *reinterpret_cast<uint4 *>(dst) = lo;
+  }
+  if (threadIdx.x >= 192 && room == 16) *reinterpret_cast<uint4 *>(dst + 8) = hi;
 }
 
 void OperandList::launch(int32_t dtype, void *stream, bool late) {
@@ -290,11 +323,13 @@ void OperandList::launch(int32_t dtype, void *stream, bool late) {
   a.n = n, a.late = late ? 1 : 0;
   cudaStream_t s = as_stream(stream);
   ProfileScope prof(kCatElementwise, s);
-  const dim3 grid(static_cast<unsigned>(blocks));
-  if (dtype == MGPU_DTYPE_F16)
-    check_cuda(launch_chain(prepare_operands_kernel<__half>, grid, dim3(kEwBlock), 0, s, 1, a), "launch prepare_operands");
-  else
-    check_cuda(launch_chain(prepare_operands_kernel<__nv_bfloat16>, grid, dim3(kEwBlock), 0, s, 1, a), "launch prepare_operands");
+  bool odd = false;
+  for (int i = 0; i < n; ++i) odd |= jobs[i].tiles_n != 0 && jobs[i].pitch % 16 != 0;
+  auto launch = [&](auto kern) {
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(blocks)), dim3(kEwBlock), 0, s, 1, a), "launch prepare_operands");
+  };
+  if (dtype == MGPU_DTYPE_F16) odd ? launch(prepare_operands_kernel<__half, true>) : launch(prepare_operands_kernel<__half, false>);
+  else odd ? launch(prepare_operands_kernel<__nv_bfloat16, true>) : launch(prepare_operands_kernel<__nv_bfloat16, false>);
   launched("mdc_prepare_operands");
   clear();
 }

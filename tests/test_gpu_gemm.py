@@ -296,6 +296,25 @@ def test_packed_weights_are_exact(m, M, N, K):
     _exact_matmul(m, M, N, K, 19)
 
 
+@pytest.mark.parametrize("offset", [0, 16])
+@pytest.mark.parametrize("K,N", [(1, 1), (7, 5), (8, 64), (9, 65), (16, 3), (24, 130), (57, 66), (64, 64), (65, 1), (72, 129), (121, 64), (1000, 67)])
+def test_packed_rows_on_and_off_sectors(m, K, N, offset):
+    """Rows of an odd multiple of 16 bytes start alternately on and inside a 32-byte sector; a weight may be packed to
+    any multiple of 16 bytes.  Every value once, zeros in the padding, the neighbours untouched."""
+    rng = np.random.default_rng(K * 131 + N)
+    w, Kp = rng.standard_normal((K, N)).astype(np.float32), (K + 7) // 8 * 8
+    dw, out = m.to_device(w), m.to_device(np.full(N * Kp + 64, 0x5a5a, np.uint16))
+    for dtype in (m.F16, m.BF16):
+        m.ops().mgpuPackWeight(dw.ptr, out.ptr + 32 + offset, K, N, dtype, None)
+        got = m.to_host(out, (N * Kp + 64,), np.uint16)
+        m.check("mgpuPackWeight")
+        first = 16 + offset // 2
+        ref = np.zeros((N, Kp), np.uint16)
+        ref[:, :K] = m.encode16(np.ascontiguousarray(w.T), dtype).view(np.uint16)
+        assert np.array_equal(got[first:first + N * Kp].reshape(N, Kp), ref)
+        assert (got[:first] == 0x5a5a).all() and (got[first + N * Kp:] == 0x5a5a).all()
+
+
 @pytest.mark.parametrize("M,N,K", [
     (1, 8, 8), (1, 1, 1), (5, 17, 24), (32, 16, 128), (33, 15, 129),    # a stage, its edges, one column tile
     (16, 1000, 2048), (64, 2368, 200), (64, 2369, 200), (3, 4100, 63),  # 16 columns a CTA, 32, odd widths
