@@ -204,6 +204,9 @@ void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *output, 
 
 /* Number of kernels this library has launched since load (for launch accounting). */
 uint64_t mgpuOpsLaunchCount(void);
+/* Number of fp32 weights this library has converted to its packed form since load: a weight that the
+ * constant cache holds, or that a Gemm of a few rows reads itself, is not packed. */
+uint64_t mgpuOpsWeightPackCount(void);
 
 /* Per-kernel timing for measurements.  Between Begin and End every kernel launch of this
  * library is bracketed by two CUDA events on its stream; End waits for them and returns,

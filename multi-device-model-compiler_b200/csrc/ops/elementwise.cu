@@ -9,6 +9,7 @@
 namespace mdc {
 
 std::atomic<uint64_t> g_launch_count{0};
+static std::atomic<uint64_t> g_pack_count{0};
 
 bool pdl_enabled() {
   static const bool on = [] {
@@ -324,7 +325,10 @@ void OperandList::launch(int32_t dtype, void *stream, bool late) {
   cudaStream_t s = as_stream(stream);
   ProfileScope prof(kCatElementwise, s);
   bool odd = false;
-  for (int i = 0; i < n; ++i) odd |= jobs[i].tiles_n != 0 && jobs[i].pitch % 16 != 0;
+  uint64_t packs = 0;
+  for (int i = 0; i < n; ++i)
+    if (jobs[i].tiles_n != 0) ++packs, odd |= jobs[i].pitch % 16 != 0;
+  g_pack_count.fetch_add(packs, std::memory_order_relaxed);
   auto launch = [&](auto kern) {
     check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(blocks)), dim3(kEwBlock), 0, s, 1, a), "launch prepare_operands");
   };
@@ -339,6 +343,7 @@ void OperandList::launch(int32_t dtype, void *stream, bool late) {
 using namespace mdc;
 
 MDC_API uint64_t mgpuOpsLaunchCount(void) { return g_launch_count.load(); }
+MDC_API uint64_t mgpuOpsWeightPackCount(void) { return g_pack_count.load(); }
 
 MDC_API void mgpuOpsProfileBegin(void) {
   g_spans.clear();
