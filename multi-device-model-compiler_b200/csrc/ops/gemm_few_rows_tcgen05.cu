@@ -269,8 +269,7 @@ void gemm_few_rows(const void *a16, const float *w, const float *bias, float *ou
   p.err = err;
   CUtensorMap ta;
   if (!encode_tmap_2d(&ta, a16, MGPU_DTYPE_F16, Kp, static_cast<uint64_t>(M), Kp * 2, 64, static_cast<uint32_t>(p.box_m))) return;
-  // 16 columns spread a narrow weight over more SMs; 32 read whole lines of a wide one
-  if ((N + 15) / 16 <= di.sms) launch_few_rows<16>(ta, p, s);
+  if (few_rows_columns(N, di.sms) == 16) launch_few_rows<16>(ta, p, s);
   else launch_few_rows<32>(ta, p, s);
 }
 

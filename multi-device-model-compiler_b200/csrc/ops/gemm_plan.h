@@ -1,6 +1,7 @@
 // Tile choice of the tensor-core Gemms.
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 
@@ -21,16 +22,47 @@ constexpr int kOneWaveMaxSmem = 226 * 1024;  // the rest of the 227 KiB is the k
 
 GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms);
 
-// Whether gemm_few_rows takes a call whose fp32 weight would have to be converted first.  A CTA of it walks K
-// alone, at about 0.07 us per 16 values, so K is to be short or the columns many: 16 x 1000 x 2048 14.2 -> 10.5
-// us, 16 x 4096 x 4096 44 -> 28 (inputs out of memory), but 16 x 1000 x 4096 25.6 -> 27.6, 16 x 491 x 2136 19.4
-// -> 21.5 and 64 x 257 x 4095 25.6 -> 31.7, which stay with a conversion over the whole chip.  Rows that are not
-// loaded in vectors take a shorter K still: 16 x 906 x 1751 21.5 -> 15.4, but 32 x 1221 x 3008 23.6 -> 25.6.
-// An output that overlaps the weight stays with the conversion too: it has read the whole weight before the
+// Columns per CTA of gemm_few_rows: 16 spread a narrow weight over more SMs; 32 read whole lines of a wide one.
+inline int few_rows_columns(int64_t N, int sms) { return (N + 15) / 16 <= sms ? 16 : 32; }
+
+// Largest K that gemm_few_rows takes.  A CTA of it walks K alone, so its time grows with K and hardly with N;
+// converting the weight first goes over the whole chip, and its time grows with K and N: few rows win at a short K,
+// and at any K once there are columns enough for the SMs.  How many depends on how a row of W comes: in 16-byte
+// vectors or value by value, and for 32 columns in whole lines or not.  us a call, converted / few rows, 16 rows,
+// inputs out of memory:
+//   16 columns, vectors      256 x 1024 7.3 / 7.1     1000 x 1536 9.7 / 9.1     1000 x 3072 14.5 / 17.4
+//                            1300 x 2048 12.6 / 14.4  1800 x 3072 18.0 / 18.1   2000 x 6144 31.7 / 27.4
+//                            1000 x 2048 13.3 / 13.6, out of L2 12.2 / 10.8;  1344 x 3200 16.4 / 16.6, 14.9 / 13.9
+//   16 columns, by value     601 x 768 7.8 / 7.1      1001 x 1536 9.9 / 9.9     2001 x 1536 12.1 / 10.3
+//                            2001 x 2048 15.4 / 16.4
+//   32 columns, whole lines  2400 x 6144 32.1 / 31.2  2816 x 4096 24.4 / 23.0   4096 x 4096 30.3 / 23.6
+//   32 columns, vectors      2600 x 1280 11.1 / 10.2  2600 x 2048 15.8 / 17.5   3700 x 3072 25.2 / 25.0
+//   32 columns, by value     2369 x 1280 11.4 / 10.8  2401 x 1536 14.4 / 16.2   4401 x 3072 28.3 / 26.8
+//                            with 64 rows 2369 x 768 10.9 / 9.1, x 1024 11.7 / 13.0
+// Beyond one CTA per SM the second wave costs as much as the first (5000 x 1024 12.4 / 15.7, 32000 x 768 38.9 / 48.5),
+// until the copy of the weight no longer stays in L2: 50257 x 768 81.4 / 73.3, 32000 x 2048 107 / 94.
+inline int64_t few_rows_max_k(int64_t M, int64_t N, bool vectors, bool lines, int sms) {
+  if (few_rows_columns(N, sms) == 16) {
+    if (!vectors) return std::min<int64_t>(1536, std::max<int64_t>(512, 5 * N / 4));
+    if (N >= 1700) return 3 * N;
+    return std::max<int64_t>(1024, N % 8 == 0 ? 5 * N / 2 : std::min<int64_t>(5 * N / 2, 1792));  // rows on sectors or not
+  }
+  if (lines) return 3 * N;
+  if (vectors) return N >= 3700 ? 3 * N : 1280;
+  return N >= 4000 ? 2 * N : M <= 32 ? 1280 : 768;
+}
+
+// Whether gemm_few_rows takes a call whose fp32 weight would have to be converted first.
+// An output that overlaps the weight stays with the conversion: it has read the whole weight before the
 // first store, while here CTAs still read columns of it that others have finished and stored over.
-inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w, const float *out) {
-  if (M > 64 || N > (1 << 30) || K > (1 << 30) || (K > 1536 && K > (N % 4 == 0 ? 3 : 2) * N)) return false;
+inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w, const float *out, int sms) {
+  if (M > 64 || N > (1 << 30) || K > (1 << 30)) return false;
   const uintptr_t w0 = reinterpret_cast<uintptr_t>(w), o0 = reinterpret_cast<uintptr_t>(out);
+  if (N > 32 * sms) {
+    if (K * N < 38000000) return false;
+  } else if (K > few_rows_max_k(M, N, N % 4 == 0 && (w0 & 15u) == 0, N % 32 == 0 && (w0 & 127u) == 0, sms)) {
+    return false;
+  }
   return o0 >= w0 + static_cast<uintptr_t>(K) * N * 4 || w0 >= o0 + static_cast<uintptr_t>(M) * N * 4;
 }
 

@@ -875,7 +875,7 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   void *w16 = base + a_bytes;
   cudaStream_t s = as_stream(stream);
   OperandList list;
-  if (gemm_takes_few_rows(M, N, K, weight, output)) {
+  if (gemm_takes_few_rows(M, N, K, weight, output, di.sms)) {
     list.cast(input, a16, M, K, Kp);
     list.launch(MGPU_DTYPE_F16, stream, true);
     gemm_few_rows(a16, weight, bias, output, M, N, K, s);

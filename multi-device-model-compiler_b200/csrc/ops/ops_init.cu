@@ -63,9 +63,10 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
                         int64_t K, void *stream) {
   if (M <= 0 || N <= 0) return;
   if (K <= 0) { fail("mgpuMatmul: K must be positive"); return; }
-  if (!device_info().ok) return;
+  const DeviceInfo &di = device_info();
+  if (!di.ok) return;
   const int64_t Kp = (K + 7) / 8 * 8;
-  if (gemm_takes_few_rows(M, N, K, weight, output) && !mgpuConstantSourceOf(weight)) {
+  if (gemm_takes_few_rows(M, N, K, weight, output, di.sms) && !mgpuConstantSourceOf(weight)) {
     void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
     if (!a16) return;
     OperandList list;

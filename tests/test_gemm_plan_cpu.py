@@ -14,18 +14,36 @@ PROGRAM = r"""
 #include <cstdio>
 using mdc::gemm_takes_few_rows;
 int main() {
-  static float mem[4096];
+  alignas(16) static float mem[4096];
   float *w = mem + 1024;
   const int64_t M = 3, N = 20, K = 12;  // 240 floats of weight, 60 of output
   for (int64_t at = -1024; at + M * N <= 3072; ++at) {
     const bool overlap = at < K * N && at + M * N > 0;
-    assert(gemm_takes_few_rows(M, N, K, w, w + at) == !overlap);
+    assert(gemm_takes_few_rows(M, N, K, w, w + at, 148) == !overlap);
   }
-  const float *far = reinterpret_cast<const float *>(uintptr_t(1) << 44);
-  assert(gemm_takes_few_rows(64, 1, 1536, w, far) && !gemm_takes_few_rows(65, 1, 1, w, far));
-  assert(!gemm_takes_few_rows(1, 512, 1537, w, far) && gemm_takes_few_rows(1, 516, 1537, w, far));
-  assert(gemm_takes_few_rows(1, 1 << 30, 1 << 20, w, reinterpret_cast<const float *>(uintptr_t(1) << 60)));
-  assert(!gemm_takes_few_rows(1, 1 << 30, 1 << 20, w, reinterpret_cast<const float *>(uintptr_t(1) << 50)));
+  alignas(128) static float far_mem[64];
+  const float *out = reinterpret_cast<const float *>(uintptr_t(1) << 60), *v = far_mem;
+  auto last_k = [&](int64_t M, int64_t N, const float *w) {  // the largest K taken, all shorter ones taken too
+    int64_t k = 0;
+    while (gemm_takes_few_rows(M, N, k + 1, w, out, 148)) ++k;
+    for (int64_t longer = k + 1; longer < k + 4096; longer += 37) assert(!gemm_takes_few_rows(M, N, longer, w, out, 148));
+    return k;
+  };
+  assert(gemm_takes_few_rows(64, 1, 512, v, out, 148) && !gemm_takes_few_rows(65, 1, 1, v, out, 148));
+  // 16 columns a CTA: in vectors, off 16 bytes or an odd width value by value
+  assert(last_k(1, 64, v) == 1024 && last_k(1, 600, v) == 1500 && last_k(1, 1000, v) == 2500 && last_k(1, 1300, v) == 1792);
+  assert(last_k(1, 1700, v) == 5100 && last_k(1, 2368, v) == 7104 && last_k(1, 2368, v + 4) == 7104);
+  assert(last_k(1, 1, v) == 512 && last_k(1, 601, v) == 751 && last_k(1, 2367, v) == 1536 && last_k(1, 2368, v + 1) == 1536);
+  // 32 columns: whole lines, vectors, value by value
+  assert(last_k(64, 2400, v) == 7200 && last_k(64, 2400, v + 4) == 1280 && last_k(64, 2400, v + 1) == 768);
+  assert(last_k(33, 2372, v) == 1280 && last_k(33, 3700, v) == 11100 && last_k(33, 4092, v + 4) == 12276);
+  assert(last_k(32, 2369, v) == 1280 && last_k(33, 2369, v) == 768 && last_k(33, 4001, v) == 8002 && last_k(1, 4736, v) == 14208);
+  // more than one CTA per SM: weights that do not stay in L2
+  assert(!gemm_takes_few_rows(1, 4737, 8021, v, out, 148) && gemm_takes_few_rows(1, 4737, 8022, v, out, 148));
+  assert(!gemm_takes_few_rows(1, 32000, 1187, v, out, 148) && gemm_takes_few_rows(1, 32000, 1188, v, out, 148));
+  // ranges of bytes beyond 32 bits
+  assert(gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, out, 148));
+  assert(!gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, reinterpret_cast<const float *>(uintptr_t(1) << 50), 148));
   std::puts("ok");
 }
 """
