@@ -190,7 +190,7 @@ cast_pad_rows(const float *__restrict__ src, T16 *__restrict__ dst, int64_t R, i
 // All operands of a call in one launch; a block belongs to one job.
 //   cast: kCastItems elements of a contiguous array, or kPadItems of rows that are padded.
 //   pack: weight fp32 [K, N] (N contiguous) -> 16-bit [N, Kp] (K contiguous), zero padded to Kp, in tiles of
-//         64 x 64.  A lane reads 16 values of its column, all in flight, a line per warp and k whatever N is, and
+//         64 x 64.  A lane reads 16 values of its column, all in flight, one line or two per warp and k, and
 //         writes one whole sector; through shared memory (16-byte reads, 16-byte writes of eight values)
 //         the five operands of an 8 x 256 token layer, 1024 wide, took 2.9 us longer (98.6 -> 95.7 us a call).
 // Bound by HBM bytes (6 per element).  One launch instead of one per operand: the tail of one

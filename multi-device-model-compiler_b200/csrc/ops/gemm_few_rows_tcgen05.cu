@@ -5,12 +5,12 @@
 // to be read back, and this kernel is bound by the bytes of W (4 K N) or, where those are few, by
 // latency.  Eight warps read W straight into registers, 16 vector loads of a thread in flight (64 KB an
 // SM); a warp fills a ring stage of 128 k x 16 columns or 64 k x 32 by itself, converting to core
-// matrices of 8 columns x 8 k.  A comes by TMA.  W does not wait for the kernel that converts A: that
+// matrices of 8 columns x 8 k.  A comes by TMA.  W and the bias do not wait for the kernel that converts A: that
 // kernel lets this one start after its own wait, so what is older than it is complete.
 //
-// Whole call, before (conversion of W, of A, one-wave Gemm) and after: 16 x 1000 x 2048 14.2 -> 9.3 us one
-// after another; cold inputs: 16 x 4096 x 4096 44 -> 27.6 (2.4 TB/s), 48 x 1408 x 577 19.5 -> 13.3, 16 x 768 x 320
-// 13.4 -> 9.2.  Sixteen loading warps instead of eight: 10.9 for the first.
+// Whole call, with the weight converted and read here: 16 x 1000 x 2048 12.2 / 10.8 us one after another out of L2,
+// 13.3 / 13.6 out of memory; out of memory also 16 x 4096 x 4096 30.3 / 23.6 (2.8 TB/s), 16 x 1000 x 512 7.4 / 6.0;
+// more of them in gemm_plan.h.
 //
 // K order: one sum over K in steps of 16, as in the other Gemm kernels; a row's bits do not depend on
 // which of them takes a call.
@@ -26,6 +26,9 @@ namespace fewrows {
 constexpr int LOAD_WARPS = 8;
 constexpr int THREADS = 64 + LOAD_WARPS * 32;
 constexpr int MAX_STAGES = 24;
+constexpr int MAX_SMEM = 224 * 1024;
+// an MMA reads 128 rows of A whatever the box holds
+constexpr int fixed_bytes(int box_m) { return 1024 + (128 - box_m) * 128; }
 // Columns in groups of eight, k in groups of eight: 128-byte core matrices.  They lie 144 bytes apart along the
 // columns, which puts the eight 16-byte stores of a quarter-warp on different banks.
 constexpr int SBO = 144;
@@ -34,7 +37,17 @@ struct Cfg {
   static constexpr int STAGE_K = 2048 / BN;                      // a warp's 16 loads of 4 values per lane
   static constexpr int LBO = BN == 16 ? 288 : 4 * SBO;           // bytes from one group of eight k to the next
   static constexpr int B_BYTES = STAGE_K / 8 * LBO;              // 4608
+  static constexpr int stage_bytes(int box_m) { return STAGE_K / 64 * box_m * 128 + B_BYTES; }
+  static constexpr int stages(int box_m) {
+    const int n = (MAX_SMEM - fixed_bytes(box_m)) / stage_bytes(box_m);
+    return n < MAX_STAGES ? n : MAX_STAGES;
+  }
 };
+// Warp w fills stages' worth w, w + 8, ... of K and waits for its stage's previous use by parity alone: with fewer
+// stages than warps one would be two uses ahead and pass.
+template <int BN>
+constexpr bool ring_holds_every_warp = Cfg<BN>::stages(32) >= LOAD_WARPS && Cfg<BN>::stages(64) >= LOAD_WARPS;
+static_assert(ring_holds_every_warp<16> && ring_holds_every_warp<32>, "a stage for every loading warp");
 }  // namespace fewrows
 
 struct FewRowsParams {
@@ -59,7 +72,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
   volatile uint32_t *abort_flag = &abort_flag_s;
   uint8_t *a_s = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
   const int a_kb = p.box_m * 128, a_bytes = KBS * a_kb;
-  // an MMA reads 128 rows of A whatever the box holds: what follows the last stage's A is W's part
+  // what an MMA reads beyond the last stage's A must not be W's part
   uint8_t *b_s = a_s + p.stages * a_bytes + (128 - p.box_m) * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col0 = blockIdx.x * BN;
@@ -232,21 +245,17 @@ template <int BN>
 static void launch_few_rows(const CUtensorMap &ta, FewRowsParams &p, cudaStream_t s) {
   using C = fewrows::Cfg<BN>;
   auto kern = gemm_few_rows_kernel<BN>;
-  constexpr int kMaxSmem = 224 * 1024;
   static bool set_on[64] = {false};  // the attribute is per device
   const int dev = device_info().device;
   bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
   if (!set) {
-    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "cudaFuncSetAttribute(gemm few rows)"))
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fewrows::MAX_SMEM), "cudaFuncSetAttribute(gemm few rows)"))
       return;
     set = true;
   }
   p.steps = (p.K + C::STAGE_K - 1) / C::STAGE_K;
-  const int stage = C::STAGE_K / 64 * p.box_m * 128 + C::B_BYTES, fixed = 1024 + (128 - p.box_m) * 128;
-  p.stages = (kMaxSmem - fixed) / stage;
-  if (p.stages > fewrows::MAX_STAGES) p.stages = fewrows::MAX_STAGES;
-  if (p.stages > p.steps) p.stages = p.steps;
-  const size_t smem = static_cast<size_t>(fixed) + static_cast<size_t>(p.stages) * stage;
+  p.stages = p.steps < C::stages(p.box_m) ? p.steps : C::stages(p.box_m);  // fewer only where none is used twice
+  const size_t smem = static_cast<size_t>(fewrows::fixed_bytes(p.box_m)) + static_cast<size_t>(p.stages) * C::stage_bytes(p.box_m);
   {
     ProfileScope prof(kCatGemm, s);
     check_cuda(launch_chain(kern, dim3(static_cast<unsigned>((p.N + BN - 1) / BN)), dim3(fewrows::THREADS), smem, s, 1, ta, p),

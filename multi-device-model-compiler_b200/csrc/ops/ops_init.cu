@@ -55,7 +55,8 @@ MDC_CXX_API void checkCudaStatus(cudaError_t status) { check_cuda(status, "check
 // ---- mgpuMatmul: fp32 at the boundary, fp16 tensor-core math, fp32 accumulate ----
 // input [M,K] and weight [K,N] are converted on every call (the caller may have rewritten
 // them since the last one): input by a cast, weight by the cast + transpose that gives the
-// Gemm its K-contiguous operand.  Scratch comes from the runtime's device pool.
+// Gemm its K-contiguous operand.  Scratch comes from the runtime's device pool.  With a few rows
+// (gemm_takes_few_rows) only the input is converted ahead; the Gemm rounds the weight as it loads it.
 // Exception: a weight buffer that the runtime knows to be an unmodified copy of a registered
 // constant (mgpuRegisterConstant + mgpuMemcpy, what a lowered graph does with its weights on
 // every call) is packed once; the packed copy lives with the registration.

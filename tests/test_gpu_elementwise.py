@@ -25,6 +25,31 @@ def test_add_bit_exact(m, shape):
     assert np.array_equal(got.view(np.uint32), oracle.add(a, b).view(np.uint32))
 
 
+def test_chain_without_waits(m):
+    """Each kernel is set up while the one ahead of it drains: values and buffers handed on and used again."""
+    rows, cols, planes = 3000, 1030, 3000  # planes of 10 x 103
+    rng = np.random.default_rng(9)
+    a, bias = rng.uniform(-1, 1, (rows, cols)).astype(np.float32), rng.uniform(-1, 1, cols).astype(np.float32)
+    adds = [rng.uniform(-1, 1, (rows, cols)).astype(np.float32) for _ in range(3)]
+    n, pooled = rows * cols, planes * 5 * 51
+    da, dbias, dadds = m.to_device(a), m.to_device(bias), [m.to_device(t) for t in adds]
+    x, y = m.DeviceBuffer(n * 4), m.DeviceBuffer(n * 4)
+    outs = [(m.DeviceBuffer(n * 4), m.DeviceBuffer(pooled * 4)) for _ in range(6)]
+    ops = m.ops()
+    for i, (act, pool) in enumerate(outs):
+        ops.mgpuAdd(da.ptr, dadds[i % 3].ptr, x.ptr, n, None)
+        ops.mgpuPool2d(x.ptr, pool.ptr, 1, planes, 10, 103, 5, 51, 2, 2, 0, 0, 0, 0, 2, 2, 0, None)
+        ops.mgpuBiasAdd(x.ptr, dbias.ptr, y.ptr, rows, cols, None)
+        ops.mgpuActivation(y.ptr, act.ptr, n, m.ACT_RELU, None)
+    m.runtime().mgpuStreamSynchronize(None)
+    m.check("chain")
+    for i, (act, pool) in enumerate(outs):
+        s = a + adds[i % 3]
+        assert np.array_equal(m.to_host(act, (rows, cols), np.float32), np.maximum(s + bias, 0))
+        p = s.reshape(planes, 10, 103)[:, :, :102].reshape(planes, 5, 2, 51, 2).max(axis=(2, 4))
+        assert np.array_equal(m.to_host(pool, (planes, 5, 51), np.float32), p)
+
+
 def test_add_empty_and_unaligned(m):
     assert m.add(np.zeros(0, np.float32), np.zeros(0, np.float32)).size == 0
     # pointers offset by one float: the kernel must take its scalar path

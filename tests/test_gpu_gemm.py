@@ -358,6 +358,39 @@ def test_output_may_overlap_the_weight(m, entry, M, N, K):
         assert np.array_equal(got, a @ w + b), at
 
 
+@pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
+@pytest.mark.parametrize("M,N,K", [(16, 1000, 1024), (40, 2400, 500)])  # 16 and 32 columns a CTA
+def test_few_rows_read_what_is_queued_ahead(m, entry, M, N, K):
+    """Nothing waits between the calls: the weight and the bias are written by kernels queued ahead of the Gemm (in
+    either order, so that each is directly ahead once) and written again by those behind it."""
+    rng = np.random.default_rng(43)
+    rt, ops = m.runtime(), m.ops()
+    ints = lambda lo, hi, *shape: rng.integers(lo, hi, shape).astype(np.float32)
+    a, w0, b0 = ints(-3, 4, M, K), ints(-2, 3, K, N), ints(-4, 5, N)
+    dw, db = [ints(-2, 3, K, N) for _ in range(3)], [ints(-4, 5, N) for _ in range(3)]
+    da, dw0, db0 = m.to_device(a), m.to_device(w0), m.to_device(b0)
+    ddw, ddb = [m.to_device(t) for t in dw], [m.to_device(t) for t in db]
+    w, b = m.to_device(np.zeros_like(w0)), m.to_device(np.zeros_like(b0))
+    outs = [m.to_device(np.zeros((M, N), np.float32)) for _ in range(12)]
+    for stream in (None, rt.mgpuStreamCreate()):
+        for i, out in enumerate(outs):
+            writes = [(dw0.ptr, ddw[i % 3].ptr, w.ptr, K * N), (db0.ptr, ddb[i % 3].ptr, b.ptr, N)]
+            for x, y, z, n in writes if i % 2 else reversed(writes):
+                ops.mgpuAdd(x, y, z, n, stream)
+            getattr(ops, entry)(da.ptr, w.ptr, b.ptr, out.ptr, M, N, K, stream)
+        rt.mgpuStreamSynchronize(stream)
+        m.check(entry)
+        for i, out in enumerate(outs):
+            got = m.to_host(out, (M, N), np.float32)
+            assert np.array_equal(got, a @ (w0 + dw[i % 3]) + (b0 + db[i % 3])), i
+        assert ops.mgpuOpsCheckDeviceStatus(stream) == 0
+        if stream:
+            rt.mgpuStreamDestroy(stream)
+        for out in outs:
+            rt.mgpuMemset32(out.ptr, 0, M * N, None)
+        rt.mgpuStreamSynchronize(None)
+
+
 def test_few_rows_keep_infinities_to_themselves(m):
     # a row or column with an infinity leaves the others alone
     rng = np.random.default_rng(31)
@@ -372,7 +405,9 @@ def test_few_rows_keep_infinities_to_themselves(m):
     assert not np.isfinite(got[4]).any() and np.isnan(got[:, 13]).all()
 
 
-@pytest.mark.parametrize("N,K", [(768, 3072), (1000, 1000), (72, 333)])
+# 768 x 3072 is never read by the Gemm of a few rows; 1000 x 1000 and 1760 x 3210 are in its form with 16 columns,
+# 2400 x 3000 in the one with 32, the latter two with more stages than its ring holds
+@pytest.mark.parametrize("N,K", [(768, 3072), (1000, 1000), (72, 333), (1760, 3210), (2400, 3000)])
 def test_matmul_rows_do_not_depend_on_their_number(m, N, K):
     # few rows, one wave, CTA pairs: the same sum over K in the same order
     rng = np.random.default_rng(37)

@@ -419,8 +419,9 @@ def test_pool_guard_bands_catch_a_write_past_the_end():
 
 @pytest.mark.parametrize("nbytes,offset", [((1 << 20) + 3, 1), (9 << 20, 4095), ((17 << 20) + 5, 64)])
 def test_download_into_unmapped_pages(m, nbytes, offset):
-    """A large download brings the pages of its destination in beforehand: a fresh mapping, off its page
-    boundaries, gets the bytes and its neighbours keep theirs; so does memory that is in use."""
+    """A large download first brings in the pages of its destination, also where they hold other data: a fresh
+    mapping, off its page boundaries, gets the bytes and its neighbours keep theirs; so does memory that is in use.
+    (That the pages came in ahead of the copy shows in the time only.)"""
     import ctypes
     import mmap
     rt = m.runtime()
