@@ -94,7 +94,8 @@ __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
 // the tile fastest, a sequence of two or four of them gives a CTA, and an SM, the same tile every time: one key
 // tile for some and four for others under a causal mask.  Where a CTA takes more than one item, causal tiles
 // therefore run slowest, the longest first: 32 x 512 tokens, 12 x 64, 59.8 -> 46.3 us; 16 x 512, 8 x 128, 46.5 -> 33.2;
-// with padding 48 x 512 67.5 -> 59.0.  Padding alone does not gain (32 x 384 37.6 us, 39.3 in this order), nor does
+// with padding 48 x 512 67.5 -> 59.0; whole layers of 64 x 512 tokens, whose K and V do not stay in L2, 654 -> 640
+// (12 x 64) and 983 -> 958 (8 x 128).  Padding alone does not gain (32 x 384 37.6 us, 39.3 in this order), nor does
 // one item per CTA (3 x 300 11.9, 12.3).
 __device__ __forceinline__ int attn_tile(const AttnParams &p, int item, int q_tiles, int &rest) {
   const int d = p.tiles_outer ? p.heads * p.batch : q_tiles, quot = item / d, r = item - quot * d;
@@ -483,7 +484,7 @@ constexpr size_t SMEM_BYTES = 3 * TILE_BYTES + 4 * 4096 + 1024;
 struct AttnItem64 {
   int q0, head, b, kv_end, n_kv;
 };
-// kOuter: p.tiles_outer, compiled in (as a run-time choice it cost the short items of this kernel 2 to 6 %)
+// kOuter: the order of tiles_outer, compiled in (as a run-time choice it cost the short items of this kernel 2 to 6 %)
 template <bool kOuter>
 __device__ __forceinline__ AttnItem64 attn_item64(const AttnParams &p, int item, int q_tiles) {
   AttnItem64 it;
@@ -814,8 +815,8 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
 }
 
 template <typename T16, bool kOuter>
-static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &tmo, AttnParams p, int64_t n_items,
-                               const DeviceInfo &di, cudaStream_t s) {
+static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &tmo, const AttnParams &p, int64_t n_items,
+                                     const DeviceInfo &di, cudaStream_t s) {
   auto kern = attention_d64_kernel<T16, kOuter>;
   static bool set_on[64] = {false};  // the attribute is per device
   bool &set = set_on[(di.device >= 0 && di.device < 64) ? di.device : 0];
@@ -826,7 +827,6 @@ static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &t
     set = true;
   }
   const int64_t slots = static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM;
-  p.tiles_outer = kOuter;
   dim3 grid(static_cast<unsigned>(n_items < slots ? n_items : slots));
   check_cuda(launch_chain(kern, grid, dim3(attn64::THREADS), attn64::SMEM_BYTES, s, 1, tm, tmo, p), "launch attention");
 }

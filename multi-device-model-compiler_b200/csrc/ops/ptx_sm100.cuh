@@ -216,7 +216,6 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-constexpr int kStepKMajor = 2;
 // Two operand descriptors of 64-wide k-blocks: their low words move, the high ones are constant.
 struct KblockDesc {
   uint32_t a_lo, a_hi, b_lo, b_hi;
@@ -232,11 +231,11 @@ __device__ __forceinline__ KblockDesc kblock_desc(uint64_t a, uint64_t b) {
 // arithmetic and four k-blocks per election instead of 64-bit adds and an election each.
 #define MDC_KBLOCK(CGS, A, B, P)                                             \
   "add.u32 x1, " A ", 2;\n"                                                  \
-  "add.u32 y1, " B ", %9;\n"                                                  \
+  "add.u32 y1, " B ", %9;\n"                                                 \
   "add.u32 x2, " A ", 4;\n"                                                  \
-  "add.u32 y2, " B ", %10;\n"                                                  \
+  "add.u32 y2, " B ", %10;\n"                                                \
   "add.u32 x3, " A ", 6;\n"                                                  \
-  "add.u32 y3, " B ", %11;\n"                                                  \
+  "add.u32 y3, " B ", %11;\n"                                                \
   "mov.b64 da, {" A ", %2};\n"                                               \
   "mov.b64 db, {" B ", %4};\n"                                               \
   "@e tcgen05.mma.cta_group::" CGS ".kind::f16 [%0], da, db, %5, " P ";\n"   \
@@ -270,7 +269,7 @@ __device__ __forceinline__ KblockDesc kblock_desc(uint64_t a, uint64_t b) {
   "add.u32 ka3, ka2, %7;\n"                                                  \
   "add.u32 kb3, kb2, %8;\n" MDC_KBLOCK(CGS, "%1", "%3", "p")                 \
   MDC_KBLOCK(CGS, "ka1", "kb1", "1") MDC_KBLOCK(CGS, "ka2", "kb2", "1") MDC_KBLOCK(CGS, "ka3", "kb3", "1") "}\n"
-template <int CG, int NKB, int B_STEP = kStepKMajor>
+template <int CG, int NKB, int B_STEP = 2>
 __device__ __forceinline__ void umma_f16_ss_kblocks(uint32_t d_tmem, const KblockDesc &d, uint32_t idesc, uint32_t accumulate,
                                                     uint32_t a_kb = 0, uint32_t b_kb = 0) {
   static_assert((CG == 1 || CG == 2) && (NKB == 1 || NKB == 4), "");
