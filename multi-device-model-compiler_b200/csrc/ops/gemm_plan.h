@@ -40,7 +40,9 @@ inline int few_rows_columns(int64_t N, int sms) { return (N + 15) / 16 <= sms ? 
 //   32 columns, by value     2369 x 1280 11.4 / 10.8  2401 x 1536 14.4 / 16.2   4401 x 3072 28.3 / 26.8
 //                            with 64 rows 2369 x 768 10.9 / 9.1, x 1024 11.7 / 13.0
 // Beyond one CTA per SM the second wave costs as much as the first (5000 x 1024 12.4 / 15.7, 32000 x 768 38.9 / 48.5),
-// until the copy of the weight no longer stays in L2: 50257 x 768 81.4 / 73.3, 32000 x 2048 107 / 94.
+// until the copy of the weight no longer stays in L2: 50257 x 768 81.4 / 73.3, 32000 x 2048 107 / 94.  A second wave
+// that is at least two thirds full still wins at a short K: 7500 x 512 14.2 / 12.2, 9001 x 512 14.5 / 13.5, but 7008 x 512
+// 11.0 / 12.1 and 8500 x 768 13.4 / 14.8.
 inline int64_t few_rows_max_k(int64_t M, int64_t N, bool vectors, bool lines, int sms) {
   if (few_rows_columns(N, sms) == 16) {
     if (!vectors) return std::min<int64_t>(1536, std::max<int64_t>(512, 5 * N / 4));
@@ -59,7 +61,7 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w,
   if (M > 64 || N > (1 << 30) || K > (1 << 30)) return false;
   const uintptr_t w0 = reinterpret_cast<uintptr_t>(w), o0 = reinterpret_cast<uintptr_t>(out);
   if (N > 32 * sms) {
-    if (K * N < 38000000) return false;
+    if (K * N < 38000000 && (K > 640 || N < 50 * sms || N > 64 * sms)) return false;
   } else if (K > few_rows_max_k(M, N, N % 4 == 0 && (w0 & 15u) == 0, N % 32 == 0 && (w0 & 127u) == 0, sms)) {
     return false;
   }

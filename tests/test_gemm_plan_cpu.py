@@ -41,6 +41,10 @@ int main() {
   // more than one CTA per SM: weights that do not stay in L2
   assert(!gemm_takes_few_rows(1, 4737, 8021, v, out, 148) && gemm_takes_few_rows(1, 4737, 8022, v, out, 148));
   assert(!gemm_takes_few_rows(1, 32000, 1187, v, out, 148) && gemm_takes_few_rows(1, 32000, 1188, v, out, 148));
+  // a second wave that is two thirds full
+  assert(!gemm_takes_few_rows(1, 7399, 256, v, out, 148) && gemm_takes_few_rows(1, 7400, 640, v, out, 148));
+  assert(!gemm_takes_few_rows(1, 7400, 641, v, out, 148) && gemm_takes_few_rows(1, 9472, 1, v, out, 148));
+  assert(!gemm_takes_few_rows(1, 9473, 640, v, out, 148));
   // ranges of bytes beyond 32 bits
   assert(gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, out, 148));
   assert(!gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, reinterpret_cast<const float *>(uintptr_t(1) << 50), 148));

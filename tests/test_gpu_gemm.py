@@ -319,7 +319,7 @@ def test_packed_rows_on_and_off_sectors(m, K, N, offset):
     (1, 8, 8), (1, 1, 1), (5, 17, 24), (32, 16, 128), (33, 15, 129),    # a stage, its edges, one column tile
     (16, 1000, 2048), (64, 2368, 200), (64, 2369, 200), (3, 4100, 63),  # 16 columns a CTA, 32, odd widths
     (7, 1100, 3210), (40, 2400, 3333), (7, 48, 6001),                   # the ring goes round; a long K that it leaves
-    (7, 1760, 3210), (33, 4001, 1999), (2, 5000, 8100)])                # round with 16 columns, by value, in two waves
+    (7, 1760, 3210), (33, 4001, 1999), (2, 5000, 8100), (9, 7402, 130)])  # round with 16 columns, by value, in two waves
 def test_few_rows_are_exact(m, M, N, K):
     """Up to 64 rows the weight is read in fp32 by the Gemm itself."""
     _exact_matmul(m, M, N, K, 23)
