@@ -148,7 +148,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
   uint8_t *sQ = tiles, *sK = tiles + QS * TILE_BYTES, *sV = sK + KS * TILE_BYTES;
   uint8_t *sOut = sV + KS * TILE_BYTES;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q_tiles = (p.seq + BQ - 1) / BQ;
   const int n_items = q_tiles * p.heads * p.batch;
   const int hd = p.heads * HD;
@@ -522,7 +522,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
   uint8_t *sQ = tiles, *sK = tiles + TILE_BYTES, *sV = tiles + 2 * TILE_BYTES;
   uint8_t *sOut = tiles + 3 * TILE_BYTES;  // 4 warps x 32 rows x 128 bytes of staged output
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q_tiles = (p.seq + BQ - 1) / BQ;
   const int n_items = q_tiles * p.heads * p.batch;
   const int hd = p.heads * D;

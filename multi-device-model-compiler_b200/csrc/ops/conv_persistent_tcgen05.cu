@@ -80,7 +80,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   volatile uint32_t *abort_flag = &abort_flag_s;
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int b_bytes = p.bn * BK * 2;
   const int stage_bytes = A_BYTES + (p.resident ? 0 : b_bytes);
   uint8_t *filter_s = tiles + p.stages * stage_bytes;
@@ -219,7 +219,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     }
     if (!kGather || !p.resident) {
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, looked = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
         const int mt = tile / p.n_tiles, n0 = (tile - mt * p.n_tiles) * p.bn;
@@ -227,11 +227,13 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         const int h0 = oh * p.SH - p.PHL, w0 = (pix - oh * p.OW) * p.SW - p.PWL;
         int c0 = 0, kh = 0, kw = 0;  // k-blocks run over the taps of 64 channels, then the next 64
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
+          if (!mbar_wait_looked(looked, &empty_bar[stage], phase ^ 1, abort_flag)) {
             atomicCAS(p.err, 0u, 0x51000000u | static_cast<uint32_t>(stage));
             ok = false;
             break;
           }
+          const int next = stage + 1 == p.stages ? 0 : stage + 1;
+          looked = mbar_look(&empty_bar[next], next ? phase ^ 1 : phase);
           if (elect_one()) {
             uint8_t *sa = tiles + stage * stage_bytes;
             mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>((kGather ? 0 : A_BYTES) + (p.resident ? 0 : b_bytes)));
@@ -254,7 +256,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     const uint64_t a0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
     const uint64_t f0 = make_smem_desc_sw128(smem_u32(filter_s), 16, 1024);
     int stage = 0, acc = 0;
-    uint32_t phase = 0, acc_phase = 0;
+    uint32_t phase = 0, acc_phase = 0, looked = 0;
     bool ok = true;
     if (p.resident && !mbar_wait_all(&filter_bar, 0, abort_flag)) {
       atomicCAS(p.err, 0u, 0x55000000u);
@@ -271,12 +273,14 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       tc_fence_after();
       const uint32_t d = tmem_base + acc * (p.tmem_cols / 2);
       for (int kb = 0; kb < p.num_kb; ++kb) {
-        if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_looked(looked, &full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x53000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
         tc_fence_after();
+        const int next = stage + 1 == p.stages ? 0 : stage + 1;
+        looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
         const uint64_t ad = a0 + static_cast<uint64_t>(stage * (stage_bytes / 16));
         const uint64_t bd = p.resident ? f0 + static_cast<uint64_t>(kb * (b_bytes / 16)) : ad + A_BYTES / 16;
         if (kb < partial_from) {

@@ -95,7 +95,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
   volatile uint32_t *abort_flag = &abort_flag_s;
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int bn = p.bn;
   const int stage_bytes = A_BYTES + bn * BK * 2;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * bn;

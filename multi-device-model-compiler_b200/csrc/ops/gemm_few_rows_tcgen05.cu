@@ -74,7 +74,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
   const int a_kb = p.box_m * 128, a_bytes = KBS * a_kb;
   // what an MMA reads beyond the last stage's A must not be W's part
   uint8_t *b_s = a_s + p.stages * a_bytes + (128 - p.box_m) * 128;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int col0 = blockIdx.x * BN;
 
   if (threadIdx.x == 0) {
@@ -101,12 +101,14 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
     // ------------------------------ A ------------------------------
     pdl_wait();
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, looked = 0;
     for (int i = 0; i < p.steps; ++i) {
-      if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
+      if (!mbar_wait_looked(looked, &empty_bar[stage], phase ^ 1, abort_flag)) {
         atomicCAS(p.err, 0u, 0x91000000u | static_cast<uint32_t>(stage));
         break;
       }
+      const int next = stage + 1 == p.stages ? 0 : stage + 1;
+      looked = mbar_look(&empty_bar[next], next ? phase ^ 1 : phase);
       if (elect_one()) {
         mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(a_bytes));
 #pragma unroll
@@ -123,15 +125,17 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
     const uint64_t b0 = static_cast<uint64_t>(smem_u32(b_s) >> 4) | static_cast<uint64_t>(C::LBO / 16) << 16 |
                         static_cast<uint64_t>(SBO / 16) << 32 | static_cast<uint64_t>(1) << 46;
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, looked = 0;
     bool ok = true;
     for (int i = 0; i < p.steps; ++i) {
-      if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
+      if (!mbar_wait_looked(looked, &full_bar[stage], phase, abort_flag)) {
         atomicCAS(p.err, 0u, 0x92000000u | static_cast<uint32_t>(stage));
         ok = false;
         break;
       }
       tc_fence_after();
+      const int next = stage + 1 == p.stages ? 0 : stage + 1;
+      looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
       const uint64_t ad = a0 + static_cast<uint64_t>(stage * (a_bytes >> 4)), bd = b0 + static_cast<uint64_t>(stage * (C::B_BYTES >> 4));
 #pragma unroll
       for (int kb = 0; kb < KBS; ++kb)

@@ -64,7 +64,7 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int half = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;  // which 128 rows of a pair's 256
   const bool leader = half == 0;
   const int tile = static_cast<int>(blockIdx.x) / CG;
@@ -143,12 +143,14 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, looked = 0;
     for (int i = 0; i < steps; ++i) {
-      if (i >= early && !mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
+      if (i >= early && !mbar_wait_looked(looked, &empty_bar[stage], phase ^ 1, abort_flag)) {
         atomicCAS(p.err, 0u, 0x81000000u | static_cast<uint32_t>(stage));
         break;
       }
+      const int next = stage + 1 == stages ? 0 : stage + 1;
+      looked = mbar_look(&empty_bar[next], next ? phase ^ 1 : phase);
       if (elect_one()) {
         if (i >= early) {
           expect(stage);
@@ -167,15 +169,17 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                            make_smem_desc_sw128(smem_u32(tiles) + static_cast<uint32_t>(a_bytes), 16, 1024));
       const uint32_t a_kb16 = static_cast<uint32_t>(a_kb_bytes) >> 4, b_kb16 = static_cast<uint32_t>(b_kb_bytes) >> 4;
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, looked = 0;
       bool ok = true;
       for (int i = 0; i < steps; ++i) {
-        if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_looked(looked, &full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x82000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
         tc_fence_after();
+        const int next = stage + 1 == stages ? 0 : stage + 1;
+        looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
         KblockDesc kd = desc0;
         kd.a_lo += static_cast<uint32_t>(stage * stage_bytes) >> 4;
         kd.b_lo += static_cast<uint32_t>(stage * stage_bytes) >> 4;

@@ -109,7 +109,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // 128-byte-swizzled tiles need 1024-byte aligned bases
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // CG == 2: the two CTAs of a cluster work on one 256-row tile; rank 0 leads
   const int cta_rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
   const bool leader = cta_rank == 0;
@@ -162,16 +162,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp == 0) {
     // ------------------------------ TMA producer (whole warp, elected lane issues) ------------------------------
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, looked = 0;
     bool ok = true;
     for (int tile = worker; ok && tile < num_tiles; tile += num_workers) {
       const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        if (!mbar_wait_looked(looked, &empty_bar[stage], phase ^ 1, abort_flag)) {
           atomicCAS(p.err, 0u, 0x10000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;
         }
+        const int next = stage + 1 == STAGES ? 0 : stage + 1;
+        looked = mbar_look(&empty_bar[next], next ? phase ^ 1 : phase);
         if (elect_one()) {
           uint8_t *sa = tiles + stage * STAGE_BYTES;
           uint8_t *sb = sa + A_BYTES;
@@ -197,7 +199,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                                             std::is_same<T16, __nv_bfloat16>::value, false, false);
       const uint64_t desc0 = make_smem_desc_sw128(smem_u32(tiles), 16, 1024);
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, looked = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
@@ -209,12 +211,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_all(&full_bar[stage], phase, abort_flag)) {
+          if (!mbar_wait_looked(looked, &full_bar[stage], phase, abort_flag)) {
             atomicCAS(p.err, 0u, 0x20000000u | static_cast<uint32_t>(stage));
             ok = false;
             break;
           }
           tc_fence_after();
+          const int next = stage + 1 == STAGES ? 0 : stage + 1;
+          looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
           // (descriptors hold addresses in units of 16 bytes)
           const uint64_t a_desc = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES / 16));
           const uint64_t b_desc = a_desc + A_BYTES / 16;
