@@ -539,7 +539,7 @@ static bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
 // A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels only, and
 // the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56, stride 2: 108 us
 // with the whole input rewritten, 65 sampled.)
-static bool conv_sampled(ConvShape &c) {
+bool conv_sampled(ConvShape &c) {
   if (conv_gathers(c) || c.KH * c.KW != 1 || (c.SH == 1 && c.SW == 1)) return false;
   c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
   return true;
@@ -559,6 +559,32 @@ bool conv_persistent_takes(const ConvShape &call) {
   const int64_t up_w = conv_upper_w(c), up_h = conv_upper_h(c);
   return c.SW <= 8 && c.SH <= 8 && c.PWL <= 127 && c.PHL <= 127 && up_w >= -128 && up_w <= 127 && up_h >= -128 &&
          up_h <= 127 && span_w <= 255 && span_h <= 255 && encode_im2col() != nullptr;
+}
+
+bool conv_prepare(const ConvShape &c, const ConvShape &call, bool sampled, int64_t copy_h, int64_t copy_w, void *x16, void *w16,
+                  cudaStream_t s) {
+  const bool gather = conv_gathers(c);
+  const int64_t taps = c.KH * c.KW, ncb = (c.IC + 63) / 64, K = c.IC * taps;
+  ConvPrepareParams q;
+  q.x = call.x, q.w = call.w, q.w16 = static_cast<__half *>(w16), q.x16 = static_cast<__half *>(x16);
+  q.IC = int(c.IC), q.HW = int(copy_h * copy_w), q.Cp = int((c.IC + 7) / 8 * 8), q.taps = int(taps), q.ncb = gather ? 0 : int(ncb);
+  q.K = int(K), q.Kp = int((K + 7) / 8 * 8);
+  q.sampled = sampled || copy_h != c.H || copy_w != c.W ? 1 : 0;
+  q.H = int(call.H), q.W = int(call.W);
+  // a copy with margins is one of stride 1: pixel for pixel
+  q.SH = sampled ? int(call.SH) : 1, q.SW = sampled ? int(call.SW) : 1;
+  q.PHL = sampled ? int(call.PHL) : 0, q.PWL = sampled ? int(call.PWL) : 0;
+  q.by_w = Divisor(copy_w);
+  q.pixel_tiles = int((copy_h * copy_w + 63) / 64), q.channel_tiles = int(ncb);
+  q.input_blocks = gather ? 0 : c.N * q.pixel_tiles * q.channel_tiles;
+  const int64_t blocks = q.input_blocks + c.OC * (gather ? 1 : ncb);
+  if (blocks > INT32_MAX) return false;
+  {
+    ProfileScope prof(kCatElementwise, s);
+    check_cuda(launch_chain(conv_prepare_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, 1, q), "launch conv_prepare_kernel");
+  }
+  launched("conv_prepare_kernel");
+  return true;
 }
 
 bool conv_persistent(const ConvShape &call, cudaStream_t s) {
@@ -612,20 +638,8 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
     if (before == 0) mgpuClearLastError();  // an earlier failure's status stays
     return false;
   }
-  ConvPrepareParams q;
-  q.x = c.x, q.w = c.w, q.w16 = reinterpret_cast<__half *>(ws), q.x16 = reinterpret_cast<__half *>(ws + w_bytes);
-  q.IC = int(c.IC), q.HW = int(c.H * c.W), q.Cp = int(Cp), q.taps = int(taps), q.ncb = gather ? 0 : int(ncb);
-  q.K = int(K), q.Kp = int(Kp);
-  q.sampled = sampled ? 1 : 0;
-  q.H = int(call.H), q.W = int(call.W), q.SH = int(call.SH), q.SW = int(call.SW), q.PHL = int(call.PHL), q.PWL = int(call.PWL);
-  q.by_w = Divisor(c.W);
-  q.pixel_tiles = int((c.H * c.W + 63) / 64), q.channel_tiles = int(ncb);
-  q.input_blocks = gather ? 0 : c.N * q.pixel_tiles * q.channel_tiles;
-  const int64_t blocks = q.input_blocks + c.OC * (gather ? 1 : ncb);
-
   CUtensorMap tx = {}, tw;
-  bool ok = blocks <= INT32_MAX &&
-            encode_tmap_2d(&tw, ws, MGPU_DTYPE_F16, static_cast<uint64_t>(Kp), static_cast<uint64_t>(c.OC),
+  bool ok = encode_tmap_2d(&tw, ws, MGPU_DTYPE_F16, static_cast<uint64_t>(Kp), static_cast<uint64_t>(c.OC),
                            static_cast<uint64_t>(Kp) * 2, BK, static_cast<uint32_t>(p.bn));
   if (ok && !gather) {
     const cuuint64_t gdim[4] = {cuuint64_t(Cp), cuuint64_t(c.W), cuuint64_t(c.H), cuuint64_t(c.N)};
@@ -636,13 +650,8 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
+  ok = ok && conv_prepare(c, call, sampled, c.H, c.W, ws + w_bytes, ws, s);
   if (ok) {
-    {
-      ProfileScope prof(kCatElementwise, s);
-      check_cuda(launch_chain(conv_prepare_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, 1, q),
-                 "launch conv_prepare_kernel");
-    }
-    launched("conv_prepare_kernel");
     if (gather && p.add) launch_persistent<true, true>(tx, tw, p, smem, di.sms, s);
     else if (gather) launch_persistent<true, false>(tx, tw, p, smem, di.sms, s);
     else if (p.add) launch_persistent<false, true>(tx, tw, p, smem, di.sms, s);

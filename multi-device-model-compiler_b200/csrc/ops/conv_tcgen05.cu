@@ -371,7 +371,7 @@ MDC_API void mgpuConv2d(float *input, float *weight, float *bias, float *output,
   // MDC_CONV_DIRECT selects the direct gather for every shape (for comparisons)
   const ConvShape c{input, weight, bias, hasPostAdd ? postAdd : nullptr, output, N, IC, H, W, OC, KH, KW, OH, OW,
                     PHL, PWL, SH, SW, DH, DW, hasContainRelu};
-  if (getenv("MDC_CONV_DIRECT") == nullptr && conv_persistent(c, s)) return;
+  if (getenv("MDC_CONV_DIRECT") == nullptr && (conv_halo(c, s) || conv_persistent(c, s))) return;
   const bool tap_major = IC % 32 == 0;
   const int blocks64 = conv_persistent_takes(c) ? int(IC / 64) : 0;
   const int64_t Kp = (K + 7) / 8 * 8;  // filter rows padded to 16-byte multiples for TMA

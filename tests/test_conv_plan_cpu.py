@@ -1,0 +1,102 @@
+"""The tiles of the convolution kernel whose taps share one region of the input (conv_plan.h), compiled for the host: every
+live output's every tap finds its input pixel, or padding, where the kernel looks for it."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+OPS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "multi-device-model-compiler_b200", "csrc", "ops")
+CUDA_INCLUDE = "/usr/local/cuda/include"
+
+PROGRAM = r"""
+#include "conv_plan.h"
+#include <cassert>
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+using namespace mdc;
+int main() {
+  srand(1);
+  auto pick = [](int lo, int hi) { return lo + rand() % (hi - lo + 1); };
+  int rects = 0, flats = 0, strided = 0;
+  for (int i = 0; i < 1500; ++i) {
+    ConvShape c = {};
+    c.N = pick(1, 4), c.IC = 1, c.OC = 1, c.H = pick(1, 24), c.W = pick(1, 24), c.KH = pick(1, 5), c.KW = pick(1, 5);
+    c.SH = pick(1, 3), c.SW = pick(1, 3), c.DH = pick(1, 3), c.DW = pick(1, 3), c.PHL = pick(0, 4), c.PWL = pick(0, 4);
+    const int64_t span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
+    c.OH = (c.H + c.PHL + pick(0, 4) - span_h - 1) / c.SH + 1, c.OW = (c.W + c.PWL + pick(0, 4) - span_w - 1) / c.SW + 1;
+    if (c.OH < 1 || c.OW < 1 || c.H + c.PHL + 4 < span_h + 1 || c.W + c.PWL + 4 < span_w + 1) continue;
+    c.OH -= c.OH > 1 ? pick(0, 1) : 0, c.OW -= c.OW > 1 ? pick(0, 1) : 0;
+    for (int flat = 0; flat < 2; ++flat) {
+      HaloPlan h;
+      if (!halo_plan(c, flat, &h)) {
+        assert(c.SH > 2 || c.SW > 2 || (flat && (c.SH > 1 || c.SW > 1)));
+        continue;
+      }
+      flat ? ++flats : c.SH * c.SW > 1 ? ++strided : ++rects;
+      std::vector<int> seen(c.N * c.OH * c.OW, 0);
+      for (int64_t tile = 0; tile < h.m_tiles; ++tile) {
+        // the region's pixels by their place, as the input warps write them: image, row, column, or -1 for padding
+        std::vector<int64_t> at(h.plane_px, -2);
+        for (int64_t q = 0; q < h.px; ++q) {
+          int64_t row, col, place = q;
+          if (flat) {
+            const int64_t px = tile * 128 - c.PHL * h.Wv - c.PWL + q;
+            row = px < 0 ? -1 : px / h.Wv, col = px < 0 ? 0 : px % h.Wv;
+          } else {
+            const int64_t rh = q / h.IW, rw = q % h.IW;
+            row = tile / h.tiles_w * 16 * c.SH - c.PHL + rh, col = tile % h.tiles_w * 8 * c.SW - c.PWL + rw;
+            place = (rh % c.SH * c.SW + rw % c.SW) * h.class_px + rh / c.SH * h.pitch + rw / c.SW;
+          }
+          assert(place >= 0 && place < h.plane_px);
+          const int64_t img = row < 0 ? c.N : row / h.Hv, y = row < 0 ? 0 : row % h.Hv;
+          at[place] = img < c.N && y < c.H && col >= 0 && col < c.W ? (img * c.H + y) * c.W + col : -1;
+        }
+        for (int64_t r = 0; r < 128; ++r) {
+          const int64_t vr = flat ? (tile * 128 + r) / h.Wv : tile / h.tiles_w * 16 + r / 8;
+          const int64_t ow = flat ? (tile * 128 + r) % h.Wv : tile % h.tiles_w * 8 + r % 8;
+          const int64_t img = vr / h.HvO, oh = vr % h.HvO;
+          const bool live = img < c.N && oh < c.OH && ow < c.OW;
+          if (live) ++seen[(img * c.OH + oh) * c.OW + ow];
+          for (int64_t kh = 0; kh < c.KH; ++kh)
+            for (int64_t kw = 0; kw < c.KW; ++kw) {
+              const int64_t rh = kh * c.DH, rw = kw * c.DW;
+              const int64_t place = (rh % c.SH * c.SW + rw % c.SW) * h.class_px + rh / c.SH * h.pitch + rw / c.SW +
+                                    (flat ? r : r / 8 * h.pitch + r % 8);
+              assert(place < h.plane_px);  // whatever the pixel: the tensor core reads all 128
+              if (!live) continue;
+              const int64_t y = oh * c.SH - c.PHL + rh, x = ow * c.SW - c.PWL + rw;
+              assert(at[place] == (y >= 0 && y < c.H && x >= 0 && x < c.W ? (img * c.H + y) * c.W + x : -1));
+            }
+        }
+      }
+      for (int n : seen) assert(n == 1);
+    }
+  }
+  assert(rects > 50 && flats > 50 && strided > 100);
+  // where the kernel takes a call
+  ConvShape c = {};
+  auto form = [&](int N, int IC, int H, int W, int OC, int K, int S) {
+    c.N = N, c.IC = IC, c.H = H, c.W = W, c.OC = OC, c.KH = c.KW = K, c.SH = c.SW = S, c.DH = c.DW = 1, c.PHL = c.PWL = K / 2;
+    c.OH = (H + K / 2 * 2 - K) / S + 1, c.OW = (W + K / 2 * 2 - K) / S + 1;
+    return conv_form(c, 148);
+  };
+  assert(form(16, 3, 256, 256, 64, 3, 1) == ConvForm::kOther && form(16, 3, 224, 224, 32, 7, 1) == ConvForm::kDirectRect);
+  assert(form(21, 3, 29, 37, 352, 3, 1) == ConvForm::kDirectFlat && form(8, 15, 20, 20, 8, 5, 3) == ConvForm::kOther);
+  assert(form(32, 64, 56, 56, 64, 3, 1) == ConvForm::kCopyRect && form(32, 64, 57, 57, 64, 3, 1) == ConvForm::kCopyFlat);
+  assert(form(32, 128, 28, 28, 128, 3, 1) == ConvForm::kOther && form(32, 512, 7, 7, 512, 3, 1) == ConvForm::kCopyFlat);
+  assert(form(32, 64, 56, 56, 256, 1, 1) == ConvForm::kCopyFlat && form(1, 160, 9, 7, 96, 3, 1) == ConvForm::kCopyFlat);
+  assert(form(2, 32, 22, 23, 32, 7, 2) == ConvForm::kDirectRect && form(2, 64, 22, 23, 32, 7, 2) == ConvForm::kOther);
+  printf("ok\n");
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or not os.path.isdir(CUDA_INCLUDE), reason="no host compiler or CUDA headers")
+def test_halo_tiles_find_every_tap(tmp_path):
+    src = tmp_path / "plan.cpp"
+    src.write_text(PROGRAM)
+    exe = str(tmp_path / "plan")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout == "ok\n"

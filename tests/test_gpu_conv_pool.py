@@ -203,6 +203,67 @@ def test_conv_persistent_edges(m, shape):
     assert np.array_equal(m.conv2d(x, w, b, **kw), oracle.conv2d(x, w, b, **kw))
 
 
+@pytest.mark.parametrize("shape", [
+    # N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
+    (3, 16, 9, 16, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False),      # rect out of a copy: tiles of two images
+    (2, 72, 33, 24, 33, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),     # rect: a block of 8 channels, three rounds of rows
+    (40, 64, 24, 24, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True),     # rect: filter kept, several tiles per CTA
+    (5, 40, 7, 9, 20, 3, 5, (1, 1), (0, 3, 2, 1), (2, 1), True, False),       # flat out of a copy: asymmetric
+    (60, 100, 13, 11, 60, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),  # flat: filter streamed, 36 channels in the last block
+    (9, 20, 19, 17, 300, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, True),     # flat, 1 x 1: two channel tiles
+    (7, 48, 15, 14, 260, 1, 1, (2, 3), (0, 0, 0, 0), (1, 1), False, True),    # the same, sampled
+    (2, 3, 21, 70, 24, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, False),      # straight from the input: rect, a tap without a partner
+    (3, 8, 12, 10, 40, 6, 6, (1, 1), (3, 2, 2, 3), (1, 1), False, True),      # flat, pairs only
+    (70, 1, 30, 31, 33, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), False, False),    # stride 2: classes of rows and columns
+    (2, 5, 23, 64, 300, 3, 3, (2, 1), (0, 1, 1, 1), (2, 3), True, False),     # strides and dilations apart, two channel tiles
+    (3, 15, 14, 9, 17, 5, 5, (1, 2), (2, 2, 2, 2), (1, 3), False, True),      # two groups of channels, columns in two classes
+    (4, 32, 18, 21, 64, 7, 5, (2, 2), (3, 2, 3, 2), (1, 1), True, True),      # stride 2, 32 channels
+])
+def test_conv_halo_forms(m, shape):
+    """The kernel whose tiles share one region of the input between taps, in every form of conv_form: small integers,
+    equal bit for bit (see test_conv_exact_on_small_integers)."""
+    test_conv_persistent_edges(m, shape)
+
+
+@pytest.mark.parametrize("IC,W", [(3, 60), (3, 20), (12, 20), (64, 20), (64, 24)])
+def test_conv_keeps_infinities_to_their_windows(m, IC, W):
+    """An infinity next to a window, where the tile's region holds it and the weights of a padded tap are zero, must not
+    turn into NaN: outputs whose window does not hold it are those of the input without it."""
+    rng = np.random.default_rng(W)
+    x = rng.integers(-4, 5, size=(2, IC, 20, W)).astype(np.float32)
+    w = rng.integers(1, 4, size=(9, IC, 5, 5)).astype(np.float32)
+    b = np.zeros(9, np.float32)
+    clean = m.conv2d(x, w, b, pad=(2, 2, 2, 2))
+    x[1, IC - 1, 9, 13] = np.inf
+    got = m.conv2d(x, w, b, pad=(2, 2, 2, 2))
+    hit = np.zeros(clean.shape, bool)
+    hit[1, :, 7:12, 11:16] = True
+    assert np.array_equal(got[~hit], clean[~hit])
+    assert np.all(np.isposinf(got[hit]))
+
+
+@pytest.mark.parametrize("IC,OC,size,kernel,stride", [(24, 24, 20, 5, 1), (32, 32, 20, 5, 2), (64, 64, 24, 3, 1), (32, 16, 33, 1, 1)])
+def test_conv_output_over_its_input(m, IC, OC, size, kernel, stride):
+    """From 16 channels on the output may lie over the input: a launch ahead has copied it, or the call is routed so."""
+    rng = np.random.default_rng(IC)
+    x = rng.integers(-4, 5, size=(3, IC, size, size)).astype(np.float32)
+    w = rng.integers(-3, 4, size=(OC, IC, kernel, kernel)).astype(np.float32)
+    pad = kernel // 2
+    out = (size - 1) // stride + 1
+    ref = oracle.conv2d(x, w, None, stride=(stride, stride), pad=(pad,) * 4)
+    for offset in (0, 4 * 64 * size):  # the same start, and inside
+        buf, dw = m.DeviceBuffer(x.nbytes + 4 * 64 * size + ref.nbytes), m.to_device(w)
+        m.runtime().mgpuMemcpy(buf.ptr, x.ctypes.data, x.nbytes, None)
+        m.runtime().mgpuStreamSynchronize(None)
+        m.ops().mgpuConv2d(buf.ptr, dw.ptr, None, buf.ptr + offset, None, 3, IC, size, size, OC, kernel, kernel, out, out, pad, pad,
+                           pad, pad, stride, stride, 1, 1, False, False, None)
+        m.check("conv")
+        got = np.empty_like(ref)
+        m.runtime().mgpuMemcpy(got.ctypes.data, buf.ptr + offset, ref.nbytes, None)
+        m.runtime().mgpuStreamSynchronize(None)
+        assert np.array_equal(got, ref)
+
+
 @pytest.mark.parametrize("earlier_failure", [False, True])
 def test_conv_without_memory_for_the_copy(m, earlier_failure):
     """With no device memory left for the NHWC copy of the input the direct kernel takes over, whether
