@@ -5,8 +5,10 @@
 // to be read back, and this kernel is bound by the bytes of W (4 K N) or, where those are few, by
 // latency.  Eight warps read W straight into registers, 16 vector loads of a thread in flight (64 KB an
 // SM); a warp fills a ring stage of 128 k x 16 columns or 64 k x 32 by itself, converting to core
-// matrices of 8 columns x 8 k.  A comes by TMA.  W and the bias do not wait for the kernel that converts A: that
-// kernel lets this one start after its own wait, so what is older than it is complete.
+// matrices of 8 columns x 8 k.  A comes by TMA, converted by a launch ahead; W and the bias do not wait for it: that
+// kernel lets this one start after its own wait, so what is older than it is complete.  Where A is small (kConvert,
+// few_rows_convert) eight more warps read and round it here instead, and there is no launch ahead: 16 x 768 x 768 6.9 ->
+// 5.1 us a call, 16 x 256 x 256 6.8 -> 4.1.
 //
 // Whole call, with the weight converted and read here: 16 x 1000 x 2048 12.2 / 10.8 us one after another out of L2,
 // 13.3 / 13.6 out of memory; out of memory also 16 x 4096 x 4096 30.3 / 23.6 (2.8 TB/s), 16 x 1000 x 512 7.4 / 6.0;
@@ -24,7 +26,8 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
 
 namespace fewrows {
 constexpr int LOAD_WARPS = 8;
-constexpr int THREADS = 64 + LOAD_WARPS * 32;
+// with the input converted here, as many warps again for it
+constexpr int threads(bool convert) { return 64 + LOAD_WARPS * (convert ? 64 : 32); }
 constexpr int MAX_STAGES = 24;
 constexpr int MAX_SMEM = 224 * 1024;
 // an MMA reads 128 rows of A whatever the box holds
@@ -51,16 +54,18 @@ static_assert(ring_holds_every_warp<16> && ring_holds_every_warp<32>, "a stage f
 }  // namespace fewrows
 
 struct FewRowsParams {
+  const float *x;  // kConvert: the input, M x K
   const float *w, *bias;
   float *out;
   int M, N, K;
   int box_m, stages, steps;  // steps: stages' worth of K
   int w_vec, out_vec;        // rows of W / of out and the bias in 16-byte vectors
+  int x_vec;                 // rows of x
   uint32_t *err;
 };
 
-template <int BN>
-__global__ void __launch_bounds__(fewrows::THREADS, 1)
+template <int BN, bool kConvert>
+__global__ void __launch_bounds__(fewrows::threads(kConvert), 1)
 gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsParams p) {
   using namespace fewrows;
   using namespace ptx;
@@ -79,9 +84,9 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
 
   if (threadIdx.x == 0) {
     abort_flag_s = 0;
-    tma_prefetch_desc(&tmap_a);
+    if (!kConvert) tma_prefetch_desc(&tmap_a);
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(&full_bar[s], 2);  // A's bytes, and the warp that brings W
+      mbar_init(&full_bar[s], 2);  // A's bytes, or the warp that brings them, and the warp that brings W
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&acc_bar, 1);
@@ -96,8 +101,11 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   pdl_launch_dependents();  // after this CTA holds its tensor memory (see gemm_tcgen05.cu)
+  if (kConvert) pdl_wait();  // no conversion ahead that would have waited
 
-  if (warp == 0) {
+  if (kConvert && warp == 0) {
+    // nothing to fetch
+  } else if (warp == 0) {
     // ------------------------------ A ------------------------------
     pdl_wait();
     int stage = 0;
@@ -146,6 +154,67 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
     if (ok) umma_commit_warp(&acc_bar);
+  } else if (kConvert && warp >= 2 + LOAD_WARPS) {
+    // ------------------------------ A out of the fp32 input ------------------------------
+    // A warp fills a stage's worth of rows by itself, in pieces of 16 rows x 64 k (eight lanes a row, four rows a load),
+    // two pieces' loads in flight.
+    const int aw = warp - 2 - LOAD_WARPS, chunk = lane & 7;
+    const int pieces = (p.M + 15) / 16 * KBS;
+    auto load = [&](int i, int piece, float4 (&v)[4][2]) __attribute__((always_inline)) {
+      const int k = i * C::STAGE_K + piece % KBS * 64 + chunk * 8;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = piece / KBS * 16 + r * 4 + (lane >> 3);
+        const float *src = p.x + static_cast<int64_t>(m) * p.K + k;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+          const int left = m < p.M ? p.K - k - 4 * h : 0;  // values of the row from here on
+          if (p.x_vec) {
+            if (left > 0) q = __ldg(reinterpret_cast<const float4 *>(src + 4 * h));
+          } else {
+            if (left > 0) q.x = __ldg(src + 4 * h);
+            if (left > 1) q.y = __ldg(src + 4 * h + 1);
+            if (left > 2) q.z = __ldg(src + 4 * h + 2);
+            if (left > 3) q.w = __ldg(src + 4 * h + 3);
+          }
+          v[r][h] = q;
+        }
+      }
+    };
+    auto store = [&](int stage, int piece, const float4 (&v)[4][2]) __attribute__((always_inline)) {
+      uint8_t *dst = a_s + stage * a_bytes + piece % KBS * a_kb;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = piece / KBS * 16 + r * 4 + (lane >> 3);
+        const float4 lo = v[r][0], hi = v[r][1];
+        if (m < p.M)  // 128-byte swizzle: 16-byte chunk c of row m lies at c ^ (m % 8)
+          *reinterpret_cast<uint4 *>(dst + m * 128 + ((chunk ^ (m & 7)) << 4)) =
+              make_uint4(pack_pair<__half>(lo.x, lo.y), pack_pair<__half>(lo.z, lo.w), pack_pair<__half>(hi.x, hi.y), pack_pair<__half>(hi.z, hi.w));
+      }
+    };
+    for (int i = aw; i < p.steps; i += LOAD_WARPS) {
+      const int stage = i % p.stages;
+      const uint32_t phase = static_cast<uint32_t>(i / p.stages) & 1u;
+      bool gone = false;
+      for (int piece = 0; piece < pieces; piece += 2) {
+        float4 va[4][2], vb[4][2];
+        load(i, piece, va);
+        if (piece + 1 < pieces) load(i, piece + 1, vb);
+        // the loads are in flight; only now does the stage have to be free
+        if (piece == 0 && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
+          if (lane == 0) atomicCAS(p.err, 0u, 0x94000000u | static_cast<uint32_t>(stage));
+          gone = true;
+          break;
+        }
+        store(stage, piece, va);
+        if (piece + 1 < pieces) store(stage, piece + 1, vb);
+      }
+      if (gone) break;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[stage]);
+    }
   } else {
     // ------------------------------ W, then the epilogue ------------------------------
     const int lw = warp - 2;
@@ -245,10 +314,10 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
   if (warp == 1) tmem_dealloc(tmem_base, 32);
 }
 
-template <int BN>
+template <int BN, bool kConvert>
 static void launch_few_rows(const CUtensorMap &ta, FewRowsParams &p, cudaStream_t s) {
   using C = fewrows::Cfg<BN>;
-  auto kern = gemm_few_rows_kernel<BN>;
+  auto kern = gemm_few_rows_kernel<BN, kConvert>;
   static bool set_on[64] = {false};  // the attribute is per device
   const int dev = device_info().device;
   bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
@@ -262,28 +331,31 @@ static void launch_few_rows(const CUtensorMap &ta, FewRowsParams &p, cudaStream_
   const size_t smem = static_cast<size_t>(fewrows::fixed_bytes(p.box_m)) + static_cast<size_t>(p.stages) * C::stage_bytes(p.box_m);
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>((p.N + BN - 1) / BN)), dim3(fewrows::THREADS), smem, s, 1, ta, p),
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>((p.N + BN - 1) / BN)), dim3(fewrows::threads(kConvert)), smem, s, 1, ta, p),
                "launch gemm few rows");
   }
   launched("gemm_few_rows_kernel");
 }
 
-void gemm_few_rows(const void *a16, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K, cudaStream_t s) {
+void gemm_few_rows(const void *a16, const float *x, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K,
+                   cudaStream_t s) {
   const DeviceInfo &di = device_info();
   uint32_t *err = device_error_slot();
   if (!err) return;
   const uint64_t Kp = static_cast<uint64_t>((K + 7) / 8 * 8);
   FewRowsParams p;
-  p.w = w, p.bias = bias, p.out = out;
+  p.x = x, p.w = w, p.bias = bias, p.out = out;
   p.M = static_cast<int>(M), p.N = static_cast<int>(N), p.K = static_cast<int>(K);
   p.box_m = M <= 32 ? 32 : 64;
   p.w_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
   p.out_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.x_vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
   p.err = err;
-  CUtensorMap ta;
-  if (!encode_tmap_2d(&ta, a16, MGPU_DTYPE_F16, Kp, static_cast<uint64_t>(M), Kp * 2, 64, static_cast<uint32_t>(p.box_m))) return;
-  if (few_rows_columns(N, di.sms) == 16) launch_few_rows<16>(ta, p, s);
-  else launch_few_rows<32>(ta, p, s);
+  CUtensorMap ta = {};
+  if (a16 && !encode_tmap_2d(&ta, a16, MGPU_DTYPE_F16, Kp, static_cast<uint64_t>(M), Kp * 2, 64, static_cast<uint32_t>(p.box_m))) return;
+  const bool narrow = few_rows_columns(N, di.sms) == 16;
+  if (a16) narrow ? launch_few_rows<16, false>(ta, p, s) : launch_few_rows<32, false>(ta, p, s);
+  else narrow ? launch_few_rows<16, true>(ta, p, s) : launch_few_rows<32, true>(ta, p, s);
 }
 
 }  // namespace mdc

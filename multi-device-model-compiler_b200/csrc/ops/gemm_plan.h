@@ -68,10 +68,30 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w,
   return o0 >= w0 + static_cast<uintptr_t>(K) * N * 4 || w0 >= o0 + static_cast<uintptr_t>(M) * N * 4;
 }
 
-// out[M, N] = a16[M, Kp] . w[K, N] + bias, fp16 operands, the weight as the caller has it
-// (gemm_few_rows_tcgen05.cu).  It follows the launch that converts a16, which lets it start after its own
-// wait (OperandList::launch with `late`): the weight is read ahead of that launch's end.
-void gemm_few_rows(const void *a16, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K, cudaStream_t s);
+// Whether gemm_few_rows converts the input too, every CTA for itself, instead of a launch ahead: a launch and its scratch
+// less, for M * K values more that a CTA reads.  us a call, two launches / one, inputs out of memory:
+//   K = 256, 256 columns   16 rows 6.8 / 4.1, 32 rows 7.1 / 4.7, 48 rows 7.0 / 5.8, 64 rows 6.9 / 7.1
+//   K = 768, 768 columns   16 rows 6.9 / 5.1, 32 rows 7.0 / 6.1, 48 rows 6.9 / 7.2
+//   K = 1500, 2000 columns 16 rows 8.8 / 7.8, 24 rows 8.4 / 8.9
+//   K = 2048, 1000 columns  8 rows 12.8 / 12.3, 16 rows 12.6 / 12.9;  K = 4096, 4096 columns 8 rows 21.7 / 21.2, 16 rows 21.3 / 22.3
+//   input read value by value: 770, 500 columns 16 rows 7.0 / 6.2, 24 rows 7.1 / 7.3;  1501, 1000 columns 8 rows 8.4 / 8.0, 12 rows 8.2 / 8.4
+// Below 256 nothing was measured and the launch ahead stays, as it does for an output that overlaps the input: it has read
+// the input before the first store.
+inline bool few_rows_convert(const float *x, const float *out, int64_t M, int64_t N, int64_t K) {
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), o0 = reinterpret_cast<uintptr_t>(out);
+  if (o0 < x0 + static_cast<uintptr_t>(M) * K * 4 && x0 < o0 + static_cast<uintptr_t>(M) * N * 4) return false;
+  if (K < 256) return false;
+  if (M <= 8) return true;
+  if (K % 4 || (x0 & 15u)) return M <= 16 && K <= 768;
+  return (M <= 16 && K <= 1536) || (M <= 32 && K <= 768) || (M <= 48 && K <= 512);
+}
+
+// out[M, N] = x[M, K] . w[K, N] + bias, operands rounded to fp16, the weight as the caller has it
+// (gemm_few_rows_tcgen05.cu).  a16: x as fp16 [M, Kp], or null where the kernel converts it (few_rows_convert).  With a16
+// it follows the launch that converts it, which lets it start after its own wait (OperandList::launch with `late`): the
+// weight is read ahead of that launch's end.
+void gemm_few_rows(const void *a16, const float *x, const float *w, const float *bias, float *out, int64_t M, int64_t N, int64_t K,
+                   cudaStream_t s);
 
 // One call of the one-wave kernel.  w_ready: W was complete before this launch was issued (it does
 // not come from a kernel still queued), so it may be read ahead of the dependency wait.

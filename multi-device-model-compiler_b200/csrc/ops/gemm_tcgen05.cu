@@ -880,9 +880,13 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   cudaStream_t s = as_stream(stream);
   OperandList list;
   if (gemm_takes_few_rows(M, N, K, weight, output, di.sms)) {
+    if (few_rows_convert(input, output, M, N, K)) {
+      gemm_few_rows(nullptr, input, weight, bias, output, M, N, K, s);
+      return;
+    }
     list.cast(input, a16, M, K, Kp);
     list.launch(MGPU_DTYPE_F16, stream, true);
-    gemm_few_rows(a16, weight, bias, output, M, N, K, s);
+    gemm_few_rows(a16, input, weight, bias, output, M, N, K, s);
     return;
   }
   list.pack(weight, w16, K, N);

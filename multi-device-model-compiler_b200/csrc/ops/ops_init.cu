@@ -68,12 +68,16 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   if (!di.ok) return;
   const int64_t Kp = (K + 7) / 8 * 8;
   if (gemm_takes_few_rows(M, N, K, weight, output, di.sms) && !mgpuConstantSourceOf(weight)) {
+    if (few_rows_convert(input, output, M, N, K)) {
+      gemm_few_rows(nullptr, input, weight, bias, output, M, N, K, as_stream(stream));
+      return;
+    }
     void *a16 = mgpuMemAllocAsync(static_cast<uint64_t>(M) * Kp * 2, stream);
     if (!a16) return;
     OperandList list;
     list.cast(input, a16, M, K, Kp);
     list.launch(MGPU_DTYPE_F16, stream, true);
-    gemm_few_rows(a16, weight, bias, output, M, N, K, as_stream(stream));
+    gemm_few_rows(a16, input, weight, bias, output, M, N, K, as_stream(stream));
     mgpuMemFreeAsync(a16, stream);
     return;
   }

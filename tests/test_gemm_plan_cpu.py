@@ -48,6 +48,16 @@ int main() {
   // ranges of bytes beyond 32 bits
   assert(gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, out, 148));
   assert(!gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, reinterpret_cast<const float *>(uintptr_t(1) << 50), 148));
+  // where the input is converted in the Gemm: rows and K, the input's alignment, no overlap with the output
+  using mdc::few_rows_convert;
+  alignas(16) static float in[64];
+  assert(few_rows_convert(in, out, 8, 10, 1 << 20) && few_rows_convert(in + 1, out, 8, 10, 1 << 20));
+  assert(few_rows_convert(in, out, 16, 10, 1536) && !few_rows_convert(in, out, 16, 10, 1540) && !few_rows_convert(in, out, 17, 10, 772));
+  assert(few_rows_convert(in, out, 32, 10, 768) && few_rows_convert(in, out, 48, 10, 512) && !few_rows_convert(in, out, 49, 10, 256));
+  assert(few_rows_convert(in, out, 1, 10, 256) && !few_rows_convert(in, out, 1, 10, 255));
+  assert(few_rows_convert(in, out, 16, 10, 767) && !few_rows_convert(in, out, 17, 10, 767) && !few_rows_convert(in + 1, out, 16, 10, 772));
+  for (int64_t at = -1024; at + 60 <= 3072; ++at)
+    assert(few_rows_convert(w, w + at, 3, 20, 256) == !(at < 768 && at + 60 > 0));
   std::puts("ok");
 }
 """

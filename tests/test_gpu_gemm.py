@@ -359,6 +359,29 @@ def test_output_may_overlap_the_weight(m, entry, M, N, K):
 
 
 @pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
+@pytest.mark.parametrize("offset", [0, 4])  # bytes of the input from its boundary: vectors, value by value
+@pytest.mark.parametrize("M,N,K", [(1, 17, 255), (1, 17, 257), (8, 1000, 2048), (9, 40, 259), (16, 2400, 768), (16, 2500, 1532), (17, 300, 300),
+                                   (32, 2400, 508), (33, 16, 512), (48, 200, 500), (48, 2401, 512), (64, 64, 256)])
+def test_few_rows_with_the_input_converted_inside(m, entry, offset, M, N, K):
+    """Either side of the line to a launch that converts the input, with tails of rows, columns and K, and with the output
+    over the input, which keeps that launch: exact on small integers."""
+    rng = np.random.default_rng(M * N + K)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    ref, dw, db = a @ w + b, m.to_device(w), m.to_device(b)
+    pad = np.zeros(offset // 4, np.float32)
+    mem, out = m.to_device(np.concatenate([pad, a.ravel(), np.zeros(M * N, np.float32)])), m.DeviceBuffer(M * N * 4)
+    for dst, at in ((out, 0), (mem, offset), (mem, offset + 4 * (M * K // 2))):
+        getattr(m.ops(), entry)(mem.ptr + offset, dw.ptr, db.ptr, dst.ptr + at, M, N, K, None)
+        got = m.to_host(dst, (M, N), np.float32, offset_bytes=at)
+        assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+        m.check(entry)
+        assert np.array_equal(got, ref)
+        m.runtime().mgpuMemcpy(mem.ptr + offset, a.ctypes.data, a.nbytes, None)
+        m.runtime().mgpuStreamSynchronize(None)
+
+
+@pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
 @pytest.mark.parametrize("M,N,K", [(16, 1000, 1024), (40, 2400, 500)])  # 16 and 32 columns a CTA
 def test_few_rows_read_what_is_queued_ahead(m, entry, M, N, K):
     """Nothing waits between the calls: the weight and the bias are written by kernels queued ahead of the Gemm (in
