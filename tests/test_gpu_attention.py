@@ -92,6 +92,15 @@ def test_causal(m, S, D):
     _case(m, 2, S, 2, np.array([S, max(1, S // 2)], np.int32), True, m.F16, seed=4, D=D)
 
 
+@pytest.mark.parametrize("causal", [False, True])
+def test_partial_tiles_end_anywhere_in_a_piece(m, causal):
+    """Key tiles are read 32 keys at a time up to the last one that a row of the warp sees: lengths at the pieces' edges,
+    alone in a tile and behind a full one."""
+    edges = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128]
+    _case(m, len(edges), 128, 2, np.array(edges, np.int32), causal, m.F16, seed=31)
+    _case(m, len(edges), 256, 2, np.array([128 + e for e in edges], np.int32), causal, m.F16, seed=32)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_bf16(m, D):
     _case(m, 2, 256, 2, np.array([256, 130], np.int32), False, m.BF16, seed=5, D=D)
