@@ -184,7 +184,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
 
   if (warp == 5) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t t = 0, qn = 0, code = 0;
       for (int item = blockIdx.x; item < n_items && !code; item += gridDim.x) {
         const AttnItem it = attn_item(p, item, q_tiles);
@@ -217,7 +217,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
     }
   } else if (warp == 4) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr bool kBf16 = std::is_same<T16, __nv_bfloat16>::value;
       constexpr uint32_t idesc_s = make_idesc_f16(BQ, BKV, kBf16, false, false);
       constexpr uint32_t idesc_o = make_idesc_f16(BQ, 64, kBf16, false, true);  // V is MN-major
@@ -552,7 +552,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
 
   if (warp == 4) {
     // ------------------------------ loads + MMA issue ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr bool kBf16 = std::is_same<T16, __nv_bfloat16>::value;
       constexpr uint32_t idesc_s = make_idesc_f16(BQ, BKV, kBf16, false, false);
       constexpr uint32_t idesc_o = make_idesc_f16(BQ, D, kBf16, false, true);  // V is MN-major

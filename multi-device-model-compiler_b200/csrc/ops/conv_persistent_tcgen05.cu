@@ -17,16 +17,16 @@
 //     thread per pixel; where k lies in the window comes from a table in shared memory.
 // The filter stays in shared memory for the CTA's life when it fits there.
 //
-// Bound: bytes (input once, output once) for few channels, L2 -> shared memory bandwidth of the
-// patch loads (each input element once per tap) for many.
+// Bound: instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, 340
+// cycles where the MMAs of 64 columns take 192 (conv_plan.h says which calls conv_halo_kernel takes instead).
 // Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
 // changing from call to call:
-//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  73 us (43 of HBM time)
-//   32 x 64 x 56 x 56 -> 64, 3 x 3, residual, ReLU        74 ->  32 us
+//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  64 us (43 of HBM time)
+//   32 x 128 x 28 x 28 -> 128, 3 x 3                            19 us
 // L2 flushed between calls:
-//   26 x 352 x 37 x 46 -> 32, 3 x 3                      155 ->  81 us
 //   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            116 ->  34 us
-//   1 x 128 x 16 x 25 -> 64, 3 x 3                        34 ->  17 us
+// With warp roles by an index that the compiler knows to be uniform and the next barrier looked at ahead (ptx_sm100.cuh)
+// the first shape went from 73 to 64 us, 32 x 256 x 14 x 14 -> 256 from 22.9 to 16.9, 32 x 512 x 7 x 7 -> 512 from 32 to 25.
 // The gather was bound by instruction issue: run-time divisions and per-channel tests in the
 // epilogue, 2.7 us a tile of 128 x 64; with multiplicative division, whole-group stores and the
 // two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).

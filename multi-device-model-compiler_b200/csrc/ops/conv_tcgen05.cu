@@ -277,7 +277,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
     }
   } else if (warp == GATHER_WARPS) {
     // ------------------------- filter loader -------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       const uint32_t tx = static_cast<uint32_t>(bn * BK * 2);
@@ -293,7 +293,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
     }
   } else {
     // ------------------------- MMA issuer -------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(BM, static_cast<uint32_t>(bn), false, false, false);
       int stage = 0;
       uint32_t phase = 0;
