@@ -190,7 +190,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         const AttnItem it = attn_item(p, item, q_tiles);
         if (it.n_kv == 0) continue;
         const uint32_t qs = qn % QS;
-        if (!mbar_wait(&q_empty[qs], ((qn / QS) & 1) ^ 1, abort_flag)) { code = 0x71000000u; break; }
+        if (!mbar_wait_elected(&q_empty[qs], ((qn / QS) & 1) ^ 1, abort_flag)) { code = 0x71000000u; break; }
         mbar_arrive_expect_tx(&q_full[qs], TILE_BYTES);
 #pragma unroll
         for (int blk = 0; blk < C::BLOCKS; ++blk)
@@ -199,13 +199,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         ++qn;
         for (int j = 0; j < it.n_kv; ++j, ++t) {
           const uint32_t st = t % KS, ph = ((t / KS) & 1) ^ 1;
-          if (!mbar_wait(&k_empty[st], ph, abort_flag)) { code = 0x72000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&k_empty[st], ph, abort_flag)) { code = 0x72000000u | (t & 0xffff); break; }
           mbar_arrive_expect_tx(&k_full[st], TILE_BYTES);
 #pragma unroll
           for (int blk = 0; blk < C::BLOCKS; ++blk)
             tma_load_3d(sK + st * TILE_BYTES + blk * BLOCK_BYTES, &tmap_qkv, &k_full[st],
                         hd + it.head * HD + blk * 64, j * BKV, it.b);
-          if (!mbar_wait(&v_empty[st], ph, abort_flag)) { code = 0x73000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&v_empty[st], ph, abort_flag)) { code = 0x73000000u | (t & 0xffff); break; }
           mbar_arrive_expect_tx(&v_full[st], TILE_BYTES);
 #pragma unroll
           for (int blk = 0; blk < C::BLOCKS; ++blk)
@@ -227,12 +227,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         const AttnItem it = attn_item(p, item, q_tiles);
         if (it.n_kv == 0) continue;
         const uint32_t qs = qn % QS;
-        if (!mbar_wait(&q_full[qs], (qn / QS) & 1, abort_flag)) { code = 0x51000000u; break; }
+        if (!mbar_wait_elected(&q_full[qs], (qn / QS) & 1, abort_flag)) { code = 0x51000000u; break; }
         for (int j = 0; j < it.n_kv; ++j, ++t) {
           const uint32_t st = t % KS, ph = (t / KS) & 1;
           // S = Q.K^T.  It overwrites the scores / P of the previous step, which the P.V issued
           // just before has finished reading by the time this executes (one in-order pipe).
-          if (!mbar_wait(&k_full[st], ph, abort_flag)) { code = 0x53000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&k_full[st], ph, abort_flag)) { code = 0x53000000u | (t & 0xffff); break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) {
@@ -244,8 +244,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
           umma_commit(&k_empty[st]);
           if (j == it.n_kv - 1) umma_commit(&q_empty[qs]);
           // O (+)= P.V, one N = 64 MMA group per 64 output columns
-          if (!mbar_wait(&p_ready, t & 1, abort_flag)) { code = 0x55000000u | (t & 0xffff); break; }
-          if (!mbar_wait(&v_full[st], ph, abort_flag)) { code = 0x56000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&p_ready, t & 1, abort_flag)) { code = 0x55000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&v_full[st], ph, abort_flag)) { code = 0x56000000u | (t & 0xffff); break; }
           tc_fence_after();
 #pragma unroll
           for (int nb = 0; nb < C::BLOCKS; ++nb) {
@@ -592,13 +592,13 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         }
         const bool has_next = n_item < n_items;
         if (j == 0) {
-          if (!mbar_wait(&bar_q, q_cnt & 1, abort_flag)) { code = 0x51000000u; break; }
+          if (!mbar_wait_elected(&bar_q, q_cnt & 1, abort_flag)) { code = 0x51000000u; break; }
           ++q_cnt;
         }
         // S overwrites the columns that held P and O of the previous step: the softmax
         // threads must have read that O (the P.V that read P has completed by then)
-        if (t > 0 && !mbar_wait(&bar_o_read, ph ^ 1, abort_flag)) { code = 0x57000000u | (t & 0xffff); break; }
-        if (!mbar_wait(&bar_k, ph, abort_flag)) { code = 0x53000000u | (t & 0xffff); break; }
+        if (t > 0 && !mbar_wait_elected(&bar_o_read, ph ^ 1, abort_flag)) { code = 0x57000000u | (t & 0xffff); break; }
+        if (!mbar_wait_elected(&bar_k, ph, abort_flag)) { code = 0x53000000u | (t & 0xffff); break; }
         tc_fence_after();
         {
           const uint64_t a_desc = make_smem_desc_sw128(q_addr, 16, 1024);
@@ -608,14 +608,14 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
             umma_f16_ss(tmem_base + S_COL, a_desc + 2 * k, b_desc + 2 * k, idesc_s, k != 0);
         }
         umma_commit(&bar_s_full);
-        if (!mbar_wait(&bar_s_full, ph, abort_flag)) { code = 0x54000000u | (t & 0xffff); break; }
+        if (!mbar_wait_elected(&bar_s_full, ph, abort_flag)) { code = 0x54000000u | (t & 0xffff); break; }
         if (has_next) {
           // K (and, when this was the item's last tile, Q) are free: prefetch the next step's
           if (n_j == 0) load_q(nxt);
           load_k(nxt, n_j);
         }
-        if (!mbar_wait(&bar_p_ready, ph, abort_flag)) { code = 0x55000000u | (t & 0xffff); break; }
-        if (!mbar_wait(&bar_v, ph, abort_flag)) { code = 0x56000000u | (t & 0xffff); break; }
+        if (!mbar_wait_elected(&bar_p_ready, ph, abort_flag)) { code = 0x55000000u | (t & 0xffff); break; }
+        if (!mbar_wait_elected(&bar_v, ph, abort_flag)) { code = 0x56000000u | (t & 0xffff); break; }
         tc_fence_after();
         {
 #pragma unroll
@@ -629,7 +629,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         umma_commit(&bar_o_full);
         if (has_next) {
           // V is free once this P.V has been computed
-          if (!mbar_wait(&bar_o_full, ph, abort_flag)) { code = 0x52000000u | (t & 0xffff); break; }
+          if (!mbar_wait_elected(&bar_o_full, ph, abort_flag)) { code = 0x52000000u | (t & 0xffff); break; }
           load_v(nxt, n_j);
         }
         ++t;

@@ -282,7 +282,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
       uint32_t phase = 0;
       const uint32_t tx = static_cast<uint32_t>(bn * BK * 2);
       for (int kb = 0; kb < p.num_kb; ++kb) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        if (!mbar_wait_elected(&empty_bar[stage], phase ^ 1, abort_flag)) {
           atomicCAS(p.err, 0u, 0x51000000u | static_cast<uint32_t>(stage));
           break;
         }
@@ -299,7 +299,7 @@ conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const conv::Para
       uint32_t phase = 0;
       bool ok = true;
       for (int kb = 0; kb < p.num_kb; ++kb) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_elected(&full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x53000000u | static_cast<uint32_t>(stage));
           ok = false;
           break;

@@ -112,6 +112,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
   }
 }
 
+// The wait of a role that one elected thread runs from end to end (`if (elect_one()) { ... }`).
+__device__ __forceinline__ bool mbar_wait_elected(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag) {
+  return mbar_wait(bar, parity, abort_flag);
+}
+
 // The same wait for a whole (converged) warp: lane 0 polls, the others are released by the
 // shuffle.  Keeps 31 of 32 threads off the barrier word and off the global timer, which is
 // slow to read when hundreds of threads do so at once.

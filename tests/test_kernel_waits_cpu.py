@@ -36,6 +36,21 @@ def test_warps_wait_with_one_verdict(name):
         assert any("lane == 0" in opener for opener in _enclosing(code, call.start())), code[call.start() - 80:call.end() + 60]
 
 
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(OPS) if f.endswith(".cu")))
+def test_elected_waits_stand_under_an_election(name):
+    """mbar_wait_elected is mbar_wait where one elected thread runs the whole role.  Nothing warp-wide may stand there
+    either: the other lanes never come to a second election, a vote or a shuffle."""
+    code = _code(name)
+    for call in re.finditer(r"\bmbar_wait_elected\(", code):
+        assert "if (elect_one())" in " ".join(_enclosing(code, call.start())), code[call.start() - 80:call.end() + 60]
+    for role in re.finditer(r"if \(elect_one\(\)\) \{", code):
+        depth, end = 1, role.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[end], 0)
+            end += 1
+        assert not re.search(r"elect_one|_sync\(0x|_warp\(|_all\(|kblocks|umma_planes|mbar_wait_looked", code[role.end():end]), code[role.start():end][:300]
+
+
 def test_the_warp_waits_are_uniform():
     code = _code("ptx_sm100.cuh")
 
