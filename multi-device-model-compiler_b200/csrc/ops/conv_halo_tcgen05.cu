@@ -12,7 +12,7 @@
 //           in turn; the next sixteen channels' loads are in flight while these are converted.  Up to eight channels make
 //           one group, and an MMA takes two taps of a filter row: the second half of its sixteen k lies as far from the
 //           first as the next tap's pixel.  The last tap of an odd row is paired with zeros, not with the pixel beyond the
-//           window: zero weights would turn an infinity there into NaN.  Strides of two keep rows and columns in classes.
+//           window: zero weights would turn an infinity there into NaN.  A sum is made in parts (halo_chain).  Strides of two keep rows and columns in classes.
 //           The filter is packed by a launch ahead; this kernel starts once that launch's own dependency is resolved and
 //           reads the input before the filter is complete.
 //   warps 0-7   epilogue: accumulator -> bias, residual, ReLU -> NCHW, alternate tiles on up to four accumulators
@@ -45,7 +45,7 @@ constexpr int MAX_STAGES = 12;
 constexpr int EPI_WARPS = 8, IN_WARPS = 12;
 constexpr int threads(bool copy) { return (EPI_WARPS + 2 + (copy ? 1 : IN_WARPS)) * 32; }
 constexpr int kMaxOC = 2048;  // bias kept in shared memory
-constexpr int kMaxTaps = 128;
+constexpr int kMaxTaps = 64;  // entries of the tables below: taps, or pairs of them (a longer list is a slower launch)
 constexpr size_t kMaxSmem = 220 * 1024;
 
 struct Params {
@@ -63,7 +63,8 @@ struct Params {
   int taps;                   // entries of `tap`
   int bn, n_tiles, num_tiles, stages, resident, filter_stages, filter_kbs, relu;
   uint32_t region_bytes, tmem_cols;
-  int accs;                   // accumulators in tensor memory
+  int accs;                   // accumulators in tensor memory, of `splits` sums each
+  int splits, chain;          // few channels: MMAs per sum (see halo_chain)
   uint32_t regions_bytes;     // of all stages
   // A's descriptor in units of 16 bytes: leading offset, high word, from sixteen channels to the next
   uint32_t lead, a_hi, a_step;
@@ -71,6 +72,7 @@ struct Params {
   // What is added to the low word of A's descriptor for a tap (a pair of taps): where its pixels start, and with a tap
   // that has no partner the way to the zeros.  In the constant bank, so that the loop over taps has no arithmetic.
   uint32_t tap[kMaxTaps];
+  uint16_t sum[kMaxTaps];  // few channels: columns to the MMA's sum, and in the top bit whether it adds to it
 };
 }  // namespace convh
 
@@ -223,6 +225,15 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         if constexpr (G == 32) tmem_ld_32x32(addr, a);
         else tmem_ld_32x16(addr, a);
         tmem_ld_wait_regs(a);
+        if constexpr (!kCopy) {
+          for (int i = 1; i < p.splits; ++i) {
+            uint32_t more[16];
+            tmem_ld_32x16(addr + static_cast<uint32_t>(i * p.bn), more);
+            tmem_ld_wait_regs(more);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] = __float_as_uint(__uint_as_float(a[j]) + __uint_as_float(more[j]));
+          }
+        }
 #pragma unroll
         for (int j = 0; j < G; j += 4) {
           float4 b = *reinterpret_cast<const float4 *>(bias_s + n0 + c0 + j);
@@ -331,19 +342,28 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           if (++f_stage == p.filter_stages) { f_stage = 0; f_phase ^= 1; }
         }
       };
-      // The MMAs of one region.  STEPS: sixteens of channels of a tap, zero for pairs of taps.
+      // The MMAs of one region.  STEPS: sixteens of channels of a tap; few channels: 0 pairs of taps, 5 single ones.
       auto taps = [&](auto steps, auto resident, uint32_t region) __attribute__((always_inline)) -> bool {
         constexpr int STEPS = decltype(steps)::value;
         constexpr bool RES = decltype(resident)::value;
         if constexpr (STEPS == 0) {
           // a k-block holds four pairs, rows of the filter one after the other
+          auto one = [&](int t, uint32_t b) __attribute__((always_inline)) {
+            umma_planes<1>(d + (p.sum[t] & 0x7fffu), region + p.tap[t], p.a_hi, 0, b, f_hi, idesc, static_cast<uint32_t>(p.sum[t] >> 15));
+          };
           for (int t = 0; t < p.taps; t += 4) {
             if (!RES && !filter_ready()) return false;
-            umma_planes<1>(d, region + p.tap[t], p.a_hi, 0, b_lo, f_hi, idesc, accumulate);
-            accumulate = 1;
-            if (t + 1 < p.taps) umma_planes<1>(d, region + p.tap[t + 1], p.a_hi, 0, b_lo + 2, f_hi, idesc, 1);
-            if (t + 2 < p.taps) umma_planes<1>(d, region + p.tap[t + 2], p.a_hi, 0, b_lo + 4, f_hi, idesc, 1);
-            if (t + 3 < p.taps) umma_planes<1>(d, region + p.tap[t + 3], p.a_hi, 0, b_lo + 6, f_hi, idesc, 1);
+            one(t, b_lo);
+            if (t + 1 < p.taps) one(t + 1, b_lo + 2);
+            if (t + 2 < p.taps) one(t + 2, b_lo + 4);
+            if (t + 3 < p.taps) one(t + 3, b_lo + 6);
+            b_lo += b_step;
+            if (!RES) filter_done();
+          }
+        } else if constexpr (STEPS == 5) {
+          for (int t = 0; t < p.taps; ++t) {
+            if (!RES && !filter_ready()) return false;
+            umma_planes<1>(d + (p.sum[t] & 0x7fffu), region + p.tap[t], p.a_hi, 0, b_lo, f_hi, idesc, static_cast<uint32_t>(p.sum[t] >> 15));
             b_lo += b_step;
             if (!RES) filter_done();
           }
@@ -364,6 +384,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         case 1: return taps(std::integral_constant<int, 1>{}, resident, region);
         case 2: return taps(std::integral_constant<int, 2>{}, resident, region);
         case 3: return taps(std::integral_constant<int, 3>{}, resident, region);
+        case 5: return taps(std::integral_constant<int, 5>{}, resident, region);
         default: return taps(std::integral_constant<int, 4>{}, resident, region);
         }
       };
@@ -377,7 +398,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const int next = stage + 1 == p.stages ? 0 : stage + 1;
         looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
         const uint32_t region = a_lo0 + static_cast<uint32_t>(stage) * region_units;
-        const int steps = p.pairs ? 0 : cb + 1 < p.ncb ? 4 : p.last_steps;
+        const int steps = p.chain ? (p.pairs ? 0 : 5) : cb + 1 < p.ncb ? 4 : p.last_steps;
         ok = p.resident ? of_steps(std::true_type{}, steps, region) : of_steps(std::false_type{}, steps, region);
         if (!ok) break;
         umma_commit_warp(&empty_bar[stage]);
@@ -616,6 +637,13 @@ void launch_halo(const CUtensorMap &tx, const CUtensorMap &tw, const convh::Para
   launched("conv_halo_kernel");
 }
 
+// The tensor core adds to its fp32 sum once per MMA, and rounds there.  With few channels an MMA holds padding and a sum takes
+// more of them than one over a dense patch, as the gather kernel builds it, would: 28 instead of 10 for 7 x 7 x 3, which
+// was 5.3e-7 off a sum in 64 bits where the dense one is 2.3e-7 (2-norm, relative).  So such a sum is made in as many
+// parts as it takes to have no more MMAs in each, added in the epilogue.  0: one sum (16 channels or more: no other kernel
+// is denser).
+int halo_chain(const ConvShape &c) { return c.IC < 16 ? static_cast<int>((c.IC * c.KH * c.KW + 15) / 16) : 0; }
+
 // Tile width, by the cycles of the busiest CTA; fills in what follows from the shape.  False where nothing fits.
 bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Params *best, size_t *smem) {
   const int64_t ncb = (c.IC + 63) / 64, taps = c.KH * c.KW, pair_taps = c.KH * ((c.KW + 1) / 2);
@@ -623,9 +651,11 @@ bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Param
   const int64_t num_kb = pairs ? (pair_taps + 3) / 4 : ncb * taps;
   const int last_steps = static_cast<int>((c.IC - (ncb - 1) * 64 + 15) / 16), steps = ncb > 1 ? 4 : last_steps;
   const int64_t mmas = pairs ? pair_taps : ((ncb - 1) * 4 + last_steps) * taps;
-  if (c.OC > convh::kMaxOC || taps > convh::kMaxTaps || ncb * taps > (1 << 16) || c.OH * c.OW > INT32_MAX) return false;
+  if (c.OC > convh::kMaxOC || (pairs ? pair_taps : taps) > convh::kMaxTaps || ncb * taps > (1 << 16) || c.OH * c.OW > INT32_MAX) return false;
   convh::Params p;
   p.ncb = static_cast<int>(ncb), p.last_steps = last_steps, p.pairs = pairs ? 1 : 0, p.num_kb = static_cast<int>(num_kb);
+  p.chain = halo_chain(c);
+  p.splits = p.chain ? static_cast<int>((mmas + p.chain - 1) / p.chain) : 1;
   if (!halo_plan(c, flat, &p.h)) return false;
   p.qb = (p.h.px + 31) / 32;
   if (copy) {
@@ -639,7 +669,7 @@ bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Param
   }
   double best_cost = 1e300;
   for (int bn = 256; bn >= 32; bn -= 32) {
-    if (bn > 32 && bn >= c.OC + 32) continue;
+    if ((bn > 32 && bn >= c.OC + 32) || 2 * p.splits * bn > 512) continue;
     size_t need;
     if (!fit_halo(&p, copy, c.OC, num_kb, bn, sms, &need)) continue;
     const int64_t tiles = p.h.m_tiles * ((c.OC + bn - 1) / bn);
@@ -653,7 +683,7 @@ bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Param
     const double l2 = (copy ? static_cast<double>(ncb) * p.region_bytes : 0.0) / 64.0 + (p.resident ? 0.0 : num_kb * bn * 2.0);
     const double loads = copy ? 0.0 : p.qb * (pairs ? static_cast<double>(c.IC) : (ncb - 1) * 64.0 + last_steps * 16.0);
     const double work = copy ? 0.0 : p.qb * ((ncb - 1) * 4.0 + last_steps) * 100.0 + p.qb * ncb * 60.0;
-    const double epi = bn * (c.add ? 1024.0 : 512.0) / 24.0;
+    const double epi = bn * ((c.add ? 1024.0 : 512.0) / 24.0 + 4.0 * (p.splits - 1));
     const double lsu = loads * in_lines + bn * 4.0 * out_lines * (c.add ? 2.0 : 1.0);
     const double cost = rounds * (std::max({mma, l2, lsu, epi, work}) + 300.0) + epi + (copy ? l2 : 3.0 * loads);
     if (cost < best_cost * 0.98) best_cost = cost, *best = p, *smem = need;
@@ -698,9 +728,9 @@ const HaloChoice &halo_choice(const ConvShape &call, int sms) {
   p.by_ntiles = Divisor(p.n_tiles), p.by_tiles_w = Divisor(p.h.tiles_w), p.by_iw = Divisor(p.h.IW);
   p.by_hv = Divisor(p.h.Hv), p.by_hvo = Divisor(p.h.HvO);
   p.alternate = p.num_tiles > sms ? 1 : 0;
-  p.accs = p.bn <= 128 ? 4 : 2;
+  p.accs = p.splits * p.bn <= 128 ? 4 : 2;
   p.tmem_cols = 32;
-  while (p.tmem_cols < static_cast<uint32_t>(p.accs * p.bn)) p.tmem_cols *= 2;
+  while (p.tmem_cols < static_cast<uint32_t>(p.accs * p.splits * p.bn)) p.tmem_cols *= 2;
   auto pixel = [&](int64_t rh, int64_t rw) {  // of the region, that a tap starts at
     return static_cast<uint32_t>(((rh % c.SH) * c.SW + rw % c.SW) * p.h.class_px + rh / c.SH * p.h.pitch + rw / c.SW);
   };
@@ -717,6 +747,8 @@ const HaloChoice &halo_choice(const ConvShape &call, int sms) {
     for (int64_t kw = 0; kw < c.KW; kw += p.pairs ? 2 : 1)
       p.tap[p.taps++] = pixel(kh * c.DH, kw * c.DW) * (copy ? 8 : 1) +
                         (p.pairs && kw + 1 == c.KW ? (static_cast<uint32_t>(p.h.plane_px) - p.lead) << 16 : 0u);
+  for (int t = 0; p.chain && t < p.taps; ++t)
+    p.sum[t] = static_cast<uint16_t>(t / p.chain * p.bn | (t % p.chain ? 1 << 15 : 0));
   return e;
 }
 }  // namespace
@@ -724,6 +756,12 @@ const HaloChoice &halo_choice(const ConvShape &call, int sms) {
 bool conv_halo(const ConvShape &call, cudaStream_t s) {
   using namespace convh;
   const DeviceInfo &di = device_info();
+  {
+    // most small calls are not for this kernel: no look at the table for them
+    ConvShape sampled = call;
+    conv_sampled(sampled);
+    if (conv_form(sampled, di.sms) == ConvForm::kOther) return false;
+  }
   const HaloChoice &e = halo_choice(call, di.sms);
   if (e.form == ConvForm::kOther) return false;
   const bool copy = e.form == ConvForm::kCopyRect || e.form == ConvForm::kCopyFlat;

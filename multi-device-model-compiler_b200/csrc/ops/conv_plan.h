@@ -84,11 +84,14 @@ bool conv_prepare(const ConvShape &c, const ConvShape &call, bool sampled, int64
 //   copy, 1 x 1                         32x64x56x56->256 73 / 58, 45x192x47x35->32 26 / 21, 2x32x179x207->131 38 / 24
 //   copy, up to 64 outputs              16x16x112x112->16 31 / 16, 32x64x56x56->64 with residual 26.9 / 25.1
 //   copy, few tiles and many channels   17x448x13x9->113 18.2 / 16.4, 1x160x9x7->96 10.3 / 9.2, 32x512x7x7->512 25.0 / 23.1
-// elsewhere the im2col kernel's stores win, whose 32 pixels of a warp are neighbours in memory: 32x128x28x28->128 19.2 / 20.4,
+// A call of one round of tiles and up to ten k-blocks is bound by its launches, and this kernel's parameters are the longer
+// ones: 2x32x20x20->32 7.9 / 8.0, 9x96x21x30->32 1x1 stride 2 7.9 / 8.1.
+// Elsewhere the im2col kernel's stores win, whose 32 pixels of a warp are neighbours in memory: 32x128x28x28->128 19.2 / 20.4,
 // 25x224x38x43->192 49.8 / 54.2, 34x32x23x21->352 22.2 / 23.8.  Rect keeps to whole sectors where rows of the output are
 // multiples of eight pixels (32x64x56x56->64 19.2, flat 25.2); flat wastes less elsewhere (32x256x14x14->256 17.4, rect 20.7).
-//   direct, up to 15 channels           16x3x224x224->32 7x7 142 / 66, 21x3x29x37->352 3x3 21.9 / 15.6; but 16x3x256x256->64
-//                                       3x3 64 / 69, 30x3x250x256->32 3x3 stride 2 44 / 57
+//   direct, up to 15 channels           16x3x224x224->32 7x7 143 / 79, 16x3x128x128->64 5x5 43 / 33, 4x12x100x100->64 5x5 29 / 11.5;
+//                                       but 16x3x256x256->64 3x3 64 / 69, 30x3x250x256->32 3x3 stride 2 44 / 57, and windows
+//                                       that reach far: 18x3x18x29->96 7x7 dilation 2 12.3 / 12.8
 //   direct, stride 2, up to 32 channels 42x32x97x102->32 5x5 54 / 46, 2x32x22x23->32 7x7 15.5 / 13.5; but 1x32x165x248->192 28 / 31
 enum class ConvForm { kOther, kCopyRect, kCopyFlat, kDirectRect, kDirectFlat };
 inline ConvForm conv_form(const ConvShape &c, int sms) {
@@ -99,9 +102,10 @@ inline ConvForm conv_form(const ConvShape &c, int sms) {
     if (c.SH > 2 || c.SW > 2) return ConvForm::kOther;
     return unit && c.OW < 48 && halo_plan(c, true, &h) ? ConvForm::kDirectFlat : ConvForm::kDirectRect;
   };
-  if (c.IC < 16) return taps >= 25 || c.OC > 256 ? direct() : ConvForm::kOther;
+  if (c.IC < 16) return taps >= 25 && (c.KH - 1) * c.DH <= 8 && (c.KW - 1) * c.DW <= 8 ? direct() : ConvForm::kOther;
   if (!unit) return c.IC <= 32 && taps >= 25 && (c.OC <= 64 || pixels < 5000) ? direct() : ConvForm::kOther;
   const bool few = (pixels + 127) / 128 * ((c.OC + 63) / 64) <= sms;
+  if (few && (c.IC + 63) / 64 * taps <= 10) return ConvForm::kOther;
   if (taps > 1 && c.OC > 64 && c.IC < 384 && !(taps >= 25 && (c.OC <= 128 || c.IC >= 64)) && !(few && c.IC >= 64)) return ConvForm::kOther;
   if (taps > 1 && c.OW % 8 == 0) return ConvForm::kCopyRect;
   return halo_plan(c, true, &h) && h.px <= 512 ? ConvForm::kCopyFlat : ConvForm::kCopyRect;

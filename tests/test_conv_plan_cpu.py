@@ -83,10 +83,12 @@ int main() {
     return conv_form(c, 148);
   };
   assert(form(16, 3, 256, 256, 64, 3, 1) == ConvForm::kOther && form(16, 3, 224, 224, 32, 7, 1) == ConvForm::kDirectRect);
-  assert(form(21, 3, 29, 37, 352, 3, 1) == ConvForm::kDirectFlat && form(8, 15, 20, 20, 8, 5, 3) == ConvForm::kOther);
+  assert(form(21, 3, 29, 37, 352, 5, 1) == ConvForm::kDirectFlat && form(8, 15, 20, 20, 8, 5, 3) == ConvForm::kOther);
+  assert(form(8, 3, 29, 37, 32, 9, 1) == ConvForm::kDirectFlat && form(8, 3, 29, 37, 32, 11, 1) == ConvForm::kOther);
   assert(form(32, 64, 56, 56, 64, 3, 1) == ConvForm::kCopyRect && form(32, 64, 57, 57, 64, 3, 1) == ConvForm::kCopyFlat);
   assert(form(32, 128, 28, 28, 128, 3, 1) == ConvForm::kOther && form(32, 512, 7, 7, 512, 3, 1) == ConvForm::kCopyFlat);
   assert(form(32, 64, 56, 56, 256, 1, 1) == ConvForm::kCopyFlat && form(1, 160, 9, 7, 96, 3, 1) == ConvForm::kCopyFlat);
+  assert(form(2, 64, 20, 20, 32, 3, 1) == ConvForm::kOther && form(2, 65, 20, 20, 32, 3, 1) == ConvForm::kCopyFlat);
   assert(form(2, 32, 22, 23, 32, 7, 2) == ConvForm::kDirectRect && form(2, 64, 22, 23, 32, 7, 2) == ConvForm::kOther);
   printf("ok\n");
 }

@@ -205,17 +205,18 @@ def test_conv_persistent_edges(m, shape):
 
 @pytest.mark.parametrize("shape", [
     # N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
-    (3, 16, 9, 16, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False),      # rect out of a copy: tiles of two images
+    (3, 16, 9, 16, 16, 5, 3, (1, 1), (2, 1, 2, 1), (1, 1), True, False),      # rect out of a copy: tiles of two images
     (2, 72, 33, 24, 33, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),     # rect: a block of 8 channels, three rounds of rows
     (40, 64, 24, 24, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True),     # rect: filter kept, several tiles per CTA
-    (5, 40, 7, 9, 20, 3, 5, (1, 1), (0, 3, 2, 1), (2, 1), True, False),       # flat out of a copy: asymmetric
+    (5, 80, 7, 9, 20, 3, 5, (1, 1), (0, 3, 2, 1), (2, 1), True, False),       # flat out of a copy: asymmetric
     (60, 100, 13, 11, 60, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),  # flat: filter streamed, 36 channels in the last block
-    (9, 20, 19, 17, 300, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, True),     # flat, 1 x 1: two channel tiles
-    (7, 48, 15, 14, 260, 1, 1, (2, 3), (0, 0, 0, 0), (1, 1), False, True),    # the same, sampled
+    (60, 20, 19, 17, 300, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, True),    # flat, 1 x 1: two channel tiles
+    (150, 48, 15, 14, 260, 1, 1, (2, 3), (0, 0, 0, 0), (1, 1), False, True),  # the same, sampled
     (2, 3, 21, 70, 24, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, False),      # straight from the input: rect, a tap without a partner
     (3, 8, 12, 10, 40, 6, 6, (1, 1), (3, 2, 2, 3), (1, 1), False, True),      # flat, pairs only
     (70, 1, 30, 31, 33, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), False, False),    # stride 2: classes of rows and columns
-    (2, 5, 23, 64, 300, 3, 3, (2, 1), (0, 1, 1, 1), (2, 3), True, False),     # strides and dilations apart, two channel tiles
+    (2, 5, 23, 64, 300, 5, 5, (2, 1), (0, 1, 1, 1), (1, 2), True, False),     # strides and dilations apart, several channel tiles
+    (2, 1, 20, 50, 48, 9, 9, (1, 1), (4, 4, 4, 4), (1, 1), False, False),     # one channel: eight parts of a sum, 32 columns a tile
     (3, 15, 14, 9, 17, 5, 5, (1, 2), (2, 2, 2, 2), (1, 3), False, True),      # two groups of channels, columns in two classes
     (4, 32, 18, 21, 64, 7, 5, (2, 2), (3, 2, 3, 2), (1, 1), True, True),      # stride 2, 32 channels
 ])
