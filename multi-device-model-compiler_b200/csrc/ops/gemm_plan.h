@@ -71,10 +71,13 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w,
 // Whether gemm_few_rows converts the input too, every CTA for itself, instead of a launch ahead: a launch and its scratch
 // less, for M * K values more that a CTA reads.  us a call, two launches / one, inputs out of memory:
 //   K = 256, 256 columns   16 rows 6.8 / 4.1, 32 rows 7.1 / 4.7, 48 rows 7.0 / 5.8, 64 rows 6.9 / 7.1
+//   K = 512, 1000 columns  16 rows 6.9 / 4.4, 32 rows 7.2 / 5.3, 48 rows 7.0 / 6.4
 //   K = 768, 768 columns   16 rows 6.9 / 5.1, 32 rows 7.0 / 6.1, 48 rows 6.9 / 7.2
 //   K = 1500, 2000 columns 16 rows 8.8 / 7.8, 24 rows 8.4 / 8.9
 //   K = 2048, 1000 columns  8 rows 12.8 / 12.3, 16 rows 12.6 / 12.9;  K = 4096, 4096 columns 8 rows 21.7 / 21.2, 16 rows 21.3 / 22.3
 //   input read value by value: 770, 500 columns 16 rows 7.0 / 6.2, 24 rows 7.1 / 7.3;  1501, 1000 columns 8 rows 8.4 / 8.0, 12 rows 8.2 / 8.4
+// Two launches never take less than the host needs for them, 7 us here and 6 on a faster one (48 rows, K = 448: 6.1 / 6.3),
+// so the line is drawn where one launch takes less than 6.
 // Below 256 nothing was measured and the launch ahead stays, as it does for an output that overlaps the input: it has read
 // the input before the first store.
 inline bool few_rows_convert(const float *x, const float *out, int64_t M, int64_t N, int64_t K) {
@@ -83,7 +86,7 @@ inline bool few_rows_convert(const float *x, const float *out, int64_t M, int64_
   if (K < 256) return false;
   if (M <= 8) return true;
   if (K % 4 || (x0 & 15u)) return M <= 16 && K <= 768;
-  return (M <= 16 && K <= 1536) || (M <= 32 && K <= 768) || (M <= 48 && K <= 512);
+  return (M <= 16 && K <= 1536) || (M <= 32 && K <= 512);
 }
 
 // out[M, N] = x[M, K] . w[K, N] + bias, operands rounded to fp16, the weight as the caller has it

@@ -53,7 +53,7 @@ int main() {
   alignas(16) static float in[64];
   assert(few_rows_convert(in, out, 8, 10, 1 << 20) && few_rows_convert(in + 1, out, 8, 10, 1 << 20));
   assert(few_rows_convert(in, out, 16, 10, 1536) && !few_rows_convert(in, out, 16, 10, 1540) && !few_rows_convert(in, out, 17, 10, 772));
-  assert(few_rows_convert(in, out, 32, 10, 768) && few_rows_convert(in, out, 48, 10, 512) && !few_rows_convert(in, out, 49, 10, 256));
+  assert(few_rows_convert(in, out, 32, 10, 512) && !few_rows_convert(in, out, 32, 10, 516) && !few_rows_convert(in, out, 33, 10, 256));
   assert(few_rows_convert(in, out, 1, 10, 256) && !few_rows_convert(in, out, 1, 10, 255));
   assert(few_rows_convert(in, out, 16, 10, 767) && !few_rows_convert(in, out, 17, 10, 767) && !few_rows_convert(in + 1, out, 16, 10, 772));
   for (int64_t at = -1024; at + 60 <= 3072; ++at)
