@@ -41,38 +41,27 @@ bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t 
 
 namespace convh {
 constexpr int BM = 128, BK = 64;
-constexpr int MAX_STAGES = 12;
-constexpr int EPI_WARPS = 8, IN_WARPS = 12;
+constexpr int MAX_STAGES = kHaloFilterStages;
+constexpr int EPI_WARPS = 8, IN_WARPS = kHaloInputWarps;
 constexpr int threads(bool copy) { return (EPI_WARPS + 2 + (copy ? 1 : IN_WARPS)) * 32; }
-constexpr int kMaxOC = 2048;  // bias kept in shared memory
-constexpr int kMaxTaps = 64;  // entries of the tables below: taps, or pairs of them (a longer list is a slower launch)
-constexpr size_t kMaxSmem = 220 * 1024;
 
-struct Params {
+struct Params : HaloTile {
   const float *x, *bias, *add;
   float *out;
   int N, IC, H, W, OC, KH, KW, OH, OW, PHL, PWL, SH, SW, DH, DW;
-  HaloPlan h;
   Divisor by_ntiles, by_tiles_w, by_iw, by_hv, by_hvo;
-  int ncb, last_steps;        // blocks of 64 channels; sixteens of the last one's channels
-  int pairs;                  // up to eight channels: MMAs of two taps
-  int num_kb;                 // filter blocks of 64 k
-  int qb;                     // 32-pixel pieces of a region
-  int boxes, box_px;          // loads that make up a copy's region, and the pixels of one
   int alternate;              // epilogue: the two warps of a lane quarter take alternate tiles instead of alternate channels
   int taps;                   // entries of `tap`
-  int bn, n_tiles, num_tiles, stages, resident, filter_stages, filter_kbs, relu;
-  uint32_t region_bytes, tmem_cols;
+  int n_tiles, num_tiles, relu;
+  uint32_t tmem_cols;
   int accs;                   // accumulators in tensor memory, of `splits` sums each
-  int splits, chain;          // few channels: MMAs per sum (see halo_chain)
-  uint32_t regions_bytes;     // of all stages
   // A's descriptor in units of 16 bytes: leading offset, high word, from sixteen channels to the next
   uint32_t lead, a_hi, a_step;
   uint32_t *err;
   // What is added to the low word of A's descriptor for a tap (a pair of taps): where its pixels start, and with a tap
   // that has no partner the way to the zeros.  In the constant bank, so that the loop over taps has no arithmetic.
-  uint32_t tap[kMaxTaps];
-  uint16_t sum[kMaxTaps];  // few channels: columns to the MMA's sum, and in the top bit whether it adds to it
+  uint32_t tap[kHaloMaxTaps];
+  uint16_t sum[kHaloMaxTaps];  // few channels: columns to the MMA's sum, and in the top bit whether it adds to it
 };
 }  // namespace convh
 
@@ -590,40 +579,14 @@ __global__ void __launch_bounds__(256) conv_filter_kernel(const FilterPackParams
 }
 
 namespace {
-// Shared memory: regions, then the filter whole or a ring of its k-blocks, several to a stage where they are short (a
-// hand-over costs as much as the MMAs of 64 columns).  False where it does not fit.
-bool fit_halo(convh::Params *p, bool copy, int64_t OC, int64_t num_kb, int bn, int sms, size_t *smem) {
-  const int64_t fixed = 2048 + (OC + 31) / 32 * 128, room = static_cast<int64_t>(convh::kMaxSmem) - fixed;
-  const int64_t b_bytes = bn * convh::BK * 2, filter = num_kb * b_bytes, region = p->region_bytes;
-  const int64_t most = region <= 16 * 1024 ? 8 : 4;
-  const int64_t tiles = p->h.m_tiles * ((OC + bn - 1) / bn);
-  const bool resident = OC <= bn && tiles > sms && filter + 2 * region <= room;
-  int64_t kbs = 32 * 1024 / b_bytes;
-  if (kbs > 4) kbs = 4;
-  if (kbs > num_kb) kbs = num_kb;
-  const int64_t blocks = (num_kb + kbs - 1) / kbs, least = blocks < 3 ? blocks : 3;
-  int64_t n = (room - (resident ? filter : least * kbs * b_bytes)) / region;
-  if (n > most) n = most;
-  // as many stages as regions that the input warps' pieces reach over: a stage's barrier is then never two uses behind
-  const int64_t reach = copy ? 0 : (convh::IN_WARPS + p->qb - 1) / p->qb;
-  if (n < 2 || n < reach) return false;
-  int64_t fs = (room - n * region) / (kbs * b_bytes);
-  if (fs > convh::MAX_STAGES) fs = convh::MAX_STAGES;
-  p->bn = bn, p->resident = resident ? 1 : 0, p->stages = static_cast<int>(n);
-  p->filter_stages = resident ? 0 : static_cast<int>(fs), p->filter_kbs = static_cast<int>(kbs);
-  p->regions_bytes = static_cast<uint32_t>((n * region + 1023) / 1024 * 1024);
-  *smem = static_cast<size_t>(1024 + p->regions_bytes + (resident ? filter : fs * kbs * b_bytes) + (OC + 31) / 32 * 128);
-  return true;
-}
-
 template <bool kCopy, bool kAdd>
-void launch_halo(const CUtensorMap &tx, const CUtensorMap &tw, const convh::Params &p, size_t smem, int sms, cudaStream_t s) {
+void launch_halo(const CUtensorMap &tx, const CUtensorMap &tw, const convh::Params &p, int sms, cudaStream_t s) {
   auto kern = conv_halo_kernel<kCopy, kAdd>;
   static bool set_on[64] = {false};  // the attribute is per device
   const int dev = device_info().device;
   bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
   if (!set) {
-    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(convh::kMaxSmem)),
+    if (!check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kHaloMaxSmem)),
                     "cudaFuncSetAttribute(conv)"))
       return;
     set = true;
@@ -632,63 +595,9 @@ void launch_halo(const CUtensorMap &tx, const CUtensorMap &tw, const convh::Para
   const int rounds = (p.num_tiles + sms - 1) / sms, grid = (p.num_tiles + rounds - 1) / rounds;
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convh::threads(kCopy)), smem, s, 1, tx, tw, p), "launch conv_halo_kernel");
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convh::threads(kCopy)), p.smem, s, 1, tx, tw, p), "launch conv_halo_kernel");
   }
   launched("conv_halo_kernel");
-}
-
-// The tensor core adds to its fp32 sum once per MMA, and rounds there.  With few channels an MMA holds padding and a sum takes
-// more of them than one over a dense patch, as the gather kernel builds it, would: 28 instead of 10 for 7 x 7 x 3, which
-// was 5.3e-7 off a sum in 64 bits where the dense one is 2.3e-7 (2-norm, relative).  So such a sum is made in as many
-// parts as it takes to have no more MMAs in each, added in the epilogue.  0: one sum (16 channels or more: no other kernel
-// is denser).
-int halo_chain(const ConvShape &c) { return c.IC < 16 ? static_cast<int>((c.IC * c.KH * c.KW + 15) / 16) : 0; }
-
-// Tile width, by the cycles of the busiest CTA; fills in what follows from the shape.  False where nothing fits.
-bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Params *best, size_t *smem) {
-  const int64_t ncb = (c.IC + 63) / 64, taps = c.KH * c.KW, pair_taps = c.KH * ((c.KW + 1) / 2);
-  const bool pairs = c.IC <= 8;
-  const int64_t num_kb = pairs ? (pair_taps + 3) / 4 : ncb * taps;
-  const int last_steps = static_cast<int>((c.IC - (ncb - 1) * 64 + 15) / 16), steps = ncb > 1 ? 4 : last_steps;
-  const int64_t mmas = pairs ? pair_taps : ((ncb - 1) * 4 + last_steps) * taps;
-  if (c.OC > convh::kMaxOC || (pairs ? pair_taps : taps) > convh::kMaxTaps || ncb * taps > (1 << 16) || c.OH * c.OW > INT32_MAX) return false;
-  convh::Params p;
-  p.ncb = static_cast<int>(ncb), p.last_steps = last_steps, p.pairs = pairs ? 1 : 0, p.num_kb = static_cast<int>(num_kb);
-  p.chain = halo_chain(c);
-  p.splits = p.chain ? static_cast<int>((mmas + p.chain - 1) / p.chain) : 1;
-  if (!halo_plan(c, flat, &p.h)) return false;
-  p.qb = (p.h.px + 31) / 32;
-  if (copy) {
-    p.boxes = flat ? (p.h.px + 255) / 256 : 1;
-    p.box_px = flat ? (p.h.px + p.boxes * 8 - 1) / (p.boxes * 8) * 8 : p.h.px;
-    if (!flat && (p.h.IW > 256 || p.h.px / p.h.IW > 256)) return false;
-    p.region_bytes = static_cast<uint32_t>((p.boxes * p.box_px * 128 + 1023) / 1024 * 1024);
-  } else {
-    p.boxes = p.box_px = 0;
-    p.region_bytes = static_cast<uint32_t>(p.h.plane_px * 32 * (pairs ? 1 : steps));
-  }
-  double best_cost = 1e300;
-  for (int bn = 256; bn >= 32; bn -= 32) {
-    if ((bn > 32 && bn >= c.OC + 32) || 2 * p.splits * bn > 512) continue;
-    size_t need;
-    if (!fit_halo(&p, copy, c.OC, num_kb, bn, sms, &need)) continue;
-    const int64_t tiles = p.h.m_tiles * ((c.OC + bn - 1) / bn);
-    if (tiles > (1 << 30)) continue;
-    const double rounds = static_cast<double>((tiles + sms - 1) / sms);
-    // Cycles of a tile's engines: MMAs; bytes out of L2 (regions of a copy, the filter where it does not stay) at 64 a
-    // cycle; lines through the load / store unit (pixels of one channel lie in rows of the region's width); stores;
-    // instructions of the input warps.
-    const double in_lines = flat ? 1.8 : 1.0 + 26.0 / p.h.IW, out_lines = flat ? 1.8 : 4.0;
-    const double mma = static_cast<double>(mmas) * (bn < 64 ? 46.0 : bn < 128 ? 54.0 : bn / 2.0);
-    const double l2 = (copy ? static_cast<double>(ncb) * p.region_bytes : 0.0) / 64.0 + (p.resident ? 0.0 : num_kb * bn * 2.0);
-    const double loads = copy ? 0.0 : p.qb * (pairs ? static_cast<double>(c.IC) : (ncb - 1) * 64.0 + last_steps * 16.0);
-    const double work = copy ? 0.0 : p.qb * ((ncb - 1) * 4.0 + last_steps) * 100.0 + p.qb * ncb * 60.0;
-    const double epi = bn * ((c.add ? 1024.0 : 512.0) / 24.0 + 4.0 * (p.splits - 1));
-    const double lsu = loads * in_lines + bn * 4.0 * out_lines * (c.add ? 2.0 : 1.0);
-    const double cost = rounds * (std::max({mma, l2, lsu, epi, work}) + 300.0) + epi + (copy ? l2 : 3.0 * loads);
-    if (cost < best_cost * 0.98) best_cost = cost, *best = p, *smem = need;
-  }
-  return best_cost < 1e300;
 }
 
 // What follows from a call's shape, kept for the next call of that shape (a plan, not a result; working it out takes
@@ -696,31 +605,26 @@ bool choose_halo(const ConvShape &c, bool copy, bool flat, int sms, convh::Param
 struct HaloChoice {
   int64_t shape[17];
   int sms = 0;
-  ConvForm form;  // kOther where conv_halo does not take the shape
+  ConvForm form;  // kOther: for the other kernels
   bool sampled;
   ConvShape c;  // after conv_sampled; its pointers are the call's that made the entry and are not used
   convh::Params p;
-  size_t smem;
 };
 const HaloChoice &halo_choice(const ConvShape &call, int sms) {
-  static thread_local HaloChoice cache[16];
+  static thread_local HaloChoice cache[64];
   const int64_t shape[17] = {call.N,  call.IC, call.H,   call.W,   call.OC, call.KH, call.KW, call.OH,          call.OW,
                              call.SH, call.SW, call.PHL, call.PWL, call.DH, call.DW, call.relu, call.add != nullptr};
   uint64_t key = 0;
   for (int64_t v : shape) key = (key ^ static_cast<uint64_t>(v)) * 0x9E3779B97F4A7C15ull;
-  HaloChoice &e = cache[key >> 60];
+  HaloChoice &e = cache[key >> 58];
   if (e.sms == sms && std::equal(shape, shape + 17, e.shape)) return e;
   std::copy(shape, shape + 17, e.shape);
   e.sms = sms, e.c = call, e.sampled = conv_sampled(e.c);
-  e.form = conv_form(e.c, sms);
-  const bool copy = e.form == ConvForm::kCopyRect || e.form == ConvForm::kCopyFlat;
-  if (e.form != ConvForm::kOther &&
-      ((!copy && e.sampled) ||  // (conv_form keeps 1 x 1 windows of 16 channels or more to copies)
-       !choose_halo(e.c, copy, e.form == ConvForm::kCopyFlat || e.form == ConvForm::kDirectFlat, sms, &e.p, &e.smem)))
-    e.form = ConvForm::kOther;
+  e.form = conv_form(e.c, sms, conv_persistent_takes(call), &e.p);
   if (e.form == ConvForm::kOther) return e;
   const ConvShape &c = e.c;
   convh::Params &p = e.p;
+  const bool copy = form_copies(e.form);
   p.N = int(c.N), p.IC = int(c.IC), p.H = int(c.H), p.W = int(c.W), p.OC = int(c.OC), p.KH = int(c.KH), p.KW = int(c.KW);
   p.OH = int(c.OH), p.OW = int(c.OW), p.PHL = int(c.PHL), p.PWL = int(c.PWL), p.SH = int(c.SH), p.SW = int(c.SW);
   p.DH = int(c.DH), p.DW = int(c.DW), p.relu = c.relu ? 1 : 0;
@@ -756,15 +660,9 @@ const HaloChoice &halo_choice(const ConvShape &call, int sms) {
 bool conv_halo(const ConvShape &call, cudaStream_t s) {
   using namespace convh;
   const DeviceInfo &di = device_info();
-  {
-    // most small calls are not for this kernel: no look at the table for them
-    ConvShape sampled = call;
-    conv_sampled(sampled);
-    if (conv_form(sampled, di.sms) == ConvForm::kOther) return false;
-  }
   const HaloChoice &e = halo_choice(call, di.sms);
   if (e.form == ConvForm::kOther) return false;
-  const bool copy = e.form == ConvForm::kCopyRect || e.form == ConvForm::kCopyFlat;
+  const bool copy = form_copies(e.form);
   // An output that overlaps the input: a launch that copies the input has read it before the first store.
   const uintptr_t x0 = reinterpret_cast<uintptr_t>(call.x), o0 = reinterpret_cast<uintptr_t>(call.out);
   if (!copy && call.IC >= 16 && o0 < x0 + static_cast<uintptr_t>(call.N * call.IC * call.H * call.W) * 4 &&
@@ -811,7 +709,7 @@ bool conv_halo(const ConvShape &call, cudaStream_t s) {
   }
   if (ok) {
     auto launch = copy ? (p.add ? launch_halo<true, true> : launch_halo<true, false>) : (p.add ? launch_halo<false, true> : launch_halo<false, false>);
-    launch(tx, tw, p, e.smem, di.sms, s);
+    launch(tx, tw, p, di.sms, s);
   }
   mgpuMemFreeAsync(ws, s);
   return ok;

@@ -486,29 +486,6 @@ EncodeIm2col encode_im2col() {
   return fn;
 }
 
-// Tile width, by the cycles of the busiest CTA: rounds x the slowest of a tile's three engines.
-// Loads: about 64 bytes per cycle and SM out of L2 (a gathered k-block about 400 cycles with three
-// groups at work); MMAs: 2 cycles per column and k-block, at least what reading A takes; epilogue:
-// about 24 bytes per cycle and SM of HBM.  E.g. 6272 pixels x 256 channels: 147 tiles of 96 columns
-// in one round (224 units of load) beat 98 of 128 in one (256) and 49 of 256 (384).
-int choose_conv_bn(int64_t m_tiles, int64_t OC, int num_kb, bool gather, bool add, int sms) {
-  int best = 32;
-  double best_cost = 1e300;
-  for (int bn = 256; bn >= 32; bn -= 32) {
-    if (bn > 32 && bn >= OC + 32) continue;
-    const int64_t n_tiles = (OC + bn - 1) / bn;
-    const int64_t rounds = (m_tiles * n_tiles + sms - 1) / sms;
-    const double load = num_kb * ((gather ? 400.0 : 256.0) + bn * 2.0);
-    const double mma = num_kb * (bn < 64 ? 160.0 : bn < 96 ? 192.0 : 2.0 * bn);
-    const double epi = bn * (add ? 1024.0 : 512.0) / 24.0;
-    double tile = load > mma ? load : mma;
-    if (epi > tile) tile = epi;
-    const double cost = static_cast<double>(rounds) * tile + epi;
-    if (cost < best_cost * 0.97) best_cost = cost, best = bn;
-  }
-  return best;
-}
-
 template <bool kGather, bool kAdd>
 void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp::Params &p, size_t smem, int sms,
                        cudaStream_t s) {
@@ -532,9 +509,6 @@ void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp
   launched("conv_persistent_kernel");
 }
 }  // namespace
-
-// 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks.
-static bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
 
 // A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels only, and
 // the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56, stride 2: 108 us
@@ -614,9 +588,8 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   p.by_p = Divisor(p.P), p.by_ow = Divisor(p.OW), p.by_ntiles = Divisor(p.n_tiles);
   p.tmem_cols = 32;
   while (p.tmem_cols < 2u * p.bn) p.tmem_cols *= 2;
-  // the filter stays when it is one tile wide, there is a second tile to use it, and it leaves the ring room
   const int64_t filter_bytes = num_kb * p.bn * BK * 2;
-  p.resident = p.n_tiles == 1 && p.num_tiles > di.sms && filter_bytes <= 100 * 1024;
+  p.resident = conv_filter_stays(num_kb, p.bn, p.n_tiles, p.num_tiles, di.sms);
   const int64_t stage_bytes = A_BYTES + (p.resident ? 0 : p.bn * BK * 2);
   const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128 + (gather ? num_kb * BK * 8 : 0);
   int64_t stages = (static_cast<int64_t>(kMaxSmem) - 4096 - fixed) / stage_bytes;

@@ -2,6 +2,8 @@
 // (conv_persistent_tcgen05.cu) share.
 #pragma once
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -77,40 +79,232 @@ bool conv_sampled(ConvShape &c);
 bool conv_prepare(const ConvShape &c, const ConvShape &call, bool sampled, int64_t copy_h, int64_t copy_w, void *x16, void *w16,
                   cudaStream_t s);
 
-// Where conv_halo_kernel takes a call, and in which form; `c` after conv_sampled.  The other kernels are the im2col
-// kernel (16 channels or more) and the gather kernel.  us a call, inputs changing, theirs / the form's:
-//   copy, windows of 25 taps and more   26x192x60x37->32 5x5 73 / 57, 16x32x113x91->32 7x7 105 / 66, 3x352x54x33->165 7x7
-//                                       79 / 64: a k-block costs the im2col kernel at least 340 cycles, these 46 to 64 an MMA
-//   copy, 1 x 1                         32x64x56x56->256 73 / 58, 45x192x47x35->32 26 / 21, 2x32x179x207->131 38 / 24
-//   copy, up to 64 outputs              16x16x112x112->16 31 / 16, 32x64x56x56->64 with residual 26.9 / 25.1
-//   copy, few tiles and many channels   17x448x13x9->113 18.2 / 16.4, 1x160x9x7->96 10.3 / 9.2, 32x512x7x7->512 25.0 / 23.1
-// A call of one round of tiles and up to ten k-blocks is bound by its launches, and this kernel's parameters are the longer
-// ones: 2x32x20x20->32 7.9 / 8.0, 9x96x21x30->32 1x1 stride 2 7.9 / 8.1.
-// Elsewhere the im2col kernel's stores win, whose 32 pixels of a warp are neighbours in memory: 32x128x28x28->128 19.2 / 20.4,
-// 25x224x38x43->192 49.8 / 54.2, 34x32x23x21->352 22.2 / 23.8.  Rect keeps to whole sectors where rows of the output are
-// multiples of eight pixels (32x64x56x56->64 19.2, flat 25.2); flat wastes less elsewhere (32x256x14x14->256 17.4, rect 20.7).
-//   direct, up to 15 channels           16x3x224x224->32 7x7 143 / 79, 16x3x128x128->64 5x5 43 / 33, 4x12x100x100->64 5x5 29 / 11.5;
-//                                       but 16x3x256x256->64 3x3 64 / 69, 30x3x250x256->32 3x3 stride 2 44 / 57, and windows
-//                                       that reach far: 18x3x18x29->96 7x7 dilation 2 12.3 / 12.8
-//   direct, stride 2, up to 32 channels 42x32x97x102->32 5x5 54 / 46, 2x32x22x23->32 7x7 15.5 / 13.5; but 1x32x165x248->192 28 / 31
-enum class ConvForm { kOther, kCopyRect, kCopyFlat, kDirectRect, kDirectFlat };
-inline ConvForm conv_form(const ConvShape &c, int sms) {
-  const int64_t taps = c.KH * c.KW, pixels = c.N * c.OH * c.OW;
-  const bool unit = c.SH == 1 && c.SW == 1;
-  HaloPlan h;
-  auto direct = [&]() {
-    if (c.SH > 2 || c.SW > 2) return ConvForm::kOther;
-    return unit && c.OW < 48 && halo_plan(c, true, &h) ? ConvForm::kDirectFlat : ConvForm::kDirectRect;
-  };
-  if (c.IC < 16) return taps >= 25 && (c.KH - 1) * c.DH <= 8 && (c.KW - 1) * c.DW <= 8 ? direct() : ConvForm::kOther;
-  if (!unit) return c.IC <= 32 && taps >= 25 && (c.OC <= 64 || pixels < 5000) ? direct() : ConvForm::kOther;
-  const bool few = (pixels + 127) / 128 * ((c.OC + 63) / 64) <= sms;
-  if (few && (c.IC + 63) / 64 * taps <= 10) return ConvForm::kOther;
-  if (taps > 1 && c.OC > 64 && c.IC < 384 && !(taps >= 25 && (c.OC <= 128 || c.IC >= 64)) && !(few && c.IC >= 64)) return ConvForm::kOther;
-  if (taps > 1 && c.OW % 8 == 0) return ConvForm::kCopyRect;
-  return halo_plan(c, true, &h) && h.px <= 512 ? ConvForm::kCopyFlat : ConvForm::kCopyRect;
+// The persistent kernels' tile: width, by the cycles of the busiest CTA: rounds x the slowest of a tile's three engines.
+// Loads: about 64 bytes per cycle and SM out of L2 (a gathered k-block about 400 cycles with three
+// groups at work); MMAs: 2 cycles per column and k-block, at least what reading A takes; epilogue:
+// about 24 bytes per cycle and SM of HBM.  E.g. 6272 pixels x 256 channels: 147 tiles of 96 columns
+// in one round (224 units of load) beat 98 of 128 in one (256) and 49 of 256 (384).
+inline int choose_conv_bn(int64_t m_tiles, int64_t OC, int64_t num_kb, bool gather, bool add, int sms) {
+  int best = 32;
+  double best_cost = 1e300;
+  for (int bn = 256; bn >= 32; bn -= 32) {
+    if (bn > 32 && bn >= OC + 32) continue;
+    const int64_t n_tiles = (OC + bn - 1) / bn;
+    const int64_t rounds = (m_tiles * n_tiles + sms - 1) / sms;
+    const double load = num_kb * ((gather ? 400.0 : 256.0) + bn * 2.0);
+    const double mma = num_kb * (bn < 64 ? 160.0 : bn < 96 ? 192.0 : 2.0 * bn);
+    const double epi = bn * (add ? 1024.0 : 512.0) / 24.0;
+    double tile = load > mma ? load : mma;
+    if (epi > tile) tile = epi;
+    const double cost = static_cast<double>(rounds) * tile + epi;
+    if (cost < best_cost * 0.97) best_cost = cost, best = bn;
+  }
+  return best;
+}
+// 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks.
+inline bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
+// The filter stays in shared memory when it is one tile wide, there is a second tile to use it, and it leaves the ring room.
+inline bool conv_filter_stays(int64_t num_kb, int bn, int64_t n_tiles, int64_t tiles, int sms) {
+  return n_tiles == 1 && tiles > sms && num_kb * bn * 128 <= 100 * 1024;
 }
 
+// How conv_halo_kernel runs a call: in a copy of the input or directly (see there), by rect or flat tiles.
+enum class ConvForm { kOther, kCopyRect, kCopyFlat, kDirectRect, kDirectFlat };
+inline bool form_copies(ConvForm f) { return f == ConvForm::kCopyRect || f == ConvForm::kCopyFlat; }
+inline bool form_flat(ConvForm f) { return f == ConvForm::kCopyFlat || f == ConvForm::kDirectFlat; }
+
+constexpr int kHaloMaxOC = 2048;           // bias kept in shared memory
+constexpr int kHaloMaxTaps = 64;           // entries of its table of taps, or pairs of them
+constexpr int kHaloFilterStages = 12;
+constexpr int kHaloInputWarps = 12;        // of the direct forms
+constexpr size_t kHaloMaxSmem = 220 * 1024;
+
+// A tile of conv_halo_kernel and what follows from it.
+struct HaloTile {
+  HaloPlan h;
+  int ncb, last_steps;        // blocks of 64 channels; sixteens of the last one's channels
+  int pairs;                  // up to eight channels: MMAs of two taps
+  int num_kb;                 // filter blocks of 64 k
+  int mmas;                   // of a tile
+  int chain, splits;          // few channels: MMAs per sum, and sums (see halo_chain)
+  int qb;                     // 32-pixel pieces of a region
+  int boxes, box_px;          // loads that make up a copy's region, and the pixels of one
+  int bn, resident, stages, filter_stages, filter_kbs;
+  uint32_t region_bytes, regions_bytes;  // of a stage / of all
+  size_t smem;
+};
+
+// Shared memory: regions, then the filter whole or a ring of its k-blocks, several to a stage where they are short (a
+// hand-over costs as much as the MMAs of 64 columns).  False where it does not fit.
+inline bool fit_halo(HaloTile *t, bool copy, int64_t OC, int bn, int sms) {
+  const int64_t fixed = 2048 + (OC + 31) / 32 * 128, room = static_cast<int64_t>(kHaloMaxSmem) - fixed;
+  const int64_t num_kb = t->num_kb, b_bytes = bn * 128, filter = num_kb * b_bytes, region = t->region_bytes;
+  const int64_t most = region <= 16 * 1024 ? 8 : 4;
+  const int64_t tiles = t->h.m_tiles * ((OC + bn - 1) / bn);
+  const bool resident = OC <= bn && tiles > sms && filter + 2 * region <= room;
+  int64_t kbs = 32 * 1024 / b_bytes;
+  if (kbs > 4) kbs = 4;
+  if (kbs > num_kb) kbs = num_kb;
+  const int64_t blocks = (num_kb + kbs - 1) / kbs, least = blocks < 3 ? blocks : 3;
+  int64_t n = (room - (resident ? filter : least * kbs * b_bytes)) / region;
+  if (n > most) n = most;
+  // as many stages as regions that the input warps' pieces reach over: a stage's barrier is then never two uses behind
+  const int64_t reach = copy ? 0 : (kHaloInputWarps + t->qb - 1) / t->qb;
+  if (n < 2 || n < reach) return false;
+  int64_t fs = (room - n * region) / (kbs * b_bytes);
+  if (fs > kHaloFilterStages) fs = kHaloFilterStages;
+  t->bn = bn, t->resident = resident ? 1 : 0, t->stages = static_cast<int>(n);
+  t->filter_stages = resident ? 0 : static_cast<int>(fs), t->filter_kbs = static_cast<int>(kbs);
+  t->regions_bytes = static_cast<uint32_t>((n * region + 1023) / 1024 * 1024);
+  t->smem = static_cast<size_t>(1024 + t->regions_bytes + (resident ? filter : fs * kbs * b_bytes) + (OC + 31) / 32 * 128);
+  return true;
+}
+
+// The tensor core adds to its fp32 sum once per MMA, and rounds there.  With few channels an MMA holds padding and a sum takes
+// more of them than one over a dense patch, as the gather kernel builds it, would: 28 instead of 10 for 7 x 7 x 3, which
+// was 5.3e-7 off a sum in 64 bits where the dense one is 2.3e-7 (2-norm, relative).  So such a sum is made in as many
+// parts as it takes to have no more MMAs in each, added in the epilogue.  0: one sum (16 channels or more: no other kernel
+// is denser).
+inline int halo_chain(const ConvShape &c) { return c.IC < 16 ? static_cast<int>((c.IC * c.KH * c.KW + 15) / 16) : 0; }
+
+// The tile of a form, its width by the cycles of the busiest CTA.  False where the form does not take the shape.
+inline bool halo_tile(const ConvShape &c, ConvForm form, int sms, HaloTile *best) {
+  const bool copy = form_copies(form), flat = form_flat(form);
+  const int64_t ncb = (c.IC + 63) / 64, taps = c.KH * c.KW, pair_taps = c.KH * ((c.KW + 1) / 2);
+  const bool pairs = c.IC <= 8;
+  const int64_t num_kb = pairs ? (pair_taps + 3) / 4 : ncb * taps;
+  const int last_steps = static_cast<int>((c.IC - (ncb - 1) * 64 + 15) / 16), steps = ncb > 1 ? 4 : last_steps;
+  const int64_t mmas = pairs ? pair_taps : ((ncb - 1) * 4 + last_steps) * taps;
+  if (c.OC > kHaloMaxOC || (pairs ? pair_taps : taps) > kHaloMaxTaps || ncb * taps > (1 << 16) || c.OH * c.OW > INT32_MAX) return false;
+  HaloTile t;
+  t.ncb = static_cast<int>(ncb), t.last_steps = last_steps, t.pairs = pairs ? 1 : 0, t.num_kb = static_cast<int>(num_kb);
+  t.mmas = static_cast<int>(mmas), t.chain = halo_chain(c);
+  t.splits = t.chain ? static_cast<int>((mmas + t.chain - 1) / t.chain) : 1;
+  if (!halo_plan(c, flat, &t.h)) return false;
+  t.qb = (t.h.px + 31) / 32;
+  if (copy) {
+    t.boxes = flat ? (t.h.px + 255) / 256 : 1;
+    t.box_px = flat ? (t.h.px + t.boxes * 8 - 1) / (t.boxes * 8) * 8 : t.h.px;
+    if (!flat && (t.h.IW > 256 || t.h.px / t.h.IW > 256)) return false;
+    t.region_bytes = static_cast<uint32_t>((t.boxes * t.box_px * 128 + 1023) / 1024 * 1024);
+  } else {
+    t.boxes = t.box_px = 0;
+    t.region_bytes = static_cast<uint32_t>(t.h.plane_px * 32 * (pairs ? 1 : steps));
+  }
+  double best_cost = 1e300;
+  for (int bn = 256; bn >= 32; bn -= 32) {
+    if ((bn > 32 && bn >= c.OC + 32) || 2 * t.splits * bn > 512) continue;
+    if (!fit_halo(&t, copy, c.OC, bn, sms)) continue;
+    const int64_t tiles = t.h.m_tiles * ((c.OC + bn - 1) / bn);
+    if (tiles > (1 << 30)) continue;
+    const double rounds = static_cast<double>((tiles + sms - 1) / sms);
+    // Cycles of a tile's engines: MMAs; bytes out of L2 (regions of a copy, the filter where it does not stay) at 64 a
+    // cycle; lines through the load / store unit (pixels of one channel lie in rows of the region's width); stores;
+    // instructions of the input warps.
+    const double in_lines = flat ? 1.8 : 1.0 + 26.0 / t.h.IW, out_lines = flat ? 1.8 : 4.0;
+    const double mma = static_cast<double>(mmas) * (bn < 64 ? 46.0 : bn < 128 ? 54.0 : bn / 2.0);
+    const double l2 = (copy ? static_cast<double>(ncb) * t.region_bytes : 0.0) / 64.0 + (t.resident ? 0.0 : num_kb * bn * 2.0);
+    const double loads = copy ? 0.0 : t.qb * (pairs ? static_cast<double>(c.IC) : (ncb - 1) * 64.0 + last_steps * 16.0);
+    const double work = copy ? 0.0 : t.qb * ((ncb - 1) * 4.0 + last_steps) * 100.0 + t.qb * ncb * 60.0;
+    const double epi = bn * ((c.add ? 1024.0 : 512.0) / 24.0 + 4.0 * (t.splits - 1));
+    const double lsu = loads * in_lines + bn * 4.0 * out_lines * (c.add ? 2.0 : 1.0);
+    const double cost = rounds * (std::max({mma, l2, lsu, epi, work}) + 300.0) + epi + (copy ? l2 : 3.0 * loads);
+    if (cost < best_cost * 0.98) best_cost = cost, *best = t;
+  }
+  return best_cost < 1e300;
+}
+
+// What a call takes on the persistent kernels, and on conv_halo_kernel, in us: estimates to choose by.  Their constants were
+// fitted to 2500 shapes timed on all of these kernels (16 to 1024 channels under 1 x 1 to 7 x 7 windows, 1 to 32 channels
+// under 25 to 81 taps; strides 1 and 2, dilations, maps of one row or column and square ones, 1 to 65536 tiles): absolute
+// times are met within 10 % for half of them, and what is chosen is rarely the slower one (conv_form).  A CTA's tiles pass
+// one after another, each as slow as the slowest of its engines; or all CTAs wait for memory.  Cycles at 1.85 GHz; no call
+// is over before its two launches.
+constexpr double kConvLaunches = 7.9;
+inline double conv_us(double bytes_rewritten, double cycles) {
+  return std::max(kConvLaunches, 4.5 + bytes_rewritten / 8.0e6 + cycles / 1850.0);
+}
+inline double dense_us(const ConvShape &c, int sms) {
+  const double out = 4.0 * c.N * c.OC * c.OH * c.OW * (c.add ? 2 : 1);
+  const int64_t taps = c.KH * c.KW, ncb = (c.IC + 63) / 64, m_tiles = (c.N * c.OH * c.OW + 127) / 128, Cp8 = (c.IC + 7) / 8;
+  const bool gather = conv_gathers(c);
+  const int64_t num_kb = gather ? (c.IC * taps + 63) / 64 : ncb * taps;
+  const int bn = choose_conv_bn(m_tiles, c.OC, num_kb, gather, c.add != nullptr, sms);
+  const int64_t n_tiles = (c.OC + bn - 1) / bn, tiles = m_tiles * n_tiles;
+  const double rounds = static_cast<double>((tiles + sms - 1) / sms);
+  if (gather) return conv_us(0.0, rounds * num_kb * 2600.0 + 4000.0);  // instructions of the gather
+  // an im2col k-block: the hand-over of its stage, or 70 bytes a cycle; rows of the copy that end inside a sector are read
+  // at half that rate
+  const double kb = std::max(400.0, (16384.0 + (conv_filter_stays(num_kb, bn, n_tiles, tiles, sms) ? 0 : bn * 128)) / 70.0);
+  const double loads = kb * (num_kb + (Cp8 % 2 ? 0.8 * taps : 0.0)), epi = bn * (c.add ? 1024.0 : 512.0) / 35.0;
+  const double rewritten = 6.0 * (static_cast<double>(c.N) * c.IC * c.H * c.W + static_cast<double>(c.OC) * c.IC * taps);
+  const double memory = out / 3000.0 + 2.0 * c.N * c.H * c.W * Cp8 * 8 / 1150.0;
+  return conv_us(rewritten, std::max(rounds * (1450.0 + std::max(loads, epi)), memory) + epi);
+}
+inline double halo_us(const ConvShape &c, ConvForm form, const HaloTile &t, int sms) {
+  const bool copy = form_copies(form), flat = form_flat(form);
+  const int64_t tiles = t.h.m_tiles * ((c.OC + t.bn - 1) / t.bn);
+  const double rounds = static_cast<double>((tiles + sms - 1) / sms);
+  const double blocks = t.resident ? 0 : (t.num_kb + t.filter_kbs - 1) / t.filter_kbs;  // stages of the filter
+  // rows of eight pixels that do not start on a sector are stored in parts of two
+  const double parts = flat || c.OW % 8 == 0 ? 1.0 : 1.5;
+  double mma = t.mmas * (t.bn < 64 ? 42.0 : std::max(58.0, t.bn / 2.0));
+  if (!copy) {
+    mma += blocks * 490.0;
+    const double in = t.qb * t.last_steps * 120.0, epi = t.bn * (512.0 * parts * (c.add ? 3.5 : 1.0) / 30.0 + 6.0 * (t.splits - 1));
+    return conv_us(0.0, rounds * (1800.0 + std::max({mma, in, epi})) + epi + in);
+  }
+  mma += blocks * 330.0 + t.ncb * 960.0;
+  const double l2 = (static_cast<double>(t.ncb) * t.region_bytes + (t.resident ? 0.0 : t.num_kb * t.bn * 128.0)) / 43.0;
+  const double stored = parts * (c.add ? (flat ? 1.5 : 2.0) : 1.0), epi = t.bn * 512.0 * stored / (flat ? 19.0 : 39.0);
+  const double rewritten = 6.0 * (static_cast<double>(c.N) * c.IC * c.H * c.W + static_cast<double>(c.OC) * c.IC * c.KH * c.KW);
+  const double memory = 4.0 * c.N * c.OC * c.OH * c.OW * stored / 2000.0;
+  return conv_us(rewritten, std::max(rounds * (530.0 + std::max({mma, l2, epi})), memory) + epi + t.region_bytes / 43.0);
+}
+
+// Where conv_halo_kernel takes a call, in which form and with which tile; `c` after conv_sampled.  dense: whether the
+// persistent kernels take it too (im2col with 16 channels or more, gather below).  The quicker one by the estimates above: a
+// region's tiles hold the margins between images too, and rect ones whatever 16 rows x 8 pixels leave empty.
+// us a call, inputs changing, theirs / rect / flat:
+//   a k-block costs im2col 400 cycles or more, a region's MMAs 42 to 58 each below 128 columns:
+//     32x64x56x56->64 3x3 24 / 19 / 26, 16x16x77x77->16 20 / 12 / 12, 33x32x55x55->32 5x5 46 / 20 / 22, 33x192x55x55->32 5x5 113 / 90 / 94
+//   a block of 64 channels costs a region 960 beside them and 43 bytes a cycle, so wide tiles and many blocks go dense:
+//     32x128x28x28->128 3x3 19.1 / 20.0 / 20.7, 32x512x14x14->512 35 / 48 / 46, 8x384x56x56->384 67 / 87 / 101, 32x512x28x28->512 108 / 141 / 137
+//   rows of eight pixels off the sectors: 14x64x85x93->448 5x1 67 / 201 / 70, 25x64x52x87->256 1x3 44 / 108 / 51
+//   empty tiles: 1x64x1x65536->64 1x3 15 / 56 / 17, 1x64x4x8192->64 3x3 13 / 19, 206x32x2x112->64 5x5 dilation 3 24 / 69
+//   1 x 1: 32x64x56x56->256 40 / 34 / 30, 117x128x43x60->32 with residual 91 / 65 / 60, but 10x96x220x8->142 12 / 15 / 15
+//   few channels, gather / rect / flat: 16x3x224x224->32 7x7 143 / 78, 16x3x18x256->64 7x7 26 / 17 / 31, 1x16x1x160000->32 1x9 27 / 94 / 15,
+//     but 256x1x28x28->32 5x5 19 / 25 / 25, 21x3x29x37->352 5x5 21 / 24 / 24, 1x3x4x40000->32 5x5 28 / 46
+//   stride 2, 16 to 32 channels, im2col / rect: 16x24x150x153->32 5x5 78 / 30, 4x32x200x203->32 5x5 27 / 19, but 4x16x120x123->256 7x7 24 / 32
+// Below 25 taps few channels and strides stay where they are: nearly all that was measured there is slower (16x3x256x256->64
+// 3x3 64 / 93).
+// Over 1648 shapes with copies the choice takes 0.901 of the dense kernels' time (geometric mean; always the best one, 0.890)
+// and 40 are more than 4 % slower; over 871 others 0.814 (0.804) and 39.  Over 1050 that the estimates were not fitted to,
+// 0.910 (0.893), 14 of 700, and 0.804 (0.790), 16 of 350.
+inline ConvForm conv_form(const ConvShape &c, int sms, bool dense = true, HaloTile *tile = nullptr) {
+  const bool unit = c.SH == 1 && c.SW == 1, direct = c.IC < 16 || (!unit && c.IC <= 32);
+  ConvForm best = ConvForm::kOther;
+  if (direct ? c.KH * c.KW < 25 : !unit) return best;
+  double us = dense ? dense_us(c, sms) : 1e300;
+  auto consider = [&](ConvForm form) {
+    HaloTile t;
+    if (!halo_tile(c, form, sms, &t)) return;
+    // the remaining kernel (conv_tcgen05.cu) is slower than either, by how much was not measured: not on mostly empty tiles
+    if (!dense && t.h.m_tiles > 2 * ((c.N * c.OH * c.OW + 127) / 128)) return;
+    const double e = halo_us(c, form, t, sms);
+    if (e >= us) return;
+    us = e, best = form;
+    if (tile) *tile = t;
+  };
+  if (c.KH * c.KW > 1) consider(direct ? ConvForm::kDirectRect : ConvForm::kCopyRect);  // (1 x 1 has no margins to read)
+  // Where rect wastes little: a copy whose rows are whole sectors is stored as such, which flat tiles do not; a flat region
+  // of long rows is read for pixels that most of its tile has no use for.
+  HaloPlan rect, flat;
+  const bool keep = c.KH * c.KW > 1 && (direct ? c.KH > 1 && c.OW >= 48 : c.OW % 8 == 0) && halo_plan(c, false, &rect) && halo_plan(c, true, &flat) &&
+                    rect.m_tiles * 5 <= flat.m_tiles * 6;
+  if (unit && !keep) consider(direct ? ConvForm::kDirectFlat : ConvForm::kCopyFlat);
+  return best;
+}
 // Runs the convolution on conv_halo_kernel; false (and nothing launched) when the shape is not one for it.
 bool conv_halo(const ConvShape &c, cudaStream_t s);
 

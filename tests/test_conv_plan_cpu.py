@@ -77,19 +77,43 @@ int main() {
   assert(rects > 50 && flats > 50 && strided > 100);
   // where the kernel takes a call
   ConvShape c = {};
-  auto form = [&](int N, int IC, int H, int W, int OC, int K, int S) {
-    c.N = N, c.IC = IC, c.H = H, c.W = W, c.OC = OC, c.KH = c.KW = K, c.SH = c.SW = S, c.DH = c.DW = 1, c.PHL = c.PWL = K / 2;
-    c.OH = (H + K / 2 * 2 - K) / S + 1, c.OW = (W + K / 2 * 2 - K) / S + 1;
-    return conv_form(c, 148);
+  auto form = [&](int N, int IC, int H, int W, int OC, int K, int S, int KH = 0, int D = 1, bool dense = true) {
+    if (!KH) KH = K;
+    c.N = N, c.IC = IC, c.H = H, c.W = W, c.OC = OC, c.KH = KH, c.KW = K, c.SH = c.SW = S, c.DH = c.DW = D;
+    c.PHL = KH / 2 * D, c.PWL = K / 2 * D;
+    c.OH = (H + 2 * c.PHL - (KH - 1) * D - 1) / S + 1, c.OW = (W + 2 * c.PWL - (K - 1) * D - 1) / S + 1;
+    return conv_form(c, 148, dense);
   };
   assert(form(16, 3, 256, 256, 64, 3, 1) == ConvForm::kOther && form(16, 3, 224, 224, 32, 7, 1) == ConvForm::kDirectRect);
-  assert(form(21, 3, 29, 37, 352, 5, 1) == ConvForm::kDirectFlat && form(8, 15, 20, 20, 8, 5, 3) == ConvForm::kOther);
-  assert(form(8, 3, 29, 37, 32, 9, 1) == ConvForm::kDirectFlat && form(8, 3, 29, 37, 32, 11, 1) == ConvForm::kOther);
+  assert(form(21, 3, 29, 37, 352, 5, 1) == ConvForm::kOther && form(8, 15, 20, 20, 8, 5, 3) == ConvForm::kOther);
+  assert(form(8, 3, 29, 37, 32, 9, 1) == ConvForm::kDirectRect && form(8, 3, 29, 37, 32, 11, 1) == ConvForm::kOther);
   assert(form(32, 64, 56, 56, 64, 3, 1) == ConvForm::kCopyRect && form(32, 64, 57, 57, 64, 3, 1) == ConvForm::kCopyFlat);
-  assert(form(32, 128, 28, 28, 128, 3, 1) == ConvForm::kOther && form(32, 512, 7, 7, 512, 3, 1) == ConvForm::kCopyFlat);
-  assert(form(32, 64, 56, 56, 256, 1, 1) == ConvForm::kCopyFlat && form(1, 160, 9, 7, 96, 3, 1) == ConvForm::kCopyFlat);
-  assert(form(2, 64, 20, 20, 32, 3, 1) == ConvForm::kOther && form(2, 65, 20, 20, 32, 3, 1) == ConvForm::kCopyFlat);
+  assert(form(32, 128, 28, 28, 128, 3, 1) == ConvForm::kOther && form(32, 512, 14, 14, 512, 3, 1) == ConvForm::kOther);
+  assert(form(32, 64, 56, 56, 256, 1, 1) == ConvForm::kCopyFlat && form(1, 160, 9, 7, 96, 3, 1) == ConvForm::kCopyRect);
+  assert(form(2, 64, 20, 20, 32, 3, 1) == ConvForm::kOther && form(2, 65, 20, 20, 32, 3, 1) != ConvForm::kOther);
   assert(form(2, 32, 22, 23, 32, 7, 2) == ConvForm::kDirectRect && form(2, 64, 22, 23, 32, 7, 2) == ConvForm::kOther);
+  // mostly empty tiles (one or a few rows of many pixels; rect 2 to 16 times the dense tiles), and many channels on large
+  // maps: the dense kernels take 0.2 to 0.8 of the region kernel's time on these
+  for (int w : {65536, 65535, 49152}) assert(form(1, 64, 1, w, 64, 3, 1, 1) != ConvForm::kCopyRect);
+  assert(form(1, 16, 1, 160000, 32, 9, 1, 1) == ConvForm::kCopyFlat && form(4, 64, 1, 16384, 64, 3, 1, 1) == ConvForm::kOther);
+  assert(form(1, 64, 4, 8192, 64, 3, 1) == ConvForm::kOther && form(1, 64, 17, 2048, 64, 3, 1) == ConvForm::kOther);
+  assert(form(1, 3, 4, 40000, 32, 5, 1) == ConvForm::kOther && form(206, 32, 2, 112, 64, 5, 1, 5, 3) == ConvForm::kOther);
+  assert(form(32, 512, 28, 28, 512, 3, 1) == ConvForm::kOther && form(8, 384, 56, 56, 128, 3, 1) == ConvForm::kOther);
+  assert(form(14, 64, 85, 93, 448, 1, 1, 5) != ConvForm::kCopyRect && form(4, 16, 120, 123, 256, 7, 2) == ConvForm::kOther);
+  // a dilation that the im2col map cannot describe goes to a region, unless most of its tiles were empty
+  assert(form(1, 64, 1, 20000, 64, 9, 1, 1, 32, false) == ConvForm::kCopyFlat);
+  assert(form(64, 64, 1, 64, 64, 9, 1, 1, 32, false) == ConvForm::kOther);
+  // a tile and its memory belong to the form, and keep to the kernel's limits
+  for (int i = 0; i < 4000; ++i) {
+    const int K = pick(0, 2) ? pick(1, 9) : 1, S = pick(1, 2), size = pick(1, 3) * pick(1, 90) + K;
+    if (form(pick(1, 9), i % 2 ? pick(1, 40) : pick(1, 700), size, pick(1, 300) + K, pick(1, 2100), K, S) == ConvForm::kOther) continue;
+    HaloTile t;
+    const ConvForm f = conv_form(c, 148, true, &t);
+    assert(form_flat(f) == (t.h.flat != 0) && (form_copies(f) ? c.IC >= 16 && S == 1 : c.IC <= 32));
+    assert(t.smem <= kHaloMaxSmem && t.stages >= 2 && t.bn % 32 == 0 && t.bn <= 256 && 2 * t.splits * t.bn <= 512);
+    assert(t.resident ? c.OC <= t.bn : t.filter_stages >= 1 && t.filter_stages <= kHaloFilterStages);
+    assert(form_copies(f) || t.stages * t.qb >= kHaloInputWarps);
+  }
   printf("ok\n");
 }
 """
