@@ -107,6 +107,12 @@ void *mgpuTensorMapEncodeTiledMemref(int64_t tensorRank, void *descriptor, int t
 
 /* ---- additions (no counterpart in the reference) ---- */
 
+/* mgpuTensorMapEncodeTiled with a verdict of its own: returns the driver's status (0: encoded) and does not record it, for
+ * callers that have another way, or that must not take an earlier or another thread's status for this call's. */
+int32_t mgpuTensorMapTryEncodeTiled(void *tensorMap, int tensorDataType, uint32_t tensorRank, void *globalAddress,
+                                    const uint64_t *globalDim, const uint64_t *globalStrides, const uint32_t *boxDim,
+                                    const uint32_t *elementStrides, int interleave, int swizzle, int l2Promotion, int oobFill);
+
 /* Sticky status: 0 when no wrapper has failed since the last clear, otherwise the CUDA
  * error code of the first failure.  The reference only prints (CudaRuntimeWrappers.cpp:3-12). */
 int32_t mgpuGetLastError(void);

@@ -74,6 +74,7 @@ RUNTIME_SIGNATURES = {
     "mgpuMemHostUnregisterMemRef": (None, [_i64, _vp, _i64]),
     "mgpuSetDefaultDevice": (None, [_i32]),
     "mgpuTensorMapEncodeTiled": (None, [_vp, C.c_int, _u32, _vp, _vp, _vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int]),
+    "mgpuTensorMapTryEncodeTiled": (_i32, [_vp, C.c_int, _u32, _vp, _vp, _vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int]),
     "mgpuTensorMapEncodeTiledMemref": (_vp, [_i64, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp]),
     "mgpuModuleOverrideKernel": (None, [C.c_char_p, C.c_char_p, _i32]),
     "mgpuModuleOverrideKernelBare": (None, [C.c_char_p, C.c_char_p, _i64]),

@@ -898,13 +898,7 @@ MDC_API void mgpuAttention(const void *qkv, const int32_t *seq_lens, void *out, 
     const uint64_t gdim[3] = {row_elems, static_cast<uint64_t>(seq_len), static_cast<uint64_t>(batch)};
     const uint64_t gstr[2] = {row_elems * 2, row_elems * 2 * static_cast<uint64_t>(seq_len)};
     const uint32_t box[3] = {64, 128, 1};
-    const uint32_t estr[3] = {1, 1, 1};
-    const int before = mgpuGetLastError();
-    mgpuTensorMapEncodeTiled(&tm, dtype == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                             3, const_cast<void *>(qkv), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (before == 0 && mgpuGetLastError() != 0) return;
+    if (!encode_tmap(&tm, dtype, 3, qkv, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B)) return;
   }
   // the output as (column, position, sequence) in boxes of 64 columns x 32 rows: a warp's
   // rows past the end of the sequence are clipped instead of landing in the next sequence
@@ -914,13 +908,7 @@ MDC_API void mgpuAttention(const void *qkv, const int32_t *seq_lens, void *out, 
     const uint64_t gdim[3] = {out_row, static_cast<uint64_t>(seq_len), static_cast<uint64_t>(batch)};
     const uint64_t gstr[2] = {out_row * 2, out_row * 2 * static_cast<uint64_t>(seq_len)};
     const uint32_t box[3] = {64, 32, 1};
-    const uint32_t estr[3] = {1, 1, 1};
-    const int before = mgpuGetLastError();
-    mgpuTensorMapEncodeTiled(&tmo, dtype == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                             3, out, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (before == 0 && mgpuGetLastError() != 0) return;
+    if (!encode_tmap(&tmo, dtype, 3, out, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B)) return;
   }
   AttnParams p;
   p.seq_lens = seq_lens;

@@ -36,8 +36,6 @@
 #include "ptx_sm100.cuh"
 
 namespace mdc {
-bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
-                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
 namespace convh {
 constexpr int BM = 128, BK = 64;
@@ -687,17 +685,14 @@ bool conv_halo(const ConvShape &call, cudaStream_t s) {
   }
   CUtensorMap tx = {}, tw;
   bool ok = encode_tmap_2d(&tw, ws, MGPU_DTYPE_F16, static_cast<uint64_t>(Kp), static_cast<uint64_t>(c.OC), static_cast<uint64_t>(Kp) * 2, BK,
-                           static_cast<uint32_t>(p.bn));
+                           static_cast<uint32_t>(p.bn), false);
   if (ok && copy) {
     const uint64_t px = static_cast<uint64_t>(Cp) * 2, rows = static_cast<uint64_t>(c.N * copy_h), width = static_cast<uint64_t>(copy_w);
     const uint64_t gdim[3] = {static_cast<uint64_t>(Cp), p.h.flat ? rows * width : width, p.h.flat ? 1 : rows};
     const uint64_t gstr[2] = {px, px * width};
     const uint32_t box[3] = {BK, static_cast<uint32_t>(p.h.flat ? p.box_px : p.h.IW), static_cast<uint32_t>(p.h.flat ? 1 : p.h.px / p.h.IW)};
-    const uint32_t estr[3] = {1, 1, 1};
-    mgpuTensorMapEncodeTiled(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, ws + w_bytes, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    ok = before != 0 || mgpuGetLastError() == 0;
-    ok = ok && conv_prepare(c, call, e.sampled, copy_h, copy_w, ws + w_bytes, ws, s);
+    ok = encode_tmap(&tx, MGPU_DTYPE_F16, 3, ws + w_bytes, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B, false) &&
+         conv_prepare(c, call, e.sampled, copy_h, copy_w, ws + w_bytes, ws, s);
   } else if (ok) {
     const int64_t ncb = p.pairs ? 1 : p.ncb;
     const FilterPackParams f{call.w, reinterpret_cast<__half *>(ws), int(c.IC), int(c.KH), int(c.KW), int(c.KH * c.KW), int(ncb), p.pairs, int(Kp)};

@@ -39,8 +39,6 @@
 #include "ptx_sm100.cuh"
 
 namespace mdc {
-bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
-                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
 namespace convp {
 constexpr int BM = 128, BK = 64;
@@ -613,7 +611,7 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   }
   CUtensorMap tx = {}, tw;
   bool ok = encode_tmap_2d(&tw, ws, MGPU_DTYPE_F16, static_cast<uint64_t>(Kp), static_cast<uint64_t>(c.OC),
-                           static_cast<uint64_t>(Kp) * 2, BK, static_cast<uint32_t>(p.bn));
+                           static_cast<uint64_t>(Kp) * 2, BK, static_cast<uint32_t>(p.bn), false);
   if (ok && !gather) {
     const cuuint64_t gdim[4] = {cuuint64_t(Cp), cuuint64_t(c.W), cuuint64_t(c.H), cuuint64_t(c.N)};
     const cuuint64_t gstr[3] = {cuuint64_t(Cp) * 2, cuuint64_t(Cp) * 2 * c.W, cuuint64_t(Cp) * 2 * c.W * c.H};

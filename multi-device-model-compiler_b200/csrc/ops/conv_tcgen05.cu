@@ -37,8 +37,6 @@
 namespace mdc {
 void cast_rows_padded(const float *src, void *dst, int64_t R, int64_t C, int64_t Cp, int32_t dtype,
                       cudaStream_t s);
-bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
-                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
 namespace conv {
 // Where the 32 values of group q (k / 32) of a TAP_MAJOR patch come from; blocks64: blocks of 64 channels

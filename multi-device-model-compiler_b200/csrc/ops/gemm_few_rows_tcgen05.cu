@@ -21,8 +21,6 @@
 #include "ops_common.h"
 
 namespace mdc {
-bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
-                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
 namespace fewrows {
 constexpr int LOAD_WARPS = 8;

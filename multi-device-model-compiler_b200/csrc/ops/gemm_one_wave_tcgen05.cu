@@ -353,13 +353,7 @@ static bool encode_operand(CUtensorMap *map, const void *base, int32_t dtype, in
                             static_cast<uint64_t>(blocked ? Kp / onewave::BK : 1)};
   const uint64_t gstr[2] = {static_cast<uint64_t>(Kp) * 2, onewave::BK * 2};
   const uint32_t box[3] = {onewave::BK, static_cast<uint32_t>(box_rows), static_cast<uint32_t>(blocked ? depth : 1)};
-  const uint32_t estr[3] = {1, 1, 1};
-  const int before = mgpuGetLastError();
-  mgpuTensorMapEncodeTiled(map, dtype == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                           3, const_cast<void *>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return before != 0 || mgpuGetLastError() == 0;
+  return encode_tmap(map, dtype, 3, base, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, const float *bias, const void *residual,

@@ -499,27 +499,11 @@ uint32_t *device_error_slot() {
   return slot;
 }
 
-// elem: MGPU_DTYPE_*; swizzle_bytes: 128 or 64 (must equal box_inner * element size)
-bool encode_tmap_2d_ex(CUtensorMap *map, const void *base, int32_t elem, uint64_t inner, uint64_t outer,
-                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle_bytes) {
-  const uint64_t gdim[2] = {inner, outer};
-  const uint64_t gstr[1] = {row_stride_bytes};
-  const uint32_t box[2] = {box_inner, box_outer};
-  const uint32_t estr[2] = {1, 1};
-  const int before = mgpuGetLastError();
-  const int dt = elem == MGPU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                 : elem == MGPU_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                          : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  mgpuTensorMapEncodeTiled(map, dt, 2, const_cast<void *>(base), gdim, gstr, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return before != 0 || mgpuGetLastError() == 0;
-}
-
-bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
-                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer) {
-  return encode_tmap_2d_ex(map, base, dtype, inner, outer, row_stride_bytes, box_inner, box_outer, 128);
+// Rows of the output or the residual in boxes of cw columns x 32 rows.
+static bool encode_rows(CUtensorMap *map, const void *base, int32_t dtype, int64_t M, int64_t N, uint32_t cw, size_t elem) {
+  const uint64_t dim[2] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M)}, stride = static_cast<uint64_t>(N) * elem;
+  const uint32_t box[2] = {cw, 32};
+  return encode_tmap(map, dtype, 2, base, dim, &stride, box, cw * elem == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <typename T16, typename TOut, int ACT, int CG, bool kWide>
@@ -574,11 +558,10 @@ static void launch_gemm_rows(const CUtensorMap &ta, const CUtensorMap &tb, GemmP
   // staged chunks of 64 columns (128-byte rows) for 16-bit output when a tile half is a multiple of
   // that, else of 32
   p.cw = sizeof(TOut) == 2 && (p.bn / 2) % 64 == 0 ? 64 : 32;
-  const uint64_t N = static_cast<uint64_t>(p.N), M = static_cast<uint64_t>(p.M);
   const uint32_t cw = static_cast<uint32_t>(p.cw);
   if (p.rows.fast) {
-    if (!encode_tmap_2d_ex(&rows.out, p.out, out_dtype, N, M, N * sizeof(TOut), cw, 32, static_cast<int>(cw * sizeof(TOut)))) return;
-    if (p.residual && !encode_tmap_2d_ex(&rows.res, p.residual, dtype, N, M, N * 2, cw, 32, static_cast<int>(cw * 2))) return;
+    if (!encode_rows(&rows.out, p.out, out_dtype, p.M, p.N, cw, sizeof(TOut))) return;
+    if (p.residual && !encode_rows(&rows.res, p.residual, dtype, p.M, p.N, cw, 2)) return;
   }
   launch_gemm_act<T16, TOut, false>(ta, tb, rows, p, grid, act, s);
 }

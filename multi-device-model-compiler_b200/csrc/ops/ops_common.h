@@ -91,6 +91,29 @@ inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// A tiled tensor map of fp16, bf16 or fp32 elements; dim and box innermost first, stride in bytes from the second dimension
+// on.  False where it is not encoded, by this call's own verdict, whatever the status says; the status then says so, unless
+// the caller has another way (`report` false).
+inline bool encode_tmap(CUtensorMap *map, int32_t dtype, uint32_t rank, const void *base, const uint64_t *dim,
+                        const uint64_t *stride, const uint32_t *box, CUtensorMapSwizzle swizzle, bool report = true) {
+  const uint32_t ones[5] = {1, 1, 1, 1, 1};
+  const int type = dtype == MGPU_DTYPE_BF16  ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                   : dtype == MGPU_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                             : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const int32_t e = mgpuTensorMapTryEncodeTiled(map, type, rank, const_cast<void *>(base), dim, stride, box, ones,
+                                                CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (e != 0 && report) mgpuSetLastError(e, "cuTensorMapEncodeTiled");
+  return e == 0;
+}
+// The same for rows of a matrix, 128-byte swizzled.
+inline bool encode_tmap_2d(CUtensorMap *map, const void *base, int32_t dtype, uint64_t inner, uint64_t outer,
+                           uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, bool report = true) {
+  const uint64_t dim[2] = {inner, outer};
+  const uint32_t box[2] = {box_inner, box_outer};
+  return encode_tmap(map, dtype, 2, base, dim, &row_stride_bytes, box, CU_TENSOR_MAP_SWIZZLE_128B, report);
+}
+
 // Optional per-launch timing: while profiling is on (mgpuOpsProfileBegin), every launch
 // site brackets its kernel with two CUDA events on the launching stream; mgpuOpsProfileEnd
 // sums the elapsed times per kernel category.  Off by default (no events, no overhead).

@@ -984,19 +984,30 @@ MDC_API uint64_t mgpuPoolInUseBytes(void) { return pool().in_use_bytes(); }
 MDC_API void mgpuPoolTrim(void) { pool().trim(); }
 
 // ---------------- tensor maps ----------------
-MDC_API void mgpuTensorMapEncodeTiled(void *tensorMap, int tensorDataType, uint32_t tensorRank,
-                                      void *globalAddress, const uint64_t *globalDim,
-                                      const uint64_t *globalStrides, const uint32_t *boxDim,
-                                      const uint32_t *elementStrides, int interleave, int swizzle,
-                                      int l2Promotion, int oobFill) {
-  if (!ensure_device() || !driver().ok) return;
-  DRV_CHECK(driver().TensorMapEncodeTiled(
+MDC_API int32_t mgpuTensorMapTryEncodeTiled(void *tensorMap, int tensorDataType, uint32_t tensorRank,
+                                            void *globalAddress, const uint64_t *globalDim,
+                                            const uint64_t *globalStrides, const uint32_t *boxDim,
+                                            const uint32_t *elementStrides, int interleave, int swizzle,
+                                            int l2Promotion, int oobFill) {
+  if (!ensure_device() || !driver().ok) return -1;
+  return static_cast<int32_t>(driver().TensorMapEncodeTiled(
       static_cast<CUtensorMap *>(tensorMap), static_cast<CUtensorMapDataType>(tensorDataType),
       tensorRank, globalAddress, reinterpret_cast<const cuuint64_t *>(globalDim),
       reinterpret_cast<const cuuint64_t *>(globalStrides), boxDim, elementStrides,
       static_cast<CUtensorMapInterleave>(interleave), static_cast<CUtensorMapSwizzle>(swizzle),
       static_cast<CUtensorMapL2promotion>(l2Promotion),
       static_cast<CUtensorMapFloatOOBfill>(oobFill)));
+}
+
+MDC_API void mgpuTensorMapEncodeTiled(void *tensorMap, int tensorDataType, uint32_t tensorRank,
+                                      void *globalAddress, const uint64_t *globalDim,
+                                      const uint64_t *globalStrides, const uint32_t *boxDim,
+                                      const uint32_t *elementStrides, int interleave, int swizzle,
+                                      int l2Promotion, int oobFill) {
+  const int32_t e = mgpuTensorMapTryEncodeTiled(tensorMap, tensorDataType, tensorRank, globalAddress, globalDim, globalStrides,
+                                                boxDim, elementStrides, interleave, swizzle, l2Promotion, oobFill);
+  // (-1: no device or driver, which is on record)
+  if (e != -1) drv_ok(static_cast<CUresult>(e), "cuTensorMapEncodeTiled");
 }
 
 MDC_API void *mgpuTensorMapEncodeTiledMemref(int64_t tensorRank, void *descriptor,

@@ -70,6 +70,23 @@ def test_no_cpu_fallback_without_a_gpu(built):
     rt.mgpuClearLastError()
 
 
+def test_tensor_map_verdict_is_its_own(built):
+    """Refused without a device, and for a rank that the driver does not know: with a status pending or without one."""
+    rt = built.runtime()
+    tmap, one = (ctypes.c_uint64 * 17)(), (ctypes.c_uint64 * 5)(8, 8, 8, 8, 8)
+    at = (ctypes.addressof(tmap) + 63) // 64 * 64
+    boxes = (ctypes.c_uint32 * 5)(8, 8, 1, 1, 1)
+
+    def encode():
+        return rt.mgpuTensorMapTryEncodeTiled(at, 6, 0, None, one, one, boxes, boxes, 0, 0, 0, 0)
+    rt.mgpuClearLastError()
+    assert encode() != 0
+    rt.mgpuSetLastError(7, b"pending")
+    status = rt.mgpuGetLastError()
+    assert status != 0 and encode() != 0 and rt.mgpuGetLastError() == status
+    rt.mgpuClearLastError()
+
+
 def test_cnn_ops_reject_bad_geometry_before_touching_a_device(built):
     rt, ops = built.runtime(), built.ops()
     rt.mgpuClearLastError()

@@ -266,24 +266,27 @@ def test_conv_output_over_its_input(m, IC, OC, size, kernel, stride):
 
 
 @pytest.mark.parametrize("earlier_failure", [False, True])
-def test_conv_without_memory_for_the_copy(m, earlier_failure):
+@pytest.mark.parametrize("OC,KH,KW,stride", [(16, 1, 2, 8), (8, 3, 3, 1)])  # an im2col call, and one of shared regions
+def test_conv_without_memory_for_the_copy(m, OC, KH, KW, stride, earlier_failure):
     """With no device memory left for the NHWC copy of the input the direct kernel takes over, whether
     or not an earlier call has left a status; that status stays."""
     import torch
     rt, ops = m.runtime(), m.ops()
-    N, IC, H, W, OC, OH, OW = 12, 32, 2048, 2048, 16, 256, 256  # 6.4 GB in, a copy of 3.2 GB
+    N, IC, H, W = 12, 32, 2048, 2048  # 6.4 GB in, a copy of 3.2 GB
+    pad = KH // 2
+    OH, OW = H // stride, W // stride
     x = torch.randint(-4, 5, (N, IC, H, W), device="cuda", dtype=torch.int8).float()
-    w = torch.randint(-3, 4, (OC, IC, 1, 2), device="cuda", dtype=torch.int8).float()
+    w = torch.randint(-3, 4, (OC, IC, KH, KW), device="cuda", dtype=torch.int8).float()
     out = torch.empty(N, OC, OH, OW, device="cuda")
 
     def call():
         out.zero_()
         torch.cuda.synchronize()
-        ops.mgpuConv2d(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), None, N, IC, H, W, OC, 1, 2, OH, OW, 0, 0, 0, 0, 8, 8, 1, 1,
-                       False, False, None)
+        ops.mgpuConv2d(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), None, N, IC, H, W, OC, KH, KW, OH, OW, pad, pad, pad, pad,
+                       stride, stride, 1, 1, False, False, None)
         rt.mgpuStreamSynchronize(None)
-        return out.clone()
-    expect = call()
+    call()
+    expect = out.clone()
     m.check("conv")
     assert float(expect.abs().max()) > 0
     torch.cuda.empty_cache()
@@ -295,8 +298,8 @@ def test_conv_without_memory_for_the_copy(m, earlier_failure):
                            False, False, None)
             ops.mgpuPool2d(None, None, 1, 1, 4, 4, 3, 3, 2, 2, 0, 0, 0, 0, 2, 2, 0, None)  # bad geometry: sets the status
             assert rt.mgpuGetLastError() != 0
-        got = call()
-        assert torch.equal(got, expect)
+        call()
+        assert torch.equal(out, expect)
         assert (rt.mgpuGetLastError() != 0) == earlier_failure
     finally:
         rt.mgpuClearLastError()

@@ -58,3 +58,14 @@ def test_the_warp_waits_are_uniform():
         return code[code.index("bool " + function):].split("\n}\n")[0]
     assert "__all_sync(0xffffffffu, mbar_wait(" in body("mbar_wait_all")
     assert "__shfl_sync(0xffffffffu, ok, 0)" in body("mbar_wait_warp")
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(OPS) if f.endswith((".cu", ".h", ".cuh"))))
+def test_a_tensor_map_is_judged_by_its_own_call(name):
+    """A kernel launched with a map that was never written faults.  The status cannot tell: it may hold an earlier call's
+    failure, or another thread's.  So the entry point that only sets the status is not for the operators."""
+    code = _code(name)
+    assert "mgpuTensorMapEncodeTiled" not in code and not re.search(r"before != 0 \|\| mgpuGetLastError", code)
+    for call in re.finditer(r"\bencode_(tmap|tmap_2d|rows|operand)\(", code):
+        before = code[max(0, call.start() - 120):call.start()]
+        assert re.search(r"(if \([^;{}]*|ok = [^;{}]*|return |\|\|\s*!|inline bool |static bool )$", before), before[-80:]
