@@ -76,16 +76,22 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w,
 //   K = 1500, 2000 columns 16 rows 8.8 / 7.8, 24 rows 8.4 / 8.9
 //   K = 2048, 1000 columns  8 rows 12.8 / 12.3, 16 rows 12.6 / 12.9;  K = 4096, 4096 columns 8 rows 21.7 / 21.2, 16 rows 21.3 / 22.3
 //   input read value by value: 770, 500 columns 16 rows 7.0 / 6.2, 24 rows 7.1 / 7.3;  1501, 1000 columns 8 rows 8.4 / 8.0, 12 rows 8.2 / 8.4
-// Two launches never take less than the host needs for them, 7 us here and 6 on a faster one (48 rows, K = 448: 6.1 / 6.3),
-// so the line is drawn where one launch takes less than 6.
+// Up to 8 rows the launch is worth more than what the CTAs read, up to 40000 values, or 16000 that come one by one; beyond
+// one CTA per SM each wave reads them again:
+//   1 row   2000 x 6000 27.8 / 23.6, 4736 x 14000 67.7 / 64.6;  8 rows  4096 x 5000 25.9 / 25.4 (40000), 2816 x 6000 28.9 / 29.7, 4096 x 10000 44.2 / 46.7
+//   by value  4 rows  1700 x 3001 18.6 / 17.4, 2816 x 7001 33.4 / 33.7;  6 rows  1700 x 3001 18.1 / 19.0;  8 rows  2000 x 3001 16.5 / 17.9
+//   two waves and more  7500 x 640 8 rows 13.0 / 11.9;  16384 x 2400 2 rows 57.0 / 55.1, 8 rows 55.9 / 56.2;  30000 x 1600 6 rows 85.2 / 89.4
+// From 9 rows to 16 the line is where one launch stops winning.  From 17 to 32 it lies below that, at 512: 32 rows at K =
+// 768 gain (7.0 / 6.1) only where the host needs 7 us for two launches, and a faster one needs 6.
 // Below 256 nothing was measured and the launch ahead stays, as it does for an output that overlaps the input: it has read
 // the input before the first store.
-inline bool few_rows_convert(const float *x, const float *out, int64_t M, int64_t N, int64_t K) {
+inline bool few_rows_convert(const float *x, const float *out, int64_t M, int64_t N, int64_t K, int sms) {
   const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), o0 = reinterpret_cast<uintptr_t>(out);
   if (o0 < x0 + static_cast<uintptr_t>(M) * K * 4 && x0 < o0 + static_cast<uintptr_t>(M) * N * 4) return false;
   if (K < 256) return false;
-  if (M <= 8) return true;
-  if (K % 4 || (x0 & 15u)) return M <= 16 && K <= 768;
+  const bool by_value = K % 4 || (x0 & 15u);
+  if (M <= 8) return M * K <= (by_value ? 16000 : 40000) / ((N + 32 * sms - 1) / (32 * sms));
+  if (by_value) return M <= 16 && K <= 768;
   return (M <= 16 && K <= 1536) || (M <= 32 && K <= 512);
 }
 

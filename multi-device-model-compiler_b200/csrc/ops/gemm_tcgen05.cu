@@ -863,7 +863,7 @@ MDC_API void mgpuMatmulNoAlloc(float *input, float *weight, float *bias, float *
   cudaStream_t s = as_stream(stream);
   OperandList list;
   if (gemm_takes_few_rows(M, N, K, weight, output, di.sms)) {
-    if (few_rows_convert(input, output, M, N, K)) {
+    if (few_rows_convert(input, output, M, N, K, di.sms)) {
       gemm_few_rows(nullptr, input, weight, bias, output, M, N, K, s);
       return;
     }

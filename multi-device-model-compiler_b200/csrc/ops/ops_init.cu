@@ -68,7 +68,7 @@ MDC_API void mgpuMatmul(float *input, float *weight, float *bias, float *output,
   if (!di.ok) return;
   const int64_t Kp = (K + 7) / 8 * 8;
   if (gemm_takes_few_rows(M, N, K, weight, output, di.sms) && !mgpuConstantSourceOf(weight)) {
-    if (few_rows_convert(input, output, M, N, K)) {
+    if (few_rows_convert(input, output, M, N, K, di.sms)) {
       gemm_few_rows(nullptr, input, weight, bias, output, M, N, K, as_stream(stream));
       return;
     }

@@ -49,9 +49,14 @@ int main() {
   assert(gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, out, 148));
   assert(!gemm_takes_few_rows(1, 1 << 30, 1 << 20, v, reinterpret_cast<const float *>(uintptr_t(1) << 50), 148));
   // where the input is converted in the Gemm: rows and K, the input's alignment, no overlap with the output
-  using mdc::few_rows_convert;
+  auto few_rows_convert = [](const float *x, const float *o, int64_t M, int64_t N, int64_t K) { return mdc::few_rows_convert(x, o, M, N, K, 148); };
   alignas(16) static float in[64];
-  assert(few_rows_convert(in, out, 8, 10, 1 << 20) && few_rows_convert(in + 1, out, 8, 10, 1 << 20));
+  // up to 8 rows: values that all waves together read of the input
+  assert(few_rows_convert(in, out, 8, 10, 5000) && !few_rows_convert(in, out, 8, 10, 5004) && few_rows_convert(in, out, 1, 4736, 14000));
+  assert(few_rows_convert(in + 1, out, 8, 10, 2000) && !few_rows_convert(in + 1, out, 8, 10, 2004));
+  assert(few_rows_convert(in, out, 5, 10, 3199) && !few_rows_convert(in, out, 5, 10, 3201) && !few_rows_convert(in, out, 8, 10, 1 << 20));
+  assert(few_rows_convert(in, out, 8, 9472, 640) && few_rows_convert(in, out, 8, 4737, 2500) && !few_rows_convert(in, out, 8, 4737, 2504));
+  assert(!few_rows_convert(in, out, 8, 1 << 30, 256) && !few_rows_convert(in, out, 6, 30000, 1600));
   assert(few_rows_convert(in, out, 16, 10, 1536) && !few_rows_convert(in, out, 16, 10, 1540) && !few_rows_convert(in, out, 17, 10, 772));
   assert(few_rows_convert(in, out, 32, 10, 512) && !few_rows_convert(in, out, 32, 10, 516) && !few_rows_convert(in, out, 33, 10, 256));
   assert(few_rows_convert(in, out, 1, 10, 256) && !few_rows_convert(in, out, 1, 10, 255));
