@@ -366,16 +366,18 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         return true;
       };
       auto of_steps = [&](auto resident, int steps, uint32_t region) __attribute__((always_inline)) -> bool {
-        switch (steps) {
-        case 0: return taps(std::integral_constant<int, 0>{}, resident, region);
-        case 1: return taps(std::integral_constant<int, 1>{}, resident, region);
-        case 2: return taps(std::integral_constant<int, 2>{}, resident, region);
-        case 3: return taps(std::integral_constant<int, 3>{}, resident, region);
-        case 5: return taps(std::integral_constant<int, 5>{}, resident, region);
-        default: return taps(std::integral_constant<int, 4>{}, resident, region);
+        if (steps == 1) return taps(std::integral_constant<int, 1>{}, resident, region);
+        if constexpr (kCopy) {
+          if (steps == 2) return taps(std::integral_constant<int, 2>{}, resident, region);
+          if (steps == 3) return taps(std::integral_constant<int, 3>{}, resident, region);
+          return taps(std::integral_constant<int, 4>{}, resident, region);
+        } else {
+          if (steps == 0) return taps(std::integral_constant<int, 0>{}, resident, region);
+          if (steps == 5) return taps(std::integral_constant<int, 5>{}, resident, region);
+          return taps(std::integral_constant<int, 2>{}, resident, region);
         }
       };
-      for (int cb = 0; cb < p.ncb; ++cb) {
+      for (int cb = 0; cb < (kCopy ? p.ncb : 1); ++cb) {
         if (!mbar_wait_looked(looked, &full_bar[stage], phase, abort_flag)) {
           atomicCAS(p.err, 0u, 0x63000000u | static_cast<uint32_t>(stage));
           ok = false;
@@ -385,7 +387,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const int next = stage + 1 == p.stages ? 0 : stage + 1;
         looked = mbar_look(&full_bar[next], next ? phase : phase ^ 1);
         const uint32_t region = a_lo0 + static_cast<uint32_t>(stage) * region_units;
-        const int steps = p.chain ? (p.pairs ? 0 : 5) : cb + 1 < p.ncb ? 4 : p.last_steps;
+        const int steps = !kCopy && p.chain ? (p.pairs ? 0 : 5) : kCopy && cb + 1 < p.ncb ? 4 : p.last_steps;
         ok = p.resident ? of_steps(std::true_type{}, steps, region) : of_steps(std::false_type{}, steps, region);
         if (!ok) break;
         umma_commit_warp(&empty_bar[stage]);
@@ -431,17 +433,15 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const uint64_t plane = static_cast<uint32_t>(HW);
     const int log_sh = p.SH - 1, log_sw = p.SW - 1;
     constexpr int kOutside = 1 << 30;  // mark of a pixel outside the image
-    // Where this warp is: tile, block of channels, piece of the region, sixteen of its channels; the region's place in
-    // the ring.
+    // Where this warp is: tile, piece of the region, sixteen of its channels; the region's place in the ring.
     struct Cursor {
-      int tile, cb, piece, step, stage;
+      int tile, piece, step, stage;
       uint32_t phase;
     };
-    auto steps_of = [&](int cb) __attribute__((always_inline)) { return cb + 1 < p.ncb ? 4 : p.last_steps; };
     auto settle = [&](Cursor &c) __attribute__((always_inline)) {  // pieces past the end are those of the next regions
       while (c.piece >= p.qb) {
         c.piece -= p.qb;
-        if (++c.cb == p.ncb) c.cb = 0, c.tile += gridDim.x;
+        c.tile += gridDim.x;
         if (++c.stage == p.stages) c.stage = 0, c.phase ^= 1;
       }
     };
@@ -467,10 +467,10 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       in = in && img < p.N && h < p.H && static_cast<unsigned>(col) < static_cast<unsigned>(p.W);
       if (at >= 0 && !in) at |= kOutside;
       // pixels outside read an element that is there and drop it: no branch per load
-      src = reinterpret_cast<const char *>(p.x + (static_cast<int64_t>(in ? img : 0) * p.IC + c.cb * 64) * HW + (in ? h * p.W + col : 0));
+      src = reinterpret_cast<const char *>(p.x + static_cast<int64_t>(in ? img : 0) * p.IC * HW + (in ? h * p.W + col : 0));
     };
     auto load = [&](const Cursor &c, float (&dst)[16]) __attribute__((always_inline)) {
-      const int n = p.IC - c.cb * 64 - c.step * 16;
+      const int n = p.IC - c.step * 16;
       if (n >= 16) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) dst[j] = __ldg(reinterpret_cast<const float *>(src + plane * (4u * j)));
@@ -479,7 +479,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         for (int j = 0; j < 16; ++j) dst[j] = j < n ? __ldg(reinterpret_cast<const float *>(src + plane * (4u * j))) : 0.f;
       }
     };
-    Cursor cur{static_cast<int>(blockIdx.x), 0, warp - EPI_WARPS - 2, 0, 0, 0};
+    Cursor cur{static_cast<int>(blockIdx.x), warp - EPI_WARPS - 2, 0, 0, 0};
     settle(cur);
     float va[16], vb[16];
     int at_a = -1, at_b = -1;
@@ -493,7 +493,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     auto turn = [&](const float (&v)[16], int at_v, float (&ahead)[16], int &at_ahead) __attribute__((always_inline)) -> bool {
       if (cur.tile >= p.num_tiles) return false;
       Cursor nx = cur;
-      const bool last = ++nx.step == steps_of(cur.cb);
+      const bool last = ++nx.step == p.last_steps;
       if (last) {
         nx.step = 0, nx.piece += IN_WARPS;
         settle(nx);
@@ -546,18 +546,17 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 }
 
 // The filter, OIHW fp32, as rows of fp16 in the order the MMAs take it, zeros where there is no weight:
-//   [OC][block of 64 channels][tap][64], or with pairs of taps [OC][filter row][pair][2][8], rows padded to 64.
-// A block of threads per output channel and block of 64 channels.
+//   [OC][tap][64], or with pairs of taps [OC][filter row][pair][2][8], rows padded to 64.
+// A block of threads per output channel.
 struct FilterPackParams {
   const float *w;
   __half *out;
-  int IC, KH, KW, taps, ncb, pairs, row;  // row: elements per output channel
+  int IC, KH, KW, taps, pairs, row;  // row: elements per output channel
 };
 __global__ void __launch_bounds__(256) conv_filter_kernel(const FilterPackParams p) {
   pdl_wait();
   pdl_launch_dependents();  // after the wait: what is older is complete for the kernel that follows
-  const int cb = static_cast<int>(blockIdx.x % static_cast<unsigned>(p.ncb));
-  const int64_t oc = blockIdx.x / static_cast<unsigned>(p.ncb);
+  const int64_t oc = blockIdx.x;
   if (p.pairs) {
     const int per_row = (p.KW + 1) / 2;
     for (int i = threadIdx.x; i < p.row; i += 256) {
@@ -568,11 +567,11 @@ __global__ void __launch_bounds__(256) conv_filter_kernel(const FilterPackParams
     return;
   }
   // the block's 64 x taps weights are contiguous in w: strided reads, served by L1 after the first touch
-  const float *w = p.w + (oc * p.IC + cb * 64) * static_cast<int64_t>(p.taps);
-  __half *out = p.out + oc * p.row + static_cast<int64_t>(cb) * p.taps * 64;
+  const float *w = p.w + oc * p.IC * p.taps;
+  __half *out = p.out + oc * p.row;
   for (int i = threadIdx.x; i < p.taps * 64; i += 256) {
     const int ic = i & 63, tap = i >> 6;
-    out[i] = __float2half_rn(cb * 64 + ic < p.IC ? __ldg(w + ic * p.taps + tap) : 0.f);
+    out[i] = __float2half_rn(ic < p.IC ? __ldg(w + ic * p.taps + tap) : 0.f);
   }
 }
 
@@ -694,11 +693,10 @@ bool conv_halo(const ConvShape &call, cudaStream_t s) {
     ok = encode_tmap(&tx, MGPU_DTYPE_F16, 3, ws + w_bytes, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B, false) &&
          conv_prepare(c, call, e.sampled, copy_h, copy_w, ws + w_bytes, ws, s);
   } else if (ok) {
-    const int64_t ncb = p.pairs ? 1 : p.ncb;
-    const FilterPackParams f{call.w, reinterpret_cast<__half *>(ws), int(c.IC), int(c.KH), int(c.KW), int(c.KH * c.KW), int(ncb), p.pairs, int(Kp)};
+    const FilterPackParams f{call.w, reinterpret_cast<__half *>(ws), int(c.IC), int(c.KH), int(c.KW), int(c.KH * c.KW), p.pairs, int(Kp)};
     {
       ProfileScope prof(kCatElementwise, s);
-      check_cuda(launch_chain(conv_filter_kernel, dim3(static_cast<unsigned>(c.OC * ncb)), dim3(256), 0, s, 1, f), "launch conv_filter_kernel");
+      check_cuda(launch_chain(conv_filter_kernel, dim3(static_cast<unsigned>(c.OC)), dim3(256), 0, s, 1, f), "launch conv_filter_kernel");
     }
     launched("conv_filter_kernel");
   }

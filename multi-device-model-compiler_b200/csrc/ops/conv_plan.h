@@ -173,8 +173,9 @@ inline bool halo_tile(const ConvShape &c, ConvForm form, int sms, HaloTile *best
   const int64_t ncb = (c.IC + 63) / 64, taps = c.KH * c.KW, pair_taps = c.KH * ((c.KW + 1) / 2);
   const bool pairs = c.IC <= 8;
   const int64_t num_kb = pairs ? (pair_taps + 3) / 4 : ncb * taps;
-  const int last_steps = static_cast<int>((c.IC - (ncb - 1) * 64 + 15) / 16), steps = ncb > 1 ? 4 : last_steps;
+  const int last_steps = static_cast<int>((c.IC - (ncb - 1) * 64 + 15) / 16);
   const int64_t mmas = pairs ? pair_taps : ((ncb - 1) * 4 + last_steps) * taps;
+  if (!copy && c.IC > 32) return false;  // one block of channels
   if (c.OC > kHaloMaxOC || (pairs ? pair_taps : taps) > kHaloMaxTaps || ncb * taps > (1 << 16) || c.OH * c.OW > INT32_MAX) return false;
   HaloTile t;
   t.ncb = static_cast<int>(ncb), t.last_steps = last_steps, t.pairs = pairs ? 1 : 0, t.num_kb = static_cast<int>(num_kb);
@@ -189,7 +190,7 @@ inline bool halo_tile(const ConvShape &c, ConvForm form, int sms, HaloTile *best
     t.region_bytes = static_cast<uint32_t>((t.boxes * t.box_px * 128 + 1023) / 1024 * 1024);
   } else {
     t.boxes = t.box_px = 0;
-    t.region_bytes = static_cast<uint32_t>(t.h.plane_px * 32 * (pairs ? 1 : steps));
+    t.region_bytes = static_cast<uint32_t>(t.h.plane_px * 32 * (pairs ? 1 : last_steps));
   }
   double best_cost = 1e300;
   for (int bn = 256; bn >= 32; bn -= 32) {
@@ -204,8 +205,8 @@ inline bool halo_tile(const ConvShape &c, ConvForm form, int sms, HaloTile *best
     const double in_lines = flat ? 1.8 : 1.0 + 26.0 / t.h.IW, out_lines = flat ? 1.8 : 4.0;
     const double mma = static_cast<double>(mmas) * (bn < 64 ? 46.0 : bn < 128 ? 54.0 : bn / 2.0);
     const double l2 = (copy ? static_cast<double>(ncb) * t.region_bytes : 0.0) / 64.0 + (t.resident ? 0.0 : num_kb * bn * 2.0);
-    const double loads = copy ? 0.0 : t.qb * (pairs ? static_cast<double>(c.IC) : (ncb - 1) * 64.0 + last_steps * 16.0);
-    const double work = copy ? 0.0 : t.qb * ((ncb - 1) * 4.0 + last_steps) * 100.0 + t.qb * ncb * 60.0;
+    const double loads = copy ? 0.0 : t.qb * (pairs ? static_cast<double>(c.IC) : last_steps * 16.0);
+    const double work = copy ? 0.0 : t.qb * (last_steps * 100.0 + 60.0);
     const double epi = bn * ((c.add ? 1024.0 : 512.0) / 24.0 + 4.0 * (t.splits - 1));
     const double lsu = loads * in_lines + bn * 4.0 * out_lines * (c.add ? 2.0 : 1.0);
     const double cost = rounds * (std::max({mma, l2, lsu, epi, work}) + 300.0) + epi + (copy ? l2 : 3.0 * loads);
