@@ -46,8 +46,6 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 12;
 constexpr int EPI_WARPS = 8;
 constexpr int GATHER_GROUPS = 3, GATHER_WARPS = GATHER_GROUPS * 4;
-constexpr int kMaxGatherK = 1024;  // table entries
-constexpr int kMaxOC = 2048;       // bias kept in shared memory
 constexpr size_t kMaxSmem = 224 * 1024;
 // warps: 0-7 epilogue, 8 TMA, 9 MMA, then the gather warps
 constexpr int threads(bool gather) { return (EPI_WARPS + 2 + (gather ? GATHER_WARPS : 0)) * 32; }
@@ -508,30 +506,7 @@ void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp
 }
 }  // namespace
 
-// A strided 1 x 1 window reads one pixel in SH x SW: the rewrite then copies the output's pixels only, and
-// the convolution is one without stride or padding on that copy.  (33 x 476 x 87 x 56, stride 2: 108 us
-// with the whole input rewritten, 65 sampled.)
-bool conv_sampled(ConvShape &c) {
-  if (conv_gathers(c) || c.KH * c.KW != 1 || (c.SH == 1 && c.SW == 1)) return false;
-  c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
-  return true;
-}
-
-// im2col: first and last window origin relative to the first and last column / row of the image.
-static int64_t conv_upper_w(const ConvShape &c) { return (c.OW - 1) * c.SW - c.PWL - (c.W - 1); }
-static int64_t conv_upper_h(const ConvShape &c) { return (c.OH - 1) * c.SH - c.PHL - (c.H - 1); }
-
-bool conv_persistent_takes(const ConvShape &call) {
-  ConvShape c = call;
-  conv_sampled(c);
-  const int64_t taps = c.KH * c.KW, span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
-  if (c.OC > convp::kMaxOC || taps > 4096 || c.N * c.OH * c.OW * c.OC > (int64_t(1) << 40)) return false;
-  if (conv_gathers(c)) return c.IC * taps <= convp::kMaxGatherK && span_h <= 32767 && span_w <= 32767;
-  // limits of the im2col tensor map: strides, corners and tap offsets
-  const int64_t up_w = conv_upper_w(c), up_h = conv_upper_h(c);
-  return c.SW <= 8 && c.SH <= 8 && c.PWL <= 127 && c.PHL <= 127 && up_w >= -128 && up_w <= 127 && up_h >= -128 &&
-         up_h <= 127 && span_w <= 255 && span_h <= 255 && encode_im2col() != nullptr;
-}
+bool conv_persistent_takes(const ConvShape &call) { return conv_dense_describes(call) && (conv_gathers(call) || encode_im2col() != nullptr); }
 
 bool conv_prepare(const ConvShape &c, const ConvShape &call, bool sampled, int64_t copy_h, int64_t copy_w, void *x16, void *w16,
                   cudaStream_t s) {

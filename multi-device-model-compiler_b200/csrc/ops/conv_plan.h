@@ -69,9 +69,37 @@ inline bool halo_plan(const ConvShape &c, bool flat, HaloPlan *h) {
   return true;
 }
 
+// 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks.
+inline bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
+
 // A strided 1 x 1 window reads one pixel in SH x SW: makes `c` the convolution without stride or padding on a copy that
-// holds the output's pixels only.  False, and nothing changed, for other shapes.
-bool conv_sampled(ConvShape &c);
+// holds the output's pixels only.  False, and nothing changed, for other shapes.  (33 x 476 x 87 x 56, stride 2: 108 us with
+// the whole input rewritten, 65 sampled.)
+inline bool conv_sampled(ConvShape &c) {
+  if (conv_gathers(c) || c.KH * c.KW != 1 || (c.SH == 1 && c.SW == 1)) return false;
+  c.H = c.OH, c.W = c.OW, c.SH = c.SW = c.DH = c.DW = 1, c.PHL = c.PWL = 0;
+  return true;
+}
+
+// im2col: first and last window origin relative to the first and last column / row of the image.
+inline int64_t conv_upper_w(const ConvShape &c) { return (c.OW - 1) * c.SW - c.PWL - (c.W - 1); }
+inline int64_t conv_upper_h(const ConvShape &c) { return (c.OH - 1) * c.SH - c.PHL - (c.H - 1); }
+
+constexpr int kDenseMaxOC = 2048;       // bias kept in shared memory
+constexpr int kDenseMaxGatherK = 1024;  // entries of the gather's table
+
+// Whether the shape is within the limits of the persistent kernels.
+inline bool conv_dense_describes(const ConvShape &call) {
+  ConvShape c = call;
+  conv_sampled(c);
+  const int64_t taps = c.KH * c.KW, span_h = (c.KH - 1) * c.DH, span_w = (c.KW - 1) * c.DW;
+  if (c.OC > kDenseMaxOC || taps > 4096 || c.N * c.OH * c.OW * c.OC > (int64_t(1) << 40)) return false;
+  if (conv_gathers(c)) return c.IC * taps <= kDenseMaxGatherK && span_h <= 32767 && span_w <= 32767;
+  // limits of the im2col tensor map: strides, corners and tap offsets
+  const int64_t up_w = conv_upper_w(c), up_h = conv_upper_h(c);
+  return c.SW <= 8 && c.SH <= 8 && c.PWL <= 127 && c.PHL <= 127 && up_w >= -128 && up_w <= 127 && up_h >= -128 &&
+         up_h <= 127 && span_w <= 255 && span_h <= 255;
+}
 
 // Launches the rewriting of the operands: the input of `call` as NHWC fp16, channels zero-padded to a multiple of 8, images
 // of copy_h x copy_w pixels (zeros beyond the input's, or the output's pixels where `sampled`); the filter as [OC][block of
@@ -101,8 +129,6 @@ inline int choose_conv_bn(int64_t m_tiles, int64_t OC, int64_t num_kb, bool gath
   }
   return best;
 }
-// 16 channels fill a quarter of a k-block; below that the gathered patch has fewer k-blocks.
-inline bool conv_gathers(const ConvShape &c) { return c.IC < 16; }
 // The filter stays in shared memory when it is one tile wide, there is a second tile to use it, and it leaves the ring room.
 inline bool conv_filter_stays(int64_t num_kb, int bn, int64_t n_tiles, int64_t tiles, int sms) {
   return n_tiles == 1 && tiles > sms && num_kb * bn * 128 <= 100 * 1024;
@@ -306,10 +332,11 @@ inline ConvForm conv_form(const ConvShape &c, int sms, bool dense = true, HaloTi
   if (unit && !keep) consider(direct ? ConvForm::kDirectFlat : ConvForm::kCopyFlat);
   return best;
 }
+
 // Runs the convolution on conv_halo_kernel; false (and nothing launched) when the shape is not one for it.
 bool conv_halo(const ConvShape &c, cudaStream_t s);
 
-// Whether the shape is one that the persistent kernels take.
+// Whether the persistent kernels take the shape here: it is within their limits, and the driver makes im2col maps.
 bool conv_persistent_takes(const ConvShape &c);
 
 // Runs the convolution on the persistent kernels; false (and nothing launched) when the shape is one

@@ -126,3 +126,48 @@ def test_halo_tiles_find_every_tap(tmp_path):
     exe = str(tmp_path / "plan")
     subprocess.run(["g++", "-std=c++17", "-O2", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
     assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout == "ok\n"
+
+
+ROUTES = r"""
+#include "conv_plan.h"
+#include <cstdio>
+using namespace mdc;
+int main() {  // per call: N IC H W OC KH KW OH OW SH SW DH DW PHL PWL post_add
+  const char *names[] = {"kOther", "kCopyRect", "kCopyFlat", "kDirectRect", "kDirectFlat"};
+  long v[16];
+  static float some;
+  for (;;) {
+    for (long &x : v)
+      if (scanf("%ld", &x) != 1) return 0;
+    ConvShape c = {};
+    c.N = v[0], c.IC = v[1], c.H = v[2], c.W = v[3], c.OC = v[4], c.KH = v[5], c.KW = v[6], c.OH = v[7], c.OW = v[8];
+    c.SH = v[9], c.SW = v[10], c.DH = v[11], c.DW = v[12], c.PHL = v[13], c.PWL = v[14], c.add = v[15] ? &some : nullptr;
+    const bool dense = conv_dense_describes(c);
+    conv_sampled(c);
+    puts(names[static_cast<int>(conv_form(c, 148, dense))]);
+  }
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or not os.path.isdir(CUDA_INCLUDE), reason="no host compiler or CUDA headers")
+def test_rows_of_the_gpu_tests_reach_their_kernels(tmp_path):
+    """The GPU tests compare results, which are the same on every kernel: here each of their rows is held to the kernel that
+    it is there for."""
+    import test_gpu_conv_pool as gpu
+    rows = gpu.CONV_EDGES + gpu.REGION_FORMS
+    rows += [(f, (n, ic, 20, w, 9, 5, 5, (1, 1), (2,) * 4, (1, 1), False, False)) for f, n, ic, w in gpu.INFINITIES]
+    rows += [(f, (3, ic, size, size, oc, k, k, (st, st), (k // 2,) * 4, (1, 1), False, False)) for f, ic, oc, size, k, st in gpu.OVERLAPS]
+    rows.append(("kCopyRect", (12, 32, 2048, 2048, 8, 3, 3, (1, 1), (1,) * 4, (1, 1), False, False)))  # without memory for its copy
+    calls = []
+    for _, (N, IC, H, W, OC, KH, KW, stride, pad, dil, add, _relu) in rows:
+        OH = (H + pad[0] + pad[2] - (KH - 1) * dil[0] - 1) // stride[0] + 1
+        OW = (W + pad[1] + pad[3] - (KW - 1) * dil[1] - 1) // stride[1] + 1
+        calls.append((N, IC, H, W, OC, KH, KW, OH, OW, *stride, *dil, pad[0], pad[1], int(add)))
+    src, exe = tmp_path / "routes.cpp", str(tmp_path / "routes")
+    src.write_text(ROUTES)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
+    told = subprocess.run([exe], input=" ".join(str(x) for c in calls for x in c), check=True, capture_output=True, text=True).stdout.split()
+    assert len(told) == len(rows)
+    assert not [(want, got, row) for (want, row), got in zip(rows, told) if want != got]
+    assert set(told) == {"kOther", "kCopyRect", "kCopyFlat", "kDirectRect", "kDirectFlat"}

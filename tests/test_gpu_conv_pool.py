@@ -170,25 +170,33 @@ def test_conv_exact_on_small_integers(m):
     assert np.array_equal(got, ref)
 
 
-@pytest.mark.parametrize("shape", [
-    # N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
-    (1, 16, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),      # one partial tile, im2col's fewest channels
-    (1, 15, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),      # the gather kernel's most channels
-    (5, 24, 9, 5, 33, 3, 2, (2, 1), (0, 1, 2, 0), (1, 2), True, True),        # asymmetric in every respect
-    (3, 20, 11, 13, 40, 5, 3, (1, 3), (2, 0, 1, 2), (2, 1), True, False),     # channels padded to 24
-    (2, 96, 10, 6, 65, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),      # a half-full block of 64 channels
-    (300, 72, 8, 8, 48, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, False),     # tiles of two images, one round and a bit
-    (60, 64, 20, 21, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True),     # filter kept, several tiles per CTA
-    (40, 128, 20, 20, 96, 3, 3, (2, 2), (1, 1, 1, 1), (1, 1), False, False),  # filter streamed
-    (1, 256, 4, 4, 300, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False),     # many k-blocks, few pixels
-    (90, 3, 17, 19, 40, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),     # one k-block, 32 of 64 values
-    (40, 5, 31, 30, 24, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), True, False),     # four k-blocks, gather groups out of step
-    (2, 14, 12, 12, 260, 7, 7, (1, 1), (3, 3, 3, 3), (1, 1), False, False),   # gathered, filter streamed, two channel tiles
-    (3, 33, 11, 14, 20, 1, 1, (2, 3), (1, 0, 0, 2), (1, 1), True, False),     # strided 1 x 1, padded: sampled copy
-    (70, 64, 20, 20, 32, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), False, True),
-    (2, 16, 30, 30, 8, 2, 2, (9, 1), (0, 0, 0, 0), (1, 1), False, False),     # stride outside the im2col map: direct kernel
-    (2, 160, 30, 30, 8, 3, 2, (9, 1), (1, 0, 0, 1), (1, 1), True, False),     # the same, 32 channels a block
-])
+# (how conv_plan.h sends the row at 148 SMs, the row); tests/test_conv_plan_cpu.py holds them to it
+# N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
+CONV_EDGES = [
+    ("kOther", (1, 16, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False)),  # one partial tile, im2col's fewest channels
+    ("kOther", (1, 15, 7, 7, 16, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False)),  # the gather kernel's most channels
+    ("kOther", (5, 24, 9, 5, 33, 3, 2, (2, 1), (0, 1, 2, 0), (1, 2), True, True)),  # asymmetric in every respect
+    ("kOther", (3, 20, 11, 13, 40, 5, 3, (1, 3), (2, 0, 1, 2), (2, 1), True, False)),  # channels padded to 24
+    ("kCopyRect", (2, 96, 10, 6, 65, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True)),  # a half-full block of 64 channels: shared regions
+    ("kOther", (300, 72, 8, 8, 48, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, False)),  # tiles of two images, one round and a bit
+    ("kOther", (60, 64, 20, 21, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True)),  # filter kept, several tiles per CTA
+    ("kOther", (40, 128, 20, 20, 96, 3, 3, (2, 2), (1, 1, 1, 1), (1, 1), False, False)),  # filter streamed
+    ("kCopyFlat", (1, 256, 4, 4, 300, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False)),  # many k-blocks, few pixels: shared regions
+    ("kOther", (90, 3, 17, 19, 40, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True)),  # one k-block, 32 of 64 values
+    ("kDirectRect", (40, 5, 31, 30, 24, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), True, False)),  # shared regions, stride 2: more tiles than SMs
+    ("kDirectFlat", (2, 14, 12, 12, 260, 7, 7, (1, 1), (3, 3, 3, 3), (1, 1), False, False)),  # shared regions, filter streamed, several channel tiles
+    ("kOther", (3, 33, 11, 14, 20, 1, 1, (2, 3), (1, 0, 0, 2), (1, 1), True, False)),  # strided 1 x 1, padded: sampled copy
+    ("kOther", (70, 64, 20, 20, 32, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), False, True)),
+    ("kOther", (2, 16, 30, 30, 8, 2, 2, (9, 1), (0, 0, 0, 0), (1, 1), False, False)),  # stride outside the im2col map: direct kernel
+    ("kOther", (2, 160, 30, 30, 8, 3, 2, (9, 1), (1, 0, 0, 1), (1, 1), True, False)),  # the same, 32 channels a block
+    ("kOther", (21, 13, 16, 26, 33, 4, 4, (1, 1), (2, 2, 2, 2), (1, 1), True, True)),  # gathered: four k-blocks, two channel tiles, more tiles than SMs
+    ("kOther", (54, 12, 21, 17, 8, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, False)),  # gathered: two k-blocks, filter kept
+    ("kOther", (3, 14, 12, 12, 260, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False)),  # gathered: filter streamed, several channel tiles
+    ("kOther", (68, 65, 22, 52, 8, 3, 3, (2, 2), (1, 1, 1, 1), (1, 1), True, True)),  # im2col: filter kept, residual, a last block of one channel
+]
+
+
+@pytest.mark.parametrize("shape", [row for _, row in CONV_EDGES])
 def test_conv_persistent_edges(m, shape):
     """Small integers (see test_conv_exact_on_small_integers): equal bit for bit."""
     N, IC, H, W, OC, KH, KW, stride, pad, dil, has_add, relu = shape
@@ -203,35 +211,62 @@ def test_conv_persistent_edges(m, shape):
     assert np.array_equal(m.conv2d(x, w, b, **kw), oracle.conv2d(x, w, b, **kw))
 
 
-@pytest.mark.parametrize("shape", [
-    # N, IC, H, W, OC, KH, KW, stride, pad(t,l,b,r), dilation, post_add, relu
-    (3, 16, 9, 16, 16, 5, 3, (1, 1), (2, 1, 2, 1), (1, 1), True, False),      # rect out of a copy: tiles of two images
-    (2, 72, 33, 24, 33, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True),     # rect: a block of 8 channels, three rounds of rows
-    (40, 64, 24, 24, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True),     # rect: filter kept, several tiles per CTA
-    (5, 80, 7, 9, 20, 3, 5, (1, 1), (0, 3, 2, 1), (2, 1), True, False),       # flat out of a copy: asymmetric
-    (60, 100, 13, 11, 60, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False),  # flat: filter streamed, 36 channels in the last block
-    (60, 20, 19, 17, 300, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, True),    # flat, 1 x 1: two channel tiles
-    (150, 48, 15, 14, 260, 1, 1, (2, 3), (0, 0, 0, 0), (1, 1), False, True),  # the same, sampled
-    (2, 3, 21, 70, 24, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, False),      # straight from the input: rect, a tap without a partner
-    (3, 8, 12, 10, 40, 6, 6, (1, 1), (3, 2, 2, 3), (1, 1), False, True),      # flat, pairs only
-    (70, 1, 30, 31, 33, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), False, False),    # stride 2: classes of rows and columns
-    (2, 5, 23, 64, 300, 5, 5, (2, 1), (0, 1, 1, 1), (1, 2), True, False),     # strides and dilations apart, several channel tiles
-    (2, 1, 20, 50, 48, 9, 9, (1, 1), (4, 4, 4, 4), (1, 1), False, False),     # one channel: eight parts of a sum, 32 columns a tile
-    (3, 15, 14, 9, 17, 5, 5, (1, 2), (2, 2, 2, 2), (1, 3), False, True),      # two groups of channels, columns in two classes
-    (4, 32, 18, 21, 64, 7, 5, (2, 2), (3, 2, 3, 2), (1, 1), True, True),      # stride 2, 32 channels
-])
+# rows of test_conv_persistent_edges for every form of conv_form
+REGION_FORMS = [
+    ("kCopyRect", (3, 16, 9, 16, 16, 5, 3, (1, 1), (2, 1, 2, 1), (1, 1), True, False)),  # rect out of a copy: tiles of two images
+    ("kCopyRect", (2, 72, 33, 24, 33, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, True)),  # rect: a block of 8 channels, three rounds of rows
+    ("kOther", (40, 64, 24, 24, 64, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True)),  # dense: filter kept, several tiles per CTA
+    ("kCopyFlat", (5, 80, 7, 9, 20, 3, 5, (1, 1), (0, 3, 2, 1), (2, 1), True, False)),  # flat out of a copy: asymmetric
+    ("kCopyRect", (60, 100, 13, 11, 60, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False)),  # rect: filter streamed, 36 channels in the last block
+    ("kCopyFlat", (60, 20, 19, 17, 300, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), True, True)),  # flat, 1 x 1: two channel tiles
+    ("kOther", (150, 48, 15, 14, 260, 1, 1, (2, 3), (0, 0, 0, 0), (1, 1), False, True)),  # dense: 1 x 1, sampled
+    ("kOther", (2, 3, 21, 70, 24, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, False)),  # dense: gathered, odd filter rows
+    ("kDirectRect", (3, 8, 12, 10, 40, 6, 6, (1, 1), (3, 2, 2, 3), (1, 1), False, True)),  # straight from the input: pairs only
+    ("kOther", (70, 1, 30, 31, 33, 7, 7, (2, 2), (3, 3, 3, 3), (1, 1), False, False)),  # dense: gathered, stride 2
+    ("kOther", (2, 5, 23, 64, 300, 5, 5, (2, 1), (0, 1, 1, 1), (1, 2), True, False)),  # dense: gathered, strides and dilations apart
+    ("kDirectRect", (2, 1, 20, 50, 48, 9, 9, (1, 1), (4, 4, 4, 4), (1, 1), False, False)),  # one channel: eight parts of a sum, 32 columns a tile
+    ("kDirectRect", (3, 15, 14, 9, 17, 5, 5, (1, 2), (2, 2, 2, 2), (1, 3), False, True)),  # two groups of channels, columns in two classes
+    ("kOther", (4, 32, 18, 21, 64, 7, 5, (2, 2), (3, 2, 3, 2), (1, 1), True, True)),  # dense: stride 2, 32 channels
+    ("kCopyRect", (31, 18, 23, 25, 8, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), True, True)),  # rect: filter kept, several tiles per CTA, residual
+    ("kCopyRect", (1, 86, 11, 9, 33, 3, 3, (1, 1), (1, 1, 1, 1), (1, 1), False, False)),  # rect: filter streamed, two channel tiles
+    ("kCopyFlat", (72, 19, 33, 9, 8, 2, 2, (1, 1), (1, 1, 0, 0), (1, 1), True, True)),  # flat: filter kept, several tiles per CTA, residual
+    ("kCopyFlat", (33, 69, 11, 24, 65, 2, 2, (1, 1), (1, 1, 1, 1), (1, 1), True, True)),  # flat: filter streamed, a last block of five channels, three channel tiles
+    ("kCopyFlat", (55, 16, 36, 78, 34, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), True, False)),  # flat: 1 x 1, sampled, two channel tiles
+    ("kCopyFlat", (8, 32, 1, 8000, 32, 1, 7, (1, 1), (0, 3, 0, 3), (1, 1), False, False)),  # flat: images of one row
+    ("kCopyFlat", (2, 48, 1, 3000, 20, 1, 9, (1, 1), (0, 130, 0, 132), (1, 33), True, False)),  # flat: taps beyond the im2col map's offsets
+    ("kOther", (6, 48, 1, 70, 20, 1, 9, (1, 1), (0, 132, 0, 132), (1, 33), True, False)),  # the same on tiles of mostly margins: direct kernel
+    ("kDirectRect", (56, 3, 11, 32, 11, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, True)),  # straight: a tap without a partner, several tiles per CTA, residual
+    ("kDirectRect", (74, 3, 29, 38, 8, 5, 5, (2, 2), (2, 2, 2, 2), (1, 1), False, True)),  # straight: classes of rows and columns, filter kept
+    ("kDirectRect", (55, 9, 23, 58, 8, 5, 5, (2, 2), (2, 2, 2, 2), (1, 1), True, False)),  # straight: two groups of channels in classes, filter kept, several tiles per CTA
+    ("kDirectRect", (1, 11, 5, 32, 39, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), False, False)),  # straight: two groups, filter streamed, two channel tiles
+    ("kDirectRect", (1, 17, 7, 7, 11, 6, 6, (2, 2), (3, 3, 3, 3), (1, 1), True, True)),  # straight: stride 2, two sixteens of channels
+    ("kDirectRect", (73, 16, 18, 55, 8, 5, 5, (2, 2), (2, 2, 2, 2), (1, 1), False, False)),  # straight: stride 2, one sixteen, several tiles per CTA
+    ("kDirectRect", (1, 3, 5, 5, 96, 5, 5, (2, 1), (2, 2, 2, 2), (1, 2), False, False)),  # straight: strides and dilations apart, several channel tiles
+    ("kDirectFlat", (78, 2, 5, 45, 8, 6, 6, (1, 1), (3, 3, 3, 3), (1, 1), True, True)),  # flat, straight: pairs, four parts of a sum, several tiles per CTA
+    ("kDirectFlat", (79, 9, 33, 5, 10, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), False, True)),  # flat, straight: two groups of channels, several tiles per CTA
+    ("kDirectFlat", (2, 12, 20, 20, 70, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, False)),  # flat, straight: two groups, several channel tiles
+]
+
+
+@pytest.mark.parametrize("shape", [row for _, row in REGION_FORMS])
 def test_conv_halo_forms(m, shape):
     """The kernel whose tiles share one region of the input between taps, in every form of conv_form: small integers,
     equal bit for bit (see test_conv_exact_on_small_integers)."""
     test_conv_persistent_edges(m, shape)
 
 
-@pytest.mark.parametrize("IC,W", [(3, 60), (3, 20), (12, 20), (64, 20), (64, 24)])
-def test_conv_keeps_infinities_to_their_windows(m, IC, W):
+INFINITIES = [  # form, N, IC, W (20 rows, 9 channels out, 5 x 5)
+    ("kDirectRect", 2, 3, 60), ("kDirectRect", 2, 3, 20), ("kDirectFlat", 2, 12, 20), ("kCopyRect", 2, 64, 20), ("kCopyRect", 2, 64, 24),
+    ("kDirectFlat", 23, 3, 33), ("kCopyFlat", 23, 64, 33),
+]
+
+
+@pytest.mark.parametrize("N,IC,W", [row[1:] for row in INFINITIES])
+def test_conv_keeps_infinities_to_their_windows(m, N, IC, W):
     """An infinity next to a window, where the tile's region holds it and the weights of a padded tap are zero, must not
     turn into NaN: outputs whose window does not hold it are those of the input without it."""
     rng = np.random.default_rng(W)
-    x = rng.integers(-4, 5, size=(2, IC, 20, W)).astype(np.float32)
+    x = rng.integers(-4, 5, size=(N, IC, 20, W)).astype(np.float32)
     w = rng.integers(1, 4, size=(9, IC, 5, 5)).astype(np.float32)
     b = np.zeros(9, np.float32)
     clean = m.conv2d(x, w, b, pad=(2, 2, 2, 2))
@@ -243,7 +278,13 @@ def test_conv_keeps_infinities_to_their_windows(m, IC, W):
     assert np.all(np.isposinf(got[hit]))
 
 
-@pytest.mark.parametrize("IC,OC,size,kernel,stride", [(24, 24, 20, 5, 1), (32, 32, 20, 5, 2), (64, 64, 24, 3, 1), (32, 16, 33, 1, 1)])
+OVERLAPS = [  # form, IC, OC, size, kernel, stride (three images)
+    ("kCopyRect", 24, 24, 20, 5, 1), ("kOther", 32, 32, 20, 5, 2), ("kOther", 64, 64, 24, 3, 1), ("kOther", 32, 16, 33, 1, 1),
+    ("kCopyRect", 96, 64, 24, 3, 1), ("kCopyFlat", 16, 161, 73, 1, 1), ("kDirectRect", 16, 8, 5, 5, 2),
+]
+
+
+@pytest.mark.parametrize("IC,OC,size,kernel,stride", [row[1:] for row in OVERLAPS])
 def test_conv_output_over_its_input(m, IC, OC, size, kernel, stride):
     """From 16 channels on the output may lie over the input: a launch ahead has copied it, or the call is routed so."""
     rng = np.random.default_rng(IC)
