@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "conv_epilogue.cuh"
 #include "conv_plan.h"
 #include "fast_div.h"
 #include "gemm_common.cuh"
@@ -182,17 +183,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       float extra[kAdd ? G : 1];
       auto fetch = [&](int c0) __attribute__((always_inline)) {
         if constexpr (kAdd) {
-          if (live) {
-            const float *src = p.add + out_base + static_cast<int64_t>(c0) * P;
-            if (c0 + G <= nc) {
-#pragma unroll
-              for (int j = 0; j < G; ++j, src += P) extra[j] = __ldg(src);
-            } else {
-#pragma unroll
-              for (int j = 0; j < G; ++j, src += P)
-                if (c0 + j < nc) extra[j] = __ldg(src);
-            }
-          }
+          if (live) conv_fetch(extra, p.add + out_base + static_cast<int64_t>(c0) * P, P, nc - c0);
         }
       };
       if constexpr (kAdd) {
@@ -221,31 +212,9 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             for (int j = 0; j < 16; ++j) a[j] = __float_as_uint(__uint_as_float(a[j]) + __uint_as_float(more[j]));
           }
         }
-#pragma unroll
-        for (int j = 0; j < G; j += 4) {
-          float4 b = *reinterpret_cast<const float4 *>(bias_s + n0 + c0 + j);
-          if constexpr (kAdd) b.x += extra[j], b.y += extra[j + 1], b.z += extra[j + 2], b.w += extra[j + 3];
-          a[j] = __float_as_uint(__uint_as_float(a[j]) + b.x);
-          a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + b.y);
-          a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + b.z);
-          a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + b.w);
-        }
-        if (p.relu) {
-#pragma unroll
-          for (int j = 0; j < G; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
-        }
+        conv_finish<G, kAdd>(a, bias_s + n0 + c0, extra, p.relu != 0);
         if (c0 + c_step < nc) fetch(c0 + c_step);
-        if (live) {
-          float *dst = p.out + out_base + static_cast<int64_t>(c0) * P;
-          if (c0 + G <= nc) {
-#pragma unroll
-            for (int j = 0; j < G; ++j, dst += P) *dst = __uint_as_float(a[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < G; ++j, dst += P)
-              if (c0 + j < nc) *dst = __uint_as_float(a[j]);
-          }
-        }
+        if (live) conv_store(p.out + out_base + static_cast<int64_t>(c0) * P, a, P, nc - c0);
       }
       tc_fence_before();
       __syncwarp();

@@ -32,6 +32,7 @@
 // two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).
 #include <cuda_fp16.h>
 
+#include "conv_epilogue.cuh"
 #include "conv_plan.h"
 #include "fast_div.h"
 #include "gemm_common.cuh"
@@ -143,17 +144,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       float extra[kAdd ? G : 1];
       auto fetch = [&](int c0) __attribute__((always_inline)) {
         if constexpr (kAdd) {
-          if (live) {
-            const float *src = p.add + out_base + static_cast<int64_t>(c0) * p.P;
-            if (c0 + G <= nc) {
-#pragma unroll
-              for (int j = 0; j < G; ++j, src += p.P) extra[j] = __ldg(src);
-            } else {
-#pragma unroll
-              for (int j = 0; j < G; ++j, src += p.P)
-                if (c0 + j < nc) extra[j] = __ldg(src);
-            }
-          }
+          if (live) conv_fetch(extra, p.add + out_base + static_cast<int64_t>(c0) * p.P, p.P, nc - c0);
         }
       };
       if constexpr (kAdd) {
@@ -173,31 +164,9 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         if constexpr (G == 32) tmem_ld_32x32(addr, a);
         else tmem_ld_32x16(addr, a);
         tmem_ld_wait_regs(a);
-#pragma unroll
-        for (int j = 0; j < G; j += 4) {
-          float4 b = *reinterpret_cast<const float4 *>(bias_s + n0 + c0 + j);
-          if constexpr (kAdd) b.x += extra[j], b.y += extra[j + 1], b.z += extra[j + 2], b.w += extra[j + 3];
-          a[j] = __float_as_uint(__uint_as_float(a[j]) + b.x);
-          a[j + 1] = __float_as_uint(__uint_as_float(a[j + 1]) + b.y);
-          a[j + 2] = __float_as_uint(__uint_as_float(a[j + 2]) + b.z);
-          a[j + 3] = __float_as_uint(__uint_as_float(a[j + 3]) + b.w);
-        }
-        if (p.relu) {
-#pragma unroll
-          for (int j = 0; j < G; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
-        }
+        conv_finish<G, kAdd>(a, bias_s + n0 + c0, extra, p.relu != 0);
         if (c0 + c_step < nc) fetch(c0 + c_step);
-        if (live) {
-          float *dst = p.out + out_base + static_cast<int64_t>(c0) * p.P;
-          if (c0 + G <= nc) {
-#pragma unroll
-            for (int j = 0; j < G; ++j, dst += p.P) *dst = __uint_as_float(a[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < G; ++j, dst += p.P)
-              if (c0 + j < nc) *dst = __uint_as_float(a[j]);
-          }
-        }
+        if (live) conv_store(p.out + out_base + static_cast<int64_t>(c0) * p.P, a, p.P, nc - c0);
       }
       tc_fence_before();
       __syncwarp();
