@@ -7,20 +7,22 @@
 // fetches each input element once per tap out of L2 and hands over a stage per tap.)
 //   kCopy   conv_prepare_kernel has rewritten the input as NHWC fp16, with zeros between images; a region is one or a few
 //           tiled TMA boxes, 128 bytes a pixel, swizzled by the address, which a shifted start keeps consistent.
-//   else    few channels: twelve warps read the NCHW input and write regions by channel groups of eight,
+//   else    up to 32 channels: twelve warps read the NCHW input and write regions by channel groups of eight,
 //           [group][pixel][16 bytes], unswizzled: eight neighbouring pixels are a core matrix.  A unit is 32 pixels, dealt
-//           in turn; the next sixteen channels' loads are in flight while these are converted.  Up to eight channels make
-//           one group, and an MMA takes two taps of a filter row: the second half of its sixteen k lies as far from the
-//           first as the next tap's pixel.  The last tap of an odd row is paired with zeros, not with the pixel beyond the
-//           window: zero weights would turn an infinity there into NaN.  A sum is made in parts (halo_chain).  Strides of two keep rows and columns in classes.
-//           The filter is packed by a launch ahead; this kernel starts once that launch's own dependency is resolved and
-//           reads the input before the filter is complete.
+//           in turn; the next sixteen channels' loads are in flight while these are converted.  With a stride of two, rows
+//           and columns are kept in classes.
+//           Up to eight channels make one group, and an MMA takes two taps of a filter row: the second half of its sixteen
+//           k lies as far from the first as the next tap's pixel.  The last tap of an odd row is paired with zeros, not with
+//           the pixel beyond the window: zero weights would turn an infinity there into NaN.  Below sixteen channels a sum
+//           is made in parts (halo_chain).
+//           The filter is packed by a launch ahead, which lets this one start after its own wait: input, bias and residual,
+//           older than that launch, are read before the filter is complete.
 //   warps 0-7   epilogue: accumulator -> bias, residual, ReLU -> NCHW, alternate tiles on up to four accumulators
 //   warp 8      filter blocks of 64 k by TMA, kept for the CTA's life where they fit
 //   warp 9      MMA issuer; where a tap's pixels start is read from the constant bank
 //   warps 10-   input
 //
-// Bound: a copy's regions leave the MMAs (46 to 64 cycles each below 128 channels) or the stores, a warp's 32 pixels
+// Bound: a copy's regions leave the MMAs (42 to 58 cycles each below 128 channels) or the stores, a warp's 32 pixels
 // being four rows of a channel; straight from the input, the load / store unit: four lines to a load and to a store.
 // conv_plan.h has the times and the line to the other kernels.  Offsets computed per tap, and elections per MMA, cost 300
 // cycles a k-block: 16x32x113x91->32 7x7 134 us that way, 71 with a loop over rows and columns, 66 from the constant bank.
@@ -561,7 +563,8 @@ void launch_halo(const CUtensorMap &tx, const CUtensorMap &tw, const convh::Para
   const int rounds = (p.num_tiles + sms - 1) / sms, grid = (p.num_tiles + rounds - 1) / rounds;
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convh::threads(kCopy)), p.smem, s, 1, tx, tw, p), "launch conv_halo_kernel");
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convh::threads(kCopy)), p.smem, s, 1, tx, tw, p),
+               "launch conv_halo_kernel");
   }
   launched("conv_halo_kernel");
 }
@@ -670,7 +673,8 @@ bool conv_halo(const ConvShape &call, cudaStream_t s) {
     launched("conv_filter_kernel");
   }
   if (ok) {
-    auto launch = copy ? (p.add ? launch_halo<true, true> : launch_halo<true, false>) : (p.add ? launch_halo<false, true> : launch_halo<false, false>);
+    auto launch = copy ? (p.add ? launch_halo<true, true> : launch_halo<true, false>)
+                       : (p.add ? launch_halo<false, true> : launch_halo<false, false>);
     launch(tx, tw, p, di.sms, s);
   }
   mgpuMemFreeAsync(ws, s);

@@ -17,8 +17,8 @@
 //     thread per pixel; where k lies in the window comes from a table in shared memory.
 // The filter stays in shared memory for the CTA's life when it fits there.
 //
-// Bound: instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, 340
-// cycles where the MMAs of 64 columns take 192 (conv_plan.h says which calls conv_halo_kernel takes instead).
+// Bound: instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, about
+// 400 cycles a k-block where the MMAs of 64 columns take 193 (conv_plan.h says which calls conv_halo_kernel takes instead).
 // Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
 // changing from call to call:
 //   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  64 us (43 of HBM time)

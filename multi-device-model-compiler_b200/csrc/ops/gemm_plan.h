@@ -78,7 +78,8 @@ inline bool gemm_takes_few_rows(int64_t M, int64_t N, int64_t K, const float *w,
 //   input read value by value: 770, 500 columns 16 rows 7.0 / 6.2, 24 rows 7.1 / 7.3;  1501, 1000 columns 8 rows 8.4 / 8.0, 12 rows 8.2 / 8.4
 // Up to 8 rows the launch is worth more than what the CTAs read, up to 40000 values, or 16000 that come one by one; beyond
 // one CTA per SM each wave reads them again:
-//   1 row   2000 x 6000 27.8 / 23.6, 4736 x 14000 67.7 / 64.6;  8 rows  4096 x 5000 25.9 / 25.4 (40000), 2816 x 6000 28.9 / 29.7, 4096 x 10000 44.2 / 46.7
+//   1 row   2000 x 6000 27.8 / 23.6, 4736 x 14000 67.7 / 64.6
+//   8 rows  4096 x 5000 25.9 / 25.4 (40000 values), 2816 x 6000 28.9 / 29.7, 4096 x 10000 44.2 / 46.7
 //   by value  4 rows  1700 x 3001 18.6 / 17.4, 2816 x 7001 33.4 / 33.7;  6 rows  1700 x 3001 18.1 / 19.0;  8 rows  2000 x 3001 16.5 / 17.9
 //   two waves and more  7500 x 640 8 rows 13.0 / 11.9;  16384 x 2400 2 rows 57.0 / 55.1, 8 rows 55.9 / 56.2;  30000 x 1600 6 rows 85.2 / 89.4
 // From 9 rows to 16 the line is where one launch stops winning.  From 17 to 32 it lies below that, at 512: 32 rows at K =

@@ -61,8 +61,10 @@ inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 // front end may set the next kernel up (and start its CTAs on SMs the previous kernel has
 // already left) while the previous kernel drains; each such kernel calls pdl_wait() (device,
 // pdl.cuh) before it touches global memory, which orders it after the whole
-// previous grid.  Two kernels read weights ahead of their wait: the one-wave Gemm where the host knows them to be
-// complete (w_ready), and gemm_few_rows behind a conversion that was launched `late`.  MDC_PDL=0 turns the attribute off (plain stream order).
+// previous grid.  Three kernels read ahead of their wait.  The one-wave Gemm: weights that the host knows to be complete
+// (w_ready).  gemm_few_rows behind a conversion, and conv_halo_kernel behind the packing of its filter where it makes no copy:
+// what is older than that launch (the weight; input, bias and residual), because it triggers only after its own wait.
+// MDC_PDL=0 turns the attribute off (plain stream order).
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -37,8 +37,8 @@ __device__ __forceinline__ bool elect_one() {
 
 // The warp's number, as a value that the compiler knows to be the same in all lanes: what a branch on it
 // encloses is then code of a converged warp, with addresses and descriptors in uniform registers.  (Without
-// it an MMA loop with a wait per k-block took 350 cycles a k-block, 290 with it, where the MMAs of
-// 128 x 64 x 64 take 192.)
+// it an MMA loop with a wait per k-block took 353 cycles a k-block, 289 with it, where the MMAs of
+// 128 x 64 x 64 take 193.)
 __device__ __forceinline__ int warp_index() {
   return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
 }
@@ -139,7 +139,7 @@ __device__ __forceinline__ bool mbar_wait_all(uint64_t *bar, uint32_t parity,
 
 // A ring's next barrier, looked at without waiting ahead of this turn's MMAs or loads, and the wait itself one
 // turn later.  The round trip to the barrier then passes behind that work: a k-block of 128 x 128 x 64 took
-// 303 cycles with the wait alone, 267 with the look ahead of it (256 of MMAs).
+// 304 cycles with the wait alone, 268 with the look ahead of it (257 of MMAs).
 __device__ __forceinline__ uint32_t mbar_look(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
