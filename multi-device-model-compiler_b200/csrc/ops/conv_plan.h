@@ -316,8 +316,10 @@ inline ConvForm conv_form(const ConvShape &c, int sms, bool dense = true, HaloTi
   auto consider = [&](ConvForm form) {
     HaloTile t;
     if (!halo_tile(c, form, sms, &t)) return;
-    // the remaining kernel (conv_tcgen05.cu) is slower than either, by how much was not measured: not on mostly empty tiles
-    if (!dense && t.h.m_tiles > 2 * ((c.N * c.OH * c.OW + 127) / 128)) return;
+    // The remaining kernel (conv_tcgen05.cu) takes twice a region's time or more (2x48x1x3000->64 1x9 dilation 33 29 us / 15), so
+    // not on tiles that are mostly empty.  It packs channels without padding: where a region would pad them, its sums take
+    // more MMAs, and are further off 64 bits (17 channels 3.3e-7 against 2.3e-7).
+    if (!dense && (t.h.m_tiles > 2 * ((c.N * c.OH * c.OW + 127) / 128) || (c.IC > 16 && c.IC % 16))) return;
     const double e = halo_us(c, form, t, sms);
     if (e >= us) return;
     us = e, best = form;

@@ -234,6 +234,7 @@ REGION_FORMS = [
     ("kCopyFlat", (55, 16, 36, 78, 34, 1, 1, (2, 2), (0, 0, 0, 0), (1, 1), True, False)),  # flat: 1 x 1, sampled, two channel tiles
     ("kCopyFlat", (8, 32, 1, 8000, 32, 1, 7, (1, 1), (0, 3, 0, 3), (1, 1), False, False)),  # flat: images of one row
     ("kCopyFlat", (2, 48, 1, 3000, 20, 1, 9, (1, 1), (0, 130, 0, 132), (1, 33), True, False)),  # flat: taps beyond the im2col map's offsets
+    ("kOther", (2, 40, 1, 3000, 20, 1, 9, (1, 1), (0, 130, 0, 132), (1, 33), True, False)),  # the same, channels that a region would pad: direct kernel
     ("kOther", (6, 48, 1, 70, 20, 1, 9, (1, 1), (0, 132, 0, 132), (1, 33), True, False)),  # the same on tiles of mostly margins: direct kernel
     ("kDirectRect", (56, 3, 11, 32, 11, 5, 5, (1, 1), (2, 2, 2, 2), (1, 1), True, True)),  # straight: a tap without a partner, several tiles per CTA, residual
     ("kDirectRect", (74, 3, 29, 38, 8, 5, 5, (2, 2), (2, 2, 2, 2), (1, 1), False, True)),  # straight: classes of rows and columns, filter kept
