@@ -69,6 +69,39 @@ __device__ __forceinline__ void store_out16(TOut *dst, const float *v, bool seco
     st_global_32B(dst, q);
   }
 }
+// 32 values of each lane's row (rows of a warp consecutive, row's parity the lane's; gcol a multiple of 32) as TOut, for rows of
+// whole 32-byte sectors: two lanes exchange 32 bytes each and store 64 bytes of one row, then of the other.  Called by a
+// whole warp.
+// What bounds a large Gemm's stores is the SM's port to L2, which operands share: stores of one sector a lane leave it at
+// 20 bytes a cycle, and operands, which need 64, at 15 to 40 meanwhile; sectors in pairs go at 32 (a stand-alone probe of
+// eight storing warps beside bulk loads; whole lines are no faster).
+template <typename TOut>
+__device__ __forceinline__ void store_row_pairs(TOut *out, const float *v, int row, int M, int gcol, int N) {
+  constexpr int PER = 64 / static_cast<int>(sizeof(TOut));  // values of 64 bytes
+  const bool odd = threadIdx.x & 1;
+  const int even_row = row & ~1;
+#pragma unroll
+  for (int g = 0; g < 32; g += PER) {
+    uint32_t q[16], first[8], second[8];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if constexpr (sizeof(TOut) == 4) q[i] = __float_as_uint(v[g + i]);
+      else q[i] = pack_pair<TOut>(v[2 * i], v[2 * i + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? q[i] : q[8 + i], 1);
+      first[i] = odd ? got : q[i];       // of the even lane's row
+      second[i] = odd ? q[8 + i] : got;  // of the odd lane's
+    }
+    const int col = gcol + g + (odd ? PER / 2 : 0);
+    if (col < N) {
+      TOut *dst = out + static_cast<size_t>(even_row) * N + col;
+      if (even_row < M) st_global_32B(dst, first);
+      if (even_row + 1 < M) st_global_32B(dst + N, second);
+    }
+  }
+}
 // 8 values of a row as TOut; dst is 16-byte aligned
 template <typename TOut>
 __device__ __forceinline__ void store_out8(TOut *dst, const float *v) {
@@ -128,12 +161,18 @@ __device__ __forceinline__ void store_row(TOut *out, const float *v, int cols, b
 // up with it; its scarce resource is the special-function unit (16 results per clock and SM,
 // shared with the 16-bit conversions).  The exact-erf GELU therefore uses ONE special-function
 // operation per element:
-//   gelu(v) = max(v, 0) - 0.5 |v| erfc(|v| / sqrt 2),     erfc(t) = 2^P(t),
-// P a degree-8 polynomial fitted (minimax, t in [0, 5.7]) to log2(erfc(t)); beyond 5.7 the
-// erfc term is below 1e-15 |v| and t is clamped.  Against the double-precision erf form the
-// result is within 1e-6 absolute and 1.1e-5 relative over [-12, 12] (fp32 evaluation), 50 times
-// below the rounding of a 16-bit output.  (The rational form of Abramowitz & Stegun 7.1.26 used
-// before needs a reciprocal as well as an exponential.)
+//   gelu(v) = max(v, 0) + h Phi(h),     h = max(-|v|, -8.06),     Phi(h) = 2^P(h),
+// P a degree-8 polynomial fitted to log2(Phi), by its largest error weighted between the relative error of Phi and
+// the absolute one of h Phi(h); beyond -8.06 h Phi(h) is below 4e-15.  A NaN stays one by the first term.  Against the double-precision erf form the result is within
+// 8e-7 absolute and 1.3e-5 relative over [-8, 12] (fp32 evaluation), 50 times below the rounding of a 16-bit output; in the
+// 2-norm 6.6e-7 for N(0, 1) arguments.  (The same fit to erfc(|v| / sqrt 2) with its factors 1/2 and 1/sqrt 2 applied
+// outside took 22 instructions a pair instead of 16 and was within 9.5e-7 / 1.4e-5 / 7.4e-7; the rational form of Abramowitz &
+// Stegun 7.1.26 used before that needs a reciprocal as well as an exponential.)
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ float ex2_approx(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -147,28 +186,26 @@ using ptx::f2_get;
 using ptx::f2_mul;
 
 __device__ __forceinline__ void gelu_erf_pair(float &va, float &vb) {
-  const float aa = fabsf(va), ab = fabsf(vb);
-  const F2 T = f2(fminf(aa * 0.70710678f, 5.7f), fminf(ab * 0.70710678f, 5.7f));
+  const F2 T = f2(fmaxf(-fabsf(va), -8.0610172f), fmaxf(-fabsf(vb), -8.0610172f));
 #define MDC_C2(x) f2(x, x)
-  F2 P = f2_fma(MDC_C2(1.1948015981033677e-06f), T, MDC_C2(-4.147788058617152e-05f));
-  P = f2_fma(P, T, MDC_C2(0.0006375535158440471f));
-  P = f2_fma(P, T, MDC_C2(-0.005785022862255573f));
-  P = f2_fma(P, T, MDC_C2(0.03505704924464226f));
-  P = f2_fma(P, T, MDC_C2(-0.1536988914012909f));
-  P = f2_fma(P, T, MDC_C2(-0.9163860082626343f));
-  P = f2_fma(P, T, MDC_C2(-1.628216028213501f));
-  P = f2_fma(P, T, MDC_C2(7.682551768084522e-06f));
+  F2 P = f2_fma(MDC_C2(6.983426459328257e-08f), T, MDC_C2(3.5143536933901487e-06f));
+  P = f2_fma(P, T, MDC_C2(7.777412247378379e-05f));
+  P = f2_fma(P, T, MDC_C2(0.001010141335427761f));
+  P = f2_fma(P, T, MDC_C2(0.008719745092093945f));
+  P = f2_fma(P, T, MDC_C2(0.05425671488046646f));
+  P = f2_fma(P, T, MDC_C2(-0.45826849341392517f));
+  P = f2_fma(P, T, MDC_C2(1.1512970924377441f));
+  P = f2_fma(P, T, MDC_C2(-0.9999945163726807f));
 #undef MDC_C2
   float pa, pb;
   f2_get(P, pa, pb);
-  const F2 E = f2(ex2_approx(pa), ex2_approx(pb));
-  const F2 G = f2_fma(f2(-0.5f * aa, -0.5f * ab), E, f2(fmaxf(va, 0.f), fmaxf(vb, 0.f)));
+  const F2 G = f2_fma(T, f2(ex2_approx(pa), ex2_approx(pb)), f2(max_nan(va, 0.f), max_nan(vb, 0.f)));
   f2_get(G, va, vb);
 }
 
 // Applies the activation to n (even) values in place.  For rows that are stored in vectors, where the
 // epilogue has to keep up with the mainloop; ragged rows, which do not, take act_apply_t: 3.7e-8
-// relative (2-norm, N(0, 1) arguments) instead of 7.3e-7.
+// relative (2-norm, N(0, 1) arguments) instead of 6.6e-7.
 template <int ACT, int N>
 __device__ __forceinline__ void act_fast_n(float *v) {
   if constexpr (ACT == kActGeluErf) {

@@ -14,9 +14,14 @@
 //   warps 2-9 epilogue: tcgen05.ld the 128 x 256 fp32 accumulator out of TMEM (each warp
 //            its 32-lane quarter, two warps per quarter splitting the columns), add bias,
 //            apply the activation, add the residual, convert and store.  Two forms (kWide):
-//            Rows that can be moved 32 bytes at a time: a thread owns a row and moves a whole
-//            sector per access, so nothing is staged.  The ring has two more stages, and the
-//            residual is fetched before the accumulator is waited for instead of after.
+//            Rows that can be moved 32 bytes at a time: a thread owns a row, and two threads store
+//            64 bytes of each other's (store_row_pairs), so nothing is staged.  The ring has two
+//            more stages, and the residual and the bias are fetched before the accumulator is waited for.
+//            A short K is bound by this epilogue: with sectors stored one by one, the bias loaded a
+//            tile late and the residual piece by piece it took 6940 cycles a tile, 10900 with residual,
+//            beside 6144 of MMAs at K = 768; 32768 x 2304 x 768 97.9 -> 94.2 us, 32768 x 768 x 768 with
+//            residual 46.1 -> 44.1, 12288 x 768 x 768 19.0 -> 16.2.  (Stores spread over the mainloop by the
+//            clock: no gain.  16 epilogue warps: 8 us slower at 32768 x 3072 x 768 with GELU.)
 //            Rows of other multiples of 16 bytes (N = 8 mod 16, or a pointer off its 32-byte
 //            boundary): each warp stages 32 rows x 128 bytes in swizzled shared memory and moves
 //            it with one TMA store, the residual arrives by a TMA load, and 96 KiB of the ring go
@@ -257,9 +262,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // the accumulator is handed back to the leader's MMA thread, in whichever CTA it lives
     const uint32_t acc_empty_addr0 = mapa_u32(smem_u32(&acc_empty_bar[0]), 0);
     const uint32_t acc_empty_addr1 = mapa_u32(smem_u32(&acc_empty_bar[1]), 0);
+    const int half_cols = bn / 2;
+    [[maybe_unused]] constexpr int MAX_SUBS = BN / 2 / 32;
+    // pieces of the residual in flight; the GELUs' code is too long to be written out four times (4096 x 3072 x 768 22.1 -> 23.7 us)
+    [[maybe_unused]] constexpr int RES_AHEAD = ACT == kActNone || ACT == kActRelu ? MAX_SUBS : 1;
+    // four bias values of a tile's columns (zeros beyond N), for the whole warp's row of them
+    [[maybe_unused]] auto load_bias = [&](int t) __attribute__((always_inline)) -> float4 {
+      const int c = (t % p.num_n_blocks) * bn + half_sel * half_cols + lane * 4;
+      return t < num_tiles && c < p.N ? __ldg(reinterpret_cast<const float4 *>(p.bias + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    [[maybe_unused]] float4 next_bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (kWide) {
+      if (p.bias) next_bias = load_bias(worker);
+    }
     for (int tile = worker; tile < num_tiles; tile += num_workers) {
       const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
-      const int half_cols = bn / 2;
       const int row = m_blk * BM + quarter * 32 + lane;
       const bool row_ok = row < p.M;
       const int gcol_base = n_blk * bn + half_sel * half_cols;
@@ -276,34 +293,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         return done;
       };
       if constexpr (kWide) {
-        // The warp owns 32 rows x half_cols accumulator columns, read from tensor memory in
-        // pieces of 32; the next piece's accumulator and residual loads are in flight while this
-        // one goes through bias / activation / residual.
-        // Bias and the first residual piece are fetched before the accumulator is waited for.
+        // The warp owns 32 rows x half_cols accumulator columns, read from tensor memory in pieces of 32; the
+        // next piece's load is in flight while this one goes through bias / activation / residual.  All of the
+        // tile's residual is requested before the accumulator is waited for, and its bias a tile earlier.
         const size_t row_off = static_cast<size_t>(row) * p.N + gcol_base;
         uint32_t raw[32];
-        uint32_t rr[16];
-        auto fetch_res = [&](int sub) __attribute__((always_inline)) {
-          if (res && row_ok) {
-            ld_global_32B(res + row_off + sub * 32, rr);
-            if (gcol_base + sub * 32 + 16 < p.N) ld_global_32B(res + row_off + sub * 32 + 16, rr + 8);
+        uint32_t rr[RES_AHEAD][16];
+        auto fetch_res = [&](int sub, uint32_t *r) __attribute__((always_inline)) {
+          if (res && row_ok && sub < n_sub) {
+            ld_global_32B(res + row_off + sub * 32, r);
+            if (gcol_base + sub * 32 + 16 < p.N) ld_global_32B(res + row_off + sub * 32 + 16, r + 8);
           }
         };
-        if (n_sub > 0) fetch_res(0);
-        if (p.bias) {
-          const int c = gcol_base + lane * 4;
-          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (c < p.N) b = __ldg(reinterpret_cast<const float4 *>(p.bias + c));
-          __syncwarp();  // the previous tile's values have been read
-          *reinterpret_cast<float4 *>(&bias_s[ew][lane * 4]) = b;
-          __syncwarp();
-        }
+#pragma unroll
+        for (int sub = 0; sub < RES_AHEAD; ++sub) fetch_res(sub, rr[sub]);
         if (!wait_acc()) break;
         if (n_sub > 0) tmem_ld_32x32(t_base, raw);
-#pragma unroll 1
-        for (int sub = 0; sub < n_sub; ++sub) {
+        if (p.bias) {
+          __syncwarp();  // the previous tile's values have been read
+          *reinterpret_cast<float4 *>(&bias_s[ew][lane * 4]) = next_bias;
+          __syncwarp();
+          next_bias = load_bias(tile + num_workers);
+        }
+        auto piece = [&](int sub, uint32_t *r) __attribute__((always_inline)) {
           const int gcol = gcol_base + sub * 32;
-          const bool second = gcol + 16 < p.N;
           tmem_ld_wait_regs(raw);
           float v[32];
 #pragma unroll
@@ -321,17 +334,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               float rv[8];
-              unpack_res8<T16>(rr + j / 2, rv);
+              unpack_res8<T16>(r + j / 2, rv);
 #pragma unroll
               for (int e = 0; e < 8; ++e) v[j + e] += rv[e];
             }
-            if (sub + 1 < n_sub) fetch_res(sub + 1);
+            if constexpr (RES_AHEAD == 1) fetch_res(sub + 1, r);
           }
-          if (row_ok) {
-            TOut *dst = out + row_off + sub * 32;
-            store_out16<TOut>(dst, v, gcol + 8 < p.N);
-            if (second) store_out16<TOut>(dst + 16, v + 16, gcol + 24 < p.N);
-          }
+          store_row_pairs<TOut>(out, v, row, p.M, gcol, p.N);
+        };
+        if constexpr (RES_AHEAD == MAX_SUBS) {
+#pragma unroll
+          for (int sub = 0; sub < MAX_SUBS; ++sub)
+            if (sub < n_sub) piece(sub, rr[sub]);
+        } else {
+#pragma unroll 1
+          for (int sub = 0; sub < n_sub; ++sub) piece(sub, rr[0]);
         }
       } else if (p.rows.fast) {
         // ---- staged rows.  Output leaves in chunks of cw columns: swizzled buffer -> one TMA store ----

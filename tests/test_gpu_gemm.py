@@ -262,6 +262,56 @@ def test_row_alignments_are_exact(m, M, N, offsets):
         assert np.array_equal(_matmul16_at(m, a, w, b, r, out_dtype, m.ACT_RELU, oo, ro, bo), ref)
 
 
+@pytest.mark.parametrize("act", [0, 1, 2])
+@pytest.mark.parametrize("M,N", [(19001, 16), (19001, 48), (6001, 400), (2499, 2064), (129, 19264)])
+def test_rows_stored_in_pairs_are_exact(m, M, N, act):
+    # whole-sector rows of the persistent kernel: two lanes store two rows, the last of which may be missing, in pieces of
+    # 32 columns, the last of which may hold 16; the residual may be the output itself.  Small integers; GELU of values
+    # from 10 is the value itself, and the residual shows what it was added to
+    rng = np.random.default_rng(23)
+    K = 64
+    a, w = rng.integers(0, 4, (M, K)).astype(np.float32), rng.integers(0, 3, (K, N)).astype(np.float32)
+    b, r = 10 + rng.integers(0, 5, N).astype(np.float32), rng.integers(-8, 9, (M, N)).astype(np.float32)
+    ref = a @ w + b + r
+    for out_dtype in (m.F16, m.F32):
+        assert np.array_equal(_matmul16_at(m, a, w, b, r, out_dtype, act), ref)
+    da, dw, db, do = m.to_device(a.astype(np.float16)), m.to_device(w), m.to_device(b), m.to_device(r.astype(np.float16))
+    dwp = m.DeviceBuffer(N * K * 2)
+    m.ops().mgpuPackWeight(dw.ptr, dwp.ptr, K, N, m.F16, None)
+    m.ops().mgpuMatmulEx16(da.ptr, dwp.ptr, db.ptr, do.ptr, do.ptr, M, N, K, m.F16, m.F16, act, None)
+    assert np.array_equal(m.to_host(do, (M, N), np.float16).astype(np.float32), ref)
+
+
+@pytest.mark.parametrize("M", [70, 19200])
+def test_gelu_of_vector_rows(m, M):
+    # the fitted form, one wave and persistent: A . W is one fp16 value.  The fit is within 8e-7 absolute and 1.3e-5
+    # relative (from -8 on; its exponent, up to 50 in 24 bits, brings another 2e-6 there, and ex2.approx 2^-22), and 6.6e-7
+    # in the 2-norm of N(0, 1) arguments, to which fp32 rounding adds 1e-7
+    from math import erfc
+    gelu = np.vectorize(lambda t: 0.5 * t * erfc(-t / np.sqrt(2.0)))  # (1 + erf loses digits from -4 on)
+    rng = np.random.default_rng(47)
+    N = 64
+    for v, whole in ((rng.standard_normal(M), True), (rng.uniform(-8, 12, M), False)):
+        v = v.astype(np.float16)
+        v[:3] = 0, -0.0, 6e4
+        a, w = np.zeros((M, 64), np.float16), np.zeros((64, N), np.float32)
+        a[:, 0], w[0] = v, 1
+        a[5, 1], b = np.nan, np.zeros(N, np.float32)
+        b[-1] = np.inf
+        da, dw, db, do, dwp = m.to_device(a), m.to_device(w), m.to_device(b), m.DeviceBuffer(M * N * 4), m.DeviceBuffer(N * 64 * 2)
+        m.ops().mgpuPackWeight(dw.ptr, dwp.ptr, 64, N, m.F16, None)
+        m.ops().mgpuMatmulEx16(da.ptr, dwp.ptr, db.ptr, None, do.ptr, M, N, 64, m.F16, m.F32, m.ACT_GELU_ERF, None)
+        got = m.to_host(do, (M, N), np.float32)
+        m.check("mgpuMatmulEx16")
+        assert np.isnan(got[5]).all()
+        got, ref = np.delete(got, 5, 0), np.repeat(gelu(np.delete(v, 5).astype(np.float64))[:, None], N - 1, axis=1)
+        assert np.all(np.isposinf(got[:, -1]))
+        err = np.abs(got[:, :-1] - ref)
+        assert np.all(err <= np.minimum(8e-7 + 1.2e-7 * np.abs(ref), 1.6e-5 * np.abs(ref)))
+        if whole and M > 10000:  # (of 66 values it depends on which: at most 8e-7 over their rms of 0.6, which the line above says)
+            assert np.linalg.norm(err[3:]) <= 7.6e-7 * np.linalg.norm(ref[3:])
+
+
 @pytest.mark.parametrize("N,offsets", [(1000, (0, 0, 0)), (768, (16, 0, 0)), (768, (0, 16, 0))])
 def test_rows_of_16_byte_multiples_are_not_slow(m, N, offsets):
     # against the next width of whole sectors: up to 1.3 times its time, 4 to 10 times when such rows
