@@ -14,12 +14,15 @@
 //     instruction per operand where K is a multiple of 64), and the ring is as deep as shared memory
 //     allows: a short K range is in flight as a whole and costs one memory latency;
 //   * A's box is as high as M needs; accumulator rows beyond it hold stale operands and are not
-//     stored;
+//     stored.  Up to 64 rows the MMA has M = 64: 25 cycles for up to 32 columns instead of 40, which a long K is bound by
+//     (99 x 768 x 3072 8.9 -> 6.9 us in a chain of launches, 512 x 768 x 3072 10.6 -> 8.4);
+//   * the first piece of the bias and the residual is fetched while the mainloop runs;
 //   * W's first stages are requested before the dependency on the previous kernel is resolved
 //     when the caller knows the weights to be complete;
 //   * results go straight from registers to global memory, 32 bytes per access.  Rows that are not
 //     aligned to that, and a K that is no multiple of 64, are left to a variant of their own (kWide =
 //     false): as run-time branches they took 2 to 3 % of a 12-layer pass over 99 tokens.
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -43,7 +46,7 @@ struct OneWaveParams {
   void *out;
   RowAccess rows;
   int n_tiles;  // column tiles
-  int bn, box_m, depth, stages;
+  int bn, box_m, mma_m, depth, stages;
   int tmem_cols;
   int k_in_x;   // operand maps are (k, row) instead of (64 k, row, k-block)
   int w_ready;  // W may be read before the dependency wait
@@ -163,7 +166,7 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader of the pair) ------------------------------
     if (leader) {
-      const uint32_t idesc = make_idesc_f16(128 * CG, static_cast<uint32_t>(p.bn), std::is_same<T16, __nv_bfloat16>::value,
+      const uint32_t idesc = make_idesc_f16(static_cast<uint32_t>(p.mma_m * CG), static_cast<uint32_t>(p.bn), std::is_same<T16, __nv_bfloat16>::value,
                                             false, false);
       const KblockDesc desc0 = kblock_desc(make_smem_desc_sw128(smem_u32(tiles), 16, 1024),
                                            make_smem_desc_sw128(smem_u32(tiles) + static_cast<uint32_t>(a_bytes), 16, 1024));
@@ -212,32 +215,19 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   // half of the warps takes the first half of the pieces, rounded up
   const int c_mid = (p.bn / 16 + 1) / 2 * 16;
   const int c_begin = half_sel ? c_mid : 0, c_end = half_sel ? p.bn : c_mid;
-  const int rows_in_tile = quarter * 32 + lane;
-  const bool live_warp = warp >= 2 && quarter * 32 < p.box_m;  // box_m is a multiple of 32
-  bool ok = true;
-  if (live_warp) {
-    if (!mbar_wait_warp(&acc_bar, 0, abort_flag)) {
-      if (lane == 0) atomicCAS(p.err, 0u, 0x83000000u);
-      ok = false;
-    }
-    tc_fence_after();
-  }
-  const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-  if (live_warp && ok) {
+  // an accumulator of 128 rows has 32 in each quarter of the lanes, one of 64 rows 16
+  const int q_rows = p.mma_m / 4;
+  const int rows_in_tile = quarter * q_rows + lane;
+  if (warp >= 2 && quarter * q_rows < p.box_m) {
+    constexpr int NC = 16;
     TOut *out = static_cast<TOut *>(p.out);
     const T16 *res = static_cast<const T16 *>(p.residual);
     const int row = row0 + rows_in_tile;
-    const bool row_ok = row < p.M;
-#pragma unroll 1
-    for (int c = c_begin; c < c_end; c += 16) {
-      constexpr int NC = 16;
-      const int gcol = col0 + c;
-      if (gcol >= p.N) break;  // uniform across the warp
-      uint32_t acc[NC];
-      tmem_ld_32x16(t_lane + static_cast<uint32_t>(c), acc);
-      const size_t off = static_cast<size_t>(row) * p.N + gcol;
-      const int cols = p.N - gcol;
-      float v[NC], rv[NC];  // bias, then the result; residual
+    const bool row_ok = lane < q_rows && rows_in_tile < p.box_m && row < p.M;
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    float v[NC], rv[NC];  // bias, then the result; residual
+    auto fetch = [&](int c) __attribute__((always_inline)) {
+      const int gcol = col0 + c, cols = p.N - gcol;
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] = rv[j] = 0.f;
       if (p.bias) {
@@ -256,15 +246,36 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         }
       }
       if (res && row_ok) {
+        const size_t off = static_cast<size_t>(row) * p.N + gcol;
         if constexpr (kWide) {
-          uint32_t rr[NC / 2];
-          ld_global_32B(res + off, rr);
+          if (cols > 0) {
+            uint32_t rr[NC / 2];
+            ld_global_32B(res + off, rr);
 #pragma unroll
-          for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
+            for (int j = 0; j < NC; j += 8) unpack_res8<T16>(rr + j / 2, rv + j);
+          }
         } else {
           load_row<T16, NC>(res + off, rv, cols, p.rows.vec);
         }
       }
+    };
+    // the first piece's bias and residual come while the mainloop runs
+    if (c_begin < c_end) fetch(c_begin);
+    bool ok = true;
+    if (!mbar_wait_warp(&acc_bar, 0, abort_flag)) {
+      if (lane == 0) atomicCAS(p.err, 0u, 0x83000000u);
+      ok = false;
+    }
+    tc_fence_after();
+#pragma unroll 1
+    for (int c = c_begin; ok && c < c_end; c += NC) {
+      const int gcol = col0 + c;
+      if (gcol >= p.N) break;  // uniform across the warp
+      uint32_t acc[NC];
+      tmem_ld_32x16(t_lane + static_cast<uint32_t>(c), acc);
+      if (c != c_begin) fetch(c);
+      const size_t off = static_cast<size_t>(row) * p.N + gcol;
+      const int cols = p.N - gcol;
       tmem_ld_wait_regs(acc);
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] += __uint_as_float(acc[j]);
@@ -371,7 +382,7 @@ void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, co
   p.bias = bias, p.residual = residual, p.out = out;
   p.rows = row_access(N, out, dtype_size(out_dtype), residual, bias);
   p.n_tiles = static_cast<int>((N + t.bn - 1) / t.bn);
-  p.bn = t.bn, p.box_m = t.box_m, p.stages = t.stages;
+  p.bn = t.bn, p.box_m = t.box_m, p.mma_m = t.mma_m, p.stages = t.stages;
   p.depth = t.depth;
   p.tmem_cols = 32;
   while (p.tmem_cols < t.bn) p.tmem_cols *= 2;
@@ -380,10 +391,12 @@ void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, co
   const int64_t m_tiles = (M + static_cast<int64_t>(t.box_m) * t.cg - 1) / (static_cast<int64_t>(t.box_m) * t.cg);
   const int grid = static_cast<int>(m_tiles * p.n_tiles * t.cg);
   const size_t stage = static_cast<size_t>(p.depth) * (t.box_m + t.bn / t.cg) * onewave::BK * 2;
-  // an MMA reads 128 rows of A whatever the box holds: past the last box that must still be this
+  // an MMA reads mma_m rows of A whatever the box holds: past the last box that must still be this
   // CTA's memory
-  const size_t ring = stage * t.stages + (t.box_m < 128 ? (128 - t.box_m) * onewave::BK * 2 : 0);
-  const size_t smem = ring + 1024;
+  const size_t ring = stage * t.stages + (t.mma_m - t.box_m) * onewave::BK * 2;
+  // never less than half of an SM's: two CTAs on one SM, of this launch or of the next, take turns at the SM's port while
+  // others idle (2337 x 256 x 256 4.1 -> 3.5 us, 1592 x 704 x 256 4.7 -> 4.0, 99 x 768 x 768 3.44 -> 3.30; nothing loses 2 %)
+  const size_t smem = std::max<size_t>(ring + 1024, 117 * 1024);
   if (dtype == MGPU_DTYPE_F16) {
     if (out_dtype == MGPU_DTYPE_F16) launch_one_wave_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
     else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);

@@ -12,7 +12,8 @@ namespace mdc {
 struct GemmTile {
   bool one_wave = false;  // gemm_one_wave_kernel; otherwise the persistent kernel of gemm_tcgen05.cu
   int cg = 2;             // CTAs per tile (2 = tcgen05 CTA pair)
-  int box_m = 128;        // rows of A per CTA
+  int box_m = 128;        // rows of A per CTA, a multiple of 8
+  int mma_m = 128;        // rows of its accumulator: 64 or 128
   int bn = 256;           // output columns per tile
   int depth = 1;          // 64-wide k-blocks per ring stage
   int stages = 4;

@@ -43,6 +43,7 @@
 // Measured, 12-layer step of 256 x 128 tokens (hidden 768): 7.38 ms with the one-lane loops and the
 // staged epilogue on 4 stages; whole-warp loops and direct stores 7.15 (4 stages); bias out of L1
 // 6.95 (4 stages), 6.89 (5), 6.88 (6); 7 stages leave L1 too small for the residual: 7.05.
+#include <cmath>
 #include <cstdlib>
 #include <type_traits>
 
@@ -624,35 +625,47 @@ static int choose_bn(int64_t M, int64_t N, int cta_group, int sms) {
   return best;
 }
 
-// Time of a one-wave tile in microseconds, at most one CTA per SM.  Terms: launch and drain; MMA issue;
-// operand bytes through the SM's load path; one barrier hand-over per ring stage; epilogue columns;
-// pairing; CTAs to place.  Fitted to 1700 measured (shape, tile) pairs (M 32 - 4096, N 768 - 4096, K 768
-// - 4096, weights from HBM, chained launches; 14 % rms), an extrapolation elsewhere: over 140 random
-// calls (M 1 - 40000, N and K 8 - 5000) none took 8 % longer than with the persistent kernel for all.
+// A figure of merit of a one-wave tile, near its time in microseconds, at most one CTA per SM.  Terms: launch and drain;
+// MMAs; operand bytes through the SM's load path; one barrier hand-over per ring stage; epilogue columns; CTAs to place;
+// pairing.  An MMA takes half a cycle per column, but no less than it needs to read A and to start: 25 cycles for 64 rows
+// and 16 to 32 columns, 40 for 128 rows (measured; a few rows are therefore cut into tiles of 64).  The weights are those
+// whose choice was best over 770 shapes and all their tiles (M 16 - 4096, N 256 - 4096, K 256 - 4096, weights from HBM,
+// dependent launches in a graph); on 300 others it takes 1.007 of the time of the best tile on average, 1.04 in 19
+// of 20.
 static float one_wave_cost(const GemmTile &t, int64_t M, int64_t N, int num_kb, int sms) {
   const int64_t m_tiles = (M + t.box_m * t.cg - 1) / (t.box_m * t.cg), n_tiles = (N + t.bn - 1) / t.bn;
   const int64_t ctas = m_tiles * n_tiles * t.cg;
   if (ctas > sms) return 1e30f;
   const int steps = (num_kb + t.depth - 1) / t.depth;
   const int rows = M < t.box_m ? static_cast<int>(M) : t.box_m;
-  const float mma = num_kb * (t.bn < 100 ? 200.f : 2.f * t.bn) / 1900.f;
-  const float bytes = num_kb * static_cast<float>(rows + t.bn / t.cg) * 128.f / 1e5f;
-  float us = 2.2f + 0.33f * mma + 0.305f * bytes + 0.194f * steps + 0.0125f * t.bn +
-             0.65f * static_cast<float>(ctas) / static_cast<float>(sms);
-  if (t.cg == 2) us += 1.2f;
+  const float bn = static_cast<float>(t.bn);
+  const float start = t.cg == 2 ? 35.f + 0.15f * bn : t.mma_m == 64 ? 21.7f + 0.17f * bn : 31.5f + 0.25f * bn;
+  const float mma = num_kb * 4 * fmaxf(start, 0.5f * bn) / 1900.f;
+  const float bytes = steps * t.depth * static_cast<float>(rows + t.bn / t.cg) * 128.f / 1e5f;  // (a stage is filled whole)
+  float us = 2.55f + 2.38f * mma + 0.282f * bytes + 0.118f * steps + 0.00855f * bn +
+             0.836f * static_cast<float>(ctas) / static_cast<float>(sms);
+  if (t.cg == 2) us += 2.38f;
   return us;
 }
 
 // The fastest one-wave tile for a problem of at most one 128 x 128 tile per SM.
-static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
+static GemmTile choose_one_wave(int64_t M, int64_t N, int64_t K, int sms) {
+  const int num_kb = static_cast<int>((K + 63) / 64);
   GemmTile best;
   float best_us = 1e30f;
   for (int cg = 1; cg <= 2; ++cg)
-    for (int box_m : {32, 64, 128}) {
-      if (box_m < 128 && (cg == 2 || M > 640)) continue;  // short boxes only pay for few rows
-      if (box_m > 32 && box_m >= 2 * M) continue;
+    for (int most : {32, 64, 128}) {
+      if (most < 128 && cg == 2) continue;
+      if (most > 32 && most >= 2 * M) continue;
+      // Boxes as high as an equal share of the rows, in whole swizzle groups: rows out of bounds are slow to fill (75 x 2304 x 768 in
+      // tiles of 64 and 11 rows 4.9 us, in two of 40 3.7).
+      const int64_t shares = (M + most * cg - 1) / (most * cg) * cg;
+      const int box_m = static_cast<int>(((M + shares - 1) / shares + 7) / 8 * 8), mma_m = cg == 1 && box_m <= 64 ? 64 : 128;
       for (int bn : {16, 32, 48, 64, 96, 128, 192, 256}) {
         if (cg == 2 && bn < 64) continue;
+        // k-blocks that come one box at a time: 16 columns a box lose (51 x 2264 x 1528 7.5 us, with 32 columns 6.2; 18 x 2280 x
+        // 1424 6.3 and 5.3; 160 shapes 1.044 of the best tile's time on average with them, 1.033 without)
+        if (bn == 16 && K % 64) continue;
         for (int depth : {4, 2, 1}) {
           if (depth > num_kb) continue;
           const int steps = (num_kb + depth - 1) / depth, stage = depth * (box_m + bn / cg) * 128;
@@ -661,12 +674,12 @@ static GemmTile choose_one_wave(int64_t M, int64_t N, int num_kb, int sms) {
           // this one, loses more than that overlap wins: 2048 x 1024 x 4096 31.7 -> 22.0 us,
           // 1000 x 1024 x 4096 25.8 -> 18.0, 99 x 768 x 3072 11.7 -> 10.5; a 12-layer pass over 99 tokens,
           // where every kernel is of this kind, 501 -> 450 us.
-          int stages = (220 * 1024 - (128 - box_m) * 128) / stage;
+          int stages = (220 * 1024 - (mma_m - box_m) * 128) / stage;
           if (stages > steps) stages = steps;
           if (stages > 16) stages = 16;
           if (stages < 1 || (stages < 2 && steps > 1)) continue;
           GemmTile t;
-          t.one_wave = true, t.cg = cg, t.box_m = box_m, t.bn = bn, t.depth = depth, t.stages = stages;
+          t.one_wave = true, t.cg = cg, t.box_m = box_m, t.mma_m = mma_m, t.bn = bn, t.depth = depth, t.stages = stages;
           const float us = one_wave_cost(t, M, N, num_kb, sms);
           if (us < best_us) best_us = us, best = t;
         }
@@ -692,7 +705,7 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   // 4096 x 768 x 3072 19.2 and 17.6.
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
-    t = choose_one_wave(M, N, static_cast<int>((K + 63) / 64), sms);
+    t = choose_one_wave(M, N, K, sms);
   if (!t.one_wave) {
     t.cg = choose_cta_group(M);
     t.bn = choose_bn(M, N, t.cg, sms);

@@ -151,6 +151,21 @@ def test_one_wave_tiles_are_exact(m, M, N, K):
     assert np.array_equal(m.matmul16(a, w, bias=b, residual=r, out_dtype=m.F32, act=m.ACT_RELU), np.maximum(ref, 0) + r)
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (8, 64, 256), (17, 768, 264), (64, 768, 768), (71, 2304, 768), (129, 768, 3072), (200, 2304, 512),  # boxes of 8 to 64 rows, one tile or several
+    (86, 1288, 520), (341, 424, 280), (456, 3136, 256), (1592, 704, 256),  # ragged K, 65 to 128 rows, less than half of the shared memory
+    (1375, 1024, 1024), (1101, 1040, 1096)])  # CTA pairs
+def test_one_wave_shares_of_rows_are_exact(m, M, N, K):
+    # tiles of an equal share of the rows, with accumulators of 64 or 128 rows of which only the box's are stored: exact on
+    # small integers, and nothing beside the result is written
+    rng = np.random.default_rng(13)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b, r = rng.integers(-4, 5, N).astype(np.float32), rng.integers(-8, 9, (M, N)).astype(np.float32)
+    ref = np.maximum(a @ w + b, 0) + r
+    assert np.array_equal(_matmul16_at(m, a, w, b, r, m.F32, m.ACT_RELU), ref)
+    assert np.array_equal(_matmul16_at(m, a, w, b, r, m.F16, m.ACT_RELU), ref.astype(np.float16).astype(np.float32))
+
+
 @pytest.mark.parametrize("bn", ["192", "128"])
 def test_forced_tile_width(bn):
     # every shape of this file again with the tile width forced (read once per process)
