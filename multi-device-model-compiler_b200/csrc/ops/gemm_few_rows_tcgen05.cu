@@ -10,9 +10,11 @@
 // few_rows_convert) eight more warps read and round it here instead, and there is no launch ahead: 16 x 768 x 768 6.9 ->
 // 5.1 us a call, 16 x 256 x 256 6.8 -> 4.1.
 //
-// Whole call, with the weight converted and read here: 16 x 1000 x 2048 12.2 / 10.8 us one after another out of L2,
-// 13.3 / 13.6 out of memory; out of memory also 16 x 4096 x 4096 30.3 / 23.6 (2.8 TB/s), 16 x 1000 x 512 7.4 / 6.0;
-// more of them in gemm_plan.h.
+// The accumulator has 64 rows: an MMA of 128 rows and 16 or 32 columns takes 40 cycles, one of 64 rows 25.  A's box is as high
+// as there are rows, and the ring leaves L1 to the loads in flight (RING_SMEM).  Whole calls out of memory, with 128 rows, boxes of
+// 32 or 64 and a ring of 220 KB / now: 16 x 1000 x 2048 12.6 / 8.1 us, 1 x 1000 x 2048 11.7 / 7.1, 64 x 1000 x 2048 12.9 / 9.2,
+// 8 x 2000 x 4000 18.3 / 11.4, 16 x 4096 x 4096 21.6 / 19.0 (3.5 TB/s), 16 x 1000 x 512 4.46 / 4.27.  Weights that are
+// converted first instead: gemm_plan.h.
 //
 // K order: one sum over K in steps of 16, as in the other Gemm kernels; a row's bits do not depend on
 // which of them takes a call.
@@ -27,9 +29,13 @@ constexpr int LOAD_WARPS = 8;
 // with the input converted here, as many warps again for it
 constexpr int threads(bool convert) { return 64 + LOAD_WARPS * (convert ? 64 : 32); }
 constexpr int MAX_STAGES = 24;
-constexpr int MAX_SMEM = 224 * 1024;
-// an MMA reads 128 rows of A whatever the box holds
-constexpr int fixed_bytes(int box_m) { return 1024 + (128 - box_m) * 128; }
+// What the ring may take.  Every load of W in flight holds its line in L1, 64 KB an SM, so L1 has to keep that much: with
+// 200 KB of ring 16 x 384 x 3968 takes 17.5 us, with 160 KB 11.4, with 128 KB 10.6, and less gains nothing (16 x 1088 x 6144 24.9,
+// 16.9, 15.9).  64 rows need 170 KB for a stage a warp.
+constexpr int RING_SMEM = 128 * 1024, MAX_SMEM = 172 * 1024;
+// an MMA reads 64 rows of A whatever the box holds
+constexpr int MMA_M = 64;
+constexpr int fixed_bytes(int box_m) { return 1024 + (MMA_M - box_m) * 128; }
 // Columns in groups of eight, k in groups of eight: 128-byte core matrices.  They lie 144 bytes apart along the
 // columns, which puts the eight 16-byte stores of a quarter-warp on different banks.
 constexpr int SBO = 144;
@@ -40,15 +46,16 @@ struct Cfg {
   static constexpr int B_BYTES = STAGE_K / 8 * LBO;              // 4608
   static constexpr int stage_bytes(int box_m) { return STAGE_K / 64 * box_m * 128 + B_BYTES; }
   static constexpr int stages(int box_m) {
-    const int n = (MAX_SMEM - fixed_bytes(box_m)) / stage_bytes(box_m);
-    return n < MAX_STAGES ? n : MAX_STAGES;
+    const int n = (RING_SMEM - fixed_bytes(box_m)) / stage_bytes(box_m);
+    return n < LOAD_WARPS ? LOAD_WARPS : n < MAX_STAGES ? n : MAX_STAGES;
   }
 };
 // Warp w fills stages' worth w, w + 8, ... of K and waits for its stage's previous use by parity alone: with fewer
 // stages than warps one would be two uses ahead and pass.
 template <int BN>
-constexpr bool ring_holds_every_warp = Cfg<BN>::stages(32) >= LOAD_WARPS && Cfg<BN>::stages(64) >= LOAD_WARPS;
+constexpr bool ring_holds_every_warp = Cfg<BN>::stages(8) >= LOAD_WARPS && Cfg<BN>::stages(MMA_M) >= LOAD_WARPS;
 static_assert(ring_holds_every_warp<16> && ring_holds_every_warp<32>, "a stage for every loading warp");
+static_assert(fixed_bytes(MMA_M) + Cfg<16>::stages(MMA_M) * Cfg<16>::stage_bytes(MMA_M) <= MAX_SMEM, "the largest ring fits");
 }  // namespace fewrows
 
 struct FewRowsParams {
@@ -56,7 +63,7 @@ struct FewRowsParams {
   const float *w, *bias;
   float *out;
   int M, N, K;
-  int box_m, stages, steps;  // steps: stages' worth of K
+  int box_m, stages, steps;  // rows of A's box, a multiple of 8; steps: stages' worth of K
   int w_vec, out_vec;        // rows of W / of out and the bias in 16-byte vectors
   int x_vec;                 // rows of x
   uint32_t *err;
@@ -76,7 +83,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
   uint8_t *a_s = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
   const int a_kb = p.box_m * 128, a_bytes = KBS * a_kb;
   // what an MMA reads beyond the last stage's A must not be W's part
-  uint8_t *b_s = a_s + p.stages * a_bytes + (128 - p.box_m) * 128;
+  uint8_t *b_s = a_s + p.stages * a_bytes + (MMA_M - p.box_m) * 128;
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int col0 = blockIdx.x * BN;
 
@@ -125,7 +132,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    const uint32_t idesc = make_idesc_f16(128, BN, false, false, false);
+    const uint32_t idesc = make_idesc_f16(MMA_M, BN, false, false, false);
     const uint64_t a0 = make_smem_desc_sw128(smem_u32(a_s), 16, 1024);
     // no swizzle (see make_smem_desc_sw128 for the fields)
     const uint64_t b0 = static_cast<uint64_t>(smem_u32(b_s) >> 4) | static_cast<uint64_t>(C::LBO / 16) << 16 |
@@ -266,10 +273,10 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
       if (lane == 0) mbar_arrive(&full_bar[stage]);
     }
     const int quarter = warp & 3;
-    if (ok && quarter * 32 < p.M) {
+    if (ok && quarter * 16 < p.M) {
       // the two warps of a lane quarter take 16 columns each; 16 columns in all are the first one's
       const int c0 = (lw >> 2) * 16;
-      const int row = quarter * 32 + lane, cols = p.N - (col0 + c0);
+      const int row = quarter * 16 + lane, cols = p.N - (col0 + c0);
       if (c0 < BN && cols > 0) {
         float b[16];
 #pragma unroll
@@ -283,7 +290,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const FewRowsPa
           tmem_ld_wait_regs(acc);
 #pragma unroll
           for (int j = 0; j < 16; ++j) b[j] += __uint_as_float(acc[j]);
-          if (row < p.M) {
+          if (lane < 16 && row < p.M) {  // an accumulator of 64 rows has 16 in each quarter of the lanes
             float *dst = p.out + static_cast<int64_t>(row) * p.N + col0 + c0;
             if (p.out_vec) {
 #pragma unroll
@@ -344,7 +351,7 @@ void gemm_few_rows(const void *a16, const float *x, const float *w, const float 
   FewRowsParams p;
   p.x = x, p.w = w, p.bias = bias, p.out = out;
   p.M = static_cast<int>(M), p.N = static_cast<int>(N), p.K = static_cast<int>(K);
-  p.box_m = M <= 32 ? 32 : 64;
+  p.box_m = static_cast<int>((M + 7) / 8 * 8);
   p.w_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
   p.out_vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   p.x_vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;

@@ -44,6 +44,9 @@ inline int few_rows_columns(int64_t N, int sms) { return (N + 15) / 16 <= sms ? 
 // until the copy of the weight no longer stays in L2: 50257 x 768 81.4 / 73.3, 32000 x 2048 107 / 94.  A second wave
 // that is at least two thirds full still wins at a short K: 7500 x 512 14.2 / 12.2, 9001 x 512 14.5 / 13.5, but 7008 x 512
 // 11.0 / 12.1 and 8500 x 768 13.4 / 14.8.
+// These times and the lines drawn from them are from before the few rows' own Gemm became 1.1 to 1.6 times faster (accumulators of 64
+// rows, more L1): inside the lines it now wins by more, and beyond most of them too (converted / few rows: 16 x 704 x 6912 17.3 / 16.4,
+// 32 x 2227 x 4354 22.6 / 18.8, 64 x 2828 x 8152 42.4 / 34.2; not 8 x 256 x 6912 14.3 / 16.2, 64 x 320 x 2432 7.8 / 9.3).
 inline int64_t few_rows_max_k(int64_t M, int64_t N, bool vectors, bool lines, int sms) {
   if (few_rows_columns(N, sms) == 16) {
     if (!vectors) return std::min<int64_t>(1536, std::max<int64_t>(512, 5 * N / 4));
