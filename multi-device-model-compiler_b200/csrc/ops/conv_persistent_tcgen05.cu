@@ -7,21 +7,21 @@
 // other and spends most of its life in memory round trips.
 //
 // Two sources of patches:
-//   * kGather = false (16 or more input channels).  conv_prepare_kernel first rewrites the input as
+//   * kIm2col (16 or more input channels).  conv_prepare_kernel first rewrites the input as
 //     NHWC fp16 (padded to 8 channels) and the filter as [OC][channel block][tap][64].  A k-block is one
 //     tap of 64 channels, fetched by a single im2col TMA instruction: no thread touches a patch
 //     element, and the padding comes from the hardware's zero fill.  The rewrite reads and writes
 //     each input element once, the patch loads then read two bytes instead of four, from L2.
-//   * kGather = true (fewer channels, where an NHWC pixel is shorter than the 16 bytes TMA can
+//   * kGather, kGatherFar (fewer channels, where an NHWC pixel is shorter than the 16 bytes TMA can
 //     address).  Three groups of four warps build alternate k-blocks from the NCHW input, one
-//     thread per pixel; where k lies in the window comes from a table in shared memory.
+//     thread per pixel; where k lies in the window comes from the constant bank.
 // The filter stays in shared memory for the CTA's life when it fits there.
 //
-// Bound: instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, about
+// Bound: of short patches and many channels the stores, else instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, about
 // 400 cycles a k-block where the MMAs of 64 columns take 193 (conv_plan.h says which calls conv_halo_kernel takes instead).
 // Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
 // changing from call to call:
-//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  64 us (43 of HBM time)
+//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  56 us (43 of HBM time)
 //   32 x 128 x 28 x 28 -> 128, 3 x 3                            19 us
 // L2 flushed between calls:
 //   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            116 ->  34 us
@@ -29,7 +29,9 @@
 // the first shape went from 73 to 64 us, 32 x 256 x 14 x 14 -> 256 from 22.9 to 16.9, 32 x 512 x 7 x 7 -> 512 from 32 to 25.
 // The gather was bound by instruction issue: run-time divisions and per-channel tests in the
 // epilogue, 2.7 us a tile of 128 x 64; with multiplicative division, whole-group stores and the
-// two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).
+// two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).  With the taps in the constant bank,
+// one test a value at the edges and no work on other groups' tiles 64 -> 56, 32 x 3 x 224 x 224 -> 64 stride 2 47 -> 36,
+// 43 x 6 x 255 x 256 -> 8 dilation 2 269 -> 156; 140 shapes of 1 to 15 channels 0.87 of the time.
 #include <cuda_fp16.h>
 
 #include "conv_epilogue.cuh"
@@ -63,13 +65,46 @@ struct Params {
   uint32_t tmem_cols;
   uint32_t *err;
 };
+// Where the patches come from.  Where a gathered k lies is read from the constant bank: kGather for patches of up to
+// TAP_TABLE values, windows of up to 16 x 15 taps and inputs that 32 bits address, kGatherFar for the others.
+enum Source { kIm2col, kGather, kGatherFar };
+constexpr int TAP_TABLE = 256;
+template <int kSource>
+struct Taps {};
+template <>
+struct Taps<kGather> {
+  uint32_t lead;             // bytes that a window may begin ahead of the input
+  uint32_t off[TAP_TABLE];   // bytes of k from the window's origin
+  uint32_t need[TAP_TABLE];  // bits 0-15 its row of the window, 16-30 its column; beyond the patch bit 31
+};
+template <>
+struct Taps<kGatherFar> {
+  uint32_t off[kDenseMaxGatherK];  // elements from the window's origin
+  uint32_t pos[kDenseMaxGatherK];  // row of the input from the origin's << 16 | column
+};
 }  // namespace convp
 
-template <bool kGather, bool kAdd>
-__global__ void __launch_bounds__(convp::threads(kGather), 1)
+// The value where `in`, else zero; never a branch.
+__device__ __forceinline__ float ldg_if(bool in, const float *src) {
+  float v;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "mov.f32 %0, 0f00000000;\n"
+      "@p ld.global.nc.f32 %0, [%2];\n"
+      "}\n"
+      : "=f"(v)
+      : "r"(static_cast<uint32_t>(in)), "l"(src));
+  return v;
+}
+
+template <int kSource, bool kAdd>
+__global__ void __launch_bounds__(convp::threads(kSource != convp::kIm2col), 1)
 conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                       const convp::Params p) {
+                       const convp::Params p, const __grid_constant__ convp::Taps<kSource> taps) {
   using namespace convp;
+  constexpr bool gather = kSource != kIm2col;
   using namespace ptx;
   extern __shared__ uint8_t smem_dyn[];
   __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_full_bar[2], acc_empty_bar[2], filter_bar;
@@ -82,21 +117,19 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   const int stage_bytes = A_BYTES + (p.resident ? 0 : b_bytes);
   uint8_t *filter_s = tiles + p.stages * stage_bytes;
   float *bias_s = reinterpret_cast<float *>(filter_s + (p.resident ? p.num_kb * b_bytes : 0));
-  // 16-byte aligned: everything in front is a multiple of 1 KiB, the bias a multiple of 32 floats
-  int2 *table = reinterpret_cast<int2 *>(bias_s + (p.OC + 31) / 32 * 32);
 
   if (threadIdx.x == 0) {
     abort_flag_s = 0;
-    if (!kGather) tma_prefetch_desc(&tmap_x);
+    if (!gather) tma_prefetch_desc(&tmap_x);
     tma_prefetch_desc(&tmap_w);
-    const uint32_t loaders = kGather ? (p.resident ? 4u : 5u) : 1u;
+    const uint32_t loaders = gather ? (p.resident ? 4u : 5u) : 1u;
     for (int i = 0; i < p.stages; ++i) {
       mbar_init(&full_bar[i], loaders);
       mbar_init(&empty_bar[i], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full_bar[a], 1);
-      mbar_init(&acc_empty_bar[a], kGather ? EPI_WARPS / 2 : EPI_WARPS);
+      mbar_init(&acc_empty_bar[a], gather ? EPI_WARPS / 2 : EPI_WARPS);
     }
     mbar_init(&filter_bar, 1);
     mbar_init_fence();
@@ -104,15 +137,6 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
   if (warp == EPI_WARPS + 1) {
     tmem_alloc(&tmem_slot, p.tmem_cols);
     tmem_relinquish();
-  }
-  if (kGather) {
-    // k -> (offset from the window's origin, tap position); entries past K are marked -1
-    const int hw = p.H * p.W;
-    for (int k = threadIdx.x; k < p.num_kb * BK; k += threads(true)) {
-      const int ic = k / p.taps, r = k - ic * p.taps, kh = r / p.KW, kw = r - kh * p.KW;
-      table[k] = k < p.K ? make_int2(ic * hw + kh * p.DH * p.W + kw * p.DW, (kh * p.DH) << 16 | (kw * p.DW))
-                         : make_int2(-1, 0);
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -128,13 +152,13 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     for (int i = threadIdx.x; i < (p.OC + 31) / 32 * 32; i += EPI_WARPS * 32)
       bias_s[i] = p.bias && i < p.OC ? __ldg(p.bias + i) : 0.f;
     asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-    constexpr int G = kGather ? 16 : 32;  // channels per group: as many as the registers allow
+    constexpr int G = gather ? 16 : 32;  // channels per group: as many as the registers allow
     const int quarter = warp & 3, half = warp >> 2;
-    const int c_first = kGather ? 0 : half * G, c_step = kGather ? G : 2 * G;
+    const int c_first = gather ? 0 : half * G, c_step = gather ? G : 2 * G;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    int acc = kGather ? half : 0;
+    int acc = gather ? half : 0;
     uint32_t acc_phase = 0;
-    for (int tile = blockIdx.x + (kGather ? half * gridDim.x : 0); tile < p.num_tiles; tile += (kGather ? 2 : 1) * gridDim.x) {
+    for (int tile = blockIdx.x + (gather ? half * gridDim.x : 0); tile < p.num_tiles; tile += (gather ? 2 : 1) * gridDim.x) {
       const int mt = p.by_ntiles.div(tile), n0 = p.by_ntiles.mod(tile, mt) * p.bn;
       const int m = mt * BM + quarter * 32 + lane;
       const bool live = m < p.M;
@@ -171,7 +195,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
-      if (kGather || (acc ^= 1) == 0) acc_phase ^= 1;
+      if (gather || (acc ^= 1) == 0) acc_phase ^= 1;
     }
   } else if (warp == EPI_WARPS) {
     // ---------------- TMA: filter blocks, and the patches when they are not gathered ----------------
@@ -182,7 +206,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       }
       __syncwarp();
     }
-    if (!kGather || !p.resident) {
+    if (!gather || !p.resident) {
       int stage = 0;
       uint32_t phase = 0, looked = 0;
       bool ok = true;
@@ -201,8 +225,8 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
           looked = mbar_look(&empty_bar[next], next ? phase ^ 1 : phase);
           if (elect_one()) {
             uint8_t *sa = tiles + stage * stage_bytes;
-            mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>((kGather ? 0 : A_BYTES) + (p.resident ? 0 : b_bytes)));
-            if (!kGather)
+            mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>((gather ? 0 : A_BYTES) + (p.resident ? 0 : b_bytes)));
+            if (!gather)
               tma_load_im2col_4d(sa, &tmap_x, &full_bar[stage], c0, w0, h0, img, static_cast<uint16_t>(kw * p.DW),
                                  static_cast<uint16_t>(kh * p.DH));
             if (!p.resident) tma_load_2d(sa + A_BYTES, &tmap_w, &full_bar[stage], kb * BK, n0);
@@ -228,7 +252,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       ok = false;
     }
     // the blocks that may be partial: the last one of a gathered patch, all taps of the last 64 channels
-    const int partial_from = p.last_k == BK ? p.num_kb : p.num_kb - (kGather ? 1 : p.taps);
+    const int partial_from = p.last_k == BK ? p.num_kb : p.num_kb - (gather ? 1 : p.taps);
     const int partial_steps = (p.last_k + 15) / 16;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
       if (!mbar_wait_all(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
@@ -261,81 +285,104 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
       umma_commit_warp(&acc_full_bar[acc]);
       if ((acc ^= 1) == 0) acc_phase ^= 1;
     }
-  } else if constexpr (kGather) {
+  } else if constexpr (gather) {
     // ---------------- gather: one thread per pixel, groups of four warps take alternate k-blocks ----------------
+    // Where k lies is the same for all lanes: out of the constant bank a value costs its load and an addition of the uniform
+    // datapath.  Out of a table in shared memory it took a load of that, a 64-bit addition and a test more (64 us at
+    // 16x3x256x256->64 3x3, now 55); and every group worked out every tile's pixels, where a third of the tiles are its own.
     const int group = (warp - EPI_WARPS - 2) >> 2;
     const int row = ((warp - EPI_WARPS - 2) & 3) * 32 + lane;
     const uint32_t row_off = static_cast<uint32_t>(row) * 128u, swz = static_cast<uint32_t>(row & 7);
-    const int max_dh = (p.taps / p.KW - 1) * p.DH, max_dw = (p.KW - 1) * p.DW;
-    int turn = 0, stage = 0;  // turn: which group's k-block this is
-    uint32_t phase = 0;
+    const int KH = p.taps / p.KW, max_dh = (KH - 1) * p.DH, max_dw = (p.KW - 1) * p.DW;
+    int block = group, tile_block = 0;  // this group's next k-block, and the tile's first, counted over all tiles of the CTA
+    int stage = group % p.stages;
+    uint32_t phase = static_cast<uint32_t>(group / p.stages) & 1u;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
+    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, tile_block += p.num_kb) {
+      if (block >= tile_block + p.num_kb) continue;  // short patches: not every tile has one for every group
       const int m = p.by_ntiles.div(tile) * BM + row;
       const bool live = m < p.M;
-      int h0 = 0, w0 = 0;
-      const float *origin = p.x;  // of the window; may lie outside the image, then only live taps are read
+      int h0 = 0, w0 = 0, img = 0;
       if (live) {
-        const int img = p.by_p.div(m), pix = p.by_p.mod(m, img), oh = p.by_ow.div(pix);
+        img = p.by_p.div(m);
+        const int pix = p.by_p.mod(m, img), oh = p.by_ow.div(pix);
         h0 = oh * p.SH - p.PHL;
         w0 = p.by_ow.mod(pix, oh) * p.SW - p.PWL;
-        origin += static_cast<int64_t>(img) * p.IC * p.H * p.W + h0 * p.W + w0;
       }
       // windows of the whole warp inside the image: no bounds tests
       const bool interior = __all_sync(0xffffffffu, live && h0 >= 0 && w0 >= 0 && h0 + max_dh < p.H && w0 + max_dw < p.W);
-      for (int kb = 0; kb < p.num_kb; ++kb) {
-        if (turn == group) {
-          const int pieces = kb == p.num_kb - 1 ? (p.last_k + 31) / 32 : 2;  // of 32 values
-          uint8_t *sa = tiles + stage * stage_bytes + row_off;
-          for (int h = 0; h < pieces; ++h) {
-            const int4 *t4 = reinterpret_cast<const int4 *>(table + kb * BK + h * 32);
-            float v[32];
-            if (interior) {
+      // The window's origin, which may lie outside the image (then only live taps are read): bytes from the front of the
+      // input, or its address.  And which rows and columns of the window lie outside.
+      [[maybe_unused]] const char *front = nullptr;
+      [[maybe_unused]] uint32_t at = 0, outside = 0x80000000u;
+      [[maybe_unused]] const float *origin = p.x;
+      if constexpr (kSource == kGather) {
+        front = reinterpret_cast<const char *>(p.x) - taps.lead;
+        at = taps.lead + static_cast<uint32_t>((img * p.IC * p.H + h0) * p.W + w0) * 4u;
+        if (!interior) {
+          for (int kh = 0; kh < KH; ++kh)
+            if (!live || static_cast<unsigned>(h0 + kh * p.DH) >= static_cast<unsigned>(p.H)) outside |= 1u << kh;
+          for (int kw = 0; kw < p.KW; ++kw)
+            if (static_cast<unsigned>(w0 + kw * p.DW) >= static_cast<unsigned>(p.W)) outside |= 0x10000u << kw;
+        }
+      } else {
+        origin += (static_cast<int64_t>(img) * p.IC * p.H + h0) * p.W + w0;
+      }
+      for (; block < tile_block + p.num_kb; block += GATHER_GROUPS) {
+        const int kb = block - tile_block;
+        const int pieces = kb == p.num_kb - 1 ? (p.last_k + 31) / 32 : 2;  // of 32 values
+        uint8_t *sa = tiles + stage * stage_bytes + row_off;
+        for (int h = 0; h < pieces; ++h) {
+          float v[32];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int4 t = t4[j];
-                v[2 * j] = t.x >= 0 ? __ldg(origin + t.x) : 0.f;
-                v[2 * j + 1] = t.z >= 0 ? __ldg(origin + t.z) : 0.f;
+          for (int c = 0; c < 32; c += 8) {
+            const int k = kb * BK + h * 32 + c;
+            if (interior && k + 8 <= p.K) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if constexpr (kSource == kGather) v[c + j] = __ldg(reinterpret_cast<const float *>(front + taps.off[k + j] + at));
+                else v[c + j] = __ldg(origin + taps.off[k + j]);
+              }
+            } else if (k < p.K) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if constexpr (kSource == kGather) {
+                  v[c + j] = ldg_if((outside & taps.need[k + j]) == 0, reinterpret_cast<const float *>(front + taps.off[k + j] + at));
+                } else {
+                  const uint32_t pos = taps.pos[k + j];
+                  v[c + j] = ldg_if(live && k + j < p.K && static_cast<unsigned>(h0 + static_cast<int>(pos >> 16)) < static_cast<unsigned>(p.H) &&
+                                        static_cast<unsigned>(w0 + static_cast<int>(pos & 0xffff)) < static_cast<unsigned>(p.W),
+                                    origin + taps.off[k + j]);
+                }
               }
             } else {
-              auto tap = [&](int off, int pos) __attribute__((always_inline)) {
-                const bool in = live && off >= 0 && static_cast<unsigned>(h0 + (pos >> 16)) < static_cast<unsigned>(p.H) &&
-                                static_cast<unsigned>(w0 + (pos & 0xffff)) < static_cast<unsigned>(p.W);
-                return in ? __ldg(origin + off) : 0.f;
-              };
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int4 t = t4[j];
-                v[2 * j] = tap(t.x, t.y);
-                v[2 * j + 1] = tap(t.z, t.w);
-              }
-            }
-            // the loads are in flight; only now does the stage have to be free
-            if (h == 0 && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
-              atomicCAS(p.err, 0u, 0x50000000u | static_cast<uint32_t>(stage));
-              ok = false;
-              break;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const __half2 h0_ = __floats2half2_rn(v[c * 8 + 0], v[c * 8 + 1]), h1_ = __floats2half2_rn(v[c * 8 + 2], v[c * 8 + 3]);
-              const __half2 h2_ = __floats2half2_rn(v[c * 8 + 4], v[c * 8 + 5]), h3_ = __floats2half2_rn(v[c * 8 + 6], v[c * 8 + 7]);
-              uint4 q;
-              q.x = *reinterpret_cast<const uint32_t *>(&h0_);
-              q.y = *reinterpret_cast<const uint32_t *>(&h1_);
-              q.z = *reinterpret_cast<const uint32_t *>(&h2_);
-              q.w = *reinterpret_cast<const uint32_t *>(&h3_);
-              // 128-byte swizzle: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
-              *reinterpret_cast<uint4 *>(sa + ((static_cast<uint32_t>(h * 4 + c) ^ swz) << 4)) = q;
+              for (int j = 0; j < 8; ++j) v[c + j] = 0.f;
             }
           }
-          if (!ok) break;
-          fence_proxy_async_smem();  // the tensor core reads these rows through the async proxy
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&full_bar[stage]);
+          // the loads are in flight; only now does the stage have to be free
+          if (h == 0 && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) {
+            atomicCAS(p.err, 0u, 0x50000000u | static_cast<uint32_t>(stage));
+            ok = false;
+            break;
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint4 q;
+            q.x = pack_pair<__half>(v[c * 8 + 0], v[c * 8 + 1]);
+            q.y = pack_pair<__half>(v[c * 8 + 2], v[c * 8 + 3]);
+            q.z = pack_pair<__half>(v[c * 8 + 4], v[c * 8 + 5]);
+            q.w = pack_pair<__half>(v[c * 8 + 6], v[c * 8 + 7]);
+            // 128-byte swizzle: 16-byte chunk c of row r lives at chunk (c ^ (r & 7))
+            *reinterpret_cast<uint4 *>(sa + ((static_cast<uint32_t>(h * 4 + c) ^ swz) << 4)) = q;
+          }
         }
-        if (++turn == GATHER_GROUPS) turn = 0;
-        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        if (!ok) break;
+        fence_proxy_async_smem();  // the tensor core reads these rows through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_bar[stage]);
+        stage += GATHER_GROUPS;
+        while (stage >= p.stages) stage -= p.stages, phase ^= 1;
       }
     }
   }
@@ -451,10 +498,10 @@ EncodeIm2col encode_im2col() {
   return fn;
 }
 
-template <bool kGather, bool kAdd>
-void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp::Params &p, size_t smem, int sms,
-                       cudaStream_t s) {
-  auto kern = conv_persistent_kernel<kGather, kAdd>;
+template <bool kAdd, int kSource>
+void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp::Params &p, const convp::Taps<kSource> &taps, size_t smem,
+                       int sms, cudaStream_t s) {
+  auto kern = conv_persistent_kernel<kSource, kAdd>;
   static bool set_on[64] = {false};  // the attribute is per device
   const int dev = device_info().device;
   bool &set = set_on[(dev >= 0 && dev < 64) ? dev : 0];
@@ -468,7 +515,7 @@ void launch_persistent(const CUtensorMap &tx, const CUtensorMap &tw, const convp
   const int rounds = (p.num_tiles + sms - 1) / sms, grid = (p.num_tiles + rounds - 1) / rounds;
   {
     ProfileScope prof(kCatGemm, s);
-    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convp::threads(kGather)), smem, s, 1, tx, tw, p),
+    check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(grid)), dim3(convp::threads(kSource != convp::kIm2col)), smem, s, 1, tx, tw, p, taps),
                "launch conv_persistent_kernel");
   }
   launched("conv_persistent_kernel");
@@ -509,9 +556,9 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   ConvShape c = call;
   const bool sampled = conv_sampled(c), gather = conv_gathers(c);
   const DeviceInfo &di = device_info();
-  const int64_t taps = c.KH * c.KW, K = c.IC * taps, M = c.N * c.OH * c.OW;
+  const int64_t window = c.KH * c.KW, K = c.IC * window, M = c.N * c.OH * c.OW;
   const int64_t Cp = (c.IC + 7) / 8 * 8, ncb = (c.IC + 63) / 64;
-  const int64_t num_kb = gather ? (K + BK - 1) / BK : ncb * taps;
+  const int64_t num_kb = gather ? (K + BK - 1) / BK : ncb * window;
   const int64_t Kp = gather ? (K + 7) / 8 * 8 : num_kb * BK;
   const int64_t m_tiles = (M + BM - 1) / BM;
   if (num_kb > (1 << 20)) return false;
@@ -520,7 +567,7 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   p.x = c.x, p.bias = c.bias, p.add = c.add, p.out = c.out;
   p.IC = int(c.IC), p.H = int(c.H), p.W = int(c.W), p.OC = int(c.OC), p.KW = int(c.KW), p.OH = int(c.OH), p.OW = int(c.OW);
   p.PHL = int(c.PHL), p.PWL = int(c.PWL), p.SH = int(c.SH), p.SW = int(c.SW), p.DH = int(c.DH), p.DW = int(c.DW);
-  p.taps = int(taps), p.M = int(M), p.P = int(c.OH * c.OW), p.K = int(K), p.num_kb = int(num_kb), p.ncb = int(ncb);
+  p.taps = int(window), p.M = int(M), p.P = int(c.OH * c.OW), p.K = int(K), p.num_kb = int(num_kb), p.ncb = int(ncb);
   p.last_k = int(gather ? K - (num_kb - 1) * BK : c.IC - (ncb - 1) * BK);
   p.relu = c.relu ? 1 : 0;
   p.bn = choose_conv_bn(m_tiles, c.OC, p.num_kb, gather, c.add != nullptr, di.sms);
@@ -531,9 +578,12 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   p.tmem_cols = 32;
   while (p.tmem_cols < 2u * p.bn) p.tmem_cols *= 2;
   const int64_t filter_bytes = num_kb * p.bn * BK * 2;
+  const bool near = K <= TAP_TABLE && c.KH <= 16 && c.KW <= 15 &&
+                    (c.N * c.IC * c.H * c.W + c.PHL * c.W + c.PWL) * 4 < (int64_t(1) << 32) &&
+                    (((c.IC - 1) * c.H + (c.KH - 1) * c.DH) * c.W + (c.KW - 1) * c.DW) * 4 < (int64_t(1) << 32);
   p.resident = conv_filter_stays(num_kb, p.bn, p.n_tiles, p.num_tiles, di.sms);
   const int64_t stage_bytes = A_BYTES + (p.resident ? 0 : p.bn * BK * 2);
-  const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128 + (gather ? num_kb * BK * 8 : 0);
+  const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128;
   int64_t stages = (static_cast<int64_t>(kMaxSmem) - 4096 - fixed) / stage_bytes;
   // gathered patches are read nine-fold through L1: leave it most of the memory
   const int64_t cap = gather ? 4 : MAX_STAGES;
@@ -567,10 +617,27 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   }
   ok = ok && conv_prepare(c, call, sampled, c.H, c.W, ws + w_bytes, ws, s);
   if (ok) {
-    if (gather && p.add) launch_persistent<true, true>(tx, tw, p, smem, di.sms, s);
-    else if (gather) launch_persistent<true, false>(tx, tw, p, smem, di.sms, s);
-    else if (p.add) launch_persistent<false, true>(tx, tw, p, smem, di.sms, s);
-    else launch_persistent<false, false>(tx, tw, p, smem, di.sms, s);
+    auto launch = [&](const auto &t) { p.add ? launch_persistent<true>(tx, tw, p, t, smem, di.sms, s) : launch_persistent<false>(tx, tw, p, t, smem, di.sms, s); };
+    if (!gather) {
+      launch(Taps<kIm2col>());
+    } else if (near) {
+      Taps<kGather> t;
+      t.lead = static_cast<uint32_t>((c.PHL * c.W + c.PWL) * 4);
+      for (int64_t k = 0; k < num_kb * BK; ++k) {
+        const int64_t ic = k / window, kh = k % window / c.KW, kw = k % window % c.KW;
+        t.off[k] = k < K ? static_cast<uint32_t>(((ic * c.H + kh * c.DH) * c.W + kw * c.DW) * 4) : 0;
+        t.need[k] = k < K ? 1u << kh | 0x10000u << kw : 0x80000000u;
+      }
+      launch(t);
+    } else {
+      Taps<kGatherFar> t;
+      for (int64_t k = 0; k < num_kb * BK; ++k) {
+        const int64_t ic = k / window, kh = k % window / c.KW, kw = k % window % c.KW;
+        t.off[k] = k < K ? static_cast<uint32_t>((ic * c.H + kh * c.DH) * c.W + kw * c.DW) : 0;
+        t.pos[k] = k < K ? static_cast<uint32_t>(kh * c.DH << 16 | kw * c.DW) : 0;
+      }
+      launch(t);
+    }
   }
   mgpuMemFreeAsync(ws, s);
   return ok;

@@ -211,6 +211,41 @@ def test_conv_persistent_edges(m, shape):
     assert np.array_equal(m.conv2d(x, w, b, **kw), oracle.conv2d(x, w, b, **kw))
 
 
+@pytest.mark.parametrize("shape", [
+    (2, 1, 9, 7, 8, 1, 1, (1, 1), (0, 0, 0, 0), (1, 1), False, False),         # one value of eight
+    (3, 14, 12, 11, 24, 3, 6, (1, 1), (1, 2, 1, 3), (1, 1), True, False),      # 252 values: the table's last 64, partly
+    (3, 15, 12, 11, 24, 3, 6, (1, 1), (1, 2, 1, 3), (1, 1), False, True),      # 270: the larger table
+    (40, 3, 40, 33, 16, 16, 1, (1, 1), (15, 0, 15, 0), (1, 1), False, False),  # 16 rows and 15 columns of a window have bits ...
+    (2, 3, 33, 40, 16, 1, 15, (1, 2), (0, 14, 0, 14), (1, 1), True, False),
+    (2, 3, 40, 33, 16, 17, 1, (2, 1), (16, 0, 16, 0), (1, 1), False, False),   # ... 17 and 16 have none
+    (40, 3, 33, 40, 16, 1, 16, (1, 1), (0, 15, 0, 15), (1, 1), True, True),
+    (3, 2, 3, 4, 9, 3, 3, (1, 1), (9, 7, 8, 6), (4, 3), False, False),         # margins wider than the image
+    (200, 3, 10, 45, 64, 3, 3, (1, 2), (1, 1, 1, 1), (1, 1), True, True),      # several tiles for each group of warps
+])
+def test_conv_gathered_patches(m, shape):
+    """Up to 15 channels, below 25 taps: where k lies by either table, windows partly and wholly outside.  Small integers; an
+    infinity reaches the outputs of its windows and no others."""
+    N, IC, H, W, OC, KH, KW, stride, pad, dil, has_add, relu = shape
+    rng = np.random.default_rng(IC * 1000 + KH * 10 + KW)
+    x = rng.integers(-4, 5, size=(N, IC, H, W)).astype(np.float32)
+    w = rng.integers(1, 4, size=(OC, IC, KH, KW)).astype(np.float32)
+    b = rng.integers(-8, 9, size=OC).astype(np.float32)
+    OH = (H + pad[0] + pad[2] - (KH - 1) * dil[0] - 1) // stride[0] + 1
+    OW = (W + pad[1] + pad[3] - (KW - 1) * dil[1] - 1) // stride[1] + 1
+    add = rng.integers(-8, 9, size=(N, OC, OH, OW)).astype(np.float32) if has_add else None
+    kw = dict(post_add=add, stride=stride, pad=pad, dilation=dil, relu=relu)
+    clean = m.conv2d(x, w, b, **kw)
+    assert np.array_equal(clean, oracle.conv2d(x, w, b, **kw))
+    at = (N - 1, IC - 1, H // 2, W // 2)
+    x[at] = np.inf
+    got = m.conv2d(x, w, b, **kw)
+    y, v = at[2] + pad[0] - stride[0] * np.arange(OH), at[3] + pad[1] - stride[1] * np.arange(OW)
+    in_window = lambda t, d, n: (t >= 0) & (t % d == 0) & (t // d < n)
+    hit = np.zeros(clean.shape, bool)
+    hit[N - 1] = in_window(y, dil[0], KH)[:, None] & in_window(v, dil[1], KW)[None, :]
+    assert np.array_equal(got[~hit], clean[~hit]) and np.all(np.isposinf(got[hit]))
+
+
 # rows of test_conv_persistent_edges for every form of conv_form
 REGION_FORMS = [
     ("kCopyRect", (3, 16, 9, 16, 16, 5, 3, (1, 1), (2, 1, 2, 1), (1, 1), True, False)),  # rect out of a copy: tiles of two images
