@@ -144,6 +144,7 @@ constexpr int kHaloMaxTaps = 64;           // entries of its table of taps, or p
 constexpr int kHaloFilterStages = 12;
 constexpr int kHaloInputWarps = 12;        // of the direct forms
 constexpr size_t kHaloMaxSmem = 220 * 1024;
+constexpr int64_t kHaloAddSmem = 150 * 1024;  // beside a residual, where fewer stages do
 
 // A tile of conv_halo_kernel and what follows from it.
 struct HaloTile {
@@ -162,7 +163,7 @@ struct HaloTile {
 
 // Shared memory: regions, then the filter whole or a ring of its k-blocks, several to a stage where they are short (a
 // hand-over costs as much as the MMAs of 64 columns).  False where it does not fit.
-inline bool fit_halo(HaloTile *t, bool copy, int64_t OC, int bn, int sms) {
+inline bool fit_halo(HaloTile *t, bool copy, bool add, int64_t OC, int bn, int sms) {
   const int64_t fixed = 2048 + (OC + 31) / 32 * 128, room = static_cast<int64_t>(kHaloMaxSmem) - fixed;
   const int64_t num_kb = t->num_kb, b_bytes = bn * 128, filter = num_kb * b_bytes, region = t->region_bytes;
   const int64_t most = region <= 16 * 1024 ? 8 : 4;
@@ -177,8 +178,17 @@ inline bool fit_halo(HaloTile *t, bool copy, int64_t OC, int bn, int sms) {
   // as many stages as regions that the input warps' pieces reach over: a stage's barrier is then never two uses behind
   const int64_t reach = copy ? 0 : (kHaloInputWarps + t->qb - 1) / t->qb;
   if (n < 2 || n < reach) return false;
+  // No more stages than the busiest CTA fills, so that the next call's CTAs fit beside those of a short one: 33x6x13x14->8 5x5
+  // 8.0 -> 6.9 us, 150 direct shapes 0.96 of the time, the slowest 1.02.
+  const int64_t rounds = (tiles + sms - 1) / sms;
+  n = std::min(n, std::max({int64_t(2), reach, rounds * t->ncb}));
   int64_t fs = (room - n * region) / (kbs * b_bytes);
-  if (fs > kHaloFilterStages) fs = kHaloFilterStages;
+  fs = std::min({fs, int64_t(kHaloFilterStages), blocks * rounds});
+  // A residual's loads in flight hold their lines in L1, four sectors to a line, and 220 KB leave it 30: 32x64x56x56->64 3x3
+  // 25.0 -> 24.0 us, -> 256 1x1 56.9 -> 50.9.  Not where the filter streams by for every tile, which then is what
+  // takes the time: 1x176x15x14->136 7x7 23.4 -> 24.6, 8x16x89x83->16 7x7 27.8 -> 29.0.
+  if (add && copy && (resident || blocks <= 4))
+    while (n > 3 && n * region + (resident ? filter : fs * kbs * b_bytes) + fixed > kHaloAddSmem) --n;
   t->bn = bn, t->resident = resident ? 1 : 0, t->stages = static_cast<int>(n);
   t->filter_stages = resident ? 0 : static_cast<int>(fs), t->filter_kbs = static_cast<int>(kbs);
   t->regions_bytes = static_cast<uint32_t>((n * region + 1023) / 1024 * 1024);
@@ -221,7 +231,7 @@ inline bool halo_tile(const ConvShape &c, ConvForm form, int sms, HaloTile *best
   double best_cost = 1e300;
   for (int bn = 256; bn >= 32; bn -= 32) {
     if ((bn > 32 && bn >= c.OC + 32) || 2 * t.splits * bn > 512) continue;
-    if (!fit_halo(&t, copy, c.OC, bn, sms)) continue;
+    if (!fit_halo(&t, copy, c.add != nullptr, c.OC, bn, sms)) continue;
     const int64_t tiles = t.h.m_tiles * ((c.OC + bn - 1) / bn);
     if (tiles > (1 << 30)) continue;
     const double rounds = static_cast<double>((tiles + sms - 1) / sms);
