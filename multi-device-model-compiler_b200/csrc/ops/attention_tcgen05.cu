@@ -505,8 +505,13 @@ __device__ __forceinline__ AttnItem64 attn_item64(const AttnParams &p, int item,
 // per step (parity t & 1), so loads for step t+1 (of the same or of the next item) are issued
 // while step t is still in its softmax: K (and the next item's Q) as soon as S = Q.K^T of
 // step t has been computed, V as soon as P.V of step t has.
-template <typename T16, bool kOuter>
-__global__ void __launch_bounds__(attn64::THREADS, attn64::CTAS_PER_SM)
+//
+// kFew: no more items than SMs.  Then one item's latency is the kernel's time and a CTA has an SM's registers: a row's scores are
+// read once, all in flight, and kept (the three-CTA form reads them twice, 32 at a time where a tile is partly visible), and
+// the output goes from registers to memory, without the way through shared memory and TMA.  The same operations in the
+// same order.  1 x 99 tokens, 12 heads, causal 5.41 -> 4.95 us, 8 x 64 5.18 -> 4.41, 1 x 512 causal 12.1 -> 11.8.
+template <typename T16, bool kOuter, bool kFew>
+__global__ void __launch_bounds__(attn64::THREADS, kFew ? 1 : attn64::CTAS_PER_SM)
 attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
                      const __grid_constant__ CUtensorMap tmap_out, const AttnParams p) {
   using namespace attn64;
@@ -673,7 +678,23 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         const int n_max = __reduce_max_sync(0xffffffffu, ncol);
         // pass 1: row maximum
         float m_tile = -INFINITY;
-        if (full_tile) {
+        uint32_t sc[kFew ? BKV / 32 : 1][32];  // kFew: the row's scores, those that it does not see -inf
+        if constexpr (kFew) {
+#pragma unroll
+          for (int c = 0; c < BKV / 32; ++c)
+            if (c * 32 < n_max) tmem_ld_32x32(tmem_base + lane_addr + S_COL + c * 32, sc[c]);
+#pragma unroll
+          for (int c = 0; c < BKV / 32; ++c) {
+            if (c * 32 < n_max) {
+              tmem_ld_wait_regs(sc[c]);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                if (!full_tile && c * 32 + i >= ncol) sc[c][i] = 0xff800000u;
+                m_tile = fmaxf(m_tile, __uint_as_float(sc[c][i]));
+              }
+            }
+          }
+        } else if (full_tile) {
           // 16 columns at a time, the next load in flight while the current piece is reduced
           uint32_t sa[16], sb[16];
           const uint32_t s_addr = tmem_base + lane_addr + S_COL;
@@ -709,7 +730,24 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         // goes to columns [16c, 16c+16), over S columns this thread has already consumed
         float l_tile = 0.f;
         const float mc = m_ref * p.scale_log2e;
-        if (full_tile) {
+        if constexpr (kFew) {
+#pragma unroll
+          for (int c = 0; c < BKV / 32; ++c) {
+            uint32_t packed[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) packed[i] = 0;
+            if (c * 32 < n_max) {
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                const float p0 = ex2_fast(fmaf(__uint_as_float(sc[c][i]), p.scale_log2e, -mc));
+                const float p1 = ex2_fast(fmaf(__uint_as_float(sc[c][i + 1]), p.scale_log2e, -mc));
+                l_tile += p0 + p1;
+                packed[i >> 1] = pack16<T16>(p0, p1);
+              }
+            }
+            tmem_st_32x16(tmem_base + lane_addr + P_COL + c * 16, packed);
+          }
+        } else if (full_tile) {
           // the same pipelining; two 16-column pieces of S make one 16-register piece of P
           uint32_t sa[16], sb[16];
           const uint32_t s_addr = tmem_base + lane_addr + S_COL;
@@ -791,6 +829,17 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         // O / l -> shared memory (swizzled 128-byte rows) -> one TMA store of the warp's 32 rows:
         // whole lines, and rows past the end of the sequence are clipped by the tensor map
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+        if constexpr (kFew) {
+          if (q_local < p.seq) {
+            T16 *dst = static_cast<T16 *>(p.out) + (static_cast<int64_t>(it.b) * p.seq + q_local) * hd + it.head * D;
+#pragma unroll
+            for (int g = 0; g < D / 8; ++g)
+              *reinterpret_cast<uint4 *>(dst + 8 * g) =
+                  make_uint4(pack16<T16>(o_acc[8 * g + 0] * inv, o_acc[8 * g + 1] * inv), pack16<T16>(o_acc[8 * g + 2] * inv, o_acc[8 * g + 3] * inv),
+                             pack16<T16>(o_acc[8 * g + 4] * inv, o_acc[8 * g + 5] * inv), pack16<T16>(o_acc[8 * g + 6] * inv, o_acc[8 * g + 7] * inv));
+          }
+          continue;
+        }
         uint8_t *my_out = sOut + warp * 4096;
         if (lane == 0) tma_store_wait_read<0>();  // the previous store has left the staging buffer
         __syncwarp();
@@ -811,7 +860,7 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
         }
       }
     }
-    if (lane == 0) tma_store_wait<0>();  // all staged output has left shared memory
+    if (!kFew && lane == 0) tma_store_wait<0>();  // all staged output has left shared memory
   }
 
   if (*abort_flag) {
@@ -825,10 +874,10 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
   if (warp == 4) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-template <typename T16, bool kOuter>
+template <typename T16, bool kOuter, bool kFew>
 static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &tmo, const AttnParams &p, int64_t n_items,
                                      const DeviceInfo &di, cudaStream_t s) {
-  auto kern = attention_d64_kernel<T16, kOuter>;
+  auto kern = attention_d64_kernel<T16, kOuter, kFew>;
   static bool set_on[64] = {false};  // the attribute is per device
   bool &set = set_on[(di.device >= 0 && di.device < 64) ? di.device : 0];
   if (!set) {
@@ -845,8 +894,9 @@ static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &t
 template <typename T16>
 static void launch_attention64(const CUtensorMap &tm, const CUtensorMap &tmo, const AttnParams &p, int64_t n_items,
                                const DeviceInfo &di, cudaStream_t s) {
-  if (p.causal && n_items > static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM) launch_attention64_order<T16, true>(tm, tmo, p, n_items, di, s);
-  else launch_attention64_order<T16, false>(tm, tmo, p, n_items, di, s);
+  if (n_items <= di.sms) launch_attention64_order<T16, false, true>(tm, tmo, p, n_items, di, s);
+  else if (p.causal && n_items > static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM) launch_attention64_order<T16, true, false>(tm, tmo, p, n_items, di, s);
+  else launch_attention64_order<T16, false, false>(tm, tmo, p, n_items, di, s);
 }
 
 template <typename T16, int HD>

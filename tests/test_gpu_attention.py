@@ -143,3 +143,19 @@ def test_causal_item_order(m, heads, head_dim, batch, padded):
         one = m.attention(qkv[b * S:(b + 1) * S], None if lens is None else lens[b:b + 1], 1, S, heads, head_dim, causal=True)
         n = S if lens is None else lens[b]
         assert np.array_equal(got.reshape(batch, S, -1)[b, :n], one.reshape(S, -1)[:n]), b
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S", [1, 31, 33, 64, 99, 128, 129, 200])
+def test_few_items_give_the_same_bits(m, S, causal):
+    """Up to one item an SM a row's scores stay in registers: the bits of a batch that has more, tails of tiles and of pieces
+    of 32 keys, sequences of no tokens and rows beyond the end among them."""
+    rng = np.random.default_rng(S)
+    H, B = 3, 52  # 156 items and more; eight sequences are 24 to 48
+    qkv = rng.standard_normal((B * S, 3, H, 64)).astype(np.float32)
+    lens = rng.integers(0, S + 1, B).astype(np.int32)
+    lens[:3] = 0, S, max(1, S // 2)
+    for ln in (None, lens):
+        many = m.attention(qkv, ln, B, S, H, 64, causal=causal).reshape(B, S, -1)
+        few = m.attention(qkv[:8 * S], None if ln is None else ln[:8], 8, S, H, 64, causal=causal).reshape(8, S, -1)
+        assert np.array_equal(many[:8], few)
