@@ -104,15 +104,23 @@ constexpr int kLnWarpsPerBlock = 4;
 // (short 16-bit rows would otherwise leave too few bytes in flight per SM).  n must be a
 // multiple of EPC, rows 16-byte aligned, and n <= 32 * MAXI * EPC.  Lane l owns chunks
 // l, l+32, ... (coalesced 512-byte warp accesses).
-// FULL: the row is exactly 32 * MAXI chunks, so no lane ever skips a chunk and the per-chunk
+// kLnFull: the row is exactly 32 * MAXI chunks, so no lane ever skips a chunk and the per-chunk
 // tests (and the instructions of chunks that would be predicated off) disappear.
-template <typename TIn, typename TOut, int MAXI, bool RES, bool FULL>
+// kLnFew: such rows, one to a warp.  While they come out of L2 a warp's latency is the kernel's time: without the tests its
+// loads are all in flight, and gamma and beta are asked for with the row instead of behind the statistics; no block
+// budget has the registers spill.  Chained launches, bf16, against the persistent form: 99 x 768 2.51 -> 1.65 us, 99 x 1024
+// 2.60 -> 1.67, 2048 x 768 3.55 -> 2.86, 8192 x 768 7.47 -> 6.46, 12288 x 768 9.41 -> 8.90, 8192 x 1024 8.57 -> 8.33; beyond 10
+// million values the persistent form's prefetch wins: 16384 x 1024 14.0 / 14.7, 131072 x 768 79.8 / 86.7.
+enum LnForm { kLnAny, kLnFull, kLnFew };
+constexpr int64_t kLnFewValues = 10 * 1000 * 1000;
+template <typename TIn, typename TOut, int MAXI, bool RES, int FORM>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32,
-                                  (MAXI >= 8 || sizeof(TIn) == 4) ? 2 : ((RES || (FULL && MAXI >= 4)) ? 4 : 6))
+                                  FORM == kLnFew ? 1 : (MAXI >= 8 || sizeof(TIn) == 4) ? 2 : ((RES || (FORM == kLnFull && MAXI >= 4)) ? 4 : 6))
 layernorm_warp_kernel(const TIn *__restrict__ x, const TIn *__restrict__ residual,
                       const float *__restrict__ gamma, const float *__restrict__ beta,
                       TIn *__restrict__ sum_out, TOut *__restrict__ y, float eps, int64_t m, int n) {
   constexpr int EPC = LnTraits<TIn>::EPC;
+  constexpr bool FULL = FORM != kLnAny, FEW = FORM == kLnFew;
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -122,7 +130,7 @@ layernorm_warp_kernel(const TIn *__restrict__ x, const TIn *__restrict__ residua
   const int nchunks = n / EPC;
   const float inv_n = 1.f / static_cast<float>(n);
   constexpr bool has_res = RES;
-  constexpr bool kPrefetch = sizeof(TIn) == 2;
+  constexpr bool kPrefetch = sizeof(TIn) == 2 && !FEW;
 
   uint4 raw[MAXI], raw_res[RES ? MAXI : 1];
   auto fetch = [&](int64_t rw) {
@@ -142,6 +150,25 @@ layernorm_warp_kernel(const TIn *__restrict__ x, const TIn *__restrict__ residua
     }
   };
   fetch(row);
+  [[maybe_unused]] float4 early_g[FEW ? MAXI : 1][EPC / 4], early_b[FEW ? MAXI : 1][EPC / 4];
+  if constexpr (FEW) {
+#pragma unroll
+    for (int i = 0; i < MAXI; ++i) {
+#pragma unroll
+      for (int e4 = 0; e4 < EPC / 4; ++e4) {
+        if (gamma) early_g[i][e4] = __ldg(reinterpret_cast<const float4 *>(gamma) + (lane + 32 * i) * (EPC / 4) + e4);
+        if (beta) early_b[i][e4] = __ldg(reinterpret_cast<const float4 *>(beta) + (lane + 32 * i) * (EPC / 4) + e4);
+      }
+    }
+  }
+  auto gamma_at = [&](int i, int c, int e4) __attribute__((always_inline)) -> float4 {
+    if constexpr (FEW) return early_g[i][e4];
+    else return __ldg(reinterpret_cast<const float4 *>(gamma) + c * (EPC / 4) + e4);
+  };
+  auto beta_at = [&](int i, int c, int e4) __attribute__((always_inline)) -> float4 {
+    if constexpr (FEW) return early_b[i][e4];
+    else return __ldg(reinterpret_cast<const float4 *>(beta) + c * (EPC / 4) + e4);
+  };
 
   using ptx::F2;
   using ptx::f2;
@@ -220,16 +247,16 @@ layernorm_warp_kernel(const TIn *__restrict__ x, const TIn *__restrict__ residua
         for (int e4 = 0; e4 < EPC / 4; ++e4) {
           F2 y0 = f2_mul(v[i][2 * e4], rstd2), y1 = f2_mul(v[i][2 * e4 + 1], rstd2);
           if (gamma && beta) {
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma) + c * (EPC / 4) + e4);
-            const float4 b = __ldg(reinterpret_cast<const float4 *>(beta) + c * (EPC / 4) + e4);
+            const float4 g = gamma_at(i, c, e4);
+            const float4 b = beta_at(i, c, e4);
             y0 = f2_fma(y0, f2(g.x, g.y), f2(b.x, b.y));
             y1 = f2_fma(y1, f2(g.z, g.w), f2(b.z, b.w));
           } else if (gamma) {
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma) + c * (EPC / 4) + e4);
+            const float4 g = gamma_at(i, c, e4);
             y0 = f2_mul(y0, f2(g.x, g.y));
             y1 = f2_mul(y1, f2(g.z, g.w));
           } else if (beta) {
-            const float4 b = __ldg(reinterpret_cast<const float4 *>(beta) + c * (EPC / 4) + e4);
+            const float4 b = beta_at(i, c, e4);
             y0 = f2_add(y0, f2(b.x, b.y));
             y1 = f2_add(y1, f2(b.z, b.w));
           }
@@ -320,6 +347,17 @@ static void launch_layernorm(const void *x, const void *residual, const float *g
         (sizeof(TIn) == 2 && blocks_needed > blocks_cap) ? blocks_cap : blocks_needed);
     const int threads = kLnWarpsPerBlock * 32;
     const int ni = static_cast<int>(n);
+    if constexpr (sizeof(TIn) == 2) {
+      // (beta alone stays with the other form: there the two are not compiled to the same last bit)
+      if (!ri && (gamma || !beta) && per_lane >= 2 && per_lane <= 4 && nchunks_host == 32 * per_lane && m * n <= kLnFewValues) {
+        auto kern = per_lane == 2 ? layernorm_warp_kernel<TIn, TOut, 2, false, kLnFew>
+                    : per_lane == 3 ? layernorm_warp_kernel<TIn, TOut, 3, false, kLnFew> : layernorm_warp_kernel<TIn, TOut, 4, false, kLnFew>;
+        check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(blocks_needed)), dim3(threads), 0, s, 1, xi, ri, gamma, beta, so, yo, eps, m, ni),
+                   "launch layernorm");
+        launched("layernorm_warp_kernel");
+        return;
+      }
+    }
 #define MDC_LN_LAUNCH2(MAXI_, FULL_)                                                                  \
   do {                                                                                            \
     if (ri)                                                                                       \
@@ -329,8 +367,8 @@ static void launch_layernorm(const void *x, const void *residual, const float *g
   } while (0)
 #define MDC_LN_LAUNCH(MAXI_)                                                                          \
   do {                                                                                            \
-    if (nchunks_host == 32 * (MAXI_) && !(sizeof(TIn) == 2 && (MAXI_) == 3)) MDC_LN_LAUNCH2(MAXI_, true); \
-    else MDC_LN_LAUNCH2(MAXI_, false);                                                            \
+    if (nchunks_host == 32 * (MAXI_) && !(sizeof(TIn) == 2 && (MAXI_) == 3)) MDC_LN_LAUNCH2(MAXI_, kLnFull); \
+    else MDC_LN_LAUNCH2(MAXI_, kLnAny);                                                            \
   } while (0)
     if (per_lane <= 2) MDC_LN_LAUNCH(2);
     else if (per_lane <= 3) MDC_LN_LAUNCH(3);

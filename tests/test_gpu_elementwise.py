@@ -166,3 +166,18 @@ def test_layernorm_16bit_large(m, rows, n, dtype_name):
     tol = 2 ** -9 if dt == m.F16 else 2 ** -6  # one output ulp at |y| < 8
     assert np.max(np.abs(y16 - ref)) <= tol
     assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+
+
+@pytest.mark.parametrize("affine", ["both", "gamma", "beta", "none"])
+@pytest.mark.parametrize("n", [512, 768, 1024])
+def test_layernorm_16bit_rows_do_not_depend_on_their_number(m, n, affine):
+    # one row to a warp up to ten million values, persistent warps beyond
+    rng = np.random.default_rng(n)
+    rows = 10_000_000 // n + 3
+    x = m.encode16(rng.standard_normal((rows, n)).astype(np.float32), m.F16)
+    g = (1 + 0.1 * rng.standard_normal(n)).astype(np.float32) if affine in ("both", "gamma") else None
+    b = (0.1 * rng.standard_normal(n)).astype(np.float32) if affine in ("both", "beta") else None
+    for out in (m.F16, m.F32):
+        whole = m.layernorm(x, g, b, 1e-5, io_dtype=m.F16, out_dtype=out)
+        for few in (1, 5, 593, 4097):
+            assert np.array_equal(m.layernorm(x[:few], g, b, 1e-5, io_dtype=m.F16, out_dtype=out), whole[:few]), few
