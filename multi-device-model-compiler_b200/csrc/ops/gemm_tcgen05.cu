@@ -706,7 +706,14 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
     t = choose_one_wave(M, N, K, sms);
-  if (!t.one_wave) {
+  // A long K in tiles of 128 columns: the persistent kernel's ring of single k-blocks turns faster than one of several, where
+  // its pairs of 256 x 128 come in one round.  One-wave / persistent, us: 2341 x 768 x 3072 14.6 / 13.3, 1711 x 1024 x 3712 17.1 / 15.3,
+  // 1718 x 1024 x 4096 18.1 / 16.3, 2978 x 768 x 1920 11.0 / 10.1; below K = 1400 0.98 of the time instead, and with tiles of 96
+  // columns 1.0, of 64 0.88.
+  if (t.one_wave && t.bn >= 128 && K >= 1400 && M > gemm::BM && ((M + 255) / 256) * ((N + 127) / 128) <= sms / 2) {
+    t = GemmTile();
+    t.cg = 2, t.bn = 128;
+  } else if (!t.one_wave) {
     t.cg = choose_cta_group(M);
     t.bn = choose_bn(M, N, t.cg, sms);
   }

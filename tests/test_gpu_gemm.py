@@ -405,6 +405,25 @@ def test_few_rows_off_their_boundaries(m, offset):
     assert np.array_equal(got, a @ w + b)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1000, 2496), (8, 1000, 2500), (9, 2000, 6000), (17, 1000, 2333), (41, 2400, 7001), (57, 1000, 2499), (64, 2400, 7168)])
+def test_few_rows_rings_are_exact(m, M, N, K):
+    # boxes of 8 to 64 rows, rings of 8 stages to 24 that go round, both widths of a CTA, the last stage partly past K
+    rng = np.random.default_rng(53)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b = rng.integers(-4, 5, N).astype(np.float32)
+    assert np.array_equal(m.matmul(a, w, b), a @ w + b)
+
+
+@pytest.mark.parametrize("M,N,K", [(2341, 768, 3072), (1711, 1024, 1400), (2399, 720, 1400), (300, 4090, 1408), (2976, 768, 1408), (2977, 768, 1392)])
+def test_one_round_of_pairs_is_exact(m, M, N, K):
+    # either side of the line between one-wave tiles of 128 columns and one round of the persistent kernel
+    rng = np.random.default_rng(59)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b, r = rng.integers(-4, 5, N).astype(np.float32), rng.integers(-8, 9, (M, N)).astype(np.float32)
+    got = m.matmul16(a, w, bias=b, residual=r, out_dtype=m.F32, act=m.ACT_RELU)
+    assert np.array_equal(got, np.maximum(a @ w + b, 0) + r)
+
+
 @pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
 @pytest.mark.parametrize("M,N,K", [(16, 1000, 1024), (40, 2400, 500)])
 def test_output_may_overlap_the_weight(m, entry, M, N, K):
