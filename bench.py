@@ -62,9 +62,9 @@ def bytes_touched_per_step(batch):
 # residual, output) scaled and the weights kept.
 GEMM_DRAM_TRAFFIC = {
     # tokens: {shape: bytes}
-    32768: {"gemm_qkv": 53904640 + 99526400, "gemm_proj": 51540224 + 11512576,
-            "gemm_ffn1": 55092992 + 148391424, "gemm_ffn2": 206821632 + 36534272},
-    4096: {"gemm_qkv": 9863168, "gemm_proj": 7498240, "gemm_ffn1": 11051264, "gemm_ffn2": 29911296},
+    32768: {"gemm_qkv": 53913600 + 98738176, "gemm_proj": 51549440 + 11584512,
+            "gemm_ffn1": 55092736 + 150355712, "gemm_ffn2": 206891264 + 36219392},
+    4096: {"gemm_qkv": 9873152, "gemm_proj": 7507456, "gemm_ffn1": 11049472, "gemm_ffn2": 29927168},
 }
 
 

@@ -700,9 +700,9 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
                     static_cast<uint64_t>(K) * 0x165667B19E3779F9ull) >> 58];
   if (e.M == M && e.N == N && e.K == K && e.sms == sms) return e.tile;
   GemmTile t;
-  // One wave: up to one 128 x 128 tile per SM.  Measured either side of the line: 1024 x 2304 x 768
-  // 7.6 us one-wave, 7.9 persistent; 1024 x 3072 x 768 9.9 and 9.2; 2048 x 768 x 3072 14.1 and 15.5;
-  // 4096 x 768 x 3072 19.2 and 17.6.
+  // One wave: up to one 128 x 128 tile per SM.  One-wave / persistent, us, at the line: 991 x 2304 x 768 with residual 7.2 / 7.4,
+  // 676 x 3072 x 768 6.6 / 6.9, 2841 x 768 x 768 6.5 / 6.8, 2433 x 768 x 768 with residual 7.10 / 7.04; beyond it the persistent
+  // kernel takes 0.94 of the best one-wave tile's time.
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
     t = choose_one_wave(M, N, K, sms);
