@@ -46,9 +46,9 @@ namespace mdc {
 namespace convp {
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int MAX_STAGES = 12;
+constexpr int MAX_STAGES = kRingMaxStages;
 constexpr int EPI_WARPS = 8;
-constexpr int GATHER_GROUPS = 3, GATHER_WARPS = GATHER_GROUPS * 4;
+constexpr int GATHER_GROUPS = kGatherGroups, GATHER_WARPS = GATHER_GROUPS * 4;
 constexpr size_t kMaxSmem = 224 * 1024;
 // warps: 0-7 epilogue, 8 TMA, 9 MMA, then the gather warps
 constexpr int threads(bool gather) { return (EPI_WARPS + 2 + (gather ? GATHER_WARPS : 0)) * 32; }
@@ -295,8 +295,8 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     const uint32_t row_off = static_cast<uint32_t>(row) * 128u, swz = static_cast<uint32_t>(row & 7);
     const int KH = p.taps / p.KW, max_dh = (KH - 1) * p.DH, max_dw = (p.KW - 1) * p.DW;
     int block = group, tile_block = 0;  // this group's next k-block, and the tile's first, counted over all tiles of the CTA
-    int stage = group % p.stages;
-    uint32_t phase = static_cast<uint32_t>(group / p.stages) & 1u;
+    int stage = group;  // (no fewer stages than groups: conv_ring_stages)
+    uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, tile_block += p.num_kb) {
       if (block >= tile_block + p.num_kb) continue;  // short patches: not every tile has one for every group
@@ -382,7 +382,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         __syncwarp();
         if (lane == 0) mbar_arrive(&full_bar[stage]);
         stage += GATHER_GROUPS;
-        while (stage >= p.stages) stage -= p.stages, phase ^= 1;
+        if (stage >= p.stages) stage -= p.stages, phase ^= 1;
       }
     }
   }
@@ -584,11 +584,8 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   p.resident = conv_filter_stays(num_kb, p.bn, p.n_tiles, p.num_tiles, di.sms);
   const int64_t stage_bytes = A_BYTES + (p.resident ? 0 : p.bn * BK * 2);
   const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128;
-  int64_t stages = (static_cast<int64_t>(kMaxSmem) - 4096 - fixed) / stage_bytes;
-  // gathered patches are read nine-fold through L1: leave it most of the memory
-  const int64_t cap = gather ? 4 : MAX_STAGES;
-  p.stages = int(stages < cap ? stages : cap);
-  if (p.stages < 2) return false;
+  p.stages = conv_ring_stages(static_cast<int64_t>(kMaxSmem) - 4096 - fixed, stage_bytes, gather);
+  if (p.stages == 0) return false;
   const size_t smem = static_cast<size_t>(fixed + p.stages * stage_bytes);
   p.err = device_error_slot();
   if (!p.err) return true;

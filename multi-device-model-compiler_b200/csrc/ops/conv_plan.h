@@ -134,6 +134,18 @@ inline bool conv_filter_stays(int64_t num_kb, int bn, int64_t n_tiles, int64_t t
   return n_tiles == 1 && tiles > sms && num_kb * bn * 128 <= 100 * 1024;
 }
 
+constexpr int kRingMaxStages = 12;
+constexpr int kGatherGroups = 3;  // of four warps, that gather alternate k-blocks
+// Stages of the persistent kernels' ring in `room` bytes; 0: too few.  Gathered patches are read nine-fold through L1, which
+// keeps most of the memory.  A group gathers every third k-block and waits for its stage's previous use by parity alone: it
+// knows that the block which its last one replaced has been used, three blocks and the ring back, so with fewer stages than
+// groups the use before the previous one would pass for it.
+inline int conv_ring_stages(int64_t room, int64_t stage_bytes, bool gather) {
+  const int64_t least = gather ? kGatherGroups : 2, most = gather ? 4 : kRingMaxStages;
+  const int64_t n = std::min(room / stage_bytes, most);
+  return n < least ? 0 : static_cast<int>(n);
+}
+
 // How conv_halo_kernel runs a call: in a copy of the input or directly (see there), by rect or flat tiles.
 enum class ConvForm { kOther, kCopyRect, kCopyFlat, kDirectRect, kDirectFlat };
 inline bool form_copies(ConvForm f) { return f == ConvForm::kCopyRect || f == ConvForm::kCopyFlat; }

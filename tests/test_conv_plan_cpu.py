@@ -171,3 +171,40 @@ def test_rows_of_the_gpu_tests_reach_their_kernels(tmp_path):
     assert len(told) == len(rows)
     assert not [(want, got, row) for (want, row), got in zip(rows, told) if want != got]
     assert set(told) == {"kOther", "kCopyRect", "kCopyFlat", "kDirectRect", "kDirectFlat"}
+
+
+RING = r"""
+#include "conv_plan.h"
+#include <cassert>
+#include <cstdio>
+using namespace mdc;
+int main() {
+  // A group's wait at block b, its last block b - 3 let in: blocks up to b - 3 - stages are known to be used, and any
+  // number more.  What passes a wait by parity must be the use that is waited for.
+  auto safe = [](int stages) {
+    for (int b = 3; b < 200; ++b)
+      for (int used = b - kGatherGroups - stages + 1; used <= b; ++used) {
+        const int use = b / stages, of = b % stages, done = used <= of ? 0 : (used - of - 1) / stages + 1;  // of b's stage
+        if ((done & 1) == (use & 1) && done < use) return false;
+      }
+    return true;
+  };
+  assert(!safe(1) && !safe(2) && safe(3) && safe(4));
+  for (int64_t room = 0; room < 300 * 1024; room += 512)
+    for (int64_t stage : {16384, 16384 + 32 * 128, 16384 + 256 * 128}) {
+      const int gather = conv_ring_stages(room, stage, true), im2col = conv_ring_stages(room, stage, false);
+      assert(gather == 0 || (safe(gather) && gather * stage <= room && gather <= 4));
+      assert(im2col == 0 || (im2col >= 2 && im2col * stage <= room && im2col <= kRingMaxStages));
+      assert((gather == 0) == (room / stage < 3) && (im2col == 0) == (room / stage < 2));
+    }
+  puts("ok");
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or not os.path.isdir(CUDA_INCLUDE), reason="no host compiler or CUDA headers")
+def test_a_gathered_ring_has_a_stage_for_every_group(tmp_path):
+    src, exe = tmp_path / "ring.cpp", str(tmp_path / "ring")
+    src.write_text(RING)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout == "ok\n"
