@@ -42,6 +42,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "gemm_common.cuh"
 #include "ops_common.h"
 #include "ptx_sm100.cuh"
 
@@ -508,8 +509,11 @@ __device__ __forceinline__ AttnItem64 attn_item64(const AttnParams &p, int item,
 //
 // kFew: no more items than SMs.  Then one item's latency is the kernel's time and a CTA has an SM's registers: a row's scores are
 // read once, all in flight, and kept (the three-CTA form reads them twice, 32 at a time where a tile is partly visible), and
-// the output goes from registers to memory, without the way through shared memory and TMA.  The same operations in the
-// same order.  1 x 99 tokens, 12 heads, causal 5.41 -> 4.95 us, 8 x 64 5.18 -> 4.41, 1 x 512 causal 12.1 -> 11.8.
+// the output goes from registers to memory in whole sectors, without the way through shared memory and TMA.  The same operations in the
+// same order.  Three-CTA form / this one, us in a chain of launches: 1 x 99 tokens, 12 heads, causal 5.55 / 4.72, 8 x 64 5.15 / 4.42,
+// 1 x 512 10.9 / 10.6, causal 12.0 / 10.8, 1 x 4096, 4 heads 79 / 66, causal 68 / 65; of 33 shapes none slower.  A test per score for the
+// mask, whole tiles too, and stores of half a sector cost it what it gains: 1 x 128, 12 heads 4.53 -> 5.19 (three-CTA form 4.55),
+// 1 x 256 6.55 -> 7.59 (6.6), 1 x 16384, one head, causal 246 -> 281 (256).
 template <typename T16, bool kOuter, bool kFew>
 __global__ void __launch_bounds__(attn64::THREADS, kFew ? 1 : attn64::CTAS_PER_SM)
 attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
@@ -683,17 +687,21 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
 #pragma unroll
           for (int c = 0; c < BKV / 32; ++c)
             if (c * 32 < n_max) tmem_ld_32x32(tmem_base + lane_addr + S_COL + c * 32, sc[c]);
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int c = 0; c < BKV / 32; ++c) {
             if (c * 32 < n_max) {
               tmem_ld_wait_regs(sc[c]);
+              if (!full_tile) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                if (!full_tile && c * 32 + i >= ncol) sc[c][i] = 0xff800000u;
-                m_tile = fmaxf(m_tile, __uint_as_float(sc[c][i]));
+                for (int i = 0; i < 32; ++i)
+                  if (c * 32 + i >= ncol) sc[c][i] = 0xff800000u;
               }
+#pragma unroll
+              for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(sc[c][i]));
             }
           }
+          m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         } else if (full_tile) {
           // 16 columns at a time, the next load in flight while the current piece is reduced
           uint32_t sa[16], sb[16];
@@ -833,10 +841,12 @@ attention_d64_kernel(const __grid_constant__ CUtensorMap tmap_qkv,
           if (q_local < p.seq) {
             T16 *dst = static_cast<T16 *>(p.out) + (static_cast<int64_t>(it.b) * p.seq + q_local) * hd + it.head * D;
 #pragma unroll
-            for (int g = 0; g < D / 8; ++g)
-              *reinterpret_cast<uint4 *>(dst + 8 * g) =
-                  make_uint4(pack16<T16>(o_acc[8 * g + 0] * inv, o_acc[8 * g + 1] * inv), pack16<T16>(o_acc[8 * g + 2] * inv, o_acc[8 * g + 3] * inv),
-                             pack16<T16>(o_acc[8 * g + 4] * inv, o_acc[8 * g + 5] * inv), pack16<T16>(o_acc[8 * g + 6] * inv, o_acc[8 * g + 7] * inv));
+            for (int g = 0; g < D / 16; ++g) {
+              uint32_t o[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = pack16<T16>(o_acc[16 * g + 2 * i] * inv, o_acc[16 * g + 2 * i + 1] * inv);
+              st_global_32B(dst + 16 * g, o);
+            }
           }
           continue;
         }
@@ -894,7 +904,8 @@ static void launch_attention64_order(const CUtensorMap &tm, const CUtensorMap &t
 template <typename T16>
 static void launch_attention64(const CUtensorMap &tm, const CUtensorMap &tmo, const AttnParams &p, int64_t n_items,
                                const DeviceInfo &di, cudaStream_t s) {
-  if (n_items <= di.sms) launch_attention64_order<T16, false, true>(tm, tmo, p, n_items, di, s);
+  // (rows of the few items' form leave in sectors: the output lies on one)
+  if (n_items <= di.sms && (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0) launch_attention64_order<T16, false, true>(tm, tmo, p, n_items, di, s);
   else if (p.causal && n_items > static_cast<int64_t>(di.sms) * attn64::CTAS_PER_SM) launch_attention64_order<T16, true, false>(tm, tmo, p, n_items, di, s);
   else launch_attention64_order<T16, false, false>(tm, tmo, p, n_items, di, s);
 }

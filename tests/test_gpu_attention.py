@@ -159,3 +159,19 @@ def test_few_items_give_the_same_bits(m, S, causal):
         many = m.attention(qkv, ln, B, S, H, 64, causal=causal).reshape(B, S, -1)
         few = m.attention(qkv[:8 * S], None if ln is None else ln[:8], 8, S, H, 64, causal=causal).reshape(8, S, -1)
         assert np.array_equal(many[:8], few)
+
+
+@pytest.mark.parametrize("offset", [16, 32])
+def test_few_items_off_a_sector(m, offset):
+    """An output off a 32-byte boundary stays with the form that stores by TMA; nothing beside it is written."""
+    B, S, H = 2, 131, 3
+    rng = np.random.default_rng(offset)
+    qkv = m.to_device(m.encode16(rng.standard_normal((B * S, 3 * H * 64)).astype(np.float32), m.F16))
+    n = B * S * H * 64
+    whole, moved = m.DeviceBuffer(2 * n), m.to_device(np.full(n + 64, 0x5a5a, np.uint16))
+    m.ops().mgpuAttention(qkv.ptr, None, whole.ptr, B, S, H, 64, True, m.F16, None)
+    m.ops().mgpuAttention(qkv.ptr, None, moved.ptr + offset, B, S, H, 64, True, m.F16, None)
+    got, first = m.to_host(moved, (n + 64,), np.uint16), offset // 2
+    m.check("mgpuAttention")
+    assert np.array_equal(got[first:first + n], m.to_host(whole, (n,), np.uint16))
+    assert (got[:first] == 0x5a5a).all() and (got[first + n:] == 0x5a5a).all()
