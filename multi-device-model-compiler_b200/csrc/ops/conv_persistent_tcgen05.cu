@@ -66,22 +66,14 @@ struct Params {
   uint32_t *err;
 };
 // Where the patches come from.  Where a gathered k lies is read from the constant bank: kGather for patches of up to
-// TAP_TABLE values, windows of up to 16 x 15 taps and inputs that 32 bits address, kGatherFar for the others.
+// kNearTaps values, windows of up to 16 x 15 taps and inputs that 32 bits address (conv_taps_near), kGatherFar for the others.
 enum Source { kIm2col, kGather, kGatherFar };
-constexpr int TAP_TABLE = 256;
 template <int kSource>
 struct Taps {};
 template <>
-struct Taps<kGather> {
-  uint32_t lead;             // bytes that a window may begin ahead of the input
-  uint32_t off[TAP_TABLE];   // bytes of k from the window's origin
-  uint32_t need[TAP_TABLE];  // bits 0-15 its row of the window, 16-30 its column; beyond the patch bit 31
-};
+struct Taps<kGather> : NearTaps {};
 template <>
-struct Taps<kGatherFar> {
-  uint32_t off[kDenseMaxGatherK];  // elements from the window's origin
-  uint32_t pos[kDenseMaxGatherK];  // row of the input from the origin's << 16 | column
-};
+struct Taps<kGatherFar> : FarTaps {};
 }  // namespace convp
 
 // The value where `in`, else zero; never a branch.
@@ -578,9 +570,6 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
   p.tmem_cols = 32;
   while (p.tmem_cols < 2u * p.bn) p.tmem_cols *= 2;
   const int64_t filter_bytes = num_kb * p.bn * BK * 2;
-  const bool near = K <= TAP_TABLE && c.KH <= 16 && c.KW <= 15 &&
-                    (c.N * c.IC * c.H * c.W + c.PHL * c.W + c.PWL) * 4 < (int64_t(1) << 32) &&
-                    (((c.IC - 1) * c.H + (c.KH - 1) * c.DH) * c.W + (c.KW - 1) * c.DW) * 4 < (int64_t(1) << 32);
   p.resident = conv_filter_stays(num_kb, p.bn, p.n_tiles, p.num_tiles, di.sms);
   const int64_t stage_bytes = A_BYTES + (p.resident ? 0 : p.bn * BK * 2);
   const int64_t fixed = 1024 + (p.resident ? filter_bytes : 0) + (c.OC + 31) / 32 * 128;
@@ -617,22 +606,13 @@ bool conv_persistent(const ConvShape &call, cudaStream_t s) {
     auto launch = [&](const auto &t) { p.add ? launch_persistent<true>(tx, tw, p, t, smem, di.sms, s) : launch_persistent<false>(tx, tw, p, t, smem, di.sms, s); };
     if (!gather) {
       launch(Taps<kIm2col>());
-    } else if (near) {
+    } else if (conv_taps_near(c)) {
       Taps<kGather> t;
-      t.lead = static_cast<uint32_t>((c.PHL * c.W + c.PWL) * 4);
-      for (int64_t k = 0; k < num_kb * BK; ++k) {
-        const int64_t ic = k / window, kh = k % window / c.KW, kw = k % window % c.KW;
-        t.off[k] = k < K ? static_cast<uint32_t>(((ic * c.H + kh * c.DH) * c.W + kw * c.DW) * 4) : 0;
-        t.need[k] = k < K ? 1u << kh | 0x10000u << kw : 0x80000000u;
-      }
+      fill_taps(c, &t);
       launch(t);
     } else {
       Taps<kGatherFar> t;
-      for (int64_t k = 0; k < num_kb * BK; ++k) {
-        const int64_t ic = k / window, kh = k % window / c.KW, kw = k % window % c.KW;
-        t.off[k] = k < K ? static_cast<uint32_t>((ic * c.H + kh * c.DH) * c.W + kw * c.DW) : 0;
-        t.pos[k] = k < K ? static_cast<uint32_t>(kh * c.DH << 16 | kw * c.DW) : 0;
-      }
+      fill_taps(c, &t);
       launch(t);
     }
   }

@@ -146,6 +146,49 @@ inline int conv_ring_stages(int64_t room, int64_t stage_bytes, bool gather) {
   return n < least ? 0 : static_cast<int>(n);
 }
 
+// Where the values k of a gathered patch lie, as kernel arguments.  Near: in bytes from the window's origin, and which row and
+// column of the window have to lie inside the input; one 32-bit sum of an offset and an origin reaches any value, counted from
+// `lead` bytes ahead of the input, where the first window may begin.
+constexpr int kNearTaps = 256;
+struct NearTaps {
+  uint32_t lead;
+  uint32_t off[kNearTaps];
+  uint32_t need[kNearTaps];  // bits 0-15 the row, 16-30 the column; beyond the patch bit 31
+};
+// Far: in elements from the window's origin, and the row of the input from the origin's << 16 | the column.
+struct FarTaps {
+  uint32_t off[kDenseMaxGatherK];
+  uint32_t pos[kDenseMaxGatherK];
+};
+inline bool conv_taps_near(const ConvShape &c) {
+  return c.IC * c.KH * c.KW <= kNearTaps && c.KH <= 16 && c.KW <= 15 &&
+         (c.N * c.IC * c.H * c.W + c.PHL * c.W + c.PWL) * 4 < (int64_t(1) << 32) &&
+         (((c.IC - 1) * c.H + (c.KH - 1) * c.DH) * c.W + (c.KW - 1) * c.DW) * 4 < (int64_t(1) << 32);
+}
+// The tables' entries up to the patch's end in whole eights, which is as far as they are read.  On every call, so counted up: a
+// division an entry is time that a small call has no GPU work to hide behind.  Host time of a call with 27 / 135 / 960 values 8.25 /
+// 8.88 / 13.9 us with divisions, 8.12 / 8.23 / 8.90 so, 7.97 / 8.00 / 7.89 when the GPU filled a table of its own; the tables' bytes,
+// 512 instead of 2048, make no difference.
+inline void fill_taps(const ConvShape &c, NearTaps *t) {
+  t->lead = static_cast<uint32_t>((c.PHL * c.W + c.PWL) * 4);
+  int64_t k = 0;
+  for (int64_t ic = 0; ic < c.IC; ++ic)
+    for (int64_t kh = 0; kh < c.KH; ++kh) {
+      const uint32_t row = static_cast<uint32_t>((ic * c.H + kh * c.DH) * c.W * 4);
+      for (int64_t kw = 0; kw < c.KW; ++kw, ++k) t->off[k] = row + static_cast<uint32_t>(kw * c.DW * 4), t->need[k] = 1u << kh | 0x10000u << kw;
+    }
+  for (; k % 8; ++k) t->off[k] = 0, t->need[k] = 0x80000000u;
+}
+inline void fill_taps(const ConvShape &c, FarTaps *t) {
+  int64_t k = 0;
+  for (int64_t ic = 0; ic < c.IC; ++ic)
+    for (int64_t kh = 0; kh < c.KH; ++kh) {
+      const uint32_t row = static_cast<uint32_t>((ic * c.H + kh * c.DH) * c.W), pos = static_cast<uint32_t>(kh * c.DH << 16);
+      for (int64_t kw = 0; kw < c.KW; ++kw, ++k) t->off[k] = row + static_cast<uint32_t>(kw * c.DW), t->pos[k] = pos | static_cast<uint32_t>(kw * c.DW);
+    }
+  for (; k % 8; ++k) t->off[k] = t->pos[k] = 0;
+}
+
 // How conv_halo_kernel runs a call: in a copy of the input or directly (see there), by rect or flat tiles.
 enum class ConvForm { kOther, kCopyRect, kCopyFlat, kDirectRect, kDirectFlat };
 inline bool form_copies(ConvForm f) { return f == ConvForm::kCopyRect || f == ConvForm::kCopyFlat; }

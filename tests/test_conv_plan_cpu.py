@@ -208,3 +208,64 @@ def test_a_gathered_ring_has_a_stage_for_every_group(tmp_path):
     src.write_text(RING)
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
     assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout == "ok\n"
+
+
+TAPS = r"""
+#include "conv_plan.h"
+#include <cassert>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+using namespace mdc;
+int main() {
+  srand(3);
+  auto pick = [](int lo, int hi) { return lo + rand() % (hi - lo + 1); };
+  int nears = 0, fars = 0;
+  for (int i = 0; i < 20000; ++i) {
+    ConvShape c = {};
+    c.IC = pick(1, 15), c.KH = pick(1, 9) * (i % 7 ? 1 : 2), c.KW = pick(1, 9) * (i % 11 ? 1 : 2), c.DH = pick(1, 40), c.DW = pick(1, 40);
+    c.H = pick(1, 300), c.W = pick(1, 300), c.N = pick(1, 5), c.PHL = pick(0, 50), c.PWL = pick(0, 50);
+    const int64_t K = c.IC * c.KH * c.KW;
+    if (K > kDenseMaxGatherK) continue;
+    static NearTaps n;
+    static FarTaps f;
+    memset(&n, 0xee, sizeof n), memset(&f, 0xee, sizeof f);
+    const bool near = conv_taps_near(c);
+    assert(near == (K <= 256 && c.KH <= 16 && c.KW <= 15));
+    if (near) fill_taps(c, &n), ++nears, assert(n.lead == (c.PHL * c.W + c.PWL) * 4);
+    fill_taps(c, &f), ++fars;
+    for (int64_t k = 0; k < (K + 7) / 8 * 8; ++k) {
+      const int64_t ic = k / (c.KH * c.KW), kh = k / c.KW % c.KH, kw = k % c.KW, off = (ic * c.H + kh * c.DH) * c.W + kw * c.DW;
+      assert(f.off[k] == (k < K ? off : 0) && f.pos[k] == (k < K ? (kh * c.DH) << 16 | (kw * c.DW) : 0));
+      if (near) assert(n.off[k] == (k < K ? off * 4 : 0) && n.need[k] == (k < K ? 1u << kh | 0x10000u << kw : 0x80000000u));
+    }
+  }
+  assert(nears > 1000 && fars > nears);
+  // where 32 bits end: the last value of the input from `lead` bytes ahead of it, and the last tap from a window's origin
+  ConvShape c = {};
+  c.N = 4, c.IC = 4, c.H = 8192, c.W = 8191, c.KH = c.KW = 3, c.DH = c.DW = 1;
+  for (int64_t w = 8191; w <= 8192; ++w)
+    for (int64_t ph : {0, 1, 2, 15})
+      for (int64_t pw : {0, 1, 7}) {
+        c.W = w, c.PHL = ph, c.PWL = pw;
+        assert(conv_taps_near(c) == ((c.N * c.IC * c.H * w + ph * w + pw) * 4 <= 0xffffffffll));
+      }
+  c.PHL = c.PWL = 0, c.W = 8191;
+  for (; c.PHL < 32; ++c.PHL) assert(conv_taps_near(c) == (c.PHL <= 16));  // 131072 values of 2^30 left, 16 rows and 16 values
+  c.N = 1, c.IC = 15, c.H = 8192, c.W = 8192, c.PHL = 0;
+  for (int64_t d : {1, 5000, 8191, 8192, 16383, 16384}) {
+    c.DH = d;
+    assert(conv_taps_near(c) == (((14 * 8192 + 2 * d) * 8192 + 2) * 4 <= 0xffffffffll));
+  }
+  puts("ok");
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or not os.path.isdir(CUDA_INCLUDE), reason="no host compiler or CUDA headers")
+def test_taps_of_a_gathered_patch(tmp_path):
+    """The tables are counted up: each entry against the division that defines it, and the line to 64-bit addresses."""
+    src, exe = tmp_path / "taps.cpp", str(tmp_path / "taps")
+    src.write_text(TAPS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", OPS, "-I", CUDA_INCLUDE, str(src), "-o", exe], check=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout == "ok\n"

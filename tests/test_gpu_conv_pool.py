@@ -480,6 +480,32 @@ def test_pool_kernel_forms(m, case, method, offset):
         assert np.max(np.abs(got - ref)) <= 1e-6 * max(1.0, kernel[0] * kernel[1] / 9)
 
 
+@pytest.mark.parametrize("width", [8191, 8192])
+def test_conv_either_side_of_32_bit_addresses(m, width):
+    """A gathered input of 4 GB less 128 KB, and of 4 GB: the ends of it, everything between is zero."""
+    N, H, OC, stride = 16, 8192, 8, 16
+    rng = np.random.default_rng(width)
+    ends = rng.integers(-3, 4, (2, H, width)).astype(np.float32)
+    w, b = rng.integers(-2, 3, (OC, 1, 3, 3)).astype(np.float32), rng.integers(-4, 5, OC).astype(np.float32)
+    OH, OW = H // stride, (width - 1) // stride + 1
+    x, out = m.DeviceBuffer(4 * N * H * width), m.DeviceBuffer(4 * N * OC * OH * OW)
+    dw, db = m.to_device(w), m.to_device(b)
+    m.runtime().mgpuMemset32(x.ptr, 0, N * H * width, None)
+    for image, at in ((0, 0), (1, N - 1)):
+        m.runtime().mgpuMemcpy(x.ptr + 4 * at * H * width, ends[image].ctypes.data, ends[image].nbytes, None)
+    m.ops().mgpuConv2d(x.ptr, dw.ptr, db.ptr, out.ptr, None, N, 1, H, width, OC, 3, 3, OH, OW, 1, 1, 1, 1, stride, stride, 1, 1, False, False, None)
+    got = m.to_host(out, (N, OC, OH, OW), np.float32)
+    assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
+    x.release()
+    padded = np.pad(ends, ((0, 0), (1, stride), (1, stride)))
+    ref = np.zeros((2, OC, OH, OW), np.float32) + b[None, :, None, None]
+    for kh in range(3):
+        for kw in range(3):
+            ref += w[None, :, 0, kh, kw, None, None] * padded[:, None, kh:kh + stride * OH:stride, kw:kw + stride * OW:stride]
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(got[-1], ref[1])
+    assert (got[1:-1] == b[None, :, None, None]).all()
+
+
 def test_pool_special_values(m):
     x = np.zeros((1, 1, 4, 4), np.float32)
     x[0, 0, 0, 0] = -np.inf
