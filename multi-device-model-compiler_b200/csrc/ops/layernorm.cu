@@ -257,8 +257,12 @@ layernorm_warp_kernel(const TIn *__restrict__ x, const TIn *__restrict__ residua
             y1 = f2_mul(y1, f2(g.z, g.w));
           } else if (beta) {
             const float4 b = beta_at(i, c, e4);
-            y0 = f2_add(y0, f2(b.x, b.y));
-            y1 = f2_add(y1, f2(b.z, b.w));
+            // Scalar additions come out the same in every form of this kernel.  Packed ones after the packed multiplication had
+            // another last bit in kLnFew than in the other forms (29 % of all values), and so had y * 1 + beta.
+            float t0, t1, t2, t3;
+            f2_get(y0, t0, t1), f2_get(y1, t2, t3);
+            y0 = f2(__fadd_rn(t0, b.x), __fadd_rn(t1, b.y));
+            y1 = f2(__fadd_rn(t2, b.z), __fadd_rn(t3, b.w));
           }
           f2_get(y0, o[4 * e4 + 0], o[4 * e4 + 1]);
           f2_get(y1, o[4 * e4 + 2], o[4 * e4 + 3]);
@@ -348,8 +352,7 @@ static void launch_layernorm(const void *x, const void *residual, const float *g
     const int threads = kLnWarpsPerBlock * 32;
     const int ni = static_cast<int>(n);
     if constexpr (sizeof(TIn) == 2) {
-      // (beta alone stays with the other form: there the two are not compiled to the same last bit)
-      if (!ri && (gamma || !beta) && per_lane >= 2 && per_lane <= 4 && nchunks_host == 32 * per_lane && m * n <= kLnFewValues) {
+      if (!ri && per_lane >= 2 && per_lane <= 4 && nchunks_host == 32 * per_lane && m * n <= kLnFewValues) {
         auto kern = per_lane == 2 ? layernorm_warp_kernel<TIn, TOut, 2, false, kLnFew>
                     : per_lane == 3 ? layernorm_warp_kernel<TIn, TOut, 3, false, kLnFew> : layernorm_warp_kernel<TIn, TOut, 4, false, kLnFew>;
         check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(blocks_needed)), dim3(threads), 0, s, 1, xi, ri, gamma, beta, so, yo, eps, m, ni),

@@ -168,16 +168,26 @@ def test_layernorm_16bit_large(m, rows, n, dtype_name):
     assert m.ops().mgpuOpsCheckDeviceStatus(None) == 0
 
 
+@pytest.mark.parametrize("dtype_name", ["f16", "bf16"])
 @pytest.mark.parametrize("affine", ["both", "gamma", "beta", "none"])
 @pytest.mark.parametrize("n", [512, 768, 1024])
-def test_layernorm_16bit_rows_do_not_depend_on_their_number(m, n, affine):
+def test_layernorm_16bit_rows_do_not_depend_on_their_number(m, n, affine, dtype_name):
     # one row to a warp up to ten million values, persistent warps beyond
     rng = np.random.default_rng(n)
-    rows = 10_000_000 // n + 3
-    x = m.encode16(rng.standard_normal((rows, n)).astype(np.float32), m.F16)
+    rows, dt = 10_000_000 // n + 3, m.F16 if dtype_name == "f16" else m.BF16
+    x = m.encode16(rng.standard_normal((rows, n)).astype(np.float32), dt)
     g = (1 + 0.1 * rng.standard_normal(n)).astype(np.float32) if affine in ("both", "gamma") else None
     b = (0.1 * rng.standard_normal(n)).astype(np.float32) if affine in ("both", "beta") else None
-    for out in (m.F16, m.F32):
-        whole = m.layernorm(x, g, b, 1e-5, io_dtype=m.F16, out_dtype=out)
+    for out in (dt, m.F32):
+        whole = m.layernorm(x, g, b, 1e-5, io_dtype=dt, out_dtype=out)
         for few in (1, 5, 593, 4097):
-            assert np.array_equal(m.layernorm(x[:few], g, b, 1e-5, io_dtype=m.F16, out_dtype=out), whole[:few]), few
+            assert np.array_equal(m.layernorm(x[:few], g, b, 1e-5, io_dtype=dt, out_dtype=out), whole[:few]), few
+
+
+@pytest.mark.parametrize("rows", [5, 13100])
+def test_layernorm_beta_alone_is_one_addition(m, rows):
+    """Beta is added to the rounded normalised value, however many rows there are."""
+    rng = np.random.default_rng(rows)
+    x, b = m.encode16(rng.standard_normal((rows, 768)).astype(np.float32), m.F16), rng.standard_normal(768).astype(np.float32)
+    plain = m.layernorm(x, None, None, 1e-5, io_dtype=m.F16, out_dtype=m.F32)
+    assert np.array_equal(m.layernorm(x, None, b, 1e-5, io_dtype=m.F16, out_dtype=m.F32), plain + b)
