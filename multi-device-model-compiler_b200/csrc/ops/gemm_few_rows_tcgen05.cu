@@ -28,7 +28,6 @@ namespace fewrows {
 constexpr int LOAD_WARPS = 8;
 // with the input converted here, as many warps again for it
 constexpr int threads(bool convert) { return 64 + LOAD_WARPS * (convert ? 64 : 32); }
-constexpr int MAX_STAGES = 24;
 // What the ring may take.  Every load of W in flight holds its line in L1, 64 KB an SM, so L1 has to keep that much: with
 // 200 KB of ring 16 x 384 x 3968 takes 17.5 us, with 160 KB 11.4, with 128 KB 10.6, and less gains nothing (16 x 1088 x 6144 24.9,
 // 16.9, 15.9).  64 rows need 170 KB for a stage a warp.
@@ -47,9 +46,11 @@ struct Cfg {
   static constexpr int stage_bytes(int box_m) { return STAGE_K / 64 * box_m * 128 + B_BYTES; }
   static constexpr int stages(int box_m) {
     const int n = (RING_SMEM - fixed_bytes(box_m)) / stage_bytes(box_m);
-    return n < LOAD_WARPS ? LOAD_WARPS : n < MAX_STAGES ? n : MAX_STAGES;
+    return n < LOAD_WARPS ? LOAD_WARPS : n;
   }
 };
+constexpr int MAX_STAGES = Cfg<32>::stages(8);  // the lowest boxes and the shorter stages: 21; with 16 columns 18
+static_assert(Cfg<16>::stages(8) <= MAX_STAGES, "a barrier for every stage");
 // Warp w fills stages' worth w, w + 8, ... of K and waits for its stage's previous use by parity alone: with fewer
 // stages than warps one would be two uses ahead and pass.
 template <int BN>

@@ -405,9 +405,11 @@ def test_few_rows_off_their_boundaries(m, offset):
     assert np.array_equal(got, a @ w + b)
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1000, 2496), (8, 1000, 2500), (9, 2000, 6000), (17, 1000, 2333), (41, 2400, 7001), (57, 1000, 2499), (64, 2400, 7168)])
+@pytest.mark.parametrize("M,N,K", [(1, 1000, 2496), (8, 1000, 2500), (9, 2000, 6000), (17, 1000, 2333), (41, 2400, 7001), (57, 1000, 2499), (64, 2400, 7168),
+                                   (8, 2400, 4096), (8, 2400, 5200)])
 def test_few_rows_rings_are_exact(m, M, N, K):
-    # boxes of 8 to 64 rows, rings of 8 stages to 24 that go round, both widths of a CTA, the last stage partly past K
+    # boxes of 8 to 64 rows, rings of 8 stages to 18 with 16 columns a CTA and of 9 to 21 with 32 that go round, the deepest with
+    # the input converted ahead and inside, the last stage partly past K
     rng = np.random.default_rng(53)
     a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
     b = rng.integers(-4, 5, N).astype(np.float32)
