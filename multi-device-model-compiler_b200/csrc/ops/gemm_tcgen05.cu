@@ -17,10 +17,14 @@
 //            Rows that can be moved 32 bytes at a time: a thread owns a row, and two threads store
 //            64 bytes of each other's (store_row_pairs), so nothing is staged.  The ring has two
 //            more stages, and the residual and the bias are fetched before the accumulator is waited for.
-//            A short K is bound by this epilogue: with sectors stored one by one, the bias loaded a
-//            tile late and the residual piece by piece it took 6940 cycles a tile, 10900 with residual,
-//            beside 6144 of MMAs at K = 768; 32768 x 2304 x 768 97.9 -> 94.2 us, 32768 x 768 x 768 with
-//            residual 46.1 -> 44.1, 12288 x 768 x 768 19.0 -> 16.2.  (Stores spread over the mainloop by the
+//            A short K is bound by this epilogue: with sectors stored one by one and the residual piece by
+//            piece it took 6940 cycles a tile, 10900 with residual, beside 6144 of MMAs at K = 768.  Graph
+//            replays, operands in turn, against that form: 32768 x 2304 x 768 117 -> 108 us, 32768 x 768 x 768
+//            with residual 59.7 -> 52.7, 12288 x 768 x 768 18.8 -> 16.2; at K up to 168 and rows off 64 bytes
+//            the exchange costs up to 4 % (28588 x 80 x 144 7.55 / 7.80, but 40000 x 176 x 64 10.4 / 10.5, 20000 x
+//            1000 x 128 36.4 / 35.5: no rule found).  (The bias a tile ahead and the pieces written out without
+//            a residual too: 5145 x 536 x 64 6.53 -> 6.66, 20450 x 112 x 168 8.32 -> 8.70, 36322 x 384 x 64 17.2 ->
+//            17.9, 32768 x 2304 x 768 108 -> 111.  Stores spread over the mainloop by the
 //            clock: no gain.  16 epilogue warps: 8 us slower at 32768 x 3072 x 768 with GELU.)
 //            Rows of other multiples of 16 bytes (N = 8 mod 16, or a pointer off its 32-byte
 //            boundary): each warp stages 32 rows x 128 bytes in swizzled shared memory and moves
@@ -267,15 +271,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     [[maybe_unused]] constexpr int MAX_SUBS = BN / 2 / 32;
     // pieces of the residual in flight; the GELUs' code is too long to be written out four times (4096 x 3072 x 768 22.1 -> 23.7 us)
     [[maybe_unused]] constexpr int RES_AHEAD = ACT == kActNone || ACT == kActRelu ? MAX_SUBS : 1;
-    // four bias values of a tile's columns (zeros beyond N), for the whole warp's row of them
-    [[maybe_unused]] auto load_bias = [&](int t) __attribute__((always_inline)) -> float4 {
-      const int c = (t % p.num_n_blocks) * bn + half_sel * half_cols + lane * 4;
-      return t < num_tiles && c < p.N ? __ldg(reinterpret_cast<const float4 *>(p.bias + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    [[maybe_unused]] float4 next_bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (kWide) {
-      if (p.bias) next_bias = load_bias(worker);
-    }
     for (int tile = worker; tile < num_tiles; tile += num_workers) {
       const int m_blk = (tile / p.num_n_blocks) * CG + cta_rank, n_blk = tile % p.num_n_blocks;
       const int row = m_blk * BM + quarter * 32 + lane;
@@ -296,7 +291,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if constexpr (kWide) {
         // The warp owns 32 rows x half_cols accumulator columns, read from tensor memory in pieces of 32; the
         // next piece's load is in flight while this one goes through bias / activation / residual.  All of the
-        // tile's residual is requested before the accumulator is waited for, and its bias a tile earlier.
+        // tile's residual, and its bias, are requested before the accumulator is waited for.
         const size_t row_off = static_cast<size_t>(row) * p.N + gcol_base;
         uint32_t raw[32];
         uint32_t rr[RES_AHEAD][16];
@@ -308,14 +303,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         };
 #pragma unroll
         for (int sub = 0; sub < RES_AHEAD; ++sub) fetch_res(sub, rr[sub]);
+        if (p.bias) {
+          const int c = gcol_base + lane * 4;
+          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (c < p.N) b = __ldg(reinterpret_cast<const float4 *>(p.bias + c));
+          __syncwarp();  // the previous tile's values have been read
+          *reinterpret_cast<float4 *>(&bias_s[ew][lane * 4]) = b;
+          __syncwarp();
+        }
         if (!wait_acc()) break;
         if (n_sub > 0) tmem_ld_32x32(t_base, raw);
-        if (p.bias) {
-          __syncwarp();  // the previous tile's values have been read
-          *reinterpret_cast<float4 *>(&bias_s[ew][lane * 4]) = next_bias;
-          __syncwarp();
-          next_bias = load_bias(tile + num_workers);
-        }
         auto piece = [&](int sub, uint32_t *r) __attribute__((always_inline)) {
           const int gcol = gcol_base + sub * 32;
           tmem_ld_wait_regs(raw);
@@ -343,10 +340,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           store_row_pairs<TOut>(out, v, row, p.M, gcol, p.N);
         };
-        if constexpr (RES_AHEAD == MAX_SUBS) {
+        // written out for a residual's registers only: a CTA of few tiles waits for its instructions
+        if (RES_AHEAD == MAX_SUBS && res) {
 #pragma unroll
           for (int sub = 0; sub < MAX_SUBS; ++sub)
-            if (sub < n_sub) piece(sub, rr[sub]);
+            if (sub < n_sub) piece(sub, rr[sub % RES_AHEAD]);
         } else {
 #pragma unroll 1
           for (int sub = 0; sub < n_sub; ++sub) piece(sub, rr[0]);
