@@ -110,9 +110,18 @@ constexpr int kLnWarpsPerBlock = 4;
 // loads are all in flight, and gamma and beta are asked for with the row instead of behind the statistics; no block
 // budget has the registers spill.  Chained launches, bf16, against the persistent form: 99 x 768 2.51 -> 1.65 us, 99 x 1024
 // 2.60 -> 1.67, 2048 x 768 3.55 -> 2.86, 8192 x 768 7.47 -> 6.46, 12288 x 768 9.41 -> 8.90, 8192 x 1024 8.57 -> 8.33; beyond 10
-// million values the persistent form's prefetch wins: 16384 x 1024 14.0 / 14.7, 131072 x 768 79.8 / 86.7.
+// million values the persistent form's prefetch wins: 16384 x 1024 14.0 / 14.7, 131072 x 768 79.8 / 86.7.  (Not for fp32 outputs,
+// 24 million values at 768 columns 29.9 / 27.4; the line is one for all.  A little past a round of blocks it loses up to 7 %:
+// 3000 x 1024 with gamma alone 4.23 / 4.52 out of memory, 2048 x 1024 3.93 / 3.04.)
+// Without gamma and beta there is less to ask for ahead and the line is at 2 million: 2048 x 1024 3.34 / 3.13, 2700 x 768 3.36 / 2.96,
+// 4096 x 512 3.10 / 3.01, but 3000 x 1024 3.80 / 4.52, 3500 x 768 3.64 / 3.98, 16000 x 512 6.82 / 7.25.  Short fp32 outputs of rows
+// of 1024 stay too: 500 rows 2.13 / 2.47 out of L2, 1000 3.50 / 3.16.
 enum LnForm { kLnAny, kLnFull, kLnFew };
-constexpr int64_t kLnFewValues = 10 * 1000 * 1000;
+constexpr int64_t kLnFewValues = 10 * 1000 * 1000, kLnFewPlain = 1 << 21;
+inline bool ln_few(int64_t m, int64_t n, bool affine, size_t out_bytes) {
+  if (affine) return m * n <= kLnFewValues;
+  return m * n <= kLnFewPlain && (n < 1024 || out_bytes == 2 || m >= 900);
+}
 template <typename TIn, typename TOut, int MAXI, bool RES, int FORM>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32,
                                   FORM == kLnFew ? 1 : (MAXI >= 8 || sizeof(TIn) == 4) ? 2 : ((RES || (FORM == kLnFull && MAXI >= 4)) ? 4 : 6))
@@ -352,7 +361,7 @@ static void launch_layernorm(const void *x, const void *residual, const float *g
     const int threads = kLnWarpsPerBlock * 32;
     const int ni = static_cast<int>(n);
     if constexpr (sizeof(TIn) == 2) {
-      if (!ri && per_lane >= 2 && per_lane <= 4 && nchunks_host == 32 * per_lane && m * n <= kLnFewValues) {
+      if (!ri && per_lane >= 2 && per_lane <= 4 && nchunks_host == 32 * per_lane && ln_few(m, n, gamma || beta, sizeof(TOut))) {
         auto kern = per_lane == 2 ? layernorm_warp_kernel<TIn, TOut, 2, false, kLnFew>
                     : per_lane == 3 ? layernorm_warp_kernel<TIn, TOut, 3, false, kLnFew> : layernorm_warp_kernel<TIn, TOut, 4, false, kLnFew>;
         check_cuda(launch_chain(kern, dim3(static_cast<unsigned>(blocks_needed)), dim3(threads), 0, s, 1, xi, ri, gamma, beta, so, yo, eps, m, ni),

@@ -172,7 +172,7 @@ def test_layernorm_16bit_large(m, rows, n, dtype_name):
 @pytest.mark.parametrize("affine", ["both", "gamma", "beta", "none"])
 @pytest.mark.parametrize("n", [512, 768, 1024])
 def test_layernorm_16bit_rows_do_not_depend_on_their_number(m, n, affine, dtype_name):
-    # one row to a warp up to ten million values, persistent warps beyond
+    # one row to a warp up to ten million values (two without gamma and beta), persistent warps beyond
     rng = np.random.default_rng(n)
     rows, dt = 10_000_000 // n + 3, m.F16 if dtype_name == "f16" else m.BF16
     x = m.encode16(rng.standard_normal((rows, n)).astype(np.float32), dt)
