@@ -426,6 +426,17 @@ def test_one_round_of_pairs_is_exact(m, M, N, K):
     assert np.array_equal(got, np.maximum(a @ w + b, 0) + r)
 
 
+@pytest.mark.parametrize("M,N,K", [(366, 337, 64), (1739, 59, 32), (2444, 46, 24), (653, 171, 64), (70, 405, 56), (130, 1, 8), (128, 9, 640)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_one_wave_rows_stored_by_value_are_exact(m, M, N, K, residual):
+    # tiles that are narrow because each value is a store of its own, 16 columns and boxes of 32 to 64 rows among them
+    rng = np.random.default_rng(61)
+    a, w = rng.integers(-3, 4, (M, K)).astype(np.float32), rng.integers(-2, 3, (K, N)).astype(np.float32)
+    b, r = rng.integers(-4, 5, N).astype(np.float32), rng.integers(-8, 9, (M, N)).astype(np.float32)
+    got = m.matmul16(a, w, bias=b, residual=r if residual else None, out_dtype=m.F32, act=m.ACT_RELU)
+    assert np.array_equal(got, np.maximum(a @ w + b, 0) + (r if residual else 0))
+
+
 @pytest.mark.parametrize("entry", ["mgpuMatmul", "mgpuMatmulNoAlloc"])
 @pytest.mark.parametrize("M,N,K", [(16, 1000, 1024), (40, 2400, 500)])
 def test_output_may_overlap_the_weight(m, entry, M, N, K):
