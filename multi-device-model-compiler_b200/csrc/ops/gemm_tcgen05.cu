@@ -100,10 +100,17 @@ struct RowMaps {
 template <>
 struct RowMaps<true> {};
 
-template <typename T16, typename TOut, int ACT, int CG, bool kWide>
+// Staged rows, or rows moved 32 bytes at a time; the latter without a residual are a kernel of their own.  Its registers (115 to
+// 142 a thread; 160 to 168 with a residual) leave an SM room for the blocks of the launch behind it, which are then in place
+// when this one ends: mgpuMatmul of 2590 x 1472 x 256, whose next call converts its operands, 13.2 -> 10.9 us in a graph and 14.3 ->
+// 12.7 in direct calls, 2272 x 2496 x 320 16.3 -> 14.9, 3200 x 1024 x 384 13.6 -> 12.1; Gemms behind one another the same.
+enum RowForm { kStagedRows, kWideRows, kWideResidual };
+
+template <typename T16, typename TOut, int ACT, int CG, int FORM>
 __global__ void __launch_bounds__(gemm::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    const __grid_constant__ RowMaps<kWide> rows, const GemmParams p) {
+                    const __grid_constant__ RowMaps<FORM != kStagedRows> rows, const GemmParams p) {
+  constexpr bool kWide = FORM != kStagedRows;
   using namespace gemm;
   using namespace ptx;
   using C = Cfg<CG, kWide>;
@@ -258,7 +265,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int quarter = warp & 3;   // TMEM lane quarter this warp may access
     const int half_sel = ew >> 2;   // which 128 accumulator columns this warp handles
     TOut *out = static_cast<TOut *>(p.out);
-    const T16 *res = static_cast<const T16 *>(p.residual);
+    const T16 *res = FORM == kWideRows ? nullptr : static_cast<const T16 *>(p.residual);
     [[maybe_unused]] uint8_t *my_out_base = tiles + STAGES * STAGE_BYTES + ew * C::EPI_WARP_BYTES;
     [[maybe_unused]] uint8_t *my_res = my_out_base + C::OUT_BUFS * EPI_BUF_BYTES;
     [[maybe_unused]] int out_buf = 0;
@@ -295,7 +302,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // tile's residual, and its bias, are requested before the accumulator is waited for.
         const size_t row_off = static_cast<size_t>(row) * p.N + gcol_base;
         uint32_t raw[32];
-        uint32_t rr[RES_AHEAD][16];
+        [[maybe_unused]] uint32_t rr[RES_AHEAD][16];
         auto fetch_res = [&](int sub, uint32_t *r) __attribute__((always_inline)) {
           if (res && row_ok && sub < n_sub) {
             ld_global_32B(res + row_off + sub * 32, r);
@@ -342,10 +349,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           store_row_pairs<TOut>(out, v, row, p.M, gcol, p.N);
         };
         // written out for a residual's registers only: a CTA of few tiles waits for its instructions
-        if (RES_AHEAD == MAX_SUBS && res) {
+        if constexpr (FORM == kWideResidual && RES_AHEAD == MAX_SUBS) {
 #pragma unroll
           for (int sub = 0; sub < MAX_SUBS; ++sub)
-            if (sub < n_sub) piece(sub, rr[sub % RES_AHEAD]);
+            if (sub < n_sub) piece(sub, rr[sub]);
         } else {
 #pragma unroll 1
           for (int sub = 0; sub < n_sub; ++sub) piece(sub, rr[0]);
@@ -523,11 +530,11 @@ static bool encode_rows(CUtensorMap *map, const void *base, int32_t dtype, int64
   return encode_tmap(map, dtype, 2, base, dim, &stride, box, cw * elem == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
-template <typename T16, typename TOut, int ACT, int CG, bool kWide>
-static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p,
+template <typename T16, typename TOut, int ACT, int CG, int FORM>
+static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<FORM != kStagedRows> &rows, const GemmParams &p,
                            int grid, cudaStream_t s) {
-  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG, kWide>;
-  constexpr size_t smem = gemm::Cfg<CG, kWide>::SMEM_BYTES;
+  auto kern = gemm_tcgen05_kernel<T16, TOut, ACT, CG, FORM>;
+  constexpr size_t smem = gemm::Cfg<CG, FORM != kStagedRows>::SMEM_BYTES;
   static bool attr_set_on[kMaxDevices] = {false};  // the attribute is per device
   bool &attr_set = attr_set_on[current_device_index()];
   if (!attr_set) {
@@ -548,8 +555,16 @@ static void launch_gemm_cg(const CUtensorMap &ta, const CUtensorMap &tb, const R
 template <typename T16, typename TOut, int ACT, bool kWide>
 static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const RowMaps<kWide> &rows, const GemmParams &p, int grid,
                         cudaStream_t s) {
-  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, kWide>(ta, tb, rows, p, grid, s);
-  else launch_gemm_cg<T16, TOut, ACT, 1, kWide>(ta, tb, rows, p, grid, s);
+  if constexpr (kWide && ACT != kActGeluTanh) {
+    if (!p.residual) {
+      if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, kWideRows>(ta, tb, rows, p, grid, s);
+      else launch_gemm_cg<T16, TOut, ACT, 1, kWideRows>(ta, tb, rows, p, grid, s);
+      return;
+    }
+  }
+  constexpr int FORM = kWide ? kWideResidual : kStagedRows;  // (or none, with the tanh GELU, whose registers are its own)
+  if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, FORM>(ta, tb, rows, p, grid, s);
+  else launch_gemm_cg<T16, TOut, ACT, 1, FORM>(ta, tb, rows, p, grid, s);
 }
 
 template <typename T16, typename TOut, bool kWide>
