@@ -396,7 +396,15 @@ void gemm_one_wave_launch(const GemmTile &t, const void *a, const void *w_nk, co
   const size_t ring = stage * t.stages + (t.mma_m - t.box_m) * onewave::BK * 2;
   // never less than half of an SM's: two CTAs on one SM, of this launch or of the next, take turns at the SM's port while
   // others idle (2337 x 256 x 256 4.1 -> 3.5 us, 1592 x 704 x 256 4.7 -> 4.0, 99 x 768 x 768 3.44 -> 3.30; nothing loses 2 %)
-  const size_t smem = std::max<size_t>(ring + 1024, 117 * 1024);
+  size_t smem = std::max<size_t>(ring + 1024, 117 * 1024);
+  // An SM's shared memory is set up in steps, and what a CTA leaves of its step is for the blocks of the launch behind it: a ring
+  // that fills one asks for the next.  With 2 KB left of 196 the conversion ahead of the next Gemm starts on idle SMs only:
+  // mgpuMatmul of 608 x 448 x 1152 9.2 -> 8.1 us a call in a graph, 9.8 -> 8.3 direct, 4096 x 512 x 512 12.7 -> 12.0, 512 x 1000 x 2048 12.1 ->
+  // 11.6; chains of Gemms alone do not mind.  Not beside a large weight, whose conversion needs the L1: 256 x 4096 x 1024
+  // 11.8 -> 12.3, 372 x 3008 x 2752 1.07 of the time.
+  if (N * Kp <= 1 << 21)
+    for (const size_t step : {132, 164, 196})
+      if (smem + 2048 <= step * 1024 && smem + 2048 + 12 * 1024 > step * 1024) smem = step * 1024;
   if (dtype == MGPU_DTYPE_F16) {
     if (out_dtype == MGPU_DTYPE_F16) launch_one_wave_act<__half, __half>(ta, tb, p, t.cg, grid, smem, act, s);
     else if (out_dtype == MGPU_DTYPE_F32) launch_one_wave_act<__half, float>(ta, tb, p, t.cg, grid, smem, act, s);
