@@ -62,9 +62,9 @@ def bytes_touched_per_step(batch):
 # residual, output) scaled and the weights kept.
 GEMM_DRAM_TRAFFIC = {
     # tokens: {shape: bytes}
-    32768: {"gemm_qkv": 53913600 + 98738176, "gemm_proj": 51549440 + 11584512,
-            "gemm_ffn1": 55092736 + 150355712, "gemm_ffn2": 206891264 + 36219392},
-    4096: {"gemm_qkv": 9873152, "gemm_proj": 7507456, "gemm_ffn1": 11049472, "gemm_ffn2": 29927168},
+    32768: {"gemm_qkv": 53938176 + 98845952, "gemm_proj": 51535872 + 12186112,
+            "gemm_ffn1": 55088896 + 147857664, "gemm_ffn2": 206647296 + 36318720},
+    4096: {"gemm_qkv": 9872384, "gemm_proj": 7494400, "gemm_ffn1": 11047680, "gemm_ffn2": 29908224},
 }
 
 

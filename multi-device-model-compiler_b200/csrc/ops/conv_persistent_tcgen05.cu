@@ -19,9 +19,9 @@
 //
 // Bound: of short patches and many channels the stores, else instruction issue of the gather; of im2col k-blocks the hand-over of a stage and the issue of its MMAs, about
 // 400 cycles a k-block where the MMAs of 64 columns take 193 (conv_plan.h says which calls conv_halo_kernel takes instead).
-// Measured, whole call, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.  Inputs
-// changing from call to call:
-//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  56 us (43 of HBM time)
+// Measured, whole call, one after another from the host, before (gather kernel of conv_tcgen05.cu, one tile per CTA) and after.
+// Inputs changing from call to call:
+//   16 x 3 x 256 x 256 -> 64, 3 x 3                      217 ->  56 us (43 of HBM time; 55 in a graph)
 //   32 x 128 x 28 x 28 -> 128, 3 x 3                            19 us
 // L2 flushed between calls:
 //   18 x 128 x 43 x 51 -> 76, 5 x 5, stride 2            116 ->  34 us
@@ -30,8 +30,9 @@
 // The gather was bound by instruction issue: run-time divisions and per-channel tests in the
 // epilogue, 2.7 us a tile of 128 x 64; with multiplicative division, whole-group stores and the
 // two epilogue halves on alternate tiles 1.3 us (150 -> 77 us for the first shape).  With the taps in the constant bank,
-// one test a value at the edges and no work on other groups' tiles 64 -> 56, 32 x 3 x 224 x 224 -> 64 stride 2 47 -> 36,
-// 43 x 6 x 255 x 256 -> 8 dilation 2 269 -> 156; 140 shapes of 1 to 15 channels 0.87 of the time.
+// one test a value at the edges, no work on other groups' tiles and a ring that is never shorter than the groups 64 -> 56,
+// 32 x 3 x 224 x 224 -> 64 stride 2 48.5 -> 34.9, 43 x 6 x 255 x 256 -> 8 dilation 2 271 -> 134; in a graph 200 shapes of 1 to 15 channels,
+// those that regions take among them, 0.79 of the time, none above 1.03.
 #include <cuda_fp16.h>
 
 #include "conv_epilogue.cuh"
@@ -281,7 +282,7 @@ conv_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     // ---------------- gather: one thread per pixel, groups of four warps take alternate k-blocks ----------------
     // Where k lies is the same for all lanes: out of the constant bank a value costs its load and an addition of the uniform
     // datapath.  Out of a table in shared memory it took a load of that, a 64-bit addition and a test more (64 us at
-    // 16x3x256x256->64 3x3, now 55); and every group worked out every tile's pixels, where a third of the tiles are its own.
+    // 16x3x256x256->64 3x3, now 56); and every group worked out every tile's pixels, where a third of the tiles are its own.
     const int group = (warp - EPI_WARPS - 2) >> 2;
     const int row = ((warp - EPI_WARPS - 2) & 3) * 32 + lane;
     const uint32_t row_off = static_cast<uint32_t>(row) * 128u, swz = static_cast<uint32_t>(row & 7);

@@ -109,7 +109,7 @@ bool conv_prepare(const ConvShape &c, const ConvShape &call, bool sampled, int64
 
 // The persistent kernels' tile: width, by the cycles of the busiest CTA: rounds x the slowest of a tile's three engines.
 // Loads: about 64 bytes per cycle and SM out of L2 (a gathered k-block about 400 cycles with three
-// groups at work); MMAs: 2 cycles per column and k-block, at least what reading A takes; epilogue:
+// groups at work, as the gather once was); MMAs: 2 cycles per column and k-block, at least what reading A takes; epilogue:
 // about 24 bytes per cycle and SM of HBM.  E.g. 6272 pixels x 256 channels: 147 tiles of 96 columns
 // in one round (224 units of load) beat 98 of 128 in one (256) and 49 of 256 (384).
 inline int choose_conv_bn(int64_t m_tiles, int64_t OC, int64_t num_kb, bool gather, bool add, int sms) {
@@ -233,14 +233,14 @@ inline bool fit_halo(HaloTile *t, bool copy, bool add, int64_t OC, int bn, int s
   // as many stages as regions that the input warps' pieces reach over: a stage's barrier is then never two uses behind
   const int64_t reach = copy ? 0 : (kHaloInputWarps + t->qb - 1) / t->qb;
   if (n < 2 || n < reach) return false;
-  // No more stages than the busiest CTA fills, so that the next call's CTAs fit beside those of a short one: 33x6x13x14->8 5x5
-  // 8.0 -> 6.9 us, 150 direct shapes 0.96 of the time, the slowest 1.02.
+  // No more stages than the busiest CTA fills, so that the next call's CTAs fit beside those of a short one.  In a graph: 33x6x13x14->8
+  // 5x5 7.3 -> 6.4 us (8.4 -> 8.3 from the host, which needs that long), 150 direct shapes 0.96 of the time, the slowest 1.02.
   const int64_t rounds = (tiles + sms - 1) / sms;
   n = std::min(n, std::max({int64_t(2), reach, rounds * t->ncb}));
   int64_t fs = (room - n * region) / (kbs * b_bytes);
   fs = std::min({fs, int64_t(kHaloFilterStages), blocks * rounds});
   // A residual's loads in flight hold their lines in L1, four sectors to a line, and 220 KB leave it 30: 32x64x56x56->64 3x3
-  // 25.0 -> 24.0 us, -> 256 1x1 56.9 -> 50.9.  Not where the filter streams by for every tile, which then is what
+  // 25.3 -> 24.3 us a call (in a graph 25.1 -> 23.9), -> 256 1x1 58.0 -> 51.6 (57.5 -> 51.4).  Not where the filter streams by for every tile, which then is what
   // takes the time: 1x176x15x14->136 7x7 23.4 -> 24.6, 8x16x89x83->16 7x7 27.8 -> 29.0.
   if (add && copy && (resident || blocks <= 4))
     while (n > 3 && n * region + (resident ? filter : fs * kbs * b_bytes) + fixed > kHaloAddSmem) --n;
@@ -324,7 +324,8 @@ inline double dense_us(const ConvShape &c, int sms) {
   const int bn = choose_conv_bn(m_tiles, c.OC, num_kb, gather, c.add != nullptr, sms);
   const int64_t n_tiles = (c.OC + bn - 1) / bn, tiles = m_tiles * n_tiles;
   const double rounds = static_cast<double>((tiles + sms - 1) / sms);
-  if (gather) return conv_us(0.0, rounds * num_kb * 2600.0 + 4000.0);  // instructions of the gather
+  // instructions of the gather, as they were when this was fitted; it takes about half of that now (see conv_form)
+  if (gather) return conv_us(0.0, rounds * num_kb * 2600.0 + 4000.0);
   // an im2col k-block: the hand-over of its stage, or 70 bytes a cycle; rows of the copy that end inside a sector are read
   // at half that rate
   const double kb = std::max(400.0, (16384.0 + (conv_filter_stays(num_kb, bn, n_tiles, tiles, sms) ? 0 : bn * 128)) / 70.0);
@@ -365,12 +366,14 @@ inline double halo_us(const ConvShape &c, ConvForm form, const HaloTile &t, int 
 //   rows of eight pixels off the sectors: 14x64x85x93->448 5x1 67 / 201 / 70, 25x64x52x87->256 1x3 44 / 108 / 51
 //   empty tiles: 1x64x1x65536->64 1x3 15 / 56 / 17, 1x64x4x8192->64 3x3 13 / 19, 206x32x2x112->64 5x5 dilation 3 24 / 69
 //   1 x 1: 32x64x56x56->256 40 / 34 / 30, 117x128x43x60->32 with residual 91 / 65 / 60, but 10x96x220x8->142 12 / 15 / 15
-//   few channels, gather / rect / flat: 16x3x224x224->32 7x7 143 / 78, 16x3x18x256->64 7x7 26 / 17 / 31, 1x16x1x160000->32 1x9 27 / 94 / 15,
-//     but 256x1x28x28->32 5x5 19 / 25 / 25, 21x3x29x37->352 5x5 21 / 24 / 24, 1x3x4x40000->32 5x5 28 / 46
+//   few channels, gather / rect / flat: 16x3x224x224->32 7x7 92 / 76, 16x6x64x64->64 7x7 35 / 14 / 15, 1x16x1x160000->32 1x9 27 / 101 / 15,
+//     but 256x1x28x28->32 5x5 12 / 24 / 24, 21x3x29x37->352 5x5 14 / 23 / 23, 1x3x4x40000->32 5x5 18 / 42
 //   stride 2, 16 to 32 channels, im2col / rect: 16x24x150x153->32 5x5 78 / 30, 4x32x200x203->32 5x5 27 / 19, but 4x16x120x123->256 7x7 24 / 32
 // Below 25 taps few channels and strides stay where they are: nearly all that was measured there is slower (16x3x256x256->64
-// 3x3 64 / 93).
-// Over 1648 shapes with copies the choice takes 0.901 of the dense kernels' time (geometric mean; always the best one, 0.890)
+// 3x3 56 / 87; not 43x6x255x256->8 3x3 dilation 2 134 / 131).  From 25 taps on the line stands too early since the gather takes half of
+// what dense_us says: 16x3x128x128->64 5x5 goes to a region that takes 31.6 where the gather would 26.3, 16x4x100x100->128 7x7 48.8 /
+// 33.3, 64x3x56x56->64 5x5 24.5 / 21.3, 16x3x224x224->64 7x7 stride 2 35.1 / 31.1, 16x3x18x256->64 7x7 16.4 / 15.4.
+// When these estimates were fitted: over 1648 shapes with copies the choice takes 0.901 of the dense kernels' time (geometric mean; always the best one, 0.890)
 // and 40 are more than 4 % slower; over 871 others 0.814 (0.804) and 39.  Over 1050 that the estimates were not fitted to,
 // 0.910 (0.893), 14 of 700, and 0.804 (0.790), 16 of 350.
 inline ConvForm conv_form(const ConvShape &c, int sms, bool dense = true, HaloTile *tile = nullptr) {

@@ -7,14 +7,15 @@
 // SM); a warp fills a ring stage of 128 k x 16 columns or 64 k x 32 by itself, converting to core
 // matrices of 8 columns x 8 k.  A comes by TMA, converted by a launch ahead; W and the bias do not wait for it: that
 // kernel lets this one start after its own wait, so what is older than it is complete.  Where A is small (kConvert,
-// few_rows_convert) eight more warps read and round it here instead, and there is no launch ahead: 16 x 768 x 768 6.9 ->
-// 5.1 us a call, 16 x 256 x 256 6.8 -> 4.1.
+// few_rows_convert) eight more warps read and round it here instead, and there is no launch ahead: 16 x 768 x 768 6.1 ->
+// 4.9 us a call, 16 x 256 x 256 6.1 -> 3.7.
 //
 // The accumulator has 64 rows: an MMA of 128 rows and 16 or 32 columns takes 40 cycles, one of 64 rows 25.  A's box is as high
 // as there are rows, and the ring leaves L1 to the loads in flight (RING_SMEM).  Whole calls out of memory, with 128 rows, boxes of
-// 32 or 64 and a ring of 220 KB / now: 16 x 1000 x 2048 12.6 / 8.1 us, 1 x 1000 x 2048 11.7 / 7.1, 64 x 1000 x 2048 12.9 / 9.2,
-// 8 x 2000 x 4000 18.3 / 11.4, 16 x 4096 x 4096 21.6 / 19.0 (3.5 TB/s), 16 x 1000 x 512 4.46 / 4.27.  Weights that are
-// converted first instead: gemm_plan.h.
+// 32 or 64 and a ring of 220 KB / now, one after another from the host (in a graph): 16 x 1000 x 2048 13.0 / 9.2 us (12.8 / 8.0),
+// 1 x 1000 x 2048 12.2 / 7.4 (11.8 / 7.0), 64 x 1000 x 2048 13.1 / 9.5 (12.9 / 9.2), 8 x 2000 x 4000 18.8 / 11.6 (18.5 / 11.3), 16 x
+// 4096 x 4096 22.1 / 19.1 (21.9 / 19.0; 3.5 TB/s), 16 x 1000 x 512 4.6 / 4.4 (4.35 / 4.13).  Weights that are converted first
+// instead: gemm_plan.h.
 //
 // K order: one sum over K in steps of 16, as in the other Gemm kernels; a row's bits do not depend on
 // which of them takes a call.

@@ -68,7 +68,7 @@ gemm_one_wave_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int half = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;  // which 128 rows of a pair's 256
+  const int half = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;  // which half of a pair's rows
   const bool leader = half == 0;
   const int tile = static_cast<int>(blockIdx.x) / CG;
   const int m_tile = tile / p.n_tiles, n_tile = tile - m_tile * p.n_tiles;

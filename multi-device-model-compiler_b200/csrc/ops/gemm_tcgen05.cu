@@ -562,7 +562,7 @@ static void launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const RowM
       return;
     }
   }
-  constexpr int FORM = kWide ? kWideResidual : kStagedRows;  // (or none, with the tanh GELU, whose registers are its own)
+  constexpr int FORM = kWide ? kWideResidual : kStagedRows;  // (the tanh GELU takes as many registers without a residual)
   if (p.cta_group == 2) launch_gemm_cg<T16, TOut, ACT, 2, FORM>(ta, tb, rows, p, grid, s);
   else launch_gemm_cg<T16, TOut, ACT, 1, FORM>(ta, tb, rows, p, grid, s);
 }
@@ -723,10 +723,12 @@ GemmTile choose_gemm_tile(int64_t M, int64_t N, int64_t K, int sms) {
   const bool forced = getenv("MDC_GEMM_BN") || getenv("MDC_GEMM_CTA_GROUP");
   if (!forced && ((M + 127) / 128) * ((N + 127) / 128) <= sms)
     t = choose_one_wave(M, N, K, sms);
-  // A long K in tiles of 128 columns: the persistent kernel's ring of single k-blocks turns faster than one of several, where
-  // its pairs of 256 x 128 come in one round.  One-wave / persistent, us: 2341 x 768 x 3072 14.6 / 13.3, 1711 x 1024 x 3712 17.1 / 15.3,
-  // 1718 x 1024 x 4096 18.1 / 16.3, 2978 x 768 x 1920 11.0 / 10.1; below K = 1400 0.98 of the time instead, and with tiles of 96
-  // columns 1.0, of 64 0.88.
+  // A long K in tiles of 128 columns goes to the persistent kernel where its pairs of 256 x 128 come in one round.  One-wave /
+  // persistent, us: 2341 x 768 x 3072 14.9 / 13.6, 1711 x 1024 x 3712 17.3 / 15.6, 1718 x 1024 x 4096 18.3 / 16.8, 2978 x 768 x 1920 11.2 /
+  // 10.5; below K = 1400 0.98 of the time instead, and with tiles of 96 columns 1.0, of 64 0.88.  It is the kernel and not the cost
+  // above: no tile of the one-wave kernel does as well.  2341 x 768 x 3072 in pairs with 4, 2 and 1 k-blocks to a stage 14.9, 16.2, 20.5,
+  // in single CTAs with 2 and 1 15.2, 15.6 (192 columns 17.5 and more).  Why its stages of one k-block turn slower than the
+  // persistent kernel's is not known.
   if (t.one_wave && t.bn >= 128 && K >= 1400 && M > gemm::BM && ((M + 255) / 256) * ((N + 127) / 128) <= sms / 2) {
     t = GemmTile();
     t.cg = 2, t.bn = 128;
